@@ -25,6 +25,10 @@ bool affine_b4_gemm_tc_enabled() { return true; }
 bool affine_b4_gemm_pair_applies(int M, int N, int K, int sms);
 int32_t affine_b4_gemm_pair_launch(scr_ctx* ctx, const CUtensorMap& x_map, const uint8_t* packed, uint16_t* y, int M, int N, int K,
                                    int gs, int out_f32, const uint16_t* bias, cudaStream_t stream, bool* launched);
+// Defined in affine_b4_skinny.cu
+bool affine_b4_skinny_applies(int M);
+int32_t affine_b4_skinny_launch(scr_ctx* ctx, const uint8_t* packed, const uint16_t* x, uint16_t* y, int M, int N, int K, int gs, int out_f32,
+                                const uint16_t* bias, cudaStream_t stream);
 size_t affine_b4_gemm_tc_workspace_plan(int M, int N, int K);
 size_t affine_b4_gemm_tc_workspace(int M, int N, int K) { return affine_b4_gemm_tc_workspace_plan(M, N, K); }
 
@@ -395,7 +399,10 @@ static AffineGemmPlan affine_gemm_plan(int M, int N, int K, int sms) {
     tc_plan_units(p.tiles, g.KC, sms, 1.0f * p.tm, &p.full, &p.ks_tail);      // ~1 us per 128-k step and 128 tokens (measured)
     return p;
 }
-size_t affine_b4_gemm_tc_workspace_plan(int M, int N, int K) { return affine_gemm_plan(M, N, K, tc_sm_count()).slab_floats() * sizeof(float); }
+size_t affine_b4_gemm_tc_workspace_plan(int M, int N, int K) {
+    if (affine_b4_skinny_applies(M)) return 0;
+    return affine_gemm_plan(M, N, K, tc_sm_count()).slab_floats() * sizeof(float);
+}
 
 template <int TM>
 static int32_t affine_gemm_launch_tm(scr_ctx* ctx, const CUtensorMap& map, const uint8_t* packed, uint16_t* y, int M, int N,
@@ -421,6 +428,7 @@ int32_t affine_b4_gemm_tc_launch(scr_ctx* ctx, const uint8_t* packed, const uint
                                  int gs, int out_f32, const uint16_t* bias, void* workspace, size_t, cudaStream_t stream) {
     if (((uintptr_t)packed & 127u) != 0) return scr_fail(ctx, SCR_E_ALIGN, "packed weights must be 128-byte aligned for the GEMM path");
     if (!scr_aligned16(y)) return scr_fail(ctx, SCR_E_ALIGN, "y must be 16-byte aligned");
+    if (affine_b4_skinny_applies(M)) return affine_b4_skinny_launch(ctx, packed, x, y, M, N, K, gs, out_f32, bias, stream);
     tc_encode_tiled_fn enc = tc_tensor_map_encoder();
     if (!enc) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled entry point not available");
     CUtensorMap map;

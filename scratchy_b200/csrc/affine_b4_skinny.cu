@@ -1,0 +1,264 @@
+// MLX affine int4: GEMM for 17 to 128 tokens on tcgen05 tensor cores, weights as the rows of the MMA (skinny.cuh).
+//
+//   y[m,n] = bf16( sum_k x[m,k] * w[n,k] (+ bias[n]) ),  w = the bit-exact bf16 dequantisation of the codes
+//
+// A unit is 128 channels by one CTA's share of the 128-k chunks; 352 threads:
+//   warps 0-7    dequantise: two groups of four warps take alternate chunks; a thread expands the 128 codes of ONE channel
+//                and writes them to TMEM with tcgen05.st, where the MMA reads its A operand: no swizzled shared-memory
+//                image, no proxy fence.  Afterwards they drain the accumulator.
+//   warp 8       producer of the packed weights (8 bulk copies of a block per chunk), which are load-time constants: it
+//                starts before the preceding kernel of the stream has finished
+//   warp 9       producer of the activations (2 tiled TMA loads of 64 k x the tokens, 128-byte swizzle, zeros outside)
+//   warp 10      owns TMEM; one thread issues 8 tcgen05.mma (128 x tokens x 16) per chunk
+//
+// What bounds it: the packed weights from HBM (9.2 KB per chunk) and, for the short k extents of a layer's linears, the start
+// of the pipeline and the two cluster barriers at its end.  Against the 128-token tile of affine_b4_gemm.cu, which it replaces
+// here (its rows were mostly padding, its dequantised image took a round trip through shared memory and its split sums a second
+// launch): 45 rows of 8192 -> 3072, 16.1 us in two launches before, about 10 us in one now; the four linears of a
+// Llama-3.2-3B layer at 32 tokens 56 us and four finishing launches before, the whole decode step 3.95 -> 3.33 ms.
+#include <cuda.h>
+
+#include "affine_b4.cuh"
+#include "skinny.cuh"
+
+namespace {
+
+constexpr int A4S_THREADS = 352;
+constexpr int A4S_SP = 6;                        // packed-weight stages
+
+template <int TN>
+struct A4SCfg {
+    static constexpr int kSX = TN == 64 ? 3 : 4;                        // activation stages
+    static constexpr int kSA = TN == 128 ? 2 : 3;                       // dequantised-weight stages in TMEM, 64 columns each
+    static constexpr uint32_t kTmemCols = 256;                          // the accumulator's TN columns and the stages
+    static constexpr uint32_t kXStage = TN * 256u;                      // 2 atoms of TN rows x 128 B
+    static constexpr uint32_t kPOff = kSX * kXStage;
+    static constexpr int kCtasPerSm = TN == 128 ? 1 : 2;
+};
+
+__device__ __forceinline__ uint4 a4s_lds_v4(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint32_t a4s_lds_u32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void a4s_tma_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar) : "memory");
+}
+
+// The 128 codes of channel `row` of a chunk -> 64 TMEM columns at `dst` (this warp's lanes).
+template <int GS, bool CHECK>
+__device__ __forceinline__ void a4s_expand(uint32_t stage, int row, uint32_t dst) {
+    const int half = (row >> 3) & 1, g = row & 7;
+    const uint32_t blk = stage + (uint32_t)((row >> 4) * aff_block_bytes(GS));
+    uint4 piece[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) piece[t] = a4s_lds_v4(blk + (uint32_t)(half * 512 + (4 * g + t) * 16));
+    uint32_t sb[1 << GS];
+#pragma unroll
+    for (int h = 0; h < (1 << GS); ++h) sb[h] = a4s_lds_u32(blk + 1024u + (uint32_t)(((g << GS) + h) * 8 + half * 4));
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        const uint32_t s = sb[t >> (2 - GS)];
+        uint32_t w[16];
+        if (CHECK) {
+            affine_dequant_piece<true>(piece[t], s, w);
+        } else {
+            const AffineScaled c = affine_scaled_consts(s);          // w * 2^-7: the sums are multiplied by 2^7
+            affine_dequant_word_scaled(piece[t].x, c, w + 0);
+            affine_dequant_word_scaled(piece[t].y, c, w + 4);
+            affine_dequant_word_scaled(piece[t].z, c, w + 8);
+            affine_dequant_word_scaled(piece[t].w, c, w + 12);
+        }
+        tmem_st_32x16(dst + 16u * t, w);
+    }
+}
+
+template <int TN, int GS>
+__global__ void __launch_bounds__(A4S_THREADS, A4SCfg<TN>::kCtasPerSm)
+affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t* __restrict__ packed, uint16_t* __restrict__ y, int M, int N, int RB,
+                        int KC, int split, int out_f32, const uint16_t* __restrict__ bias, int* __restrict__ status) {
+    using C = A4SCfg<TN>;
+    constexpr uint32_t kBlock = aff_block_bytes(GS), kPStage = 8u * kBlock, kBarOff = C::kPOff + A4S_SP * kPStage;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t bar = smem_base + kBarOff;
+    auto xfull = [&](int s) { return bar + 8u * s; };
+    auto xempty = [&](int s) { return bar + 8u * (C::kSX + s); };
+    auto pfull = [&](int s) { return bar + 8u * (2 * C::kSX + s); };
+    auto pempty = [&](int s) { return bar + 8u * (2 * C::kSX + A4S_SP + s); };
+    auto afull = [&](int s) { return bar + 8u * (2 * C::kSX + 2 * A4S_SP + s); };
+    auto aempty = [&](int s) { return bar + 8u * (2 * C::kSX + 2 * A4S_SP + C::kSA + s); };
+    constexpr int kSlots = 2 * C::kSX + 2 * A4S_SP + 2 * C::kSA;
+    const uint32_t accf = bar + 8u * kSlots;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kBarOff + 8 * (kSlots + 1));
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tile = blockIdx.x / split, rank = blockIdx.x - tile * split;
+    int kc_lo, kc_hi;
+    skinny_range(KC, rank, split, kc_lo, kc_hi);
+    const int steps = kc_hi - kc_lo;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < C::kSX; ++s) { mbar_init(xfull(s), 1); mbar_init(xempty(s), 1); }
+        for (int s = 0; s < A4S_SP; ++s) { mbar_init(pfull(s), 1); mbar_init(pempty(s), 4); }
+        for (int s = 0; s < C::kSA; ++s) { mbar_init(afull(s), 4); mbar_init(aempty(s), 1); }
+        mbar_init(accf, 1);
+        fence_mbar_init();
+    }
+    if (warp == 10) {
+        tmem_alloc(smem_u32((const void*)tmem_slot), C::kTmemCols);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    skinny_pdl_trigger();                              // not before this CTA has its TMEM: the next kernel's CTAs could take it first
+    auto a_col = [&](int s) { return tmem + (uint32_t)(TN + 64 * s); };
+
+    // Only the weights may be touched before the preceding kernel has finished.  A wait that depends on the activations
+    // comes after griddepcontrol.wait, so that its bound does not run against that kernel.
+    if (warp == 8) {
+        if (lane == 0) {
+            for (int i = 0; i < steps; ++i) {
+                const int s = i % A4S_SP;
+                if (i == A4S_SP) skinny_pdl_wait();
+                mbar_wait(pempty(s), ((uint32_t)(i / A4S_SP) & 1u) ^ 1u, status, TC_ERR_EMPTY_WAIT);
+                mbar_arrive_expect_tx(pfull(s), kPStage);
+                for (int j = 0; j < 8; ++j)
+                    bulk_g2s(smem_base + C::kPOff + s * kPStage + j * kBlock, packed + ((size_t)(tile * 8 + j) * KC + kc_lo + i) * kBlock, kBlock, pfull(s));
+            }
+        }
+    } else if (warp == 9) {
+        if (lane == 0) {
+            skinny_pdl_wait();
+            const uint32_t tokens = (uint32_t)(M + 15) & ~15u;
+            for (int i = 0; i < steps; ++i) {
+                const int s = i % C::kSX;
+                mbar_wait(xempty(s), ((uint32_t)(i / C::kSX) & 1u) ^ 1u, status, TC_ERR_EMPTY_WAIT);
+                mbar_arrive_expect_tx(xfull(s), tokens * 256u);
+                const uint32_t xs = smem_base + s * C::kXStage;
+                a4s_tma_2d(xs, &x_map, (kc_lo + i) * 128, 0, xfull(s));
+                a4s_tma_2d(xs + TN * 128u, &x_map, (kc_lo + i) * 128 + 64, 0, xfull(s));
+            }
+        }
+    } else if (warp == 10) {
+        if (lane == 0) {
+            skinny_pdl_wait();
+            const uint32_t idesc = umma_idesc(1, 1, SKINNY_ROWS, (uint32_t)(M + 15) & ~15u);
+            for (int i = 0; i < steps; ++i) {
+                const int s = i % C::kSX, a = i % C::kSA;
+                mbar_wait(xfull(s), (uint32_t)(i / C::kSX) & 1u, status, TC_ERR_FULL_WAIT);
+                mbar_wait(afull(a), (uint32_t)(i / C::kSA) & 1u, status, TC_ERR_DEQ_WAIT);
+                tc_fence_after();
+                const uint32_t xs = smem_base + s * C::kXStage;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint64_t bdesc = umma_desc_k_sw128(xs + h * TN * 128u);
+#pragma unroll
+                    for (int k4 = 0; k4 < 4; ++k4)
+                        umma_f16_ta(tmem, a_col(a) + (uint32_t)(32 * h + 8 * k4), bdesc + (uint64_t)(2 * k4), idesc, (i | h | k4) != 0);
+                }
+                umma_commit(xempty(s));
+                umma_commit(aempty(a));
+            }
+            umma_commit(accf);
+        }
+    } else {
+        const bool check = *reinterpret_cast<const unsigned int*>(packed + (size_t)RB * KC * kBlock) != 0;
+        const int row = (warp & 3) * 32 + lane;
+        const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+        bool waited = false;
+        for (int i = warp >> 2; i < steps; i += 2) {
+            const int s = i % A4S_SP, a = i % C::kSA;
+            if (i >= C::kSA && !waited) {
+                skinny_pdl_wait();
+                waited = true;
+            }
+            mbar_wait(pfull(s), (uint32_t)(i / A4S_SP) & 1u, status, TC_ERR_FULL_WAIT);
+            mbar_wait(aempty(a), ((uint32_t)(i / C::kSA) & 1u) ^ 1u, status, TC_ERR_EMPTY_WAIT);
+            tc_fence_after();
+            const uint32_t stage = smem_base + C::kPOff + s * kPStage;
+            if (check) a4s_expand<GS, true>(stage, row, a_col(a) + lanes);
+            else a4s_expand<GS, false>(stage, row, a_col(a) + lanes);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(afull(a));
+                mbar_arrive(pempty(s));
+            }
+        }
+        skinny_pdl_wait();                             // y may still be read by a preceding kernel
+        mbar_wait(accf, 0, status, TC_ERR_ACC_FULL);
+    }
+    __syncwarp();
+    const float factor = (*reinterpret_cast<const unsigned int*>(packed + (size_t)RB * KC * kBlock) != 0) ? 1.0f : AFF_SCALED_FACTOR;
+    skinny_pdl_wait();
+    skinny_finish(tmem, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, tile * SKINNY_ROWS, N, [&](int m, int n, float a, float b) {
+        const float v[2] = {a * factor, b * factor};
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int c = n + 8 * j;
+            if (c >= N) break;
+            if (out_f32) {
+                reinterpret_cast<float*>(y)[(size_t)m * N + c] = v[j];
+            } else {
+                const __nv_bfloat16 o = __float2bfloat16_rn(bias ? v[j] + __uint_as_float(uint32_t(bias[c]) << 16) : v[j]);
+                y[(size_t)m * N + c] = *reinterpret_cast<const uint16_t*>(&o);
+            }
+        }
+    });
+    __syncthreads();
+    if (warp == 10) {
+        tc_fence_after();
+        tmem_dealloc(tmem, C::kTmemCols);
+    }
+}
+
+template <int TN, int GS>
+int32_t a4s_launch(scr_ctx* ctx, const CUtensorMap& map, const uint8_t* packed, uint16_t* y, int M, int N, int K, int out_f32, const uint16_t* bias,
+                   cudaStream_t stream) {
+    using C = A4SCfg<TN>;
+    const AffineGeom g = affine_geom(N, K, 64);          // RB / KC only: the same for every group size
+    constexpr size_t smem = C::kPOff + A4S_SP * 8u * aff_block_bytes(GS) + 512 + 1024;
+    static_assert(C::kPOff + A4S_SP * 8u * aff_block_bytes(GS) >= skinny_sum_bytes(TN), "the sums fit the rings");
+    const int tiles = g.RB / 8, split = skinny_split(tiles, g.KC, ctx->sm_count, 3.0f);
+    const cudaError_t e = skinny_launch(affine_b4_skinny_kernel<TN, GS>, tiles, split, A4S_THREADS, smem, stream, map, packed, y, M, N, g.RB, g.KC, split,
+                                        out_f32, bias, ctx->dev_status);
+    if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "affine_b4_skinny: %s", cudaGetErrorString(e));
+    return scr_check_launch(ctx, "affine_b4_skinny");
+}
+
+}  // namespace
+
+// Whether the GEMM for few tokens takes this call: above the matvec's 16 tokens, up to the 128 that one accumulator and three
+// or four activation stages hold beside the weights.  (Beyond, a second token tile would expand every weight a second time.)
+bool affine_b4_skinny_applies(int M) { return M > 16 && M <= 128; }
+
+int32_t affine_b4_skinny_launch(scr_ctx* ctx, const uint8_t* packed, const uint16_t* x, uint16_t* y, int M, int N, int K, int gs, int out_f32,
+                                const uint16_t* bias, cudaStream_t stream) {
+    tc_encode_tiled_fn enc = tc_tensor_map_encoder();
+    if (!enc) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled entry point not available");
+    CUtensorMap map;
+    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
+    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+    const cuuint32_t box[2] = {64, (cuuint32_t)((M + 15) & ~15)};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t*>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+#define A4S_CASE(TN) (gs == 2 ? a4s_launch<TN, 2>(ctx, map, packed, y, M, N, K, out_f32, bias, stream) \
+                              : a4s_launch<TN, 1>(ctx, map, packed, y, M, N, K, out_f32, bias, stream))
+    if (M <= 32) return A4S_CASE(32);
+    if (M <= 64) return A4S_CASE(64);
+    return A4S_CASE(128);
+#undef A4S_CASE
+}

@@ -1,0 +1,35 @@
+"""The GEMMs for few tokens (weights as the rows of the MMA, k shared by a cluster) at the edges of their tiles and splits,
+against the oracle with the bars of the paths they stand beside."""
+import numpy as np
+import pytest
+
+import oracle
+from scratchy_b200 import synth
+from util import bf16_dev, bits_of, rel_l2, u32_dev
+
+pytestmark = pytest.mark.gpu
+REL_L2_TOL = 1e-3                    # the bar of every int4 and fp8 output: one bf16 rounding of an f32-accumulated sum
+
+
+@pytest.mark.parametrize("group", [32, 64, 128])
+@pytest.mark.parametrize("N,K,M", [(8, 128, 17), (130, 384, 32), (136, 640, 33), (128, 1152, 48), (3072, 3072, 64), (264, 2176, 65), (1000, 8192, 127),
+                                   (5120, 3072, 128)])
+def test_int4(N, K, M, group):
+    """Token counts on both sides of 32, 64 and 128; one k chunk and rings that go round; 1 to 8 CTAs per tile; ragged channels;
+    with a bias, and as unrounded partial sums."""
+    import torch
+    from scratchy_b200 import AffineQuantLinear
+    seed = synth.seed_for("few", N, K, M, group)
+    w, s, b = synth.affine_int4_weights(N, K, group, seed)
+    x = synth.activations_bf16(M, K, seed + 1)
+    bias = synth.activations_bf16(1, N, seed + 2).reshape(N)
+    want = oracle.affine_qmm_t_b4(w.view(np.uint8).reshape(-1), s, b, x, M, N, K, group)
+    layer = AffineQuantLinear.from_tensors(u32_dev(w), bf16_dev(s), bf16_dev(b), group, 4)
+    xd = bf16_dev(x).reshape(M, K)
+    y, part = layer.forward(xd), layer.forward_partial(xd)
+    layer.linear_bias = bf16_dev(bias)
+    yb = layer.forward(xd)
+    torch.cuda.synchronize()
+    assert rel_l2(bits_of(y).reshape(M, N), want) <= REL_L2_TOL
+    assert torch.equal(part.bfloat16().view(torch.int16), y.view(torch.int16))
+    assert torch.equal((part + layer.linear_bias.float()).bfloat16().view(torch.int16), yb.view(torch.int16))
