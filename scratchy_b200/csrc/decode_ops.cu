@@ -542,20 +542,22 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_kernel(
 
 
 // ---- the streaming variant: TMA tiles + tensor cores -------------------------------------------
-// In the paged layout one (block, kv head) is a contiguous run of block_size tokens x D bf16.  A
-// producer warp brings those runs (K and V) into a shared-memory ring with one 3-D TMA tile load
-// each (tensor map over the cache viewed as [token][D/64][64], 128-byte swizzle), one ring stage
-// per cache block, completion counted in bytes on the stage's mbarrier; everything the ring holds
-// is in flight at once.  Each of the eight consumer warps takes whole blocks and runs them through
-// mma.sync m16n8k16: S = Q K^T with the (up to 8) query heads of the kv head as the rows of the
-// 16-row A operand and K read by ldmatrix; an online softmax on the accumulator fragments; O += P V
-// with V read by ldmatrix.trans and P split into a bf16 head and a bf16 remainder (two MMAs), so
-// the probabilities keep ~16 mantissa bits.  Scores, the softmax state and O stay in f32.
+// In the paged layout one (block, kv head) is a contiguous run of block_size tokens x D bf16.  A run
+// (K and V) comes into shared memory with a few 3-D TMA tile loads (tensor map over the cache viewed
+// as [token][D/64][64], 128-byte swizzle), one stage per cache block, completion counted in bytes on
+// the stage's mbarrier.  Every warp has its own ring of stages, takes blocks warp, warp + warps, ..
+// and refills a stage itself once its lanes are done with it, so no warp waits for another: a producer
+// warp whose lanes fed one stage each went round in lockstep with the slowest of them.  Blocks run
+// through mma.sync m16n8k16: S = Q K^T with the (up to 8) query heads of the kv head as rows 0..7 of
+// the A operand and K read by ldmatrix; an online softmax on the accumulator fragments; O += P V with
+// V read by ldmatrix.trans, P's bf16 head in rows 0..7 and its bf16 remainder in rows 8..15 of one MMA,
+// so the probabilities keep ~16 mantissa bits.  Scores, the softmax state and O stay in f32.
 // The cluster (1, 2, 4 or 8 CTAs, chosen by the host from the batch) splits the sequence by whole
 // blocks.  Every wait is bounded and reports through the status word.
-constexpr int ATTB_THREADS = ATT_THREADS + 32;
+//
+// What bounds it: HBM (8 KB per block of 16 tokens and kv head).  Llama-3.2-3B at 32 sequences of 512 to 2048 tokens, 168 MB
+// per layer: 60 us with the producer warp and a second MMA for the remainders, 46 us (3.6 TB/s) like this, alone and cold.
 constexpr int ATT_ERR_FULL = 0x0A000001;
-constexpr int ATT_ERR_EMPTY = 0x0A000002;
 
 __device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const CUtensorMap* tmap, int c0, int c1, int c2, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
@@ -569,12 +571,10 @@ __device__ __forceinline__ void ldsm_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
-// D(16x8,f32) += A(16x16,bf16) * B(16x8,bf16).  Rows 8..15 of A are zero here (a1 = a3 = 0), so the
-// accumulator halves of those rows (z0, z1) stay zero: callers pass a few shared dummies for them.
-__device__ __forceinline__ void mma_bf16_16816(float& c0, float& c1, float& z0, float& z1, uint32_t a0, uint32_t a2, uint32_t b0,
-                                               uint32_t b1) {
+// D(16x8,f32) += A(16x16,bf16) * B(16x8,bf16); a0, a2: rows 0..7, a1, a3: rows 8..15.
+__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c0), "+f"(c1), "+f"(z0), "+f"(z1) : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ float fast_exp2(float x) {
     float y;
@@ -617,7 +617,7 @@ __device__ __forceinline__ uint32_t att_rope_pair(uint32_t x0w, uint32_t x1w, co
 }
 
 template <int D>
-__global__ void __launch_bounds__(ATTB_THREADS) attention_decode_tc_kernel(
+__global__ void __launch_bounds__(ATT_THREADS) attention_decode_tc_kernel(
     const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, const uint16_t* __restrict__ q,
     long long ld_q, const uint32_t* __restrict__ block_table, const uint32_t* __restrict__ seq_used_k,
     uint16_t* __restrict__ out, long long ld_o, int G, int num_kv_heads, int block_size, int max_blocks_per_seq,
@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(ATTB_THREADS) attention_decode_tc_kernel(
     constexpr int KSTEPS = D / 16;
     constexpr int NTILES = D / 8;
     extern __shared__ __align__(128) unsigned char att_smem[];
-    const int nwarps = int(blockDim.x >> 5) - 1;     // consumer warps; the last warp is the producer
+    const int nwarps = int(blockDim.x >> 5);
     const uint32_t chunk = uint32_t(block_size) * D * 2;                   // bytes of one block's K (or V) for one kv head
     const uint32_t half_bytes = uint32_t(block_size) * 128;                // one 64-dim half of it: [token][128 bytes], swizzled
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(att_smem) + 1023) & ~uintptr_t(1023));
@@ -635,7 +635,7 @@ __global__ void __launch_bounds__(ATTB_THREADS) attention_decode_tc_kernel(
     const size_t ring_bytes = max(size_t(stages) * 2 * chunk, size_t(nwarps) * G * STATE * sizeof(float));
     float* cl_part = reinterpret_cast<float*>(ring + ((ring_bytes + 127) & ~size_t(127)));        // [nsplit<=8][G][STATE]
     uint32_t* blocks = reinterpret_cast<uint32_t*>(cl_part + ATT_SPLITS * G * STATE);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(blocks + ((table_cap + 1) & ~1));                // full[stages], empty[stages]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(blocks + ((table_cap + 1) & ~1));                // full[stages]
 
     pdl_trigger();
     uint32_t nsplit;
@@ -668,51 +668,41 @@ __global__ void __launch_bounds__(ATTB_THREADS) attention_decode_tc_kernel(
         blocks[i] = pb;
     }
     if (threadIdx.x == 0) {
-        for (int s = 0; s < stages; ++s) {
-            mbar_init(smem_u32(&bars[s]), 1);
-            mbar_init(smem_u32(&bars[stages + s]), 1);
-        }
+        for (int s = 0; s < stages; ++s) mbar_init(smem_u32(&bars[s]), 1);
         fence_mbar_init();
     }
     __syncthreads();
     // What the previous kernels of the stream produce for this one is q and the cache slot of the newest token
-    // (position kv_len - 1, in the sequence's last block).  Every other cache block was written in earlier steps,
-    // so the producer starts streaming them at once and only the last block, and the consumers' q, wait.
+    // (position kv_len - 1, in the sequence's last block).  Every other cache block was written in earlier steps, so a warp
+    // fills its ring at once and only the last block and q wait (with the append folded in, no preceding kernel writes the
+    // cache at all).
     const int newest_blk = total_blk - 1;
-
-    if (warp == nwarps) {
-        // ---------------- producer: lane s owns ring stage s and issues, in order, every block that passes
-        // through it (a single thread's TMA issue rate would otherwise bound short sequences).  Consumer warp
-        // w owns stages [w*spw, (w+1)*spw) and takes blocks w, w+nwarps, ...; its j-th block sits in stage
-        // w*spw + j%spw.  Each side waits on one barrier strictly in phase order, so a parity wait is never
-        // more than one phase ahead of its barrier.
-        const int spw = stages / nwarps;
-        if (lane < stages) {
-            const int w = lane / spw, r = lane - w * spw;
-            const uint32_t full = smem_u32(&bars[lane]);
-            const uint32_t dst = smem_u32(ring + size_t(lane) * 2 * chunk);
-            bool waited = false;
-            for (int n = 0;; ++n) {
-                const int i = w + nwarps * (r + spw * n);
-                if (i >= nblk) break;
-                if (!rope.enabled && !waited && first_blk + i >= newest_blk) {
-                    pdl_wait();                    // (with the append folded in, no preceding kernel writes the cache)
-                    waited = true;
-                }
-                if (n >= 1 && !mbar_wait(smem_u32(&bars[stages + lane]), uint32_t((n - 1) & 1), status, ATT_ERR_EMPTY)) break;
-                const int token0 = int((blocks[i] * uint32_t(num_kv_heads) + uint32_t(kvh)) * uint32_t(block_size));
-                mbar_arrive_expect_tx(full, 2 * chunk);
+    const int spw = stages / nwarps;
+    auto load = [&](int n) {                           // lane 0: the warp's n-th block
+        const int i = warp + n * nwarps;
+        if (i >= nblk) return;
+        const int s = warp * spw + n % spw;
+        const uint32_t full = smem_u32(&bars[s]), dst = smem_u32(ring + size_t(s) * 2 * chunk);
+        const int token0 = int((blocks[i] * uint32_t(num_kv_heads) + uint32_t(kvh)) * uint32_t(block_size));
+        mbar_arrive_expect_tx(full, 2 * chunk);
 #pragma unroll
-                for (int h = 0; h < NH; ++h) {                              // [half][token][128 bytes]: ldmatrix rows 8 tokens apart never share a bank
-                    tma_load_3d(dst + h * half_bytes, &k_map, 0, h, token0, full);
-                    tma_load_3d(dst + chunk + h * half_bytes, &v_map, 0, h, token0, full);
-                }
-            }
+        for (int h = 0; h < NH; ++h) {                 // [half][token][128 bytes]: ldmatrix rows 8 tokens apart never share a bank
+            tma_load_3d(dst + h * half_bytes, &k_map, 0, h, token0, full);
+            tma_load_3d(dst + chunk + h * half_bytes, &v_map, 0, h, token0, full);
         }
-        __syncwarp();
-    } else {
-        // ---------------- consumers: warp w owns blocks w, w+8, ...
+    };
+    {
+        bool pending = false;
+        if (lane == 0)
+            for (int n = 0; n < spw; ++n) {
+                if (!rope.enabled && first_blk + warp + n * nwarps >= newest_blk) pending = true;
+                else load(n);
+            }
         pdl_wait();
+        if (pending)
+            for (int n = 0; n < spw; ++n)
+                if (first_blk + warp + n * nwarps >= newest_blk) load(n);
+        __syncwarp();
         const int row = lane >> 2, quad = lane & 3;
         uint32_t qa0[KSTEPS], qa2[KSTEPS];             // A fragments of Q: row = query head (zero beyond G), 16 dims per step
 #pragma unroll
@@ -744,14 +734,12 @@ __global__ void __launch_bounds__(ATTB_THREADS) attention_decode_tc_kernel(
         }
         const float sl2 = scale * 1.4426950408889634f;                     // scores live in the log2 domain
         float m2 = -INFINITY, lsum = 0.0f;                                 // this lane's row; lsum is the lane's share of the row sum
-        float o[NTILES][2];
+        float o[NTILES][4];                                                // [..][0..1]: the P heads' share, [2..3]: the remainders'
 #pragma unroll
-        for (int nt = 0; nt < NTILES; ++nt) o[nt][0] = o[nt][1] = 0.0f;
-        float z[4][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};   // rows 8..15: always zero, rotated to keep the MMAs independent
+        for (int nt = 0; nt < NTILES; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.0f;
         // ldmatrix lane roles: lane supplies the row address of matrix lane/8, row lane%8
         const int lm = lane >> 3, lr = lane & 7;
         bool alive = true;
-        const int spw = stages / nwarps;
         for (int i = warp, j = 0; i < nblk && alive; i += nwarps, ++j) {
             const int s = warp * spw + j % spw;
             alive = mbar_wait(smem_u32(&bars[s]), uint32_t((j / spw) & 1), status, ATT_ERR_FULL);
@@ -798,9 +786,7 @@ __global__ void __launch_bounds__(ATTB_THREADS) attention_decode_tc_kernel(
             for (int sub = 0; sub < block_size; sub += 16) {
                 if (t0 + sub >= kv_len) break;
                 // S[16 x 16 tokens] = Q K^T
-                float sc[2][2];
-#pragma unroll
-                for (int j = 0; j < 2; ++j) sc[j][0] = sc[j][1] = 0.0f;
+                float sc[2][4] = {};
 #pragma unroll
                 for (int kk = 0; kk < KSTEPS; ++kk) {
                     // matrices: (tokens 0-7, dims +0..7), (tokens 0-7, dims +8..15), (tokens 8-15, +0..7), (tokens 8-15, +8..15)
@@ -808,8 +794,8 @@ __global__ void __launch_bounds__(ATTB_THREADS) attention_decode_tc_kernel(
                     const int dchunk = kk * 2 + (lm & 1);                  // 16-byte piece of the token's D*2-byte row
                     uint32_t kb[4];
                     ldsm_x4(kst + (dchunk >> 3) * half_bytes + token * 128 + (((dchunk & 7) ^ (token & 7)) << 4), kb);
-                    mma_bf16_16816(sc[0][0], sc[0][1], z[0][0], z[0][1], qa0[kk], qa2[kk], kb[0], kb[1]);
-                    mma_bf16_16816(sc[1][0], sc[1][1], z[1][0], z[1][1], qa0[kk], qa2[kk], kb[2], kb[3]);
+                    mma_bf16_16816(sc[0], qa0[kk], 0u, qa2[kk], 0u, kb[0], kb[1]);
+                    mma_bf16_16816(sc[1], qa0[kk], 0u, qa2[kk], 0u, kb[2], kb[3]);
                 }
                 // online softmax on the row this lane holds (tokens j*8 + quad*2 + {0,1})
                 float rmax = -INFINITY;
@@ -839,6 +825,8 @@ __global__ void __launch_bounds__(ATTB_THREADS) attention_decode_tc_kernel(
                     for (int nt = 0; nt < NTILES; ++nt) {
                         o[nt][0] *= corr;
                         o[nt][1] *= corr;
+                        o[nt][2] *= corr;
+                        o[nt][3] *= corr;
                     }
                 }
                 // P as the A operand of the second product: k = tokens; bf16 head + bf16 remainder
@@ -852,14 +840,12 @@ __global__ void __launch_bounds__(ATTB_THREADS) attention_decode_tc_kernel(
                     const int dchunk = nt + (lm >> 1);
                     uint32_t vb[4];
                     ldsm_x4_trans(vst + (dchunk >> 3) * half_bytes + token * 128 + (((dchunk & 7) ^ (token & 7)) << 4), vb);
-                    mma_bf16_16816(o[nt][0], o[nt][1], z[0][0], z[0][1], ph0, ph2, vb[0], vb[1]);
-                    mma_bf16_16816(o[nt + 1][0], o[nt + 1][1], z[1][0], z[1][1], ph0, ph2, vb[2], vb[3]);
-                    mma_bf16_16816(o[nt][0], o[nt][1], z[2][0], z[2][1], pl0, pl2, vb[0], vb[1]);
-                    mma_bf16_16816(o[nt + 1][0], o[nt + 1][1], z[3][0], z[3][1], pl0, pl2, vb[2], vb[3]);
+                    mma_bf16_16816(o[nt], ph0, pl0, ph2, pl2, vb[0], vb[1]);
+                    mma_bf16_16816(o[nt + 1], ph0, pl0, ph2, pl2, vb[2], vb[3]);
                 }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&bars[stages + s]));
+            __syncwarp();                                                  // every lane is done with the stage
+            if (lane == 0) load(j + spw);
         }
         lsum += __shfl_xor_sync(0xffffffffu, lsum, 1);
         lsum += __shfl_xor_sync(0xffffffffu, lsum, 2);
@@ -870,8 +856,8 @@ __global__ void __launch_bounds__(ATTB_THREADS) attention_decode_tc_kernel(
             float* st = warp_part + (warp * G + row) * STATE;
 #pragma unroll
             for (int nt = 0; nt < NTILES; ++nt) {
-                st[nt * 8 + quad * 2] = o[nt][0];
-                st[nt * 8 + quad * 2 + 1] = o[nt][1];
+                st[nt * 8 + quad * 2] = o[nt][0] + o[nt][2];
+                st[nt * 8 + quad * 2 + 1] = o[nt][1] + o[nt][3];
             }
             if (quad == 0) {
                 st[D] = m2 * 0.6931471805599453f;                          // back to the natural-log domain of the merge
@@ -914,7 +900,7 @@ cudaError_t attention_launch(const uint16_t* q, long long ld_q, const uint16_t* 
     int nsplit = ATT_SPLITS;                         // the most splits that still run as a single wave of two CTAs per SM
     while (nsplit > 1 && (long long)batch * num_kv_heads * nsplit > 2LL * sm_count) nsplit /= 2;
     const int table_cap = max_blocks_per_seq / nsplit + 2;
-    const size_t fixed = part + size_t((table_cap + 1) & ~1) * 4 + 2 * ATT_MAX_STAGES * sizeof(uint64_t) + 1024 + 128;
+    const size_t fixed = part + size_t((table_cap + 1) & ~1) * 4 + ATT_MAX_STAGES * sizeof(uint64_t) + 1024 + 128;
     // alone on its SM: 8 consumer warps and a deep ring; otherwise 4 consumer warps and about half an SM's shared
     // memory.  The big CTA (48 K registers, ~200 KB) shares its SM with no CTA of the kernels before and after it in
     // the stream, so it pays only while the grid leaves most SMs to them: up to half the SMs.  (Llama-3.2-3B decode
@@ -954,7 +940,7 @@ cudaError_t attention_launch(const uint16_t* q, long long ld_q, const uint16_t* 
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
         cfg.gridDim = dim3(nsplit, num_kv_heads, batch);
-        cfg.blockDim = dim3((nwarps + 1) * 32);
+        cfg.blockDim = dim3(nwarps * 32);
         cfg.dynamicSmemBytes = smem;
         attr[0].val.clusterDim.x = nsplit;
         return cudaLaunchKernelEx(&cfg, kernel, maps[0], maps[1], q, ld_q, block_table, seq_used_k, out, ld_o, G, num_kv_heads,
