@@ -19,7 +19,7 @@ LIB = os.path.join(HERE, "libscratchy_cuda.so")
 MODELS_LIB = os.path.join(HERE, "libscratchy_models.so")
 
 SOURCES = ["context.cu", "abi.cu", "affine_b4.cu", "affine_b4_gemm.cu", "affine_b4_gemm_pair.cu", "affine_b4_skinny.cu", "fp8.cu", "fp8_gemm.cu", "fp8_gemm_pair.cu", "decode_ops.cu", "tp_comm.cu"]
-MODELS_COMMON = ["context.cu", "dense_linear.cu", "dense_gemm.cu", "seq_ops.cu"]
+MODELS_COMMON = ["context.cu", "dense_linear.cu", "dense_gemm.cu", "dense_skinny.cu", "seq_ops.cu"]
 # what the layers of a design run on
 DESIGNS = {
     "Vumipel": ["latent_attention.cu", "latent_attention_mma.cu", "latent_prefill.cu", "mlstm.cu", "mlstm_chunk.cu"],

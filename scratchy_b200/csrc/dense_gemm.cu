@@ -13,6 +13,17 @@
 
 #include <algorithm>
 
+// Tensor map over bf16 values [d2][d1][d0] (d0 dense, the others s1 and s2 bytes apart), boxes of 64 x b1 x b2
+bool dense_tensor_map(CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1, uint64_t s2, uint32_t b1, uint32_t b2) {
+    tc_encode_tiled_fn enc = tc_tensor_map_encoder();
+    if (!enc) return false;
+    const cuuint64_t dims[3] = {d0, d1, d2};
+    const cuuint64_t strides[2] = {s1, s2};
+    const cuuint32_t box[3] = {64, b1, b2}, one[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 namespace {
 
 constexpr int DG_THREADS = 192;
@@ -200,7 +211,6 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     const int n_tail = MT * NTB * groups - full;
     const int units = full + n_tail * ks_tail;
 
-    pdl_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::kStages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), 128); }
@@ -214,6 +224,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_trigger();                                     // not before this CTA has its TMEM: the next kernel's CTAs could take it first
     pdl_wait();
 
     if (warp == 0) {
@@ -326,22 +337,12 @@ __global__ void __launch_bounds__(256) dense_gemm_finish_kernel(const float* __r
     dense_put_two<bf16, END>(ends, m, g, n, N, a, b);
 }
 
-bool dg_map(CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1, uint64_t s2, uint32_t b1, uint32_t b2) {
-    tc_encode_tiled_fn enc = tc_tensor_map_encoder();
-    if (!enc) return false;
-    const cuuint64_t dims[3] = {d0, d1, d2};
-    const cuuint64_t strides[2] = {s1, s2};
-    const cuuint32_t box[3] = {64, b1, b2}, one[3] = {1, 1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <int BN, DenseEnd END>
 int32_t dg_launch(scr_ctx* ctx, const scr_dense& d, const DgPlan& p, float* slabs, cudaStream_t stream) {
     CUtensorMap x_map, w_map;
     const uint64_t xg = d.groups > 1 ? (uint64_t)d.x_group * 2 : (uint64_t)d.K * 2;
-    if (!dg_map(&x_map, d.x, d.K, d.groups, d.M, xg, (uint64_t)d.ldx * 2, 1, 128) ||
-        !dg_map(&w_map, d.w, d.K, d.N, d.groups, (uint64_t)d.K * 2, (uint64_t)d.N * d.K * 2, BN, 1))
+    if (!dense_tensor_map(&x_map, d.x, d.K, d.groups, d.M, xg, (uint64_t)d.ldx * 2, 1, 128) ||
+        !dense_tensor_map(&w_map, d.w, d.K, d.N, d.groups, (uint64_t)d.K * 2, (uint64_t)d.N * d.K * 2, BN, 1))
         return scr_fail(ctx, SCR_E_CUDA, "dense_gemm: tensor map (M %d N %d K %d groups %d)", d.M, d.N, d.K, d.groups);
     cudaError_t e = seq_smem(dense_gemm_kernel<BN, END>, DgSmem<BN>::kTotal);
     if (e == cudaSuccess) {

@@ -1,7 +1,8 @@
 // Full-precision linears of the sequence models: y = x W^T with the ends of `scr_dense`.
 //
 //   M <= 16, bf16   dense_matvec_kernel   weights streamed once from HBM straight into mma.sync fragments (decode)
-//   M > 16, bf16    dense_gemm.cu         tcgen05 GEMM
+//   M <= 128, bf16  dense_skinny.cu       tcgen05 GEMM, the weights as the rows of the MMA
+//   M > 128, bf16   dense_gemm.cu         tcgen05 GEMM
 //   otherwise       dense_plain_kernel    f32 arithmetic on any sizes (the f32 data type; bf16 rows that are not a
 //                                         multiple of 16 bytes)
 #include "seq_common.cuh"
@@ -10,6 +11,8 @@
 
 size_t dense_gemm_workspace(int M, int N, int K, int groups);
 int32_t dense_gemm_launch(scr_ctx* ctx, const scr_dense& d, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+bool dense_skinny_applies(int M);
+int32_t dense_skinny_launch(scr_ctx* ctx, const scr_dense& d, cudaStream_t stream);
 
 namespace {
 
@@ -228,7 +231,7 @@ bool rows_of_16_bytes(const scr_dense& d) {
 extern "C" int32_t scr_dense_workspace_size(int32_t dtype, int32_t M, int32_t N, int32_t K, int32_t groups, size_t* bytes) {
     if (!bytes) return SCR_E_ARG;
     if (M <= 0 || N <= 0 || K <= 0 || groups <= 0) return SCR_E_SHAPE;
-    *bytes = (dtype == SCR_DTYPE_BF16 && M > 16) ? dense_gemm_workspace(M, N, K, groups) : 0;
+    *bytes = (dtype == SCR_DTYPE_BF16 && !dense_skinny_applies(M)) ? dense_gemm_workspace(M, N, K, groups) : 0;
     return SCR_OK;
 }
 
@@ -257,5 +260,6 @@ extern "C" int32_t scr_dense_linear(scr_ctx* ctx, int32_t dtype, const scr_dense
     if (!rows_of_16_bytes(d)) return plain_launch<bf16>(ctx, d, st);
     if (d.M <= 16)
         return d.residual ? matvec_launch<END_RESIDUAL>(ctx, d, st) : d.n_parts ? matvec_launch<END_PARTS>(ctx, d, st) : matvec_launch<END_OWN>(ctx, d, st);
+    if (dense_skinny_applies(d.M)) return dense_skinny_launch(ctx, d, st);
     return dense_gemm_launch(ctx, d, workspace, workspace_bytes, st);
 }

@@ -1,0 +1,164 @@
+// bf16 GEMM for few rows of x on tcgen05 tensor cores, the weights as the rows of the MMA (skinny.cuh), with the ends of
+// `scr_dense` applied to the finished sums.
+//
+// A unit is 128 rows of W by one CTA's share of the 64-wide k slices; 352 threads:
+//   warps 0-7    drain the accumulator and store
+//   warp 8       producer of the weights (one tiled TMA load of 128 rows x 64 k per slice, 128-byte swizzle), load-time
+//                constants: it starts before the preceding kernel of the stream has finished
+//   warp 9       producer of x (one tiled TMA load per slice, zeros outside)
+//   warp 10      owns TMEM; one thread issues 4 tcgen05.mma (128 x rows of x x 16) per slice
+//
+// What bounds it: the weights from HBM.  16384 x 3072 at 32 rows takes 29 us alone (100 MB, 3.4 TB/s from a cold start) and
+// 128256 x 3072 143 us (5.5 TB/s).  In the decode step of the 3B Vumipel at 32 sequences it replaces the 128-row tile of
+// dense_gemm.cu and its finishing launch: 4.22 -> 3.59 ms per step.
+#include "seq_common.cuh"
+#include "skinny.cuh"
+
+namespace {
+
+constexpr int DS_THREADS = 352;
+constexpr uint32_t DS_W_STAGE = SKINNY_ROWS * 128u;          // 128 rows x 64 bf16
+
+template <int TN>
+struct DsCfg {
+    static constexpr int kSW = TN == 128 ? 8 : TN == 16 ? 6 : 5;                  // weight stages
+    static constexpr int kSX = TN == 128 ? 4 : TN == 64 ? 3 : kSW;                // x stages
+    static constexpr uint32_t kXStage = TN * 128u;
+    static constexpr uint32_t kXOff = kSW * DS_W_STAGE;
+    static constexpr uint32_t kBarOff = kXOff + kSX * kXStage;
+    static constexpr uint32_t kTotal = kBarOff + 256u + 1024u;
+    static constexpr uint32_t kTmemCols = TN < 32 ? 32 : TN;
+    static constexpr int kCtasPerSm = TN == 128 ? 1 : 2;
+};
+
+template <int TN, DenseEnd END>
+__global__ void __launch_bounds__(DS_THREADS, DsCfg<TN>::kCtasPerSm)
+dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, int M, int N, int KT, int NT, int split,
+                    DenseEnds ends, int* __restrict__ status) {
+    using C = DsCfg<TN>;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t bar = smem_base + C::kBarOff;
+    auto wfull = [&](int s) { return bar + 8u * s; };
+    auto wempty = [&](int s) { return bar + 8u * (C::kSW + s); };
+    auto xfull = [&](int s) { return bar + 8u * (2 * C::kSW + s); };
+    auto xempty = [&](int s) { return bar + 8u * (2 * C::kSW + C::kSX + s); };
+    constexpr int kSlots = 2 * C::kSW + 2 * C::kSX;
+    static_assert(8 * (kSlots + 2) <= 256, "barriers");
+    const uint32_t accf = bar + 8u * kSlots;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + C::kBarOff + 8 * (kSlots + 1));
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tile = blockIdx.x / split, rank = blockIdx.x - tile * split;
+    const int g = tile / NT, n0 = (tile - g * NT) * SKINNY_ROWS;
+    int k_lo, k_hi;
+    skinny_range(KT, rank, split, k_lo, k_hi);
+    const int steps = k_hi - k_lo;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < C::kSW; ++s) { mbar_init(wfull(s), 1); mbar_init(wempty(s), 1); }
+        for (int s = 0; s < C::kSX; ++s) { mbar_init(xfull(s), 1); mbar_init(xempty(s), 1); }
+        mbar_init(accf, 1);
+        fence_mbar_init();
+    }
+    if (warp == 10) {
+        tmem_alloc(smem_u32((const void*)tmem_slot), C::kTmemCols);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    pdl_trigger();                                     // not before this CTA has its TMEM: the next kernel's CTAs could take it first
+
+    // Only the weights may be touched before the preceding kernel has finished.  A wait that depends on x comes after
+    // griddepcontrol.wait, so that its bound does not run against that kernel.
+    if (warp == 8) {
+        if (lane == 0) {
+            for (int i = 0; i < steps; ++i) {
+                const int s = i % C::kSW;
+                if (i == C::kSW) pdl_wait();
+                mbar_wait(wempty(s), ((uint32_t)(i / C::kSW) & 1u) ^ 1u, status, TC_ERR_EMPTY_WAIT);
+                mbar_arrive_expect_tx(wfull(s), DS_W_STAGE);
+                tma_load_3d(smem_base + s * DS_W_STAGE, &w_map, (k_lo + i) * 64, n0, g, wfull(s));
+            }
+        }
+    } else if (warp == 9) {
+        if (lane == 0) {
+            pdl_wait();
+            const uint32_t rows = (uint32_t)(M + 15) & ~15u;
+            for (int i = 0; i < steps; ++i) {
+                const int s = i % C::kSX;
+                mbar_wait(xempty(s), ((uint32_t)(i / C::kSX) & 1u) ^ 1u, status, TC_ERR_EMPTY_WAIT);
+                mbar_arrive_expect_tx(xfull(s), rows * 128u);
+                tma_load_3d(smem_base + C::kXOff + s * C::kXStage, &x_map, (k_lo + i) * 64, g, 0, xfull(s));
+            }
+        }
+    } else if (warp == 10) {
+        if (lane == 0) {
+            pdl_wait();
+            const uint32_t idesc = umma_idesc(1, 1, SKINNY_ROWS, (uint32_t)(M + 15) & ~15u);
+            for (int i = 0; i < steps; ++i) {
+                const int sw = i % C::kSW, sx = i % C::kSX;
+                mbar_wait(wfull(sw), (uint32_t)(i / C::kSW) & 1u, status, TC_ERR_FULL_WAIT);
+                mbar_wait(xfull(sx), (uint32_t)(i / C::kSX) & 1u, status, TC_ERR_FULL_WAIT);
+                tc_fence_after();
+                const uint64_t adesc = umma_desc_k_sw128(smem_base + sw * DS_W_STAGE), bdesc = umma_desc_k_sw128(smem_base + C::kXOff + sx * C::kXStage);
+#pragma unroll
+                for (int k4 = 0; k4 < 4; ++k4) umma_f16(tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, (i | k4) != 0);
+                umma_commit(wempty(sw));
+                umma_commit(xempty(sx));
+            }
+            umma_commit(accf);
+        }
+    } else {
+        pdl_wait();
+        mbar_wait(accf, 0, status, TC_ERR_ACC_FULL);
+    }
+    __syncwarp();
+    pdl_wait();
+    skinny_finish(tmem, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, n0, N,
+                  [&](int m, int n, float a, float b) { dense_put_two<bf16, END>(ends, m, g, n, N, a, b); });
+    __syncthreads();
+    if (warp == 10) {
+        tc_fence_after();
+        tmem_dealloc(tmem, C::kTmemCols);
+    }
+}
+
+template <int TN, DenseEnd END>
+int32_t ds_launch(scr_ctx* ctx, const scr_dense& d, const CUtensorMap& x_map, const CUtensorMap& w_map, cudaStream_t stream) {
+    using C = DsCfg<TN>;
+    static_assert(C::kBarOff >= skinny_sum_bytes(TN), "the sums fit the rings");
+    const int nt = scr_ceil_div(d.N, SKINNY_ROWS), kt = scr_ceil_div(d.K, 64), split = skinny_split(nt * d.groups, kt, ctx->sm_count, 4.0f);
+    const cudaError_t e = skinny_launch(dense_skinny_kernel<TN, END>, nt * d.groups, split, DS_THREADS, C::kTotal, stream, x_map, w_map, d.M, d.N, kt, nt,
+                                        split, dense_ends(d), ctx->dev_status);
+    if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "dense_skinny: %s", cudaGetErrorString(e));
+    return scr_check_launch(ctx, "dense_skinny");
+}
+
+template <DenseEnd END>
+int32_t ds_launch_rows(scr_ctx* ctx, const scr_dense& d, const CUtensorMap& x_map, const CUtensorMap& w_map, cudaStream_t stream) {
+    if (d.M <= 16) return ds_launch<16, END>(ctx, d, x_map, w_map, stream);
+    if (d.M <= 32) return ds_launch<32, END>(ctx, d, x_map, w_map, stream);
+    if (d.M <= 64) return ds_launch<64, END>(ctx, d, x_map, w_map, stream);
+    return ds_launch<128, END>(ctx, d, x_map, w_map, stream);
+}
+
+}  // namespace
+
+bool dense_skinny_applies(int M) { return M <= 128; }
+
+int32_t dense_skinny_launch(scr_ctx* ctx, const scr_dense& d, cudaStream_t stream) {
+    CUtensorMap x_map, w_map;
+    const uint64_t xg = d.groups > 1 ? (uint64_t)d.x_group * 2 : (uint64_t)d.K * 2;
+    if (!dense_tensor_map(&x_map, d.x, d.K, d.groups, d.M, xg, (uint64_t)d.ldx * 2, 1, (d.M + 15) & ~15) ||
+        !dense_tensor_map(&w_map, d.w, d.K, d.N, d.groups, (uint64_t)d.K * 2, (uint64_t)d.N * d.K * 2, SKINNY_ROWS, 1))
+        return scr_fail(ctx, SCR_E_CUDA, "dense_skinny: tensor map (M %d N %d K %d groups %d)", d.M, d.N, d.K, d.groups);
+    switch (dense_end(d)) {
+        case END_PARTS: return ds_launch_rows<END_PARTS>(ctx, d, x_map, w_map, stream);
+        case END_RESIDUAL: return ds_launch_rows<END_RESIDUAL>(ctx, d, x_map, w_map, stream);
+        default: return ds_launch_rows<END_OWN>(ctx, d, x_map, w_map, stream);
+    }
+}

@@ -206,3 +206,5 @@ __device__ __forceinline__ void dense_put_two(const DenseEnds& e, int m, int g, 
     dense_put<T, END>(e, m, g, n, a);
     if (n + 8 < N) dense_put<T, END>(e, m, g, n + 8, b);
 }
+// Defined in dense_gemm.cu
+bool dense_tensor_map(CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1, uint64_t s2, uint32_t b1, uint32_t b2);

@@ -33,3 +33,24 @@ def test_int4(N, K, M, group):
     assert rel_l2(bits_of(y).reshape(M, N), want) <= REL_L2_TOL
     assert torch.equal(part.bfloat16().view(torch.int16), y.view(torch.int16))
     assert torch.equal((part + layer.linear_bias.float()).bfloat16().view(torch.int16), yb.view(torch.int16))
+
+
+@pytest.mark.parametrize("N,K,M", [(8, 8, 17), (130, 200, 32), (136, 64, 33), (520, 1032, 64), (300, 4104, 65), (3072, 3072, 128)])
+def test_dense(N, K, M):
+    """The same edges of the bf16 linear: plain and f32 outputs against 64-bit sums, and the residual end."""
+    import torch
+    from scratchy_b200.dense import Arena, DenseLinear
+    rng = np.random.default_rng(N + K + M)
+    draw = lambda *shape: torch.from_numpy(rng.standard_normal(shape).astype(np.float32)).cuda().bfloat16()
+    x, w, a = draw(M, K), draw(N, K), Arena("cuda")
+    want = (x.double() @ w.double().T).cpu()
+    lin, rel = DenseLinear(w), lambda t: float((t.double().cpu() - want).norm() / want.norm())
+    y, y16 = torch.full((M, N), float("nan"), device="cuda"), torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    lin(a, x, y)
+    lin(a, x, y16)
+    res = torch.ones((M, N), device="cuda")
+    lin.add_to(a, x, res)
+    torch.cuda.synchronize()
+    assert rel(y) < 1e-5                                          # f32 sums of at most 4104 products
+    assert torch.equal(y.bfloat16().view(torch.int16), y16.view(torch.int16))
+    assert torch.equal(res, y + 1.0)
