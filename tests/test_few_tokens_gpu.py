@@ -54,3 +54,10 @@ def test_dense(N, K, M):
     assert rel(y) < 1e-5                                          # f32 sums of at most 4104 products
     assert torch.equal(y.bfloat16().view(torch.int16), y16.view(torch.int16))
     assert torch.equal(res, y + 1.0)
+
+
+@pytest.mark.parametrize("N,K,M", [(256, 64, 256), (2560, 200, 1300), (264, 712, 260), (3072, 1096, 2000)])
+def test_dense_on_cta_pairs(N, K, M):
+    """256 x 256 tiles on pairs of SMs: odd numbers of k slices, rows and columns that end inside a CTA's half, rounds that are
+    cut along k and rounds that are not."""
+    test_dense(N, K, M)
