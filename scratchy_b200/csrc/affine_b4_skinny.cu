@@ -230,7 +230,9 @@ int32_t a4s_launch(scr_ctx* ctx, const CUtensorMap& map, const uint8_t* packed, 
     const AffineGeom g = affine_geom(N, K, 64);          // RB / KC only: the same for every group size
     constexpr size_t smem = C::kPOff + A4S_SP * 8u * aff_block_bytes(GS) + 512 + 1024;
     static_assert(C::kPOff + A4S_SP * 8u * aff_block_bytes(GS) >= skinny_sum_bytes(TN), "the sums fit the rings");
-    const int tiles = g.RB / 8, split = skinny_split(tiles, g.KC, ctx->sm_count, 3.0f);
+    static SkinnyResident resident;
+    const int tiles = g.RB / 8;
+    const int split = skinny_split(resident, affine_b4_skinny_kernel<TN, GS>, ctx->device, ctx->sm_count, tiles, g.KC, A4S_THREADS, smem, 3.0f);
     const cudaError_t e = skinny_launch(affine_b4_skinny_kernel<TN, GS>, tiles, split, A4S_THREADS, smem, stream, map, packed, y, M, N, g.RB, g.KC, split,
                                         out_f32, bias, ctx->dev_status);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "affine_b4_skinny: %s", cudaGetErrorString(e));

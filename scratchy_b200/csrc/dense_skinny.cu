@@ -131,7 +131,9 @@ template <int TN, DenseEnd END>
 int32_t ds_launch(scr_ctx* ctx, const scr_dense& d, const CUtensorMap& x_map, const CUtensorMap& w_map, cudaStream_t stream) {
     using C = DsCfg<TN>;
     static_assert(C::kBarOff >= skinny_sum_bytes(TN), "the sums fit the rings");
-    const int nt = scr_ceil_div(d.N, SKINNY_ROWS), kt = scr_ceil_div(d.K, 64), split = skinny_split(nt * d.groups, kt, ctx->sm_count, 4.0f);
+    const int nt = scr_ceil_div(d.N, SKINNY_ROWS), kt = scr_ceil_div(d.K, 64);
+    static SkinnyResident resident;
+    const int split = skinny_split(resident, dense_skinny_kernel<TN, END>, ctx->device, ctx->sm_count, nt * d.groups, kt, DS_THREADS, C::kTotal, 4.0f);
     const cudaError_t e = skinny_launch(dense_skinny_kernel<TN, END>, nt * d.groups, split, DS_THREADS, C::kTotal, stream, x_map, w_map, d.M, d.N, kt, nt,
                                         split, dense_ends(d), ctx->dev_status);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "dense_skinny: %s", cudaGetErrorString(e));

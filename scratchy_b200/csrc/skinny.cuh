@@ -5,6 +5,8 @@
 // unit each, whose sums meet through distributed shared memory in rank order: no workspace, no second kernel.
 #pragma once
 
+#include <atomic>
+
 #include "tc_common.cuh"
 
 constexpr int SKINNY_ROWS = 128;                 // output channels of a tile
@@ -80,13 +82,48 @@ __device__ __forceinline__ void skinny_finish(uint32_t d, uint32_t sums, const f
     }
 }
 
-// CTAs that share a tile's k extent.  A call lasts as long as its busiest SM: (units per SM) x (k steps per unit + what a unit
-// costs beside them), in k steps.
-static inline int skinny_split(int tiles, int steps, int sms, float unit_cost) {
+// How many clusters of `split` CTAs of a kernel run at once (a cluster needs its SMs in one GPC, so 148 SMs hold fewer clusters of
+// 5 or 6 CTAs than 148 / 6): asked once per kernel, device and size.
+constexpr int SKINNY_DEVICES = 64;
+struct SkinnyResident {
+    std::atomic<int> clusters[SKINNY_DEVICES][SKINNY_MAX_SPLIT + 1];
+};
+template <typename... KArgs>
+static inline int skinny_resident(SkinnyResident& cache, void (*kernel)(KArgs...), int device, int sms, int split, int threads, size_t smem) {
+    const bool known = device >= 0 && device < SKINNY_DEVICES;
+    int n = known ? cache.clusters[device][split].load(std::memory_order_relaxed) : 0;
+    if (n > 0) return n;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sms * split));
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = split;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+        (void)cudaGetLastError();
+        n = sms / split > 0 ? sms / split : 1;
+    }
+    if (known) cache.clusters[device][split].store(n, std::memory_order_relaxed);
+    return n;
+}
+
+// CTAs that share a tile's k extent.  A call is rounds of the clusters that run at once; a round lasts as long as a unit, whose
+// k steps share the SM with those of the units beside it and which costs `unit_cost` steps beside them.  (Without the rounds
+// in the account 24 tiles at 128 tokens were cut six ways, 22 of which run at once: 3072 x 3072 int4 took 19.0 us, now 11.1.)
+template <typename... KArgs>
+static inline int skinny_split(SkinnyResident& cache, void (*kernel)(KArgs...), int device, int sms, int tiles, int steps, int threads, size_t smem,
+                               float unit_cost) {
     int best = 1;
     float least = 1e30f;
     for (int s = 1; s <= SKINNY_MAX_SPLIT && s <= steps; ++s) {
-        const float t = (float)((tiles * (long long)s + sms - 1) / sms) * ((float)((steps + s - 1) / s) + unit_cost);
+        const int resident = skinny_resident(cache, kernel, device, sms, s, threads, smem), at_once = tiles < resident ? tiles : resident;
+        const int rounds = (tiles + resident - 1) / resident, beside = (at_once * s + sms - 1) / sms;
+        const float t = (float)rounds * ((float)(beside * ((steps + s - 1) / s)) + unit_cost);
         if (t < least * 0.999f) {
             least = t;
             best = s;
