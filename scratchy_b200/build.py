@@ -18,7 +18,7 @@ OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(HERE, "libscratchy_cuda.so")
 MODELS_LIB = os.path.join(HERE, "libscratchy_models.so")
 
-SOURCES = ["context.cu", "abi.cu", "affine_b4.cu", "affine_b4_gemm.cu", "affine_b4_gemm_pair.cu", "affine_b4_skinny.cu", "fp8.cu", "fp8_gemm.cu", "fp8_gemm_pair.cu", "decode_ops.cu", "tp_comm.cu"]
+SOURCES = ["context.cu", "abi.cu", "affine_b4.cu", "affine_b4_gemm.cu", "affine_b4_gemm_pair.cu", "affine_b4_skinny.cu", "fp8.cu", "fp8_gemm.cu", "fp8_gemm_pair.cu", "fp8_skinny.cu", "decode_ops.cu", "tp_comm.cu"]
 MODELS_COMMON = ["context.cu", "dense_linear.cu", "dense_gemm.cu", "dense_skinny.cu", "seq_ops.cu"]
 # what the layers of a design run on
 DESIGNS = {

@@ -21,6 +21,9 @@ bool fp8_gemm_tc_enabled() { return true; }
 bool fp8_gemm_pair_applies(int M, int N, int K, int sms);
 int32_t fp8_gemm_pair_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint16_t* y, int M, int N, int K,
                              const LinearEnds& ends, cudaStream_t stream, bool* launched);
+// Defined in fp8_skinny.cu
+int32_t fp8_skinny_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint16_t* y, int M, int N, int K, const LinearEnds& ends,
+                          cudaStream_t stream);
 // Channel-tile width and work units.  Wide (256-channel) tiles reuse every activation tile twice and are preferred;
 // a 128-channel tile does half the work in about three quarters of the time (measured), which can still win
 // when it quantises better over the SMs.  Units as in `tc_plan_units`.
@@ -320,6 +323,9 @@ int32_t fp8_gemm_tc_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* ac
         const int32_t st = fp8_gemm_pair_launch(ctx, wpack, act, y, M, N, K, ends, stream, &launched);
         if (st || launched) return st;
     }
+    // what one accumulator holds, where the pair kernel's tiles do not fill the GPU.  (It needs no slabs; the size query keeps what
+    // the tiles above would want, so that no caller's scratch limit moves.)
+    if (M <= 256) return fp8_skinny_launch(ctx, wpack, act, y, M, N, K, ends, stream);
     const Fp8GemmPlan plan = fp8_gemm_plan(M, N, K, ctx->sm_count);
     float* slabs = reinterpret_cast<float*>(workspace);
     if (plan.ks_tail > 1 && (!slabs || !scr_aligned16(slabs))) return scr_fail(ctx, SCR_E_WORKSPACE, "split-K needs an aligned workspace");

@@ -61,3 +61,41 @@ def test_dense_on_cta_pairs(N, K, M):
     """256 x 256 tiles on pairs of SMs: odd numbers of k slices, rows and columns that end inside a CTA's half, rounds that are
     cut along k and rounds that are not."""
     test_dense(N, K, M)
+
+
+@pytest.mark.parametrize("N,K,M", [(8, 64, 17), (130, 328, 32), (264, 1160, 33), (512, 3584, 65), (300, 18944, 128), (384, 256, 129), (3584, 2184, 250)])
+def test_fp8(N, K, M):
+    """Token counts on both sides of 32, 64 and 128, and up to the 256 of one accumulator; ragged channels and k."""
+    import torch
+    from scratchy_b200 import Fp8Linear
+    from util import to_dev
+    seed = synth.seed_for("few8", N, K, M)
+    wq, ws = oracle.fp8_quantize_weight_per_channel(synth.fp8_weights_f32(N, K, seed))
+    x = synth.activations_bf16(M, K, seed + 1)
+    layer, xd = Fp8Linear.from_tensors(to_dev(wq), to_dev(ws)), bf16_dev(x).reshape(M, K)
+    layer.linear_bias = bf16_dev(synth.activations_bf16(1, N, seed + 2).reshape(N))
+    yb, part = layer.forward(xd), layer.forward_partial(xd)
+    layer.linear_bias, bias = None, layer.linear_bias
+    y = layer.forward(xd)
+    torch.cuda.synchronize()
+    assert rel_l2(bits_of(y).reshape(M, N), oracle.fp8_dynamic_linear(x, wq, ws, M, N, K)) <= REL_L2_TOL
+    assert torch.equal(part.bfloat16().view(torch.int16), y.view(torch.int16))
+    assert torch.equal((part + bias.float()).bfloat16().view(torch.int16), yb.view(torch.int16))
+
+
+@pytest.mark.parametrize("K", [1024, 4096, 8200, 12296, 20480, 20488])
+def test_quantisation_of_every_code_and_tie(K):
+    """Every bf16 value in [-448, 448] at a scale of one (half-way cases of every binade and of the subnormal grid among them),
+    at row lengths on both sides of every count of pieces a thread holds: the oracle's bytes."""
+    from scratchy_b200 import Fp8Linear
+    every = np.arange(0x43E0 + 1, dtype=np.uint16)                 # 0 .. 448
+    every = np.concatenate([every, every | np.uint16(0x8000)])
+    M = max(17, -(-every.size // (K - 1)))
+    x = np.zeros((M, K), np.uint16)
+    x[:, 0] = 0x43E0                                               # the row's largest: scale 448 * (1 / 448) = 1
+    flat = np.resize(every, M * (K - 1)).reshape(M, K - 1)
+    x[:, 1:] = flat
+    xq, a = Fp8Linear.quantize_activation(bf16_dev(x.reshape(-1)).reshape(M, K)).unpack()
+    want_q, want_a = oracle.fp8_quant_per_token(x.reshape(-1), M, K)
+    assert (want_a == 1.0).all()
+    assert np.array_equal(a.cpu().numpy(), want_a) and np.array_equal(xq.cpu().numpy().reshape(want_q.shape), want_q)
