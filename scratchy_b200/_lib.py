@@ -198,6 +198,8 @@ _lock = threading.Lock()
 def lib() -> ctypes.CDLL:
     """Load the C-ABI library; raise (never fall back) if it has not been built."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             if not os.path.exists(_LIB_PATH):
@@ -279,8 +281,7 @@ _contexts: dict[int, Context] = {}
 
 def context(device: int) -> Context:
     """Process-wide context of ``device``."""
-    with _lock:
-        c = _contexts.get(device)
+    c = _contexts.get(device)
     if c is None:
         c = Context(device)
         with _lock:
