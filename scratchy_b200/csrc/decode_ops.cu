@@ -248,6 +248,7 @@ __global__ void __launch_bounds__(ARGMAX_THREADS) argmax_kernel(const uint16_t* 
     float best = -INFINITY;
     uint32_t best_i = 0;
     const int nv = width >> 3;
+#pragma unroll 8                                       // one SM reads the row: eight requests a thread in flight
     for (int v = threadIdx.x; v < nv; v += ARGMAX_THREADS) {
         float f[8];
         unpack8(*reinterpret_cast<const uint4*>(row + v * 8), f);

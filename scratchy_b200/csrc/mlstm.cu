@@ -5,7 +5,8 @@
 //   o = S'^T q / (max(|n'.q|, e^(-m')) + 1e-6),   q scaled by dim^(-1/2)
 // State and everything about it is f32.
 //
-//   mlstm_recur_kernel   token by token: decoding, short portions, any sizes, both data types
+//   mlstm_step_kernel    token by token: decoding, short portions, dim up to 256, both data types
+//   mlstm_recur_kernel   the same for larger dim
 //   mlstm_chunk.cu       bf16 prompts, 64 tokens at a time on the tensor cores
 //   mlstm_finish_kernel  each head's output over its root mean square, the norm's weight and the output gate
 #include "seq_common.cuh"
@@ -137,7 +138,176 @@ __global__ void __launch_bounds__(RC_T) mlstm_recur_kernel(MemoryArgs a) {
     if (tid == 0) a.state_m[copy] = m;
 }
 
+// The slice of S (and this slice's copy of n) in registers: 8 threads with 4 columns each cover a row, a thread has RPT rows, 32
+// apart.  The state is requested before the wait for the preceding kernel (no other kernel of a step touches it), and a token
+// takes one barrier: the normaliser's n.q goes round with the outputs.
+template <typename T, int RPT>
+__global__ void __launch_bounds__(RC_T) mlstm_step_kernel(MemoryArgs a) {
+    __shared__ float4 part[2][RC_T / 32][8];
+    __shared__ float part_n[2][RC_T / 32];
+    pdl_trigger();
+    const scr_mlstm_shape& s = a.s;
+    const int dim = s.dim, vdim = s.vdim;
+    const int h = blockIdx.y, b = blockIdx.z, c0 = blockIdx.x * RC_COLS;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row0 = tid >> 3;
+    const int* seg = a.st.segs + b * 4;
+    const int first = seg[0], count = seg[1], pos0 = seg[2], slot = seg[3];
+    const bool ok = count > 0 && slot >= 0 && slot < a.st.num_slots && first >= 0 && first + count <= a.st.rows;
+    const int col = c0 + (tid & 7) * 4, cols = min(4, vdim - col);           // this thread's columns that exist
+    const bool vec = cols == 4 && (vdim & 3) == 0, held = ok && pos0 > 0;
+    const size_t head = (size_t)(ok ? slot : 0) * s.heads + h, copy = head * mlstm_slices(vdim) + blockIdx.x;
+    float *gs = a.state_s + head * dim * vdim + col, *gn = a.state_n + copy * dim;
+    float4 S[RPT];
+    float n[RPT], m = held ? a.state_m[copy] : 0.0f;
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+        const int r = row0 + i * RC_ROWS;
+        S[i] = make_float4(0, 0, 0, 0);
+        n[i] = held && r < dim ? gn[r] : 0.0f;
+        if (held && r < dim) {
+            const float* p = gs + (size_t)r * vdim;
+            if (vec) S[i] = *reinterpret_cast<const float4*>(p);
+            else {
+                if (cols > 0) S[i].x = p[0];
+                if (cols > 1) S[i].y = p[1];
+                if (cols > 2) S[i].z = p[2];
+                if (cols > 3) S[i].w = p[3];
+            }
+        }
+    }
+    const float qscale = 1.0f / sqrtf(float(dim));
+    pdl_wait();
+    if (!ok) {
+        if (count > 0 && tid == 0) atomicCAS(a.status, 0, SEQ_BAD_SLOT);
+        return;
+    }
+    float q[RPT], k[RPT], v[4], gi, gf;
+    auto fetch = [&](int t) {
+        const T* p = reinterpret_cast<const T*>(a.proj) + (first + t) * a.ld;
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            const int r = row0 + i * RC_ROWS;
+            q[i] = r < dim ? to_f32(p[h * dim + r]) * qscale : 0.0f;
+            k[i] = r < dim ? to_f32(p[(s.heads + h) * dim + r]) : 0.0f;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = j < cols ? to_f32(p[2 * s.heads * dim + h * vdim + col + j]) : 0.0f;
+        gi = mlstm_gate_i(a, first + t, h);
+        gf = mlstm_gate_f(a, first + t, h);
+    };
+    fetch(0);
+    for (int t = 0; t < count; ++t) {
+        const float mn = fmaxf(gf + m, gi), keep = expf(gf + m - mn), put = expf(gi - mn);
+        m = mn;
+        float4 o = make_float4(0, 0, 0, 0);
+        float nq = 0.0f;
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            const float kp = put * k[i];
+            n[i] = keep * n[i] + kp;
+            S[i].x = keep * S[i].x + kp * v[0];
+            S[i].y = keep * S[i].y + kp * v[1];
+            S[i].z = keep * S[i].z + kp * v[2];
+            S[i].w = keep * S[i].w + kp * v[3];
+            nq = fmaf(n[i], q[i], nq);
+            o.x = fmaf(S[i].x, q[i], o.x);
+            o.y = fmaf(S[i].y, q[i], o.y);
+            o.z = fmaf(S[i].z, q[i], o.z);
+            o.w = fmaf(S[i].w, q[i], o.w);
+        }
+        if (t + 1 < count) fetch(t + 1);
+#pragma unroll
+        for (int sh = 8; sh < 32; sh <<= 1) {
+            o.x += __shfl_xor_sync(0xffffffffu, o.x, sh);
+            o.y += __shfl_xor_sync(0xffffffffu, o.y, sh);
+            o.z += __shfl_xor_sync(0xffffffffu, o.z, sh);
+            o.w += __shfl_xor_sync(0xffffffffu, o.w, sh);
+            nq += __shfl_xor_sync(0xffffffffu, nq, sh);
+        }
+        if (lane < 8) part[t & 1][warp][lane] = o;
+        if (lane == 0) part_n[t & 1][warp] = nq;
+        __syncthreads();                                     // (two buffers: the next token's sums do not wait for this one's readers)
+        if (tid < RC_COLS && c0 + tid < vdim) {
+            float sum = 0.0f, norm = 0.0f;
+#pragma unroll
+            for (int w = 0; w < RC_T / 32; ++w) {
+                sum += reinterpret_cast<const float*>(part[t & 1][w])[tid];
+                norm += part_n[t & 1][w];
+            }
+            a.out[(size_t)(first + t) * s.heads * vdim + (size_t)h * vdim + c0 + tid] = sum / (fmaxf(fabsf(norm), expf(-m)) + 1e-6f);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+        const int r = row0 + i * RC_ROWS;
+        if (r >= dim) continue;
+        float* p = gs + (size_t)r * vdim;
+        if (vec) *reinterpret_cast<float4*>(p) = S[i];
+        else {
+            if (cols > 0) p[0] = S[i].x;
+            if (cols > 1) p[1] = S[i].y;
+            if (cols > 2) p[2] = S[i].z;
+            if (cols > 3) p[3] = S[i].w;
+        }
+        if ((tid & 7) == 0) gn[r] = n[i];
+    }
+    if (tid == 0) a.state_m[copy] = m;
+}
+
+// One warp per row and head where 16 bytes line up: 8 x KEEP values a lane, held between the sum and the product.
 constexpr int FIN_T = 128;
+__device__ __forceinline__ void fin_load8(const float* p, float (&v)[8]) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+template <int KEEP>
+__global__ void __launch_bounds__(FIN_T) mlstm_finish_warp_kernel(scr_mlstm_shape s, const float* __restrict__ out, const float* __restrict__ norm,
+                                                                  const bf16* __restrict__ gate, long long ld_gate, long long pairs, bf16* __restrict__ y) {
+    pdl_trigger();
+    const int lane = threadIdx.x & 31;
+    const long long i0 = (long long)blockIdx.x * (FIN_T / 32) + (threadIdx.x >> 5);
+    if (i0 >= pairs) {
+        pdl_wait();
+        return;
+    }
+    const int r = (int)(i0 / s.heads), h = (int)(i0 - (long long)r * s.heads);
+    const size_t at = (size_t)r * s.heads * s.vdim + (size_t)h * s.vdim;
+    float v[KEEP][8], w[KEEP][8];
+    uint4 g[KEEP];
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        const int c = (k * 32 + lane) * 8;
+        if (c < s.vdim) fin_load8(norm + h * s.vdim + c, w[k]);
+    }
+    pdl_wait();
+    float ss = 0.0f;
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        const int c = (k * 32 + lane) * 8;
+        if (c >= s.vdim) continue;
+        fin_load8(out + at + c, v[k]);
+        g[k] = *reinterpret_cast<const uint4*>(gate + r * ld_gate + h * s.vdim + c);
+    }
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k)
+        if ((k * 32 + lane) * 8 < s.vdim)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) ss = fmaf(v[k][j], v[k][j], ss);
+    const float inv = 1.0f / sqrtf(warp_sum(ss) / float(s.vdim) + s.eps);
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        const int c = (k * 32 + lane) * 8;
+        if (c >= s.vdim) continue;
+        const uint32_t gw[4] = {g[k].x, g[k].y, g[k].z, g[k].w};
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            o[j] = pack_bf16x2(v[k][2 * j] * inv * w[k][2 * j] * sigmoid_f32(bf16_lo(gw[j])), v[k][2 * j + 1] * inv * w[k][2 * j + 1] * sigmoid_f32(bf16_hi(gw[j])));
+        *reinterpret_cast<uint4*>(y + at + c) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
+
+// Any sizes and alignment: one CTA per row and head.
 template <typename T>
 __global__ void __launch_bounds__(FIN_T) mlstm_finish_kernel(scr_mlstm_shape s, const float* __restrict__ out, const float* __restrict__ norm,
                                                              const T* __restrict__ gate, long long ld_gate, T* __restrict__ y) {
@@ -155,9 +325,20 @@ __global__ void __launch_bounds__(FIN_T) mlstm_finish_kernel(scr_mlstm_shape s, 
     }
 }
 
+template <typename T, int RPT>
+cudaError_t step_launch(const MemoryArgs& a, cudaStream_t stream) {
+    return launch_pdl(mlstm_step_kernel<T, RPT>, dim3(scr_ceil_div(a.s.vdim, RC_COLS), a.s.heads, a.st.batch), dim3(RC_T), 0, stream, a);
+}
+
 template <typename T>
 int32_t recur_launch(scr_ctx* ctx, const MemoryArgs& a, cudaStream_t stream) {
     const int dim = a.s.dim;
+    if (dim <= 8 * RC_ROWS) {                                // 8 rows of a thread fit its registers
+        const cudaError_t e = dim <= RC_ROWS ? step_launch<T, 1>(a, stream) : dim <= 2 * RC_ROWS ? step_launch<T, 2>(a, stream)
+                            : dim <= 4 * RC_ROWS ? step_launch<T, 4>(a, stream) : step_launch<T, 8>(a, stream);
+        if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "mlstm_step: %s", cudaGetErrorString(e));
+        return scr_check_launch(ctx, "mlstm_step");
+    }
     const size_t smem = (size_t)dim * 8 * 16 + (3 * dim + 4) * sizeof(float) + 8 * 8 * 16;
     if (smem > 220 * 1024) return scr_fail(ctx, SCR_E_UNSUPPORTED, "mlstm dim %d", dim);
     cudaError_t e = seq_smem(mlstm_recur_kernel<T>, smem);
@@ -197,6 +378,15 @@ extern "C" int32_t scr_mlstm_finish(scr_ctx* ctx, int32_t dtype, const scr_mlstm
     if (dtype != SCR_DTYPE_F32 && dtype != SCR_DTYPE_BF16) return scr_fail(ctx, SCR_E_DTYPE, "dtype %d", dtype);
     const dim3 grid(s->heads, rows);
     cudaStream_t cs = (cudaStream_t)stream;
+    if (dtype == SCR_DTYPE_BF16 && s->heads > 0 && s->vdim > 0 && s->vdim % 8 == 0 && s->vdim <= 512 && ld_gate % 8 == 0 && scr_aligned16(out) &&
+        scr_aligned16(norm) && scr_aligned16(gate) && scr_aligned16(y)) {
+        const long long pairs = (long long)rows * s->heads;
+        const dim3 warps((unsigned)((pairs + FIN_T / 32 - 1) / (FIN_T / 32)));
+        auto kernel = s->vdim <= 256 ? mlstm_finish_warp_kernel<1> : mlstm_finish_warp_kernel<2>;
+        const cudaError_t e = launch_pdl(kernel, warps, dim3(FIN_T), 0, cs, *s, out, norm, (const bf16*)gate, (long long)ld_gate, pairs, (bf16*)y);
+        if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "mlstm_finish: %s", cudaGetErrorString(e));
+        return scr_check_launch(ctx, "mlstm_finish");
+    }
     const cudaError_t e = dtype == SCR_DTYPE_F32
         ? launch_pdl(mlstm_finish_kernel<float>, grid, dim3(FIN_T), 0, cs, *s, out, norm, (const float*)gate, (long long)ld_gate, (float*)y)
         : launch_pdl(mlstm_finish_kernel<bf16>, grid, dim3(FIN_T), 0, cs, *s, out, norm, (const bf16*)gate, (long long)ld_gate, (bf16*)y);

@@ -34,7 +34,87 @@ __device__ __forceinline__ void get_vec(const float* src, float (&v)[4]) {
 }
 __device__ __forceinline__ void get_vec(const float* src, float (&v)[1]) { v[0] = *src; }
 
-// One CTA per row.  The row lives in shared memory between the passes.
+// Rows of up to 1024 x KEEP, 4 x KEEP values a thread in registers: the row, the sublayer's output and (before the wait for the
+// preceding kernel: load-time constants) the weights are all requested before the first sum.  In a decode step a launch is a
+// chain of latencies, and this takes two trips to memory out of it.
+template <typename T, int KEEP>
+__global__ void __launch_bounds__(NORM_T) seq_norm_held_kernel(scr_seq_norm_args a, int* status) {
+    __shared__ float red_a[NORM_T / 32], red_b[NORM_T / 32];
+    pdl_trigger();
+    const int W = a.width, r = blockIdx.x;
+    float wd[KEEP][4], wo[KEEP][4], bo[KEEP][4], d[KEEP][4], x[KEEP][4];
+    auto at = [&](int k) { return (k * NORM_T + (int)threadIdx.x) * 4; };          // (W is a multiple of 4)
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        if (at(k) >= W) continue;
+        if (a.delta && (a.w_delta || a.bias)) get_vec((a.w_delta ? a.w_delta : a.bias) + at(k), wd[k]);
+        if (a.out && a.w_out) get_vec(a.w_out + at(k), wo[k]);
+        if (a.out && a.b_out) get_vec(a.b_out + at(k), bo[k]);
+    }
+    pdl_wait();
+    int src = r;
+    if (a.row_index) {
+        src = a.row_index[r];
+        if (src < 0 || src >= a.x_rows) {
+            if (threadIdx.x == 0) atomicCAS(status, 0, SEQ_BAD_POSITION);
+            src = 0;
+        }
+    }
+    float* row = a.x + (size_t)src * W;
+    const bool add = !a.delta || a.w_delta;                  // x is replaced, not added to, by a delta without a norm of its own
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        if (at(k) >= W) continue;
+        if (a.delta) get_vec(a.delta + (size_t)r * W + at(k), d[k]);
+        if (add) get_vec(row + at(k), x[k]);
+    }
+    float sum = 0.0f;
+    if (a.delta) {
+        float inv = 0.0f;
+        if (a.w_delta) {
+            float ss = 0.0f;
+#pragma unroll
+            for (int k = 0; k < KEEP; ++k)
+                if (at(k) < W)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) ss = fmaf(d[k][j], d[k][j], ss);
+            inv = 1.0f / sqrtf(cta_sum<NORM_T>(ss, red_a) / float(W) + a.eps);
+        }
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) {
+            if (at(k) >= W) continue;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (a.w_delta) x[k][j] += d[k][j] * inv * (1.0f + wd[k][j]);
+                else x[k][j] = d[k][j] + (a.bias ? wd[k][j] : 0.0f);
+            }
+            put_vec(row + at(k), x[k]);
+        }
+    }
+    if (!a.out) return;
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k)
+        if (at(k) < W)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sum = fmaf(x[k][j], x[k][j], sum);
+    T* out = reinterpret_cast<T*>(a.out) + r * a.ld_out;
+    float inv = 1.0f;
+    if (a.w_out && !a.b_out) inv = 1.0f / sqrtf(cta_sum<NORM_T>(sum, red_b) / float(W) + a.eps);
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        if (at(k) >= W) continue;
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            v[j] = x[k][j];
+            if (a.b_out) v[j] = fmaf(tanhf(a.alpha * v[j]), wo[k][j], bo[k][j]);
+            else if (a.w_out) v[j] = v[j] * inv * (1.0f + wo[k][j]);
+        }
+        put_vec(out + at(k), v);
+    }
+}
+
+// Any width.  One CTA per row.  The row lives in shared memory between the passes.
 template <typename T, int VEC>
 __global__ void __launch_bounds__(NORM_T) seq_norm_kernel(scr_seq_norm_args a, int* status) {
     extern __shared__ float4 norm_row[];
@@ -132,7 +212,17 @@ __global__ void __launch_bounds__(AMAX_T) seq_argmax_kernel(const float* __restr
     const float* row = logits + blockIdx.x * ld;
     float best = -INFINITY;
     int best_i = 0x7FFFFFFF;
-    for (int i = threadIdx.x; i < width; i += AMAX_T) amax_take(row[i], i, best, best_i);
+    // one SM reads the row: four requests of 16 bytes a thread in flight
+    const int nv = (reinterpret_cast<uintptr_t>(row) & 15) == 0 ? width / 4 : 0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nv; i += AMAX_T) {
+        const float4 v = reinterpret_cast<const float4*>(row)[i];
+        amax_take(v.x, 4 * i, best, best_i);
+        amax_take(v.y, 4 * i + 1, best, best_i);
+        amax_take(v.z, 4 * i + 2, best, best_i);
+        amax_take(v.w, 4 * i + 3, best, best_i);
+    }
+    for (int i = 4 * nv + threadIdx.x; i < width; i += AMAX_T) amax_take(row[i], i, best, best_i);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float ob = __shfl_xor_sync(0xffffffffu, best, o);
@@ -272,6 +362,12 @@ extern "C" int32_t scr_seq_norm(scr_ctx* ctx, int32_t dtype, const scr_seq_norm_
     if (smem > 200 * 1024) return scr_fail(ctx, SCR_E_UNSUPPORTED, "width %d", a.width);
     const bool vec = a.width % 4 == 0 && a.ld_out % 4 == 0 && scr_aligned16(a.x) && scr_aligned16(a.delta) && scr_aligned16(a.w_delta) &&
                      scr_aligned16(a.bias) && scr_aligned16(a.w_out) && scr_aligned16(a.b_out) && scr_aligned16(a.out);
+    if (vec && a.width <= 4 * 4 * NORM_T) {
+        const int keep = scr_ceil_div(a.width, 4 * NORM_T);
+        auto held = dtype == SCR_DTYPE_F32 ? (keep == 1 ? seq_norm_held_kernel<float, 1> : keep == 2 ? seq_norm_held_kernel<float, 2> : keep == 3 ? seq_norm_held_kernel<float, 3> : seq_norm_held_kernel<float, 4>)
+                                           : (keep == 1 ? seq_norm_held_kernel<bf16, 1> : keep == 2 ? seq_norm_held_kernel<bf16, 2> : keep == 3 ? seq_norm_held_kernel<bf16, 3> : seq_norm_held_kernel<bf16, 4>);
+        SEQ_LAUNCH("seq_norm", launch_pdl(held, dim3(a.rows), dim3(NORM_T), 0, (cudaStream_t)stream, a, ctx->dev_status));
+    }
     auto kernel = dtype == SCR_DTYPE_F32 ? (vec ? seq_norm_kernel<float, 4> : seq_norm_kernel<float, 1>) : (vec ? seq_norm_kernel<bf16, 4> : seq_norm_kernel<bf16, 1>);
     cudaError_t e = seq_smem(kernel, smem);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "seq_norm: %s", cudaGetErrorString(e));

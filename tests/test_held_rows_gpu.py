@@ -1,0 +1,58 @@
+"""Row operators that hold a row in registers, at the widths where their dispatch changes, against plain 64-bit statements."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from oracle import sequence_plain as plain
+from tests import seq_util as su
+from tests.test_sequence_ops_gpu import TOL, dev, draw, healthy, host, lib, ptr, stream, torch_
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,vdim,lead,pad", [(3, 8, 8, 0), (2, 248, 0, 8), (5, 256, 8, 0), (1, 264, 0, 0), (2, 512, 8, 8), (2, 520, 0, 0), (2, 256, 4, 0),
+                                                 (2, 256, 0, 4)])
+def test_memory_readout(heads, vdim, lead, pad):
+    """A warp per row and head up to 512 values; a CTA beyond, and where the gate's rows do not start on 16 bytes."""
+    from scratchy_b200 import _lib
+    from scratchy_b200.dense import dtype_code
+    torch = torch_()
+    L, c = lib()
+    rng = np.random.default_rng(heads * vdim + lead)
+    T = 7
+    o, w = rng.standard_normal((T, heads * vdim)).astype(np.float32), rng.standard_normal(heads * vdim).astype(np.float32)
+    g = draw(rng, (T, lead + heads * vdim + pad), "bfloat16")
+    o[0] *= 1e-4
+    shape = _lib.MlstmShape(heads, 16, vdim, 1.0, 1e-5)
+    od, wd, gd, y = dev(o), dev(w), dev(g, "bfloat16"), torch.full((T, heads * vdim), float("nan"), dtype=torch.bfloat16, device="cuda")
+    c.check(L.scr_mlstm_finish(c.handle, dtype_code(y.dtype), ctypes.byref(shape), ptr(od), ptr(wd), ptr(gd, lead), g.shape[1], T, ptr(y), stream()))
+    want = plain.unit_rms(o.astype(np.float64).reshape(T, heads, vdim), 1e-5).reshape(T, -1) * w * plain.sigmoid(g[:, lead:lead + heads * vdim].astype(np.float64))
+    assert su.rel(host(y), want) < TOL["bfloat16"] and su.rel(host(y)[0], want[0]) < TOL["bfloat16"]
+    healthy()
+
+
+@pytest.mark.parametrize("W", [4, 1020, 1024, 1028, 2052, 4092, 4096, 4100])
+def test_norm_widths(W):
+    from scratchy_b200.dense import seq_norm
+    torch = torch_()
+    rng = np.random.default_rng(W)
+    T, eps = 3, 0.01
+    x, d = rng.standard_normal((T, W)).astype(np.float32), 3 * rng.standard_normal((T, W)).astype(np.float32)
+    wd, wo = (0.5 * rng.standard_normal(W).astype(np.float32) for _ in range(2))
+    xd, out = dev(x), torch.full((T, W), float("nan"), dtype=torch.bfloat16, device="cuda")
+    seq_norm(xd, eps, delta=dev(d), w_delta=dev(wd), out=out, w_out=dev(wo))
+    want = x.astype(np.float64) + plain.norm_around_zero(d.astype(np.float64), wd, eps)
+    assert su.rel(host(xd), want) < 1e-6 and su.rel(host(out), plain.norm_around_zero(want, wo, eps)) < TOL["bfloat16"]
+    healthy()
+
+
+@pytest.mark.parametrize("width,ld", [(1, 4), (5, 8), (4097, 4100), (128256, 128256), (777, 779)])
+def test_greedy_picks_the_first_of_equals_at_any_alignment(width, ld):
+    from scratchy_b200.dense import greedy
+    torch = torch_()
+    g = torch.Generator().manual_seed(width)
+    rows = torch.randint(-50, 50, (3, ld), generator=g).float()
+    rows[1, :width] = -3.0                                           # all equal: the first
+    want = rows[:, :width].numpy().argmax(axis=1)
+    assert greedy(rows.cuda()[:, :width]).cpu().numpy().tolist() == want.tolist()
