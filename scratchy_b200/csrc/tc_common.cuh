@@ -208,9 +208,10 @@ __device__ __forceinline__ void tc_unit(int unit, int full, int ks_tail, int k_s
     const int v = unit - full;
     tile = full + v / ks_tail;
     ks = v - (v / ks_tail) * ks_tail;
-    const int per = (k_steps + ks_tail - 1) / ks_tail;
-    k_lo = ks * per;
-    k_hi = min(k_steps, k_lo + per);
+    // even shares: with ceil(k_steps / ks_tail) steps each, 41 steps in 8 units left the last one none, and its slab whatever the
+    // accumulator held
+    k_lo = k_steps * ks / ks_tail;
+    k_hi = k_steps * (ks + 1) / ks_tail;
 }
 static inline int tc_sm_count() {
     static int sms = 0;

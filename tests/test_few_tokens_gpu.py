@@ -99,3 +99,12 @@ def test_quantisation_of_every_code_and_tie(K):
     want_q, want_a = oracle.fp8_quant_per_token(x.reshape(-1), M, K)
     assert (want_a == 1.0).all()
     assert np.array_equal(a.cpu().numpy(), want_a) and np.array_equal(xq.cpu().numpy().reshape(want_q.shape), want_q)
+
+
+@pytest.mark.parametrize("K", [3200, 4224, 5248])
+def test_no_unit_of_a_cut_is_left_without_steps(K):
+    """Contractions of 25, 33 and 41 steps of 128 (50, 66 and 82 of 64), cut into up to 8 units in every prefill GEMM."""
+    test_int4(256, K, 200, 64)
+    test_fp8(256, K, 300)
+    test_dense(300, K, 200)
+    test_dense(300, K // 2 + 32, 200)
