@@ -186,7 +186,10 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        // the warp goes round as a whole, one lane elected for the instructions alone: the descriptors stay in uniform registers,
+        // where a divergent thread spends about 55 cycles on each MMA it issues
+        {
+            const bool lead = elect_one();
             int sx = 0, sd = 0;
             uint32_t phx = 0, phd = 0;
             int it = 0;
@@ -204,24 +207,28 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_
                     tc_fence_after();
                     const uint32_t xs = smem_base + S::kXOff + sx * S::kXStage;
                     const uint32_t ds = smem_base + S::kDOff + sd * S::kDStage;
+                    if (lead) {
 #pragma unroll
-                    for (int h = 0; h < TM; ++h) {
+                        for (int h = 0; h < TM; ++h) {
 #pragma unroll
-                        for (int a = 0; a < 2; ++a) {
-                            const uint64_t adesc = umma_desc_k_sw128(xs + h * 32768u + a * 16384u);
-                            const uint64_t bdesc = umma_desc_k_sw128(ds + a * (uint32_t)(BN * 128));
+                            for (int a = 0; a < 2; ++a) {
+                                const uint64_t adesc = umma_desc_k_sw128(xs + h * 32768u + a * 16384u);
+                                const uint64_t bdesc = umma_desc_k_sw128(ds + a * (uint32_t)(BN * 128));
 #pragma unroll
-                            for (int k4 = 0; k4 < 4; ++k4)
-                                umma_f16(d_tmem + (uint32_t)(h * BN), adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc,
-                                         ((kc - kc_lo) | a | k4) != 0);
+                                for (int k4 = 0; k4 < 4; ++k4)
+                                    umma_f16(d_tmem + (uint32_t)(h * BN), adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc,
+                                             ((kc - kc_lo) | a | k4) != 0);
+                            }
                         }
+                        umma_commit(dempty(sd));
+                        umma_commit(xempty(sx));
                     }
-                    umma_commit(xempty(sx));
-                    umma_commit(dempty(sd));
+                    __syncwarp();
                     if (++sx == SX) { sx = 0; phx ^= 1u; }
                     if (++sd == A4G_SD) { sd = 0; phd ^= 1u; }
                 }
-                umma_commit(accf(buf));
+                if (lead) umma_commit(accf(buf));
+                __syncwarp();
             }
         }
     }

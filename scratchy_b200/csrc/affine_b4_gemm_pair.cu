@@ -175,7 +175,8 @@ affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const uint
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (leader CTA)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {                                  // (the whole warp, one lane elected for the instructions: see affine_b4_gemm.cu)
+            const bool lead = elect_one();
             int sx = 0, sd = 0;
             uint32_t phx = 0, phd = 0;
             int it = 0;
@@ -191,20 +192,24 @@ affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const uint
                     tc_fence_after();
                     const uint32_t xs = smem_base + A4P_XOFF + sx * A4P_XSTAGE;
                     const uint32_t ds = smem_base + A4P_DOFF + sd * A4P_DSTAGE;
+                    if (lead) {
 #pragma unroll
-                    for (int a = 0; a < 2; ++a) {
-                        const uint64_t adesc = umma_desc_k_sw128(xs + a * 16384u);
-                        const uint64_t bdesc = umma_desc_k_sw128(ds + a * 16384u);
+                        for (int a = 0; a < 2; ++a) {
+                            const uint64_t adesc = umma_desc_k_sw128(xs + a * 16384u);
+                            const uint64_t bdesc = umma_desc_k_sw128(ds + a * 16384u);
 #pragma unroll
-                        for (int k4 = 0; k4 < 4; ++k4)
-                            a4p_umma_f16(d_tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, (kc | a | k4) != 0);
+                            for (int k4 = 0; k4 < 4; ++k4)
+                                a4p_umma_f16(d_tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, (kc | a | k4) != 0);
+                        }
+                        a4p_commit(dempty(sd));
+                        a4p_commit(xempty(sx));
                     }
-                    a4p_commit(xempty(sx));
-                    a4p_commit(dempty(sd));
+                    __syncwarp();
                     if (++sx == A4P_SX) { sx = 0; phx ^= 1u; }
                     if (++sd == A4P_SD) { sd = 0; phd ^= 1u; }
                 }
-                a4p_commit(accf(buf));
+                if (lead) a4p_commit(accf(buf));
+                __syncwarp();
             }
         }
     } else if (warp < 2 + A4P_DQ_WARPS) {

@@ -2,14 +2,15 @@
 //
 //   y[m,n] = bf16( sum_k x[m,k] * w[n,k] (+ bias[n]) ),  w = the bit-exact bf16 dequantisation of the codes
 //
-// A unit is 128 channels by one CTA's share of the 128-k chunks; 352 threads:
+// A unit is 128 channels by one CTA's share of the 128-k chunks; 384 threads:
 //   warps 0-7    dequantise: two groups of four warps take alternate chunks; a thread expands the 128 codes of ONE channel
 //                and writes them to TMEM with tcgen05.st, where the MMA reads its A operand: no swizzled shared-memory
 //                image, no proxy fence.  Afterwards they drain the accumulator.
 //   warp 8       producer of the packed weights (8 bulk copies of a block per chunk), which are load-time constants: it
 //                starts before the preceding kernel of the stream has finished
 //   warp 9       producer of the activations (2 tiled TMA loads of 64 k x the tokens, 128-byte swizzle, zeros outside)
-//   warp 10      owns TMEM; one thread issues 8 tcgen05.mma (128 x tokens x 16) per chunk
+//   warps 10,11  (10 owns TMEM) issue 8 tcgen05.mma (128 x tokens x 16) per chunk, each the chunks of one group of warps 0-7
+//                into its own accumulator; the two are added at the end
 //
 // What bounds it: the packed weights from HBM (9.2 KB per chunk) and, for the short k extents of a layer's linears, the start
 // of the pipeline and the two cluster barriers at its end.  Against the 128-token tile of affine_b4_gemm.cu, which it replaces
@@ -23,14 +24,15 @@
 
 namespace {
 
-constexpr int A4S_THREADS = 352;
-constexpr int A4S_SP = 6;                        // packed-weight stages
+constexpr int A4S_THREADS = 384;
 
 template <int TN>
 struct A4SCfg {
-    static constexpr int kSX = TN == 64 ? 3 : 4;                        // activation stages
-    static constexpr int kSA = TN == 128 ? 2 : 3;                       // dequantised-weight stages in TMEM, 64 columns each
-    static constexpr uint32_t kTmemCols = 256;                          // the accumulator's TN columns and the stages
+    // Stages, all even in number: a stage then always belongs to one of the two groups, whose waits take its phases in order
+    static constexpr int kSP = TN == 64 ? 4 : 6;                        // packed weights
+    static constexpr int kSX = 4;                                       // activations
+    static constexpr int kSA = TN == 128 ? 4 : 2;                       // dequantised weights in TMEM, 64 columns each
+    static constexpr uint32_t kTmemCols = TN == 128 ? 512 : 256;        // two accumulators of TN columns and the stages
     static constexpr uint32_t kXStage = TN * 256u;                      // 2 atoms of TN rows x 128 B
     static constexpr uint32_t kPOff = kSX * kXStage;
     static constexpr int kCtasPerSm = TN == 128 ? 1 : 2;
@@ -84,7 +86,7 @@ __global__ void __launch_bounds__(A4S_THREADS, A4SCfg<TN>::kCtasPerSm)
 affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t* __restrict__ packed, uint16_t* __restrict__ y, int M, int N, int RB,
                         int KC, int split, int out_f32, const uint16_t* __restrict__ bias, int* __restrict__ status) {
     using C = A4SCfg<TN>;
-    constexpr uint32_t kBlock = aff_block_bytes(GS), kPStage = 8u * kBlock, kBarOff = C::kPOff + A4S_SP * kPStage;
+    constexpr uint32_t kBlock = aff_block_bytes(GS), kPStage = 8u * kBlock, kBarOff = C::kPOff + C::kSP * kPStage;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -92,10 +94,10 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t
     auto xfull = [&](int s) { return bar + 8u * s; };
     auto xempty = [&](int s) { return bar + 8u * (C::kSX + s); };
     auto pfull = [&](int s) { return bar + 8u * (2 * C::kSX + s); };
-    auto pempty = [&](int s) { return bar + 8u * (2 * C::kSX + A4S_SP + s); };
-    auto afull = [&](int s) { return bar + 8u * (2 * C::kSX + 2 * A4S_SP + s); };
-    auto aempty = [&](int s) { return bar + 8u * (2 * C::kSX + 2 * A4S_SP + C::kSA + s); };
-    constexpr int kSlots = 2 * C::kSX + 2 * A4S_SP + 2 * C::kSA;
+    auto pempty = [&](int s) { return bar + 8u * (2 * C::kSX + C::kSP + s); };
+    auto afull = [&](int s) { return bar + 8u * (2 * C::kSX + 2 * C::kSP + s); };
+    auto aempty = [&](int s) { return bar + 8u * (2 * C::kSX + 2 * C::kSP + C::kSA + s); };
+    constexpr int kSlots = 2 * C::kSX + 2 * C::kSP + 2 * C::kSA;
     const uint32_t accf = bar + 8u * kSlots;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kBarOff + 8 * (kSlots + 1));
 
@@ -107,9 +109,9 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::kSX; ++s) { mbar_init(xfull(s), 1); mbar_init(xempty(s), 1); }
-        for (int s = 0; s < A4S_SP; ++s) { mbar_init(pfull(s), 1); mbar_init(pempty(s), 4); }
+        for (int s = 0; s < C::kSP; ++s) { mbar_init(pfull(s), 1); mbar_init(pempty(s), 4); }
         for (int s = 0; s < C::kSA; ++s) { mbar_init(afull(s), 4); mbar_init(aempty(s), 1); }
-        mbar_init(accf, 1);
+        mbar_init(accf, 2);
         fence_mbar_init();
     }
     if (warp == 10) {
@@ -121,16 +123,16 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     skinny_pdl_trigger();                              // not before this CTA has its TMEM: the next kernel's CTAs could take it first
-    auto a_col = [&](int s) { return tmem + (uint32_t)(TN + 64 * s); };
+    auto a_col = [&](int s) { return tmem + (uint32_t)(2 * TN + 64 * s); };
 
     // Only the weights may be touched before the preceding kernel has finished.  A wait that depends on the activations
     // comes after griddepcontrol.wait, so that its bound does not run against that kernel.
     if (warp == 8) {
         if (lane == 0) {
             for (int i = 0; i < steps; ++i) {
-                const int s = i % A4S_SP;
-                if (i == A4S_SP) skinny_pdl_wait();
-                mbar_wait(pempty(s), ((uint32_t)(i / A4S_SP) & 1u) ^ 1u, status, TC_ERR_EMPTY_WAIT);
+                const int s = i % C::kSP;
+                if (i == C::kSP) skinny_pdl_wait();
+                mbar_wait(pempty(s), ((uint32_t)(i / C::kSP) & 1u) ^ 1u, status, TC_ERR_EMPTY_WAIT);
                 mbar_arrive_expect_tx(pfull(s), kPStage);
                 for (int j = 0; j < 8; ++j)
                     bulk_g2s(smem_base + C::kPOff + s * kPStage + j * kBlock, packed + ((size_t)(tile * 8 + j) * KC + kc_lo + i) * kBlock, kBlock, pfull(s));
@@ -149,40 +151,42 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t
                 a4s_tma_2d(xs + TN * 128u, &x_map, (kc_lo + i) * 128 + 64, 0, xfull(s));
             }
         }
-    } else if (warp == 10) {
-        if (lane == 0) {
-            skinny_pdl_wait();
-            const uint32_t idesc = umma_idesc(1, 1, SKINNY_ROWS, (uint32_t)(M + 15) & ~15u);
-            for (int i = 0; i < steps; ++i) {
-                const int s = i % C::kSX, a = i % C::kSA;
-                mbar_wait(xfull(s), (uint32_t)(i / C::kSX) & 1u, status, TC_ERR_FULL_WAIT);
-                mbar_wait(afull(a), (uint32_t)(i / C::kSA) & 1u, status, TC_ERR_DEQ_WAIT);
-                tc_fence_after();
-                const uint32_t xs = smem_base + s * C::kXStage;
+    } else if (warp >= 10) {
+        // Two warps issue the MMAs, one for each group's chunks, into an accumulator of its own: the 8 MMAs of a chunk are short, and
+        // what bounded the kernel was the time one thread takes to issue them.  The warp goes round as a whole, with one lane
+        // elected for the instructions alone, so that the descriptors stay in uniform registers.
+        skinny_pdl_wait();
+        const int g = warp - 10;
+        const bool lead = elect_one();
+        const uint32_t idesc = umma_idesc(1, 1, SKINNY_ROWS, (uint32_t)(M + 15) & ~15u), d = tmem + (uint32_t)(g * TN);
+        for (int i = g; i < steps; i += 2) {
+            const int s = i % C::kSX, a = i % C::kSA;
+            const uint32_t xs = smem_base + s * C::kXStage, ac = a_col(a);
+            const uint64_t b0 = umma_desc_k_sw128(xs), b1 = umma_desc_k_sw128(xs + TN * 128u);
+            mbar_wait(xfull(s), (uint32_t)(i / C::kSX) & 1u, status, TC_ERR_FULL_WAIT);
+            mbar_wait(afull(a), (uint32_t)(i / C::kSA) & 1u, status, TC_ERR_DEQ_WAIT);
+            tc_fence_after();
+            if (lead) {
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const uint64_t bdesc = umma_desc_k_sw128(xs + h * TN * 128u);
-#pragma unroll
-                    for (int k4 = 0; k4 < 4; ++k4)
-                        umma_f16_ta(tmem, a_col(a) + (uint32_t)(32 * h + 8 * k4), bdesc + (uint64_t)(2 * k4), idesc, (i | h | k4) != 0);
-                }
-                umma_commit(xempty(s));
+                for (int k = 0; k < 8; ++k) umma_f16_ta(d, ac + (uint32_t)(8 * k), (k < 4 ? b0 : b1) + (uint64_t)(2 * (k & 3)), idesc, i > 1 || k > 0);
                 umma_commit(aempty(a));
+                umma_commit(xempty(s));
             }
-            umma_commit(accf);
+            __syncwarp();
         }
+        if (lead) umma_commit(accf);
     } else {
         const bool check = *reinterpret_cast<const unsigned int*>(packed + (size_t)RB * KC * kBlock) != 0;
         const int row = (warp & 3) * 32 + lane;
         const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
         bool waited = false;
         for (int i = warp >> 2; i < steps; i += 2) {
-            const int s = i % A4S_SP, a = i % C::kSA;
+            const int s = i % C::kSP, a = i % C::kSA;
             if (i >= C::kSA && !waited) {
                 skinny_pdl_wait();
                 waited = true;
             }
-            mbar_wait(pfull(s), (uint32_t)(i / A4S_SP) & 1u, status, TC_ERR_FULL_WAIT);
+            mbar_wait(pfull(s), (uint32_t)(i / C::kSP) & 1u, status, TC_ERR_FULL_WAIT);
             mbar_wait(aempty(a), ((uint32_t)(i / C::kSA) & 1u) ^ 1u, status, TC_ERR_EMPTY_WAIT);
             tc_fence_after();
             const uint32_t stage = smem_base + C::kPOff + s * kPStage;
@@ -202,7 +206,7 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t
     __syncwarp();
     const float factor = (*reinterpret_cast<const unsigned int*>(packed + (size_t)RB * KC * kBlock) != 0) ? 1.0f : AFF_SCALED_FACTOR;
     skinny_pdl_wait();
-    skinny_finish(tmem, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, tile * SKINNY_ROWS, N, [&](int m, int n, float a, float b) {
+    skinny_finish<TN>(tmem, steps > 1, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, tile * SKINNY_ROWS, N, [&](int m, int n, float a, float b) {
         const float v[2] = {a * factor, b * factor};
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
@@ -228,8 +232,8 @@ int32_t a4s_launch(scr_ctx* ctx, const CUtensorMap& map, const uint8_t* packed, 
                    cudaStream_t stream) {
     using C = A4SCfg<TN>;
     const AffineGeom g = affine_geom(N, K, 64);          // RB / KC only: the same for every group size
-    constexpr size_t smem = C::kPOff + A4S_SP * 8u * aff_block_bytes(GS) + 512 + 1024;
-    static_assert(C::kPOff + A4S_SP * 8u * aff_block_bytes(GS) >= skinny_sum_bytes(TN), "the sums fit the rings");
+    constexpr size_t smem = C::kPOff + C::kSP * 8u * aff_block_bytes(GS) + 512 + 1024;
+    static_assert(C::kPOff + C::kSP * 8u * aff_block_bytes(GS) >= skinny_sum_bytes(TN), "the sums fit the rings");
     static SkinnyResident resident;
     const int tiles = g.RB / 8;
     const int split = skinny_split(resident, affine_b4_skinny_kernel<TN, GS>, ctx->device, ctx->sm_count, tiles, g.KC, A4S_THREADS, smem, 3.0f);

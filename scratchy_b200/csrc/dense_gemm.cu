@@ -277,7 +277,9 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
+            // the warp goes round as a whole, one lane elected for the instructions alone: the descriptors stay in uniform registers
+            const bool lead = elect_one();
             const uint32_t idesc = umma_idesc(1, 1, 128, BN);
             int s = 0, it = 0;
             uint32_t ph = 0;
@@ -293,13 +295,17 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
                     tc_fence_after();
                     const uint32_t sa = smem_base + s * S::kStageBytes;
                     const uint64_t adesc = umma_desc_k_sw128(sa), bdesc = umma_desc_k_sw128(sa + DG_A_BYTES);
+                    if (lead) {
 #pragma unroll
-                    for (int k4 = 0; k4 < 4; ++k4)
-                        umma_f16(d_tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, ((kt - k_lo) | k4) != 0);
-                    umma_commit(empty_bar(s));
+                        for (int k4 = 0; k4 < 4; ++k4)
+                            umma_f16(d_tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, ((kt - k_lo) | k4) != 0);
+                        umma_commit(empty_bar(s));
+                    }
+                    __syncwarp();
                     if (++s == S::kStages) { s = 0; ph ^= 1u; }
                 }
-                umma_commit(accf_bar(buf));
+                if (lead) umma_commit(accf_bar(buf));
+                __syncwarp();
             }
         }
     } else {
@@ -430,7 +436,8 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
+            const bool lead = elect_one();
             const uint32_t idesc = umma_idesc(1, 1, 256, DP_BN);
             int s = 0, it = 0;
             uint32_t ph = 0;
@@ -445,17 +452,21 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_c
                     mbar_wait(full_bar(s), ph, status, TC_ERR_FULL_WAIT);
                     tc_fence_after();
                     const int nk = min(DP_SLICES, k_hi - kt);
-                    for (int j = 0; j < nk; ++j) {
-                        const uint32_t sa = smem_base + s * DP_STAGE_BYTES + j * DP_SLICE_BYTES;
-                        const uint64_t adesc = umma_desc_k_sw128(sa), bdesc = umma_desc_k_sw128(sa + DG_A_BYTES);
+                    if (lead) {
+                        for (int j = 0; j < nk; ++j) {
+                            const uint32_t sa = smem_base + s * DP_STAGE_BYTES + j * DP_SLICE_BYTES;
+                            const uint64_t adesc = umma_desc_k_sw128(sa), bdesc = umma_desc_k_sw128(sa + DG_A_BYTES);
 #pragma unroll
-                        for (int k4 = 0; k4 < 4; ++k4)
-                            dp_umma(d_tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, ((kt + j - k_lo) | k4) != 0);
+                            for (int k4 = 0; k4 < 4; ++k4)
+                                dp_umma(d_tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, ((kt + j - k_lo) | k4) != 0);
+                        }
+                        dp_commit(empty_bar(s));
                     }
-                    dp_commit(empty_bar(s));
+                    __syncwarp();
                     if (++s == DP_STAGES) { s = 0; ph ^= 1u; }
                 }
-                dp_commit(accf_bar(buf));
+                if (lead) dp_commit(accf_bar(buf));
+                __syncwarp();
             }
         }
     } else {

@@ -8,9 +8,10 @@
 //   warp 9       producer of x (one tiled TMA load per slice, zeros outside)
 //   warp 10      owns TMEM; one thread issues 4 tcgen05.mma (128 x rows of x x 16) per slice
 //
-// What bounds it: the weights from HBM.  16384 x 3072 at 32 rows takes 29 us alone (100 MB, 3.4 TB/s from a cold start) and
-// 128256 x 3072 143 us (5.5 TB/s).  In the decode step of the 3B Vumipel at 32 sequences it replaces the 128-row tile of
-// dense_gemm.cu and its finishing launch: 4.22 -> 3.59 ms per step.
+// What bounds it: the weights from HBM; for the small linears the start and end of a launch.  16384 x 3072 (100 MB) at 32 rows
+// 28.0 us with the MMAs issued from a divergent thread, 23.2 us (4.3 TB/s) from a whole warp; 128256 x 3072 139 and 132 us (6.0
+// TB/s).  Against the 128-row tile of dense_gemm.cu and its finishing launch: a decode step of the 3B Vumipel at 32 sequences
+// 4.22 -> 3.59 ms, with that issue 3.31 -> 3.09 ms.
 #include "seq_common.cuh"
 #include "skinny.cuh"
 
@@ -96,29 +97,33 @@ dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_cons
             }
         }
     } else if (warp == 10) {
-        if (lane == 0) {
-            pdl_wait();
-            const uint32_t idesc = umma_idesc(1, 1, SKINNY_ROWS, (uint32_t)(M + 15) & ~15u);
-            for (int i = 0; i < steps; ++i) {
-                const int sw = i % C::kSW, sx = i % C::kSX;
-                mbar_wait(wfull(sw), (uint32_t)(i / C::kSW) & 1u, status, TC_ERR_FULL_WAIT);
-                mbar_wait(xfull(sx), (uint32_t)(i / C::kSX) & 1u, status, TC_ERR_FULL_WAIT);
-                tc_fence_after();
-                const uint64_t adesc = umma_desc_k_sw128(smem_base + sw * DS_W_STAGE), bdesc = umma_desc_k_sw128(smem_base + C::kXOff + sx * C::kXStage);
+        // The warp goes round as a whole, with one lane elected for the instructions alone, so that the descriptors stay in uniform
+        // registers: an MMA of few columns is shorter than its issue from a divergent thread.
+        pdl_wait();
+        const bool lead = elect_one();
+        const uint32_t idesc = umma_idesc(1, 1, SKINNY_ROWS, (uint32_t)(M + 15) & ~15u);
+        for (int i = 0; i < steps; ++i) {
+            const int sw = i % C::kSW, sx = i % C::kSX;
+            const uint64_t adesc = umma_desc_k_sw128(smem_base + sw * DS_W_STAGE), bdesc = umma_desc_k_sw128(smem_base + C::kXOff + sx * C::kXStage);
+            mbar_wait(wfull(sw), (uint32_t)(i / C::kSW) & 1u, status, TC_ERR_FULL_WAIT);
+            mbar_wait(xfull(sx), (uint32_t)(i / C::kSX) & 1u, status, TC_ERR_FULL_WAIT);
+            tc_fence_after();
+            if (lead) {
 #pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) umma_f16(tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, (i | k4) != 0);
+                for (int k4 = 0; k4 < 4; ++k4) umma_f16(tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, i > 0 || k4 > 0);
                 umma_commit(wempty(sw));
                 umma_commit(xempty(sx));
             }
-            umma_commit(accf);
+            __syncwarp();
         }
+        if (lead) umma_commit(accf);
     } else {
         pdl_wait();
         mbar_wait(accf, 0, status, TC_ERR_ACC_FULL);
     }
     __syncwarp();
     pdl_wait();
-    skinny_finish(tmem, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, n0, N,
+    skinny_finish(tmem, false, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, n0, N,
                   [&](int m, int n, float a, float b) { dense_put_two<bf16, END>(ends, m, g, n, N, a, b); });
     __syncthreads();
     if (warp == 10) {

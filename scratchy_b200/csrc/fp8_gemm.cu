@@ -157,7 +157,9 @@ fp8_gemm_tc_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ 
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
+            // the warp goes round as a whole, one lane elected for the instructions alone: the descriptors stay in uniform registers
+            const bool lead = elect_one();
             int s = 0;
             uint32_t ph = 0;
             int it = 0;
@@ -178,13 +180,17 @@ fp8_gemm_tc_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ 
                     const uint32_t sa = smem_base + s * F8GSmem<BN>::kStageBytes;
                     const uint64_t adesc = umma_desc_k_sw128(sa);
                     const uint64_t bdesc = umma_desc_k_sw128(sa + 16384u);
+                    if (lead) {
 #pragma unroll
-                    for (int k4 = 0; k4 < 4; ++k4)
-                        umma_f8f6f4(d_tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, ((kt - kt_lo) | k4) != 0);
-                    umma_commit(empty_bar(s));
+                        for (int k4 = 0; k4 < 4; ++k4)
+                            umma_f8f6f4(d_tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, ((kt - kt_lo) | k4) != 0);
+                        umma_commit(empty_bar(s));
+                    }
+                    __syncwarp();
                     if (++s == F8G_STAGES) { s = 0; ph ^= 1u; }
                 }
-                umma_commit(accf_bar(buf));
+                if (lead) umma_commit(accf_bar(buf));
+                __syncwarp();
             }
         }
     } else {

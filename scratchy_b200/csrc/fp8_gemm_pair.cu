@@ -144,7 +144,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_con
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {                                  // (the whole warp, one lane elected for the instructions: see fp8_gemm.cu)
+            const bool lead = elect_one();
             // -------------------------------------------------------------- MMA issuer (leader CTA)
             const uint32_t idesc = umma_idesc(0, 0, 256, F8P_BN);
             int s = 0;
@@ -159,18 +160,22 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_con
                     mbar_wait(full_bar(s), ph, status, TC_ERR_FULL_WAIT);
                     tc_fence_after();
                     const int nk = min(F8P_KSTEP, KT - kt);
-                    for (int j = 0; j < nk; ++j) {
-                        const uint32_t sa = smem_base + s * F8P_STAGE_BYTES + j * 32768u;
-                        const uint64_t adesc = umma_desc_k_sw128(sa);
-                        const uint64_t bdesc = umma_desc_k_sw128(sa + 16384u);
+                    if (lead) {
+                        for (int j = 0; j < nk; ++j) {
+                            const uint32_t sa = smem_base + s * F8P_STAGE_BYTES + j * 32768u;
+                            const uint64_t adesc = umma_desc_k_sw128(sa);
+                            const uint64_t bdesc = umma_desc_k_sw128(sa + 16384u);
 #pragma unroll
-                        for (int k4 = 0; k4 < 4; ++k4)
-                            umma_f8f6f4_pair(d_tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, ((kt + j) | k4) != 0);
+                            for (int k4 = 0; k4 < 4; ++k4)
+                                umma_f8f6f4_pair(d_tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, ((kt + j) | k4) != 0);
+                        }
+                        umma_commit_pair(empty_bar(s));
                     }
-                    umma_commit_pair(empty_bar(s));
+                    __syncwarp();
                     if (++s == F8P_STAGES) { s = 0; ph ^= 1u; }
                 }
-                umma_commit_pair(accf_bar(buf));
+                if (lead) umma_commit_pair(accf_bar(buf));
+                __syncwarp();
             }
         }
     } else {

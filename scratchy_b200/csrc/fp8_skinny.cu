@@ -97,29 +97,33 @@ fp8_skinny_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ w
             }
         }
     } else if (warp == 10) {
-        if (lane == 0) {
-            skinny_pdl_wait();
-            const uint32_t idesc = umma_idesc(0, 0, SKINNY_ROWS, tokens);
-            for (int i = 0; i < steps; ++i) {
-                const int sw = i % C::kSW, sx = i % C::kSX;
-                mbar_wait(wfull(sw), (uint32_t)(i / C::kSW) & 1u, status, TC_ERR_FULL_WAIT);
-                mbar_wait(xfull(sx), (uint32_t)(i / C::kSX) & 1u, status, TC_ERR_FULL_WAIT);
-                tc_fence_after();
-                const uint64_t adesc = umma_desc_k_sw128(smem_base + sw * F8S_W_STAGE), bdesc = umma_desc_k_sw128(smem_base + C::kXOff + sx * C::kXStage);
+        // The warp goes round as a whole, with one lane elected for the instructions alone, so that the descriptors stay in uniform
+        // registers: an MMA of few columns is shorter than its issue from a divergent thread.
+        skinny_pdl_wait();
+        const bool lead = elect_one();
+        const uint32_t idesc = umma_idesc(0, 0, SKINNY_ROWS, tokens);
+        for (int i = 0; i < steps; ++i) {
+            const int sw = i % C::kSW, sx = i % C::kSX;
+            const uint64_t adesc = umma_desc_k_sw128(smem_base + sw * F8S_W_STAGE), bdesc = umma_desc_k_sw128(smem_base + C::kXOff + sx * C::kXStage);
+            mbar_wait(wfull(sw), (uint32_t)(i / C::kSW) & 1u, status, TC_ERR_FULL_WAIT);
+            mbar_wait(xfull(sx), (uint32_t)(i / C::kSX) & 1u, status, TC_ERR_FULL_WAIT);
+            tc_fence_after();
+            if (lead) {
 #pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) umma_f8f6f4(tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, (i | k4) != 0);
+                for (int k4 = 0; k4 < 4; ++k4) umma_f8f6f4(tmem, adesc + (uint64_t)(2 * k4), bdesc + (uint64_t)(2 * k4), idesc, i > 0 || k4 > 0);
                 umma_commit(wempty(sw));
                 umma_commit(xempty(sx));
             }
-            umma_commit(accf);
+            __syncwarp();
         }
+        if (lead) umma_commit(accf);
     } else {
         skinny_pdl_wait();
         mbar_wait(accf, 0, status, TC_ERR_ACC_FULL);
     }
     __syncwarp();
     skinny_pdl_wait();
-    skinny_finish(tmem, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, tile * SKINNY_ROWS, N,
+    skinny_finish(tmem, false, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, tile * SKINNY_ROWS, N,
                          [&](int m, int n, float a, float b) {
         const float as = a_scale[m], v[2] = {a, b};
 #pragma unroll

@@ -37,11 +37,11 @@ __host__ __device__ constexpr size_t skinny_sum_bytes(int tokens) { return (size
 
 // The end of a unit, called by every thread of every CTA of the cluster once its role is done; warps 0..7 have seen the
 // accumulator complete, so nothing reads or fills this CTA's rings any more.  `d` = the accumulator (lane = channel, column =
-// token), `sums` = the start of the rings (shared and generic address).  The tokens are dealt to the cluster's CTAs in runs:
+// token), with `two` followed by a second one SECOND columns on, which is added, `sums` = the start of the rings (shared and generic address).  The tokens are dealt to the cluster's CTAs in runs:
 // a CTA sends every run to its owner, which adds the `split` sums of a value in rank order and passes the channels n and
 // n + 8 (n % 16 < 8: a gate and its up, where they are interleaved) to put(token, n, sum, sum8).
-template <typename Put>
-__device__ __forceinline__ void skinny_finish(uint32_t d, uint32_t sums, const float* sums_gen, int M, int split, int rank, int n0, int N, Put put) {
+template <int SECOND = 0, typename Put>
+__device__ __forceinline__ void skinny_finish(uint32_t d, bool two, uint32_t sums, const float* sums_gen, int M, int split, int rank, int n0, int N, Put put) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int per = (M + split - 1) / split;
     if (split > 1) skinny_cluster_sync();
@@ -53,6 +53,13 @@ __device__ __forceinline__ void skinny_finish(uint32_t d, uint32_t sums, const f
             uint32_t r[16];
             tmem_ld_32x16(d + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c, r);
             tmem_ld_wait();
+            if (SECOND && two) {
+                uint32_t more[16];
+                tmem_ld_32x16(d + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(SECOND + c), more);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(more[j]));
+            }
             int owner = c / per, at = c - owner * per;
 #pragma unroll
             for (int j = 0; j < 16; ++j) {

@@ -35,7 +35,8 @@ def test_int4(N, K, M, group):
     assert torch.equal((part + layer.linear_bias.float()).bfloat16().view(torch.int16), yb.view(torch.int16))
 
 
-@pytest.mark.parametrize("N,K,M", [(8, 8, 17), (130, 200, 32), (136, 64, 33), (520, 1032, 64), (300, 4104, 65), (3072, 3072, 128)])
+@pytest.mark.parametrize("N,K,M", [(8, 8, 17), (130, 200, 32), (136, 64, 33), (520, 1032, 64), (300, 4104, 65), (3072, 3072, 128), (18952, 1032, 1),
+                                   (9480, 2056, 16)])
 def test_dense(N, K, M):
     """The same edges of the bf16 linear: plain and f32 outputs against 64-bit sums, and the residual end."""
     import torch
