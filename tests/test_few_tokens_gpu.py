@@ -64,6 +64,13 @@ def test_dense_on_cta_pairs(N, K, M):
     test_dense(N, K, M)
 
 
+@pytest.mark.parametrize("group", [32, 64])
+@pytest.mark.parametrize("N,K,M", [(8, 128, 129), (130, 384, 192), (264, 640, 193), (1000, 1152, 400), (4096, 2176, 1030), (8192, 3072, 770)])
+def test_int4_prompts(N, K, M, group):
+    """The same checks on tiles of 128 to 192 tokens: counts on both sides of a tile, whole rounds, cut tails, one chunk."""
+    test_int4(N, K, M, group)
+
+
 @pytest.mark.parametrize("N,K,M", [(8, 64, 17), (130, 328, 32), (264, 1160, 33), (512, 3584, 65), (300, 18944, 128), (384, 256, 129), (3584, 2184, 250)])
 def test_fp8(N, K, M):
     """Token counts on both sides of 32, 64 and 128, and up to the 256 of one accumulator; ragged channels and k."""
