@@ -17,7 +17,9 @@
 // TMEM holds two accumulators of 192 columns (the epilogue of a tile overlaps the main loop of the next) and two stages of 64
 // columns of dequantised weights.  No multicast: every CTA issues its own loads.
 //
-// What bounds it: the tensor cores, and the activations' way from L2 (48 KB per chunk of 768 MMA cycles).
+// What bounds it: the MMAs themselves.  With A in TMEM one of 128 x N x 16 took about 110 + N / 2 cycles (measured: 125 at 32 columns,
+// 150 at 128, 195 at 192), so wide tiles pay, and 192 is what fits twice beside the stages: 1560 cycles per chunk.  128 tokens with
+// four stages took 1200 (a sixth slower per token), pairs of SMs (cta_group::2) 1900 per 256 channels.
 #include <cuda.h>
 
 #include <algorithm>

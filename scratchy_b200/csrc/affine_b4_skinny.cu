@@ -2,21 +2,21 @@
 //
 //   y[m,n] = bf16( sum_k x[m,k] * w[n,k] (+ bias[n]) ),  w = the bit-exact bf16 dequantisation of the codes
 //
-// A unit is 128 channels by one CTA's share of the 128-k chunks; 384 threads:
+// A unit is 128 channels by one CTA's share of the 128-k chunks; 352 threads:
 //   warps 0-7    dequantise: two groups of four warps take alternate chunks; a thread expands the 128 codes of ONE channel
 //                and writes them to TMEM with tcgen05.st, where the MMA reads its A operand: no swizzled shared-memory
 //                image, no proxy fence.  Afterwards they drain the accumulator.
 //   warp 8       producer of the packed weights (8 bulk copies of a block per chunk), which are load-time constants: it
 //                starts before the preceding kernel of the stream has finished
 //   warp 9       producer of the activations (2 tiled TMA loads of 64 k x the tokens, 128-byte swizzle, zeros outside)
-//   warps 10,11  (10 owns TMEM) issue 8 tcgen05.mma (128 x tokens x 16) per chunk, each the chunks of one group of warps 0-7
-//                into its own accumulator; the two are added at the end
+//   warp 10      owns TMEM; one elected lane issues 8 tcgen05.mma (128 x tokens x 16) per chunk
 //
-// What bounds it: the packed weights from HBM (9.2 KB per chunk) and, for the short k extents of a layer's linears, the start
-// of the pipeline and the two cluster barriers at its end.  Against the 128-token tile of affine_b4_gemm.cu, which it replaces
-// here (its rows were mostly padding, its dequantised image took a round trip through shared memory and its split sums a second
-// launch): 45 rows of 8192 -> 3072, 16.1 us in two launches before, about 10 us in one now; the four linears of a
-// Llama-3.2-3B layer at 32 tokens 56 us and four finishing launches before, the whole decode step 3.95 -> 3.33 ms.
+// What bounds it: for the short k extents of a layer's linears the start of the pipeline and the two cluster barriers at its end
+// (4 of the 7 us of a 3072 x 3072), for long ones the MMAs, which with A in TMEM take about 125 cycles each however few the columns
+// (1000 cycles per chunk and SM; a chunk's 9.2 KB from HBM would take 400).  Against the 128-token tile of the prefill GEMM that it
+// replaced, whose rows were mostly padding and whose split sums took a second launch: 45 rows of 8192 -> 3072 16.1 us, here 11.5;
+// the decode step of Llama-3.2-3B at 32 sequences 3.95 -> 3.33 ms, with whole-warp issue, the counted cut and sums sent 16 bytes at a
+// time 2.69 ms (together with the decode attention's step).
 #include <cuda.h>
 
 #include "affine_b4.cuh"
@@ -24,15 +24,17 @@
 
 namespace {
 
-constexpr int A4S_THREADS = 384;
+constexpr int A4S_THREADS = 352;
 
 template <int TN>
 struct A4SCfg {
-    // Stages, all even in number: a stage then always belongs to one of the two groups, whose waits take its phases in order
-    static constexpr int kSP = TN == 64 ? 4 : 6;                        // packed weights
-    static constexpr int kSX = 4;                                       // activations
-    static constexpr int kSA = TN == 128 ? 4 : 2;                       // dequantised weights in TMEM, 64 columns each
-    static constexpr uint32_t kTmemCols = TN == 128 ? 512 : 256;        // two accumulators of TN columns and the stages
+    static constexpr int kSP = 6;                                       // packed-weight stages, an even number: a stage always belongs to
+                                                                        //   one of the two groups, whose waits take its phases in order
+    static constexpr int kSX = TN == 64 ? 3 : 4;                        // activation stages
+    // Dequantised-weight stages in TMEM, 64 columns each beside the accumulator's TN (a stage's way round - expansion, hand-over,
+    // MMAs, release - is about 2000 cycles)
+    static constexpr int kSA = TN == 128 ? 6 : 3;
+    static constexpr uint32_t kTmemCols = TN == 128 ? 512 : 256;
     static constexpr uint32_t kXStage = TN * 256u;                      // 2 atoms of TN rows x 128 B
     static constexpr uint32_t kPOff = kSX * kXStage;
     static constexpr int kCtasPerSm = TN == 128 ? 1 : 2;
@@ -111,7 +113,7 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t
         for (int s = 0; s < C::kSX; ++s) { mbar_init(xfull(s), 1); mbar_init(xempty(s), 1); }
         for (int s = 0; s < C::kSP; ++s) { mbar_init(pfull(s), 1); mbar_init(pempty(s), 4); }
         for (int s = 0; s < C::kSA; ++s) { mbar_init(afull(s), 4); mbar_init(aempty(s), 1); }
-        mbar_init(accf, 2);
+        mbar_init(accf, 1);
         fence_mbar_init();
     }
     if (warp == 10) {
@@ -123,7 +125,7 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     skinny_pdl_trigger();                              // not before this CTA has its TMEM: the next kernel's CTAs could take it first
-    auto a_col = [&](int s) { return tmem + (uint32_t)(2 * TN + 64 * s); };
+    auto a_col = [&](int s) { return tmem + (uint32_t)(TN + 64 * s); };
 
     // Only the weights may be touched before the preceding kernel has finished.  A wait that depends on the activations
     // comes after griddepcontrol.wait, so that its bound does not run against that kernel.
@@ -151,15 +153,13 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t
                 a4s_tma_2d(xs + TN * 128u, &x_map, (kc_lo + i) * 128 + 64, 0, xfull(s));
             }
         }
-    } else if (warp >= 10) {
-        // Two warps issue the MMAs, one for each group's chunks, into an accumulator of its own: the 8 MMAs of a chunk are short, and
-        // what bounded the kernel was the time one thread takes to issue them.  The warp goes round as a whole, with one lane
-        // elected for the instructions alone, so that the descriptors stay in uniform registers.
+    } else if (warp == 10) {
+        // The warp goes round as a whole, with one lane elected for the instructions alone, so that the descriptors stay in uniform
+        // registers: an MMA of few columns is shorter than its issue from a divergent thread (55 cycles).
         skinny_pdl_wait();
-        const int g = warp - 10;
         const bool lead = elect_one();
-        const uint32_t idesc = umma_idesc(1, 1, SKINNY_ROWS, (uint32_t)(M + 15) & ~15u), d = tmem + (uint32_t)(g * TN);
-        for (int i = g; i < steps; i += 2) {
+        const uint32_t idesc = umma_idesc(1, 1, SKINNY_ROWS, (uint32_t)(M + 15) & ~15u);
+        for (int i = 0; i < steps; ++i) {
             const int s = i % C::kSX, a = i % C::kSA;
             const uint32_t xs = smem_base + s * C::kXStage, ac = a_col(a);
             const uint64_t b0 = umma_desc_k_sw128(xs), b1 = umma_desc_k_sw128(xs + TN * 128u);
@@ -168,7 +168,7 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t
             tc_fence_after();
             if (lead) {
 #pragma unroll
-                for (int k = 0; k < 8; ++k) umma_f16_ta(d, ac + (uint32_t)(8 * k), (k < 4 ? b0 : b1) + (uint64_t)(2 * (k & 3)), idesc, i > 1 || k > 0);
+                for (int k = 0; k < 8; ++k) umma_f16_ta(tmem, ac + (uint32_t)(8 * k), (k < 4 ? b0 : b1) + (uint64_t)(2 * (k & 3)), idesc, i > 0 || k > 0);
                 umma_commit(aempty(a));
                 umma_commit(xempty(s));
             }
@@ -206,7 +206,7 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t
     __syncwarp();
     const float factor = (*reinterpret_cast<const unsigned int*>(packed + (size_t)RB * KC * kBlock) != 0) ? 1.0f : AFF_SCALED_FACTOR;
     skinny_pdl_wait();
-    skinny_finish<TN>(tmem, steps > 1, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, tile * SKINNY_ROWS, N, [&](int m, int n, float a, float b) {
+    skinny_finish(tmem, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, tile * SKINNY_ROWS, N, [&](int m, int n, float a, float b) {
         const float v[2] = {a * factor, b * factor};
 #pragma unroll
         for (int j = 0; j < 2; ++j) {

@@ -123,7 +123,7 @@ dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_cons
     }
     __syncwarp();
     pdl_wait();
-    skinny_finish(tmem, false, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, n0, N,
+    skinny_finish(tmem, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, n0, N,
                   [&](int m, int n, float a, float b) { dense_put_two<bf16, END>(ends, m, g, n, N, a, b); });
     __syncthreads();
     if (warp == 10) {

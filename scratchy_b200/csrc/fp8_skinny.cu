@@ -123,7 +123,7 @@ fp8_skinny_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ w
     }
     __syncwarp();
     skinny_pdl_wait();
-    skinny_finish(tmem, false, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, tile * SKINNY_ROWS, N,
+    skinny_finish(tmem, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, tile * SKINNY_ROWS, N,
                          [&](int m, int n, float a, float b) {
         const float as = a_scale[m], v[2] = {a, b};
 #pragma unroll

@@ -32,18 +32,18 @@ __device__ __forceinline__ void skinny_range(int steps, int rank, int split, int
     hi = (int)((long long)steps * (rank + 1) / split);
 }
 
-// Shared memory the sums of a cluster need (they reuse the rings of the main loop).
-__host__ __device__ constexpr size_t skinny_sum_bytes(int tokens) { return (size_t)(tokens + SKINNY_MAX_SPLIT) * SKINNY_ROWS * 4; }
+// Shared memory the sums of a cluster need (they reuse the rings of the main loop): split x per tokens x 128 channels.
+__host__ __device__ constexpr size_t skinny_sum_bytes(int tokens) { return (size_t)(tokens + 4 * SKINNY_MAX_SPLIT) * SKINNY_ROWS * 4; }
 
 // The end of a unit, called by every thread of every CTA of the cluster once its role is done; warps 0..7 have seen the
 // accumulator complete, so nothing reads or fills this CTA's rings any more.  `d` = the accumulator (lane = channel, column =
-// token), with `two` followed by a second one SECOND columns on, which is added, `sums` = the start of the rings (shared and generic address).  The tokens are dealt to the cluster's CTAs in runs:
-// a CTA sends every run to its owner, which adds the `split` sums of a value in rank order and passes the channels n and
+// token), `sums` = the start of the rings (shared and generic address).  The tokens are dealt to the cluster's CTAs in runs
+// of a multiple of 4 (they travel 16 bytes at a time): a CTA sends every run to its owner, which adds the `split` sums of a value in rank order and passes the channels n and
 // n + 8 (n % 16 < 8: a gate and its up, where they are interleaved) to put(token, n, sum, sum8).
-template <int SECOND = 0, typename Put>
-__device__ __forceinline__ void skinny_finish(uint32_t d, bool two, uint32_t sums, const float* sums_gen, int M, int split, int rank, int n0, int N, Put put) {
+template <typename Put>
+__device__ __forceinline__ void skinny_finish(uint32_t d, uint32_t sums, const float* sums_gen, int M, int split, int rank, int n0, int N, Put put) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int per = (M + split - 1) / split;
+    const int per = ((M + split - 1) / split + 3) & ~3;
     if (split > 1) skinny_cluster_sync();
     else __syncthreads();
     if (warp < SKINNY_EPI_WARPS) {
@@ -53,22 +53,17 @@ __device__ __forceinline__ void skinny_finish(uint32_t d, bool two, uint32_t sum
             uint32_t r[16];
             tmem_ld_32x16(d + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c, r);
             tmem_ld_wait();
-            if (SECOND && two) {
-                uint32_t more[16];
-                tmem_ld_32x16(d + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(SECOND + c), more);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(more[j]));
-            }
+            // [sender][4 tokens][channel][token of the 4]
             int owner = c / per, at = c - owner * per;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
+            for (int j = 0; j < 16; j += 4) {
                 if (c + j < M) {
-                    uint32_t dst = sums + (uint32_t)((rank * per + at) * SKINNY_ROWS + row) * 4u;
+                    uint32_t dst = sums + (uint32_t)(((rank * per + at) >> 2) * SKINNY_ROWS + row) * 16u;
                     if (split > 1) asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(dst) : "r"(owner));
-                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(__uint_as_float(r[j])) : "memory");
+                    asm volatile("st.shared::cluster.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(r[j]), "r"(r[j + 1]), "r"(r[j + 2]), "r"(r[j + 3]) : "memory");
                 }
-                if (++at == per) { at = 0; ++owner; }
+                at += 4;
+                if (at == per) { at = 0; ++owner; }
             }
         }
         tc_fence_before();
@@ -79,13 +74,20 @@ __device__ __forceinline__ void skinny_finish(uint32_t d, bool two, uint32_t sum
     for (int i = threadIdx.x; i < mine * (SKINNY_ROWS / 2); i += blockDim.x) {
         const int t = i >> 6, p = i & 63, ch = (p >> 3) * 16 + (p & 7);
         if (n0 + ch >= N) continue;
-        const float* s = sums_gen + (size_t)t * SKINNY_ROWS + ch;
-        float a = s[0], b = s[8];
-        for (int k = 1; k < split; ++k) {
-            a += s[(size_t)k * per * SKINNY_ROWS];
-            b += s[(size_t)k * per * SKINNY_ROWS + 8];
+        const float* part = sums_gen + ((size_t)(t >> 2) * SKINNY_ROWS + ch) * 4 + (t & 3);
+        float a[SKINNY_MAX_SPLIT], b[SKINNY_MAX_SPLIT];
+#pragma unroll
+        for (int k = 0; k < SKINNY_MAX_SPLIT; ++k) {
+            a[k] = k < split ? part[(size_t)k * per * SKINNY_ROWS] : 0.0f;
+            b[k] = k < split ? part[(size_t)k * per * SKINNY_ROWS + 32] : 0.0f;
         }
-        put(rank * per + t, n0 + ch, a, b);
+#pragma unroll
+        for (int k = 1; k < SKINNY_MAX_SPLIT; ++k)
+            if (k < split) {
+                a[0] += a[k];
+                b[0] += b[k];
+            }
+        put(rank * per + t, n0 + ch, a[0], b[0]);
     }
 }
 
