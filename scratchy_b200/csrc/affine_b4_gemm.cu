@@ -29,7 +29,7 @@
 
 bool affine_b4_gemm_tc_enabled() { return true; }
 // Defined in affine_b4_gemm_pair.cu
-bool affine_b4_gemm_pair_applies(int M, int N, int K, int sms);
+float affine_b4_gemm_pair_us(int M, int N, int K, int sms);
 int32_t affine_b4_gemm_pair_launch(scr_ctx* ctx, const CUtensorMap& x_map, const uint8_t* packed, uint16_t* y, int M, int N, int K,
                                    int gs, int out_f32, const uint16_t* bias, cudaStream_t stream, bool* launched);
 // Defined in affine_b4_skinny.cu
@@ -313,10 +313,11 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_
 }
 
 // ---- host --------------------------------------------------------------------------------
-// The tokens of a tile and how the tiles are cut into work units (tc_plan_units).  A chunk takes 4 cycles per token on the tensor
-// cores, but no less than its dequantisation; the width whose rounds fill the GPU best wins.
+// The tokens of a tile and how the tiles are cut into work units (tc_plan_units).  A 128-k chunk of a tile was measured at 0.65 us
+// for 128 tokens and 0.83 us for 192; the width whose rounds fill the GPU best wins.
 struct AffineGemmPlan {
     int width, mt, tiles, full, ks_tail;
+    float us;                                            // estimate
     int n_tail() const { return tiles - full; }
     size_t slab_floats() const { return ks_tail > 1 ? (size_t)ks_tail * n_tail() * (size_t)(width * A4G_BN) : 0; }
 };
@@ -329,10 +330,10 @@ static AffineGemmPlan affine_gemm_plan(int M, int N, int K, int sms) {
         p.width = width;
         p.mt = scr_ceil_div(M, width);
         p.tiles = p.mt * (g.RB * 16 / A4G_BN);
-        const float us = (width < 144 ? 144 : width) * (1.0f / 380.0f);
-        const float t = tc_plan_units(p.tiles, g.KC, sms, us, &p.full, &p.ks_tail) * g.KC * us;
-        if (t < least * 0.99f) {
-            least = t;
+        const float us = 0.28f + 0.00286f * width;
+        p.us = tc_plan_units(p.tiles, g.KC, sms, us, &p.full, &p.ks_tail) * g.KC * us;
+        if (p.us < least * 0.99f) {
+            least = p.us;
             best = p;
         }
     }
@@ -376,13 +377,15 @@ int32_t affine_b4_gemm_tc_launch(scr_ctx* ctx, const uint8_t* packed, const uint
     tc_encode_tiled_fn enc = tc_tensor_map_encoder();
     if (!enc) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled entry point not available");
     CUtensorMap map;
-    if (affine_b4_gemm_pair_applies(M, N, K, ctx->sm_count)) {     // large, evenly tiled GEMMs: the two-CTA kernel (affine_b4_gemm_pair.cu)
+    const AffineGemmPlan plan = affine_gemm_plan(M, N, K, ctx->sm_count);
+    // Pairs (affine_b4_gemm_pair.cu) where their rounds come out clearly shorter: 2048 tokens of 3072 -> 16384 166 us against 205;
+    // 2048 of 3072 -> 8192, estimates 2 % apart, 110 against 107.
+    if (affine_b4_gemm_pair_us(M, N, K, ctx->sm_count) < 0.9f * plan.us) {
         bool launched = false;
         if (!affine_gemm_x_map(&map, enc, x, M, K, 128)) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled failed");
         const int32_t st = affine_b4_gemm_pair_launch(ctx, map, packed, y, M, N, K, gs, out_f32, bias, stream, &launched);
         if (st || launched) return st;
     }
-    const AffineGemmPlan plan = affine_gemm_plan(M, N, K, ctx->sm_count);
     float* slabs = reinterpret_cast<float*>(workspace);
     if (plan.ks_tail > 1 && (!slabs || !scr_aligned16(slabs))) return scr_fail(ctx, SCR_E_WORKSPACE, "split-K needs an aligned workspace");
     if (!affine_gemm_x_map(&map, enc, x, M, K, plan.width)) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled failed");

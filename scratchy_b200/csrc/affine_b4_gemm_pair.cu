@@ -10,7 +10,9 @@
 // channels; one `tcgen05.mma.cta_group::2` of shape 256 x 256 x 16, issued by the pair's leader CTA, reads the token rows
 // and the channel rows from both SMs' shared memory and leaves each CTA's 128 accumulator rows in that CTA's own TMEM.
 // Same MACs and the same dequantise work per SM and chunk, 44 % less L2 traffic, and room for three stages of each ring.
-// Measured: the same bits as the one-CTA kernel at the same speed (see `affine_b4_gemm_pair_applies`), so it is opt-in.
+// What bounds it: the shared-memory data pipe (operand reads, dequantised tile, activations), near the MMAs' own rate.  2048 tokens of
+// 3072 -> 16384: 166 us (1243 TFLOP/s) against 205 us on one CTA per tile with the weights in TMEM; issued from a divergent thread
+// the MMAs had held it to the one-CTA kernel's speed.
 //
 // Per CTA (704 threads), both CTAs of a pair run the same code:
 //   warp 0       producer: per chunk 2 tiled TMA loads of this CTA's activations (`.cta_group::2`, completing on the
@@ -351,23 +353,18 @@ affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const uint
 }  // namespace
 
 
-// Whether the pair kernel takes this GEMM.  It is OFF unless `SCR_AFFINE_GEMM_PAIR=1` is in the environment (read once):
-// on the Llama-3.2-3B gate shape at 2048 tokens it gives the same bits in 100.1 us against the one-CTA kernel's 99.3 us —
-// with the dequantise warps' serial chain per chunk as the limiter of both, halving the activation traffic buys nothing
-// yet.  When on: whole 256-channel pair tiles, at least one full round of pairs, and rounds that are at least 85 % full
-// (the one-CTA kernel splits its tail along k instead).
-bool affine_b4_gemm_pair_applies(int M, int N, int K, int sms) {
+// What this GEMM would take on pairs, in us (rounds of 256 x 256 tiles at 1.02 us per 128-k chunk, measured); more than anything
+// where it does not go there: whole 256-channel pair tiles only.  `SCR_AFFINE_GEMM_PAIR=0` in the environment switches the pair
+// kernel off (read once).
+float affine_b4_gemm_pair_us(int M, int N, int K, int sms) {
     static const bool enabled = [] {
         const char* e = std::getenv("SCR_AFFINE_GEMM_PAIR");
-        return e && e[0] == '1';
+        return !(e && e[0] == '0');
     }();
-    if (!enabled) return false;
     const AffineGeom g = affine_geom(N, K, 64);
-    if ((g.RB % 16) != 0 || g.KC < 1 || M <= 128) return false;
     const int pairs = sms / 2, tiles = scr_ceil_div(M, 256) * (g.RB / 16);
-    if (pairs < 1 || tiles < pairs) return false;
-    const int rounds = (tiles + pairs - 1) / pairs;
-    return (float)tiles >= 0.85f * (float)(rounds * pairs);
+    if (!enabled || (g.RB % 16) != 0 || g.KC < 1 || M <= 128 || pairs < 1) return 1e30f;
+    return 1.02f * (float)g.KC * (float)scr_ceil_div(tiles, pairs);
 }
 
 int32_t affine_b4_gemm_pair_launch(scr_ctx* ctx, const CUtensorMap& x_map, const uint8_t* packed, uint16_t* y, int M, int N, int K,
