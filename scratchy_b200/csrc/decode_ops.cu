@@ -248,12 +248,21 @@ __global__ void __launch_bounds__(ARGMAX_THREADS) argmax_kernel(const uint16_t* 
     float best = -INFINITY;
     uint32_t best_i = 0;
     const int nv = width >> 3;
-#pragma unroll 8                                       // one SM reads the row: eight requests a thread in flight
-    for (int v = threadIdx.x; v < nv; v += ARGMAX_THREADS) {
-        float f[8];
-        unpack8(*reinterpret_cast<const uint4*>(row + v * 8), f);
+    constexpr int AHEAD = 8;                           // one SM reads the row: eight requests a thread in flight
+    for (int v0 = threadIdx.x; v0 < nv; v0 += AHEAD * ARGMAX_THREADS) {
+        uint4 q[AHEAD];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) argmax_take(f[j], uint32_t(v * 8 + j), best, best_i);
+        for (int u = 0; u < AHEAD; ++u)
+            if (v0 + u * ARGMAX_THREADS < nv) q[u] = *reinterpret_cast<const uint4*>(row + (v0 + u * ARGMAX_THREADS) * 8);
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            const int v = v0 + u * ARGMAX_THREADS;
+            if (v >= nv) break;
+            float f[8];
+            unpack8(q[u], f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) argmax_take(f[j], uint32_t(v * 8 + j), best, best_i);
+        }
     }
     for (int i = (nv << 3) + threadIdx.x; i < width; i += ARGMAX_THREADS)
         argmax_take(bf16_bits_to_f32(row[i]), uint32_t(i), best, best_i);
@@ -556,8 +565,9 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_kernel(
 // The cluster (1, 2, 4 or 8 CTAs, chosen by the host from the batch) splits the sequence by whole
 // blocks.  Every wait is bounded and reports through the status word.
 //
-// What bounds it: HBM (8 KB per block of 16 tokens and kv head).  Llama-3.2-3B at 32 sequences of 512 to 2048 tokens, 168 MB
-// per layer: 60 us with the producer warp and a second MMA for the remainders, 46 us (3.6 TB/s) like this, alone and cold.
+// What bounds it: HBM (8 KB per block of 16 tokens and kv head), and the longest sequence's CTA.  Llama-3.2-3B at 32 sequences of
+// 512 to 2048 tokens, 153 MB per layer: 60 us with the producer warp and a second MMA for the remainders, 41 us with rings of
+// the warps' own, 38 us (4.0 TB/s) with the cut and the warps chosen as in `attention_launch`.
 constexpr int ATT_ERR_FULL = 0x0A000001;
 
 __device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const CUtensorMap* tmap, int c0, int c1, int c2, uint32_t bar) {
@@ -679,7 +689,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_tc_kernel(
     // cache at all).
     const int newest_blk = total_blk - 1;
     const int spw = stages / nwarps;
-    auto load = [&](int n) {                           // lane 0: the warp's n-th block
+    auto load = [&](int n) {                           // (one lane) the warp's n-th block
         const int i = warp + n * nwarps;
         if (i >= nblk) return;
         const int s = warp * spw + n % spw;
@@ -693,16 +703,11 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_tc_kernel(
         }
     };
     {
-        bool pending = false;
-        if (lane == 0)
-            for (int n = 0; n < spw; ++n) {
-                if (!rope.enabled && first_blk + warp + n * nwarps >= newest_blk) pending = true;
-                else load(n);
-            }
+        // lane n fills stage n: the lanes issue side by side, and q's loads below are not held up behind them
+        const bool waits = !rope.enabled && first_blk + warp + lane * nwarps >= newest_blk;
+        if (lane < spw && !waits) load(lane);
         pdl_wait();
-        if (pending)
-            for (int n = 0; n < spw; ++n)
-                if (first_blk + warp + n * nwarps >= newest_blk) load(n);
+        if (lane < spw && waits) load(lane);
         __syncwarp();
         const int row = lane >> 2, quad = lane & 3;
         uint32_t qa0[KSTEPS], qa2[KSTEPS];             // A fragments of Q: row = query head (zero beyond G), 16 dims per step
@@ -900,9 +905,13 @@ cudaError_t attention_launch(const uint16_t* q, long long ld_q, const uint16_t* 
     const size_t warp_part = size_t(ATT_WARPS) * G * (D + 2) * sizeof(float);
     int nsplit = ATT_SPLITS;                         // the most splits that still run as a single wave of two CTAs per SM
     while (nsplit > 1 && (long long)batch * num_kv_heads * nsplit > 2LL * sm_count) nsplit /= 2;
+    // ... but not below two for long sequences: a CTA per sequence and kv head lasts as long as the longest of them while SMs that
+    // held shorter ones idle (20 sequences of 750 to 3000 tokens 53.8 us, halved 37.4; 32 of 500 to 2000 41.1 and 38.2; 32 of 250
+    // to 1000 20.0 and 26.9)
+    if (nsplit == 1 && (long long)max_blocks_per_seq * block_size >= 1536) nsplit = 2;
     const int table_cap = max_blocks_per_seq / nsplit + 2;
     const size_t fixed = part + size_t((table_cap + 1) & ~1) * 4 + ATT_MAX_STAGES * sizeof(uint64_t) + 1024 + 128;
-    // alone on its SM: 8 consumer warps and a deep ring; otherwise 4 consumer warps and about half an SM's shared
+    // alone on its SM: 8 warps and a deep ring; otherwise 4 or 6 warps and about half an SM's shared
     // memory.  The big CTA (48 K registers, ~200 KB) shares its SM with no CTA of the kernels before and after it in
     // the stream, so it pays only while the grid leaves most SMs to them: up to half the SMs.  (Llama-3.2-3B decode
     // step, measured inside the step: batch 1, 64 CTAs — 1.074 ms with the big CTA, 1.116 with the small one; batch 2,
@@ -910,7 +919,9 @@ cudaError_t attention_launch(const uint16_t* q, long long ld_q, const uint16_t* 
     // and wants at least two of them, so that its next block loads while it works on the current one.
     const bool alone = 2LL * batch * num_kv_heads * nsplit <= sm_count;
     const size_t budget = alone ? ATT_SMEM_BUDGET_ALONE : ATT_SMEM_BUDGET;
-    int nwarps = alone ? 8 : 4, spw = 0;
+    // Six warps of two stages where a CTA has four blocks or more for each, otherwise four of three (16 sequences of up to 2048
+    // tokens 23.9 us with four warps, 20.8 with six; 4 sequences, 16 blocks a CTA, 13.0 and 14.6).
+    int nwarps = alone ? 8 : max_blocks_per_seq / nsplit >= 24 ? 6 : 4, spw = 0;
     for (; nwarps >= 2; nwarps /= 2) {
         spw = budget > fixed ? int(std::min<size_t>(3, (budget - fixed) / (2 * chunk * nwarps))) : 0;
         if (spw >= 2) break;

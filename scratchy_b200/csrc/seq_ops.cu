@@ -212,15 +212,22 @@ __global__ void __launch_bounds__(AMAX_T) seq_argmax_kernel(const float* __restr
     const float* row = logits + blockIdx.x * ld;
     float best = -INFINITY;
     int best_i = 0x7FFFFFFF;
-    // one SM reads the row: four requests of 16 bytes a thread in flight
     const int nv = (reinterpret_cast<uintptr_t>(row) & 15) == 0 ? width / 4 : 0;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < nv; i += AMAX_T) {
-        const float4 v = reinterpret_cast<const float4*>(row)[i];
-        amax_take(v.x, 4 * i, best, best_i);
-        amax_take(v.y, 4 * i + 1, best, best_i);
-        amax_take(v.z, 4 * i + 2, best, best_i);
-        amax_take(v.w, 4 * i + 3, best, best_i);
+    constexpr int AHEAD = 8;                               // one SM reads the row: eight requests of 16 bytes a thread in flight
+    for (int i0 = threadIdx.x; i0 < nv; i0 += AHEAD * AMAX_T) {
+        float4 q[AHEAD];
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u)
+            if (i0 + u * AMAX_T < nv) q[u] = reinterpret_cast<const float4*>(row)[i0 + u * AMAX_T];
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            const int i = i0 + u * AMAX_T;
+            if (i >= nv) break;
+            amax_take(q[u].x, 4 * i, best, best_i);
+            amax_take(q[u].y, 4 * i + 1, best, best_i);
+            amax_take(q[u].z, 4 * i + 2, best, best_i);
+            amax_take(q[u].w, 4 * i + 3, best, best_i);
+        }
     }
     for (int i = 4 * nv + threadIdx.x; i < width; i += AMAX_T) amax_take(row[i], i, best, best_i);
 #pragma unroll

@@ -56,3 +56,16 @@ def test_greedy_picks_the_first_of_equals_at_any_alignment(width, ld):
     rows[1, :width] = -3.0                                           # all equal: the first
     want = rows[:, :width].numpy().argmax(axis=1)
     assert greedy(rows.cuda()[:, :width]).cpu().numpy().tolist() == want.tolist()
+
+
+@pytest.mark.parametrize("longest,hq,hkv,d,bs,batch", [(1600, 8, 4, 64, 16, 40), (1600, 6, 2, 128, 32, 80), (700, 8, 4, 128, 16, 40), (300, 8, 4, 128, 16, 40),
+                                                       (1700, 4, 4, 64, 64, 12), (2100, 3, 1, 128, 16, 21)])
+def test_decode_attention_at_every_cut_and_number_of_warps(longest, hq, hkv, d, bs, batch):
+    """Sequences of all lengths up to `longest` in one launch: halved for length alone, four, six and eight warps a CTA."""
+    from scratchy_b200 import synth
+    from tests.test_decode_gpu import REL_L2_TOL, _attention_case
+    from util import rel_l2
+    rng = np.random.default_rng(longest + batch)
+    lens = [longest, 1, bs, bs + 1] + rng.integers(1, longest + 1, batch - 4).tolist()
+    got, want = _attention_case(lens, hq, hkv, d, bs, synth.seed_for("cut", longest, hq, hkv, d, bs))
+    assert rel_l2(got, want) <= REL_L2_TOL
