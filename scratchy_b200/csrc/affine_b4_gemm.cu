@@ -120,7 +120,7 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_
     static_assert(8 * (kAccSlot + 5) <= 256, "barriers");
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kBarOff + 8 * (kAccSlot + 4));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     // Work units: the first `full` tiles whole; each of the remaining (tail) tiles as ks_tail units that share its k
     // extent and leave f32 partial tiles in `slabs` for the finishing kernel.
     const int n_tail = MT * (RB / 8) - full, units = full + n_tail * ks_tail;

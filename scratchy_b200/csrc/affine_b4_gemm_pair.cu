@@ -116,7 +116,7 @@ affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const uint
     auto acce = [&](int b) { return bar_base + 8u * (kAccSlot + 2 + b); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + A4P_BAROFF + 8 * (kAccSlot + 4));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = a4p_cta_rank();                 // 0 = the pair's leader
     const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
     const int NTP = RB * 16 / A4P_BN;                     // pair tiles along the channels (RB is a multiple of 16 here)

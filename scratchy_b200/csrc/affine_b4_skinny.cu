@@ -103,7 +103,7 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t
     const uint32_t accf = bar + 8u * kSlots;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kBarOff + 8 * (kSlots + 1));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int tile = blockIdx.x / split, rank = blockIdx.x - tile * split;
     int kc_lo, kc_hi;
     skinny_range(KC, rank, split, kc_lo, kc_hi);

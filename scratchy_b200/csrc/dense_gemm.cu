@@ -238,7 +238,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     auto acce_bar = [&](int b) { return bar_base + 8u * (2 * S::kStages + 2 + b); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + S::kBarOffset + 8 * (2 * S::kStages + 4));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int n_tail = MT * NTB * groups - full;
     const int units = full + n_tail * ks_tail;
 
@@ -391,7 +391,7 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_c
     auto acce_bar = [&](int b) { return bar_base + 8u * (2 * DP_STAGES + 2 + b); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + DP_BAR_OFFSET + 8 * (2 * DP_STAGES + 4));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = dp_rank();
     const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
     const int n_tail = MT * NTB * groups - full;

@@ -50,7 +50,7 @@ dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_cons
     const uint32_t accf = bar + 8u * kSlots;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + C::kBarOff + 8 * (kSlots + 1));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int tile = blockIdx.x / split, rank = blockIdx.x - tile * split;
     const int g = tile / NT, n0 = (tile - g * NT) * SKINNY_ROWS;
     int k_lo, k_hi;

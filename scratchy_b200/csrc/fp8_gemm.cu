@@ -113,7 +113,7 @@ fp8_gemm_tc_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ 
     auto acce_bar = [&](int b) { return bar_base + 8u * (2 * F8G_STAGES + 2 + b); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + F8GSmem<BN>::kBarOffset + 8 * (2 * F8G_STAGES + 4));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int NTB = (NT * 128 + BN - 1) / BN;            // channel tiles of BN
     const int n_tail = MT * NTB - full;                  // tiles whose k extent is split ks_tail ways (see tc_plan_units)
     const int tiles = full + n_tail * ks_tail;

@@ -100,7 +100,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_con
     auto acce_bar = [&](int b) { return bar_base + 8u * (2 * F8P_STAGES + 2 + b); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + F8P_BAR_OFFSET + 8 * (2 * F8P_STAGES + 4));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = pair_cta_rank();               // 0 = the pair's leader
     const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
     const int MTP = MT >> 1, NTP = NT >> 1;              // pair tiles: 256 tokens x 256 channels

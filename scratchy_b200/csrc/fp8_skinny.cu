@@ -51,7 +51,7 @@ fp8_skinny_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ w
     const uint32_t accf = bar + 8u * kSlots;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + C::kBarOff + 8 * (kSlots + 1));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int tile = blockIdx.x / split, rank = blockIdx.x - tile * split;
     int k_lo, k_hi;
     skinny_range(KT, rank, split, k_lo, k_hi);

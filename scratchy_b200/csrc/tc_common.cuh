@@ -225,6 +225,10 @@ static inline int tc_sm_count() {
     return sms;
 }
 
+// The warp's index, broadcast from a lane so that the compiler takes branches on it, and what is computed under them, for uniform:
+// the descriptors of an MMA then stay in uniform registers.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred;
     asm volatile(
