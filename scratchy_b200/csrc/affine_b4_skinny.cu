@@ -15,8 +15,8 @@
 // (4 of the 7 us of a 3072 x 3072), for long ones the MMAs, which with A in TMEM take about 125 cycles each however few the columns
 // (1000 cycles per chunk and SM; a chunk's 9.2 KB from HBM would take 400).  Against the 128-token tile of the prefill GEMM that it
 // replaced, whose rows were mostly padding and whose split sums took a second launch: 45 rows of 8192 -> 3072 16.1 us, here 11.5;
-// the decode step of Llama-3.2-3B at 32 sequences 3.95 -> 3.33 ms, with whole-warp issue, the counted cut and sums sent 16 bytes at a
-// time 2.69 ms (together with the decode attention's step).
+// the decode step of Llama-3.2-3B at 32 sequences 3.95 -> 3.33 ms, with whole-warp issue, the counted cut, sums sent 16 bytes at
+// a time and the warp index broadcast 2.60 ms (together with the decode attention's step).
 #include <cuda.h>
 
 #include "affine_b4.cuh"
