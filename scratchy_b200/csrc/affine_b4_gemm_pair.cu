@@ -233,8 +233,12 @@ affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const uint
                 if ((c & 1) != grp) continue;
                 const int sp = c % A4P_SP, sd = c % A4P_SD;
                 const uint32_t php = (uint32_t)(c / A4P_SP) & 1u, phd = (uint32_t)(c / A4P_SD) & 1u;
-                mbar_wait(pfull(sp), php, status, TC_ERR_FULL_WAIT);
+                // `dempty` first: an odd ring hands a stage from one group to the other, so a group has not seen the fill three
+                // chunks back, and `pfull`'s parity alone would also be met two phases early.  That fill's MMAs, which
+                // `dempty` (stage for stage the same ring) waits for, cannot have run before it was complete.
+                static_assert(A4P_SP == A4P_SD, "the packed and the dequantised stages go round together");
                 mbar_wait(dempty(sd), phd ^ 1u, status, TC_ERR_EMPTY_WAIT);
+                mbar_wait(pfull(sp), php, status, TC_ERR_FULL_WAIT);
                 const uint32_t ps = smem_base + A4P_POFF + sp * A4P_PSTAGE;
                 const uint32_t ds = smem_base + A4P_DOFF + sd * A4P_DSTAGE;
 #pragma unroll
