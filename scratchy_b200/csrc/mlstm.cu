@@ -139,8 +139,8 @@ __global__ void __launch_bounds__(RC_T) mlstm_recur_kernel(MemoryArgs a) {
 }
 
 // The slice of S (and this slice's copy of n) in registers: 8 threads with 4 columns each cover a row, a thread has RPT rows, 32
-// apart.  The state is requested before the wait for the preceding kernel (no other kernel of a step touches it), and a token
-// takes one barrier: the normaliser's n.q goes round with the outputs.
+// apart.  The state's lines start for L2 before the wait for the preceding kernels and are read after it (one of those kernels may be
+// the call that leaves this one its state), and a token takes one barrier: the normaliser's n.q goes round with the outputs.
 // What bounds it: HBM, the state read and written once a step.  32 sequences of 12 heads of 128 x 256 (101 MB), alone and cold: 34.0 us
 // with the state in shared memory, asked for after the wait, and two barriers a token; 29.9 us here.
 template <typename T, int RPT>
@@ -159,6 +159,21 @@ __global__ void __launch_bounds__(RC_T) mlstm_step_kernel(MemoryArgs a) {
     const bool vec = cols == 4 && (vdim & 3) == 0, held = ok && pos0 > 0;
     const size_t head = (size_t)(ok ? slot : 0) * s.heads + h, copy = head * mlstm_slices(vdim) + blockIdx.x;
     float *gs = a.state_s + head * dim * vdim + col, *gn = a.state_n + copy * dim;
+    if (held)
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            const int r = row0 + i * RC_ROWS;
+            if (r < dim && (tid & 7) == 0) {
+                prefetch_l2(gs + (size_t)r * vdim);
+                if (row0 == 0) prefetch_l2(gn + r);              // (32 rows of n to a line)
+            }
+        }
+    const float qscale = 1.0f / sqrtf(float(dim));
+    pdl_wait();
+    if (!ok) {
+        if (count > 0 && tid == 0) atomicCAS(a.status, 0, SEQ_BAD_SLOT);
+        return;
+    }
     float4 S[RPT];
     float n[RPT], m = held ? a.state_m[copy] : 0.0f;
 #pragma unroll
@@ -176,12 +191,6 @@ __global__ void __launch_bounds__(RC_T) mlstm_step_kernel(MemoryArgs a) {
                 if (cols > 3) S[i].w = p[3];
             }
         }
-    }
-    const float qscale = 1.0f / sqrtf(float(dim));
-    pdl_wait();
-    if (!ok) {
-        if (count > 0 && tid == 0) atomicCAS(a.status, 0, SEQ_BAD_SLOT);
-        return;
     }
     float q[RPT], k[RPT], v[4], gi, gf;
     auto fetch = [&](int t) {

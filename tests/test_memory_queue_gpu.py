@@ -1,0 +1,67 @@
+"""Calls of the matrix memories that follow each other on one stream without the host between them: each goes on from the state
+that the one before it leaves.  The bits are those of the same calls with a synchronisation after each."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from tests import seq_util as su
+from tests.test_sequence_ops_gpu import DTYPES, dev, draw_memory, healthy, head_rows, lib, plain_memory, ptr, run_memory, stream, torch_
+
+pytestmark = pytest.mark.gpu
+
+# one portion per call; the state goes from a step to a step, from a prompt's chunks to a step, from a step to chunks
+PORTIONS = [[1] * 12, [70, 1, 1], [3, 64, 1, 1, 130, 2]]
+
+
+def queued(calls, captured):
+    """Issues the prepared calls back to back, as they are or as one captured graph."""
+    torch = torch_()
+    torch.cuda.synchronize()
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for call in calls:
+                call()
+        graph.replay()
+    else:
+        for call in calls:
+            call()
+    healthy()
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 16, 24), (3, 48, 72), (12, 128, 256), (1, 256, 64), (2, 300, 40)])
+@pytest.mark.parametrize("portions", PORTIONS)
+def test_gated_memory(heads, dim, vdim, portions, dtype, captured):
+    from scratchy_b200 import _lib
+    from scratchy_b200.dense import dtype_code
+    torch = torch_()
+    L, c = lib()
+    m = su.memory_spec(heads, dim, vdim)["mixer"]
+    rng = np.random.default_rng(heads * dim + vdim)
+    T, sl = sum(portions), (vdim + 31) // 32
+    proj, gates = draw_memory(rng, T, m, dtype), (2.0 * rng.standard_normal((T, 2 * heads))).astype(np.float32)
+    bi, bf = np.zeros(heads, np.float32), np.full(heads, 2.0, np.float32)
+    (want,), _ = run_memory(m, dtype, [proj], [gates], bi, bf, [[n] for n in portions], [1])
+    shape = _lib.MlstmShape(heads, dim, vdim, m["gate_cap"], 1e-5)
+    state = [torch.full(s, float("nan"), device="cuda") for s in ((2, heads, dim, vdim), (2, heads, sl, dim), (2, heads, sl))]
+    pd, gd, bid, bfd = dev(proj, dtype), dev(gates), dev(bi), dev(bf)
+    out, code = torch.full((T, heads * vdim), float("nan"), device="cuda"), dtype_code(pd.dtype)
+    calls, keep, at = [], [], 0
+    for n in portions:
+        segs = torch.tensor([[0, n, at, 1]], dtype=torch.int32, device="cuda")
+        st, need = _lib.Step(0, 0, segs.data_ptr(), 0, n, 1, n, 0, 2), ctypes.c_size_t(0)
+        c.check(L.scr_mlstm_workspace(code, ctypes.byref(shape), ctypes.byref(st), ctypes.byref(need)))
+        ws = torch.full((max(16, need.value) // 4,), float("nan"), device="cuda")
+        keep.append((segs, st, ws))
+        calls.append(lambda n=n, at=at, st=st, ws=ws, need=need: c.check(L.scr_mlstm_run(
+            c.handle, code, ctypes.byref(shape), ctypes.byref(st), ptr(pd, at * pd.shape[1]), pd.shape[1], ptr(gd, at * 2 * heads), 2 * heads, ptr(bid),
+            ptr(bfd), *[ptr(t) for t in state], ptr(out, at * out.shape[1]), ptr(ws), need, stream())))
+        at += n
+    queued(calls, captured)
+    got = out.cpu().numpy()
+    assert np.array_equal(got, want.astype(np.float32))
+    err = np.sqrt(((head_rows(got, heads) - head_rows(plain_memory(m, proj, gates, bi, bf), heads)) ** 2).mean(axis=2)).ravel()
+    assert np.median(err) < (5e-6 if dtype == "float32" else 5e-5)        # (the bar of the calls with a synchronisation after each)
