@@ -13,8 +13,8 @@ int32_t lightning_chunk_launch(scr_ctx* ctx, const MemoryArgs& a, void* workspac
 namespace {
 
 // One CTA per (32 value columns, head, sequence).  The slice of S stays in registers for the whole segment: 8 threads with
-// 4 columns each cover a row, a thread has RPT rows, 32 apart.  The state is requested before the wait for the preceding
-// kernel (no other kernel of a step touches it).
+// 4 columns each cover a row, a thread has RPT rows, 32 apart.  The state's lines start for L2 before the wait for the preceding
+// kernels and are read after it: one of those kernels may be the call that leaves this one its state.
 constexpr int LR_T = 256, LR_COLS = 32, LR_ROWS = LR_T / 8;
 
 template <typename T, int RPT>
@@ -31,12 +31,23 @@ __global__ void __launch_bounds__(LR_T) lightning_recur_kernel(MemoryArgs a) {
     const int col = c0 + (tid & 7) * 4, cols = min(4, vdim - col);           // this thread's columns that exist
     const bool vec = cols == 4 && (vdim & 3) == 0;
     float* gs = a.state_s + ((size_t)(ok ? slot : 0) * s.heads + h) * dim * vdim + col;
+    const bool held = ok && pos0 > 0;
+    if (held && (tid & 7) == 0)
+#pragma unroll
+        for (int i = 0; i < RPT; ++i)
+            if (row0 + i * LR_ROWS < dim) prefetch_l2(gs + (size_t)(row0 + i * LR_ROWS) * vdim);
+    const float decay = a.powers[(size_t)h * SCR_DECAY_POWERS + 1], rest = a.powers[(size_t)h * SCR_DECAY_POWERS + SCR_DECAY_POWERS - 1];
+    pdl_wait();
+    if (!ok) {
+        if (count > 0 && tid == 0) atomicCAS(a.status, 0, SEQ_BAD_SLOT);
+        return;
+    }
     float4 S[RPT];
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
         const int r = row0 + i * LR_ROWS;
         S[i] = make_float4(0, 0, 0, 0);
-        if (ok && pos0 > 0 && r < dim) {
+        if (held && r < dim) {
             const float* p = gs + (size_t)r * vdim;
             if (vec) S[i] = *reinterpret_cast<const float4*>(p);
             else {
@@ -46,12 +57,6 @@ __global__ void __launch_bounds__(LR_T) lightning_recur_kernel(MemoryArgs a) {
                 if (cols > 3) S[i].w = p[3];
             }
         }
-    }
-    const float decay = a.powers[(size_t)h * SCR_DECAY_POWERS + 1], rest = a.powers[(size_t)h * SCR_DECAY_POWERS + SCR_DECAY_POWERS - 1];
-    pdl_wait();
-    if (!ok) {
-        if (count > 0 && tid == 0) atomicCAS(a.status, 0, SEQ_BAD_SLOT);
-        return;
     }
     float q[RPT], k[RPT], v[4];
     auto fetch = [&](int t) {

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from tests import seq_util as su
+from tests.test_side_ops_gpu import per_head, plain_lightning, run_lightning
 from tests.test_sequence_ops_gpu import DTYPES, dev, draw_memory, healthy, head_rows, lib, plain_memory, ptr, run_memory, stream, torch_
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +66,38 @@ def test_gated_memory(heads, dim, vdim, portions, dtype, captured):
     assert np.array_equal(got, want.astype(np.float32))
     err = np.sqrt(((head_rows(got, heads) - head_rows(plain_memory(m, proj, gates, bi, bf), heads)) ** 2).mean(axis=2)).ravel()
     assert np.median(err) < (5e-6 if dtype == "float32" else 5e-5)        # (the bar of the calls with a synchronisation after each)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 16, 24), (3, 48, 72), (8, 128, 128), (1, 256, 64), (1, 300, 20)])
+@pytest.mark.parametrize("portions", PORTIONS)
+def test_decaying_memory(heads, dim, vdim, portions, dtype, captured):
+    from scratchy_b200 import _lib
+    from scratchy_b200.dense import dtype_code
+    from scratchy_b200.mixers import decay_powers
+    torch = torch_()
+    L, c = lib()
+    m = {"heads": heads, "dim": dim, "vdim": vdim, "decay": ([0.999, 0.6, 0.97] * 3)[:heads]}
+    rng = np.random.default_rng(heads * dim + vdim)
+    T = sum(portions)
+    proj = rng.standard_normal((T, heads * (2 * dim + vdim))).astype(np.float32)
+    proj = su.round_bf16(proj) if dtype == "bfloat16" else proj
+    (want,), _ = run_lightning(m, dtype, [proj], [[n] for n in portions], [1])
+    shape, powers = _lib.LightningShape(heads, dim, vdim, 1e-5, 1.0), decay_powers(np.asarray(m["decay"], np.float64)).cuda()
+    state, pd, out = torch.full((2, heads, dim, vdim), float("nan"), device="cuda"), dev(proj, dtype), torch.full((T, heads * vdim), float("nan"), device="cuda")
+    code, calls, keep, at = dtype_code(pd.dtype), [], [], 0
+    for n in portions:
+        segs = torch.tensor([[0, n, at, 1]], dtype=torch.int32, device="cuda")
+        st, need = _lib.Step(0, 0, segs.data_ptr(), 0, n, 1, n, 0, 2), ctypes.c_size_t(0)
+        c.check(L.scr_lightning_workspace(code, ctypes.byref(shape), ctypes.byref(st), ctypes.byref(need)))
+        ws = torch.full((max(16, need.value) // 4,), float("nan"), device="cuda")
+        keep.append((segs, st, ws))
+        calls.append(lambda n=n, at=at, st=st, ws=ws, need=need: c.check(L.scr_lightning_run(
+            c.handle, code, ctypes.byref(shape), ctypes.byref(st), ptr(pd, at * pd.shape[1]), pd.shape[1], ptr(powers), ptr(state),
+            ptr(out, at * out.shape[1]), ptr(ws), need, stream())))
+        at += n
+    queued(calls, captured)
+    got = out.cpu().numpy()
+    assert np.array_equal(got, want.astype(np.float32))
+    assert per_head(got, plain_lightning(m, proj), heads) < (4e-6 if dtype == "float32" else 1e-4)
