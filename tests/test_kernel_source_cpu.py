@@ -1,0 +1,51 @@
+"""Rules of the hardware that no result shows reliably, checked on the kernels' source: each would be undefined behaviour or a
+hang that depends on what else is resident."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "scratchy_b200", "csrc")
+
+
+def sources():
+    out = {}
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, name)) as f:
+                out[name] = re.sub(r"//[^\n]*", "", f.read())
+    return out
+
+
+def block(text, start):
+    """The braces' content that opens first from `start` on."""
+    lo = at = text.index("{", start)
+    depth = 0
+    while True:
+        depth += {"{": 1, "}": -1}.get(text[at], 0)
+        at += 1
+        if depth == 0:
+            return text[lo:at]
+
+
+def kernels():
+    """(file, name, body, the device functions of the repository that it calls, asm text included)"""
+    texts = sources()
+    functions = {}
+    for text in texts.values():
+        for m in re.finditer(r"__device__ __forceinline__ [\w:<> ]+?[ *&](\w+)\(", text):
+            functions.setdefault(m.group(1), []).append(block(text, m.end()))
+    for name, text in texts.items():
+        for m in re.finditer(r"__global__[^;{]*?\b(\w+_kernel)\(", text):
+            body = block(text, m.end())
+            called = "".join(f for n in sorted(set(re.findall(r"\b(\w+)\(", body))) for f in functions.get(n, []))
+            yield name, m.group(1), body, body + called
+
+
+def test_a_kernel_names_one_cta_group():
+    """All tcgen05 instructions of a kernel have the same cta_group: a pair's MMAs go with a pair's allocation."""
+    seen = {}
+    for _, kernel, _, text in kernels():
+        groups = set(re.findall(r"tcgen05\.(?:alloc|dealloc|relinquish_alloc_permit|mma|commit|cp)\.[^\"]*?cta_group::(\d)", text))
+        if groups:
+            seen[kernel] = groups
+    assert {k for k, g in seen.items() if g == {"2"}} == {"affine_b4_gemm_pair_kernel", "fp8_gemm_pair_kernel", "dense_gemm_pair_kernel"}
+    assert len(seen) >= 8 and all(len(g) == 1 for g in seen.values()), seen
