@@ -133,6 +133,7 @@ affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const uint
         tmem_alloc_pair(smem_u32((const void*)tmem_slot), 2 * A4P_BN);    // the pair's columns: the same in both CTAs
         tmem_relinquish_pair();
     }
+    __syncwarp();
     tc_fence_before();
     a4p_pair_sync();                                      // both CTAs' barriers and TMEM exist before anything crosses over
     tc_fence_after();
@@ -346,6 +347,7 @@ affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const uint
         }
     }
 
+    __syncwarp();                                         // single lanes come out of the roles above; the barrier is the whole warp's
     tc_fence_before();
     a4p_pair_sync();                                      // nobody frees TMEM or leaves while the other may still signal it
     if (warp == 1) {

@@ -406,6 +406,7 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_c
         tmem_alloc_pair(smem_u32((const void*)tmem_slot), 2 * DP_BN);
         tmem_relinquish_pair();
     }
+    __syncwarp();
     tc_fence_before();
     dp_pair_sync();                                    // both CTAs' barriers and TMEM exist before anything crosses over
     tc_fence_after();
@@ -487,6 +488,7 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_c
             else asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(dp_map(acce_bar(buf), 0)) : "memory");
         }
     }
+    __syncwarp();                                         // single lanes come out of the roles above; the barrier is the whole warp's
     tc_fence_before();
     dp_pair_sync();                                    // nobody frees TMEM or leaves while the other may still signal it
     if (warp == 1) {

@@ -115,6 +115,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_con
         tmem_alloc_pair(smem_u32((const void*)tmem_slot), 2 * F8P_BN);     // the pair's columns: the same in both CTAs
         tmem_relinquish_pair();
     }
+    __syncwarp();
     tc_fence_before();
     pair_sync();                                          // both CTAs' barriers and TMEM exist before anything crosses over
     tc_fence_after();
@@ -258,6 +259,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_con
         }
     }
 
+    __syncwarp();                                         // single lanes come out of the roles above; the barrier is the whole warp's
     tc_fence_before();
     pair_sync();                                          // nobody frees TMEM or leaves while the other may still signal it
     if (warp == 1) {

@@ -49,3 +49,24 @@ def test_a_kernel_names_one_cta_group():
             seen[kernel] = groups
     assert {k for k, g in seen.items() if g == {"2"}} == {"affine_b4_gemm_pair_kernel", "fp8_gemm_pair_kernel", "dense_gemm_pair_kernel"}
     assert len(seen) >= 8 and all(len(g) == 1 for g in seen.values()), seen
+
+
+def test_warps_are_whole_at_aligned_barriers():
+    """`barrier.cluster.*.aligned` and tcgen05's `.sync.aligned` forms are executed by a whole warp: where single lanes had roles
+    of their own before, a __syncwarp, or a barrier of the CTA, comes first."""
+    texts = sources()
+    syncs = {m.group(1) for t in texts.values() for m in re.finditer(r"(\w+)\(\) \{\s*asm volatile\(\"barrier\.cluster\.arrive\.release\.aligned", t)}
+    assert len(syncs) >= 6
+    checked = 0
+    for file, kernel, body, _ in kernels():
+        lone = [m.end() for m in re.finditer(r"if \((?:\(?threadIdx\.x == 0|lane [=<]=? ?\w+|lane == 0 && \w+ == 0)\)", body)]
+        calls = [m.start() for s in syncs for m in re.finditer(rf"\b{s}\(\)", body)] + [m.start() for m in re.finditer(r"\bskinny_finish\(", body)]
+        for at in calls:
+            before = [p for p in lone if p < at]
+            if not before:
+                continue
+            # the nearest convergence before the barrier, past the last role of a single lane
+            gap = body[before[-1]:at]
+            assert re.search(r"__syncwarp\(\)|__syncthreads\(\)|bar\.sync", gap), (file, kernel, body[at - 200:at])
+            checked += 1
+    assert checked >= 6
