@@ -79,7 +79,6 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     }
     const int nmax = max(n[0], n[1]);
 
-    pdl_trigger();
     if (threadIdx.x == 0) {
         mbar_init(q_full(), 1);
         for (int s = 0; s < 3; ++s) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 1); mbar_init(v_full(s), 1); mbar_init(v_empty(s), 1); }
@@ -94,6 +93,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_trigger();                                     // not before this CTA has its TMEM: the next kernel's CTAs could take it first
     auto s_col = [&](int t) { return tmem + 256u * t; };
     auto ph_col = [&](int t) { return tmem + 256u * t + 64u; };
     auto pl_col = [&](int t) { return tmem + 256u * t + 96u; };

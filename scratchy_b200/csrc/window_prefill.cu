@@ -78,8 +78,8 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     const int head = blockIdx.x, q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * 256, b = blockIdx.z;      // the longest first
     const int first = a.st.segs[b * 4], count = a.st.segs[b * 4 + 1], pos0 = a.st.segs[b * 4 + 2];
 
-    pdl_trigger();
     if (q0 >= count || first < 0 || first + count > a.st.rows) {
+        pdl_trigger();
         pdl_wait();
         return;
     }
@@ -119,6 +119,7 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_trigger();                                           // not before this CTA has its TMEM: the next kernel's CTAs could take it first
     auto s_col = [&](int t, int i) { return tmem + 256u * t + 64u * (i & 1); };        // S, then P: 32 columns of heads, 32 of remainders
     auto o_col = [&](int t) { return tmem + 256u * t + 128u; };
     pdl_wait();

@@ -70,3 +70,18 @@ def test_warps_are_whole_at_aligned_barriers():
             assert re.search(r"__syncwarp\(\)|__syncthreads\(\)|bar\.sync", gap), (file, kernel, body[at - 200:at])
             checked += 1
     assert checked >= 6
+
+
+def test_dependents_start_after_the_tensor_memory_is_held():
+    """A CTA of the next kernel that takes TMEM first would wait for this kernel's end, and this kernel's CTA for that TMEM: a
+    kernel lets its dependents start only when the allocation is behind it (or on a way out that takes none)."""
+    checked = set()
+    for file, kernel, body, _ in kernels():
+        if "tmem_alloc" not in body:
+            continue
+        held = body.index("*tmem_slot")
+        for m in re.finditer(r"pdl_trigger\(\)|griddepcontrol\.launch_dependents", body):
+            leaves = re.match(r"[^{}]*\breturn;", body[m.end():])
+            assert m.start() > held or leaves, (file, kernel)
+            checked.add(kernel)
+    assert {"latent_prefill_kernel", "window_prefill_kernel", "dense_gemm_kernel", "dense_skinny_kernel", "affine_b4_skinny_kernel"} <= checked
