@@ -91,11 +91,17 @@ __global__ void __launch_bounds__(LM_THREADS) latent_attention_mma_kernel(scr_la
         const int row = i / (lay.ld - D), c = D + i % (lay.ld - D);
         (row < ROWS ? Q + (size_t)row * lay.ld : reinterpret_cast<bf16*>(lm_smem + lay.tile) + (size_t)(row - ROWS) * lay.ld)[c] = __float2bfloat16_rn(0.0f);
     }
-    // cache rows before this step's are there already: their tile does not wait for the preceding kernels
-    const bool early = t_lo < t_hi && (t_lo + 1) * LM_KEYS <= pos0;
-    if (early) load_tile(t_lo, look_up(t_lo));
+    // The first tile's rows start for L2 before the wait and are read after it: a preceding kernel may be the one that stores them
+    // (the call before this one's, of the token before).
+    const long long where_first = look_up(t_lo);
+    if ((t_lo + 1) * LM_KEYS <= pos0)
+#pragma unroll
+        for (int i = 0; i < RPW; ++i) {
+            const long long off = __shfl_sync(0xffffffffu, where_first, i);
+            if (off >= 0 && lane * 64 < D) prefetch_l2(cache + off + lane * 64);
+        }
     pdl_wait();
-    if (!early && t_lo < t_hi) load_tile(t_lo, look_up(t_lo));
+    if (t_lo < t_hi) load_tile(t_lo, where_first);
     long long where_next = look_up(t_lo + 1);
     for (int i = threadIdx.x; i < ROWS * chunks; i += LM_THREADS) {
         const int row = i / chunks, c = i - row * chunks;

@@ -20,10 +20,6 @@ struct MemoryArgs {
     const float* powers;                                   // constant decay: [heads][SCR_DECAY_POWERS], otherwise unused
 };
 
-// Asks for the line of `p` in L2, where all writes meet: allowed before the wait for the preceding kernels even where one of them
-// still writes it.
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
 __host__ __device__ __forceinline__ int mlstm_slices(int vdim) { return (vdim + SCR_MLSTM_SLICE - 1) / SCR_MLSTM_SLICE; }
 
 __device__ __forceinline__ float mlstm_cap(float z, float cap) { return cap * tanhf(z / cap); }

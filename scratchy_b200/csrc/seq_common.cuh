@@ -96,6 +96,10 @@ __device__ __forceinline__ float exp2_fast(float x) {
     return y;
 }
 
+// Asks for the line of `p` in L2, where all writes meet: allowed before the wait for the preceding kernels even where one of them
+// still writes it.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // 16 bytes global -> shared (zeros unless ok), in the background
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool ok) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");

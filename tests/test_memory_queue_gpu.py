@@ -7,7 +7,7 @@ import pytest
 
 from tests import seq_util as su
 from tests.test_side_ops_gpu import per_head, plain_lightning, run_lightning
-from tests.test_sequence_ops_gpu import DTYPES, dev, draw_memory, healthy, head_rows, lib, plain_memory, ptr, run_memory, stream, torch_
+from tests.test_sequence_ops_gpu import DTYPES, Latents, dev, draw_memory, healthy, head_rows, lib, plain_memory, ptr, run_memory, stream, torch_
 
 pytestmark = pytest.mark.gpu
 
@@ -101,3 +101,43 @@ def test_decaying_memory(heads, dim, vdim, portions, dtype, captured):
     got = out.cpu().numpy()
     assert np.array_equal(got, want.astype(np.float32))
     assert per_head(got, plain_lightning(m, proj), heads) < (4e-6 if dtype == "float32" else 1e-4)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("heads,kv_rank,rot_dim", [(3, 48, 8), (24, 512, 64)])
+@pytest.mark.parametrize("start,tokens", [(0, 3), (58, 12), (126, 6), (700, 8)])
+def test_latent_cache(start, tokens, heads, kv_rank, rot_dim, captured):
+    """A token's cache row stored by one call and read by the next ones, on both sides of a key tile's end."""
+    torch = torch_()
+    L, c = lib()
+    m = su.attention_spec(heads=heads, kv_rank=kv_rank, rot_dim=rot_dim, q_rank=32, scale=(kv_rank + rot_dim) ** -0.5)["mixer"]
+    from scratchy_b200 import _lib
+    results = []
+    for synchronised in (True, False):
+        lt = Latents(m, [start], [tokens], "bfloat16", seed=start + heads)          # (the same seed: the same cache, blocks and rows)
+        rng = np.random.default_rng(start)
+        lt.cache[lt.slots[0][start:]] = float("nan")                                # the calls below store these rows
+        d, q = dev(rng.standard_normal((tokens, 32 + lt.D))), dev(rng.standard_normal((tokens, heads, lt.D)), "bfloat16")
+        wq, wkv = dev(np.ones(32)), dev(np.ones(kv_rank))
+        cq, out = (torch.full((tokens, n), float("nan"), dtype=torch.bfloat16, device="cuda") for n in (32, heads * kv_rank))
+        calls, keep = [], []
+        for t in range(tokens):
+            i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+            arrays = [i32(0), i32(start + t), i32(0, 1, start + t, 0)]
+            st = _lib.Step(*[a.data_ptr() for a in arrays], lt.dev_arrays[3].data_ptr(), 1, 1, 1, start + t + 1, 1)
+            need = ctypes.c_size_t(0)
+            c.check(L.scr_latent_attention_workspace(lt.code(), ctypes.byref(lt.shape), ctypes.byref(st), ctypes.byref(need)))
+            ws = torch.empty(max(16, need.value), dtype=torch.uint8, device="cuda")
+            keep.append((arrays, st, ws))
+
+            def call(t=t, st=st, ws=ws, need=need):
+                c.check(L.scr_latent_prepare(c.handle, lt.code(), ctypes.byref(lt.shape), ctypes.byref(st), ptr(d, t * d.shape[1]), d.shape[1], ptr(wq), ptr(wkv),
+                                             ptr(lt.cos), ptr(lt.sin), ptr(cq, t * 32), ptr(lt.cache), stream()))
+                c.check(L.scr_latent_attention(c.handle, lt.code(), ctypes.byref(lt.shape), ctypes.byref(st), ptr(q, t * heads * lt.D), ptr(lt.cache),
+                                               ptr(out, t * heads * kv_rank), ptr(ws), need, stream()))
+                if synchronised:
+                    torch.cuda.synchronize()
+            calls.append(call)
+        queued(calls, captured and not synchronised)
+        results.append(out.float().cpu().numpy())
+    assert np.isfinite(results[0]).all() and np.array_equal(*results)
