@@ -1,0 +1,53 @@
+// How a decode attention launch is laid out (decode_ops.cu); plain C++, so that the choice can be looked at without a GPU.
+#pragma once
+
+#include <stddef.h>
+
+#include <initializer_list>
+
+constexpr int ATT_SPLITS = 8;                          // CTAs of a cluster at most
+constexpr int ATT_MAX_STAGES = 24;
+// Bytes of dynamic shared memory one CTA may take so that two CTAs fit on an SM; alone on its SM.
+constexpr size_t ATT_SMEM_BUDGET = 110 * 1024;
+constexpr size_t ATT_SMEM_BUDGET_ALONE = 200 * 1024;
+
+struct AttPlan {
+    int nsplit;                                        // CTAs that share a sequence and kv head
+    int warps, stages_per_warp;                        // of the streaming kernel; no stages: the blocks do not fit it
+    int table_cap;                                     // block ids a CTA holds
+    size_t fixed;                                      // shared memory beside the ring
+};
+
+static inline AttPlan att_plan(int D, int G, int batch, int num_kv_heads, int block_size, int max_blocks_per_seq, int sm_count) {
+    AttPlan p;
+    const size_t chunk = size_t(block_size) * D * 2;
+    const size_t part = size_t(ATT_SPLITS) * G * (D + 2) * sizeof(float);
+    p.nsplit = ATT_SPLITS;                             // the most splits that still run as a single wave of two CTAs per SM
+    while (p.nsplit > 1 && (long long)batch * num_kv_heads * p.nsplit > 2LL * sm_count) p.nsplit /= 2;
+    // ... but not below two for long sequences: a CTA per sequence and kv head lasts as long as the longest of them while SMs that
+    // held shorter ones idle (20 sequences of 750 to 3000 tokens 53.8 us, halved 37.4; 32 of 500 to 2000 41.1 and 38.2; 32 of 250
+    // to 1000 20.0 and 26.9)
+    if (p.nsplit == 1 && (long long)max_blocks_per_seq * block_size >= 1536) p.nsplit = 2;
+    p.table_cap = max_blocks_per_seq / p.nsplit + 2;
+    p.fixed = part + size_t((p.table_cap + 1) & ~1) * 4 + ATT_MAX_STAGES * 8 + 1024 + 128;
+    // alone on its SM: 8 warps and a deep ring; otherwise 4 or 6 warps and about half an SM's shared
+    // memory.  The big CTA (48 K registers, ~200 KB) shares its SM with no CTA of the kernels before and after it in
+    // the stream, so it pays only while the grid leaves most SMs to them: up to half the SMs.  (Llama-3.2-3B decode
+    // step, measured inside the step: batch 1, 64 CTAs — 1.074 ms with the big CTA, 1.116 with the small one; batch 2,
+    // 128 CTAs — 1.341 ms with the big one, 1.193 with the small one.)  Every warp owns stages / warps ring stages
+    // and wants at least two of them, so that its next block loads while it works on the current one.
+    const bool alone = 2LL * batch * num_kv_heads * p.nsplit <= sm_count;
+    const size_t budget = alone ? ATT_SMEM_BUDGET_ALONE : ATT_SMEM_BUDGET;
+    // Six warps of two stages where a CTA has four blocks or more for each and they fit (the table of the cluster's sums grows with
+    // the query heads: beside it, 16-token blocks of 128 leave room for six up to 3 query heads per kv head), otherwise four of three
+    // (16 sequences of up to 2048 tokens 23.9 us with four warps, 20.8 with six; 4 sequences, 16 blocks a CTA, 13.0 and 14.6).
+    // Large blocks: two, with one stage each if it must be.
+    const int most = alone ? 8 : max_blocks_per_seq / p.nsplit >= 24 ? 6 : 4;
+    for (int w : {most, 4, 2}) {
+        const size_t fit = budget > p.fixed ? (budget - p.fixed) / (2 * chunk * w) : 0;
+        p.warps = w;
+        p.stages_per_warp = fit < 3 ? int(fit) : 3;
+        if (p.stages_per_warp >= 2) break;
+    }
+    return p;
+}

@@ -13,6 +13,7 @@
 // (fused_gate_up_silu_mul), :289-362 (rope_append), :386-460 (attention_via_cache); cache
 // addressing crates/targets/metal/src/paged_kv_layout.rs:74-115; argmax tie rule
 // crates/targets/metal/tests/argmax_split_test.rs:24-33.
+#include "attention_plan.h"
 #include "tc_common.cuh"
 
 #include <math.h>
@@ -293,7 +294,6 @@ __global__ void __launch_bounds__(ARGMAX_THREADS) argmax_kernel(const uint16_t* 
 // cluster; CTA 0 of the cluster applies inv_sum = 1 / (l + 1e-6) and stores bf16.
 constexpr int ATT_THREADS = 256;
 constexpr int ATT_WARPS = ATT_THREADS / 32;
-constexpr int ATT_SPLITS = 8;
 constexpr uint32_t ATT_NO_BLOCK = 0xFFFFFFFFu;
 
 __device__ __forceinline__ uint32_t att_cluster_rank() {
@@ -878,11 +878,6 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_tc_kernel(
     }
 }
 
-// Bytes of dynamic shared memory one CTA may take so that two CTAs fit on an SM.
-constexpr size_t ATT_SMEM_BUDGET = 110 * 1024;
-constexpr size_t ATT_SMEM_BUDGET_ALONE = 200 * 1024;
-constexpr int ATT_MAX_STAGES = 24;
-
 template <int D, int G>
 cudaError_t attention_launch(const uint16_t* q, long long ld_q, const uint16_t* cache_k, const uint16_t* cache_v,
                              const uint32_t* block_table, const uint32_t* seq_used_k, uint16_t* out, long long ld_o, int batch,
@@ -899,43 +894,18 @@ cudaError_t attention_launch(const uint16_t* q, long long ld_q, const uint16_t* 
     cfg.numAttrs = 2;
     cfg.stream = stream;
 
-    // streaming variant: blocks of a multiple of 16 tokens (one TMA box, 16-token MMA tiles), two ring stages in the budget
+    // streaming variant: blocks of a multiple of 16 tokens (one TMA box, 16-token MMA tiles)
     const size_t chunk = size_t(block_size) * D * 2;
     const size_t part = size_t(ATT_SPLITS) * G * (D + 2) * sizeof(float);
     const size_t warp_part = size_t(ATT_WARPS) * G * (D + 2) * sizeof(float);
-    int nsplit = ATT_SPLITS;                         // the most splits that still run as a single wave of two CTAs per SM
-    while (nsplit > 1 && (long long)batch * num_kv_heads * nsplit > 2LL * sm_count) nsplit /= 2;
-    // ... but not below two for long sequences: a CTA per sequence and kv head lasts as long as the longest of them while SMs that
-    // held shorter ones idle (20 sequences of 750 to 3000 tokens 53.8 us, halved 37.4; 32 of 500 to 2000 41.1 and 38.2; 32 of 250
-    // to 1000 20.0 and 26.9)
-    if (nsplit == 1 && (long long)max_blocks_per_seq * block_size >= 1536) nsplit = 2;
-    const int table_cap = max_blocks_per_seq / nsplit + 2;
-    const size_t fixed = part + size_t((table_cap + 1) & ~1) * 4 + ATT_MAX_STAGES * sizeof(uint64_t) + 1024 + 128;
-    // alone on its SM: 8 warps and a deep ring; otherwise 4 or 6 warps and about half an SM's shared
-    // memory.  The big CTA (48 K registers, ~200 KB) shares its SM with no CTA of the kernels before and after it in
-    // the stream, so it pays only while the grid leaves most SMs to them: up to half the SMs.  (Llama-3.2-3B decode
-    // step, measured inside the step: batch 1, 64 CTAs — 1.074 ms with the big CTA, 1.116 with the small one; batch 2,
-    // 128 CTAs — 1.341 ms with the big one, 1.193 with the small one.)  Every warp owns stages / warps ring stages
-    // and wants at least two of them, so that its next block loads while it works on the current one.
-    const bool alone = 2LL * batch * num_kv_heads * nsplit <= sm_count;
-    const size_t budget = alone ? ATT_SMEM_BUDGET_ALONE : ATT_SMEM_BUDGET;
-    // Six warps of two stages where a CTA has four blocks or more for each, otherwise four of three (16 sequences of up to 2048
-    // tokens 23.9 us with four warps, 20.8 with six; 4 sequences, 16 blocks a CTA, 13.0 and 14.6).
-    int nwarps = alone ? 8 : max_blocks_per_seq / nsplit >= 24 ? 6 : 4, spw = 0;
-    for (; nwarps >= 2; nwarps /= 2) {
-        spw = budget > fixed ? int(std::min<size_t>(3, (budget - fixed) / (2 * chunk * nwarps))) : 0;
-        if (spw >= 2) break;
-    }
-    if (spw < 2) {                                   // large blocks: settle for one stage per warp if that fits
-        nwarps = 2;
-        spw = budget > fixed ? int(std::min<size_t>(3, (budget - fixed) / (2 * chunk * nwarps))) : 0;
-    }
+    const AttPlan plan = att_plan(D, G, batch, num_kv_heads, block_size, max_blocks_per_seq, sm_count);
+    const int nsplit = plan.nsplit, nwarps = plan.warps, spw = plan.stages_per_warp, table_cap = plan.table_cap;
     const unsigned long long total_tokens = (unsigned long long)num_blocks * num_kv_heads * block_size;
     tc_encode_tiled_fn enc = tc_tensor_map_encoder();
     if (enc && block_size % 16 == 0 && block_size <= 256 && total_tokens < (1ull << 31) && spw >= 1) {
         const int stages = spw * nwarps;
         const size_t ring = std::max(size_t(stages) * 2 * chunk, size_t(nwarps) * G * (D + 2) * sizeof(float));
-        const size_t smem = ((ring + 127) & ~size_t(127)) + fixed;
+        const size_t smem = ((ring + 127) & ~size_t(127)) + plan.fixed;
         CUtensorMap maps[2];
         const cuuint64_t dims[3] = {64, cuuint64_t(D / 64), cuuint64_t(total_tokens)};
         const cuuint64_t strides[2] = {128, cuuint64_t(D) * 2};

@@ -1,0 +1,40 @@
+"""How a decode attention launch is laid out (scratchy_b200/csrc/attention_plan.h), compiled for the host."""
+import ctypes
+import os
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "scratchy_b200", "csrc")
+SMS = 148
+
+
+@pytest.fixture(scope="module")
+def plan(tmp_path_factory):
+    folder = tmp_path_factory.mktemp("plan")
+    source, library = folder / "plan.cpp", folder / "plan.so"
+    source.write_text('#include "attention_plan.h"\nextern "C" AttPlan plan(int d, int g, int b, int h, int bs, int mb) '
+                      f'{{ return att_plan(d, g, b, h, bs, mb, {SMS}); }}\n')
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, "-o", library, source], check=True)
+
+    class Plan(ctypes.Structure):
+        _fields_ = [(n, ctypes.c_int) for n in ("nsplit", "warps", "stages", "table_cap")] + [("fixed", ctypes.c_size_t)]
+    call = ctypes.CDLL(str(library)).plan
+    call.restype = Plan
+    return lambda d, g, batch, heads, block, blocks: call(d, g, batch, heads, block, blocks)
+
+
+@pytest.mark.parametrize("d,block", [(128, 16), (64, 16), (128, 32), (128, 48), (64, 64), (128, 128)])
+@pytest.mark.parametrize("g", range(1, 9))
+@pytest.mark.parametrize("batch,heads", [(1, 8), (2, 8), (16, 8), (32, 8), (20, 4), (64, 8)])
+def test_as_many_warps_as_fit(plan, d, block, g, batch, heads):
+    """No smaller number of warps than another that has its two stages each in the same shared memory."""
+    for tokens in (block, 640, 1040, 2048, 4112, 16384):
+        p = plan(d, g, batch, heads, block, -(-tokens // block))
+        alone = 2 * batch * heads * p.nsplit <= SMS
+        room = (200 if alone else 110) * 1024 - p.fixed
+        two = lambda warps: 4 * (block * d * 2) * warps <= room
+        assert p.warps in ((8, 4, 2) if alone else (6, 4, 2)) and p.stages <= 3
+        assert p.warps * p.stages * 2 * block * d * 2 <= room
+        assert p.warps >= 4 or not two(4), (tokens, p.warps)
+        assert p.stages >= 2 or not two(2)

@@ -69,3 +69,9 @@ def test_decode_attention_at_every_cut_and_number_of_warps(longest, hq, hkv, d, 
     lens = [longest, 1, bs, bs + 1] + rng.integers(1, longest + 1, batch - 4).tolist()
     got, want = _attention_case(lens, hq, hkv, d, bs, synth.seed_for("cut", longest, hq, hkv, d, bs))
     assert rel_l2(got, want) <= REL_L2_TOL
+
+
+@pytest.mark.parametrize("longest,hq,hkv,d,bs,batch", [(1000, 16, 4, 128, 16, 24), (1700, 28, 4, 128, 16, 20), (4500, 16, 2, 128, 16, 9), (1000, 8, 4, 128, 48, 20)])
+def test_decode_attention_with_warps_that_do_not_all_fit(longest, hq, hkv, d, bs, batch):
+    """Four or two warps where the query heads, the table or the blocks leave no room for six."""
+    test_decode_attention_at_every_cut_and_number_of_warps(longest, hq, hkv, d, bs, batch)
