@@ -24,10 +24,9 @@ static inline AttPlan att_plan(int D, int G, int batch, int num_kv_heads, int bl
     const size_t part = size_t(ATT_SPLITS) * G * (D + 2) * sizeof(float);
     p.nsplit = ATT_SPLITS;                             // the most splits that still run as a single wave of two CTAs per SM
     while (p.nsplit > 1 && (long long)batch * num_kv_heads * p.nsplit > 2LL * sm_count) p.nsplit /= 2;
-    // ... but not below two for long sequences: a CTA per sequence and kv head lasts as long as the longest of them while SMs that
-    // held shorter ones idle (20 sequences of 750 to 3000 tokens 53.8 us, halved 37.4; 32 of 500 to 2000 41.1 and 38.2; 32 of 250
-    // to 1000 20.0 and 26.9)
-    if (p.nsplit == 1 && (long long)max_blocks_per_seq * block_size >= 1536) p.nsplit = 2;
+    // (Halving sequences for the width of their table, so that none is waited for alone, was measured and is not done: the width is a
+    // capacity and not a length, and clusters of two start later.  32 sequences of 500 to 2048 tokens, in a stream of such calls, 39.7 us
+    // whole and 41.1 halved, of 250 to 1000 in a table of 2048 21.6 and 33.2; 20 of 500 to 2048 36.9 and 30.2.)
     p.table_cap = max_blocks_per_seq / p.nsplit + 2;
     p.fixed = part + size_t((p.table_cap + 1) & ~1) * 4 + ATT_MAX_STAGES * 8 + 1024 + 128;
     // alone on its SM: 8 warps and a deep ring; otherwise 4 or 6 warps and about half an SM's shared

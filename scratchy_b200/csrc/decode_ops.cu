@@ -566,8 +566,8 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_kernel(
 // blocks.  Every wait is bounded and reports through the status word.
 //
 // What bounds it: HBM (8 KB per block of 16 tokens and kv head), and the longest sequence's CTA.  Llama-3.2-3B at 32 sequences of
-// 512 to 2048 tokens, 153 MB per layer: 60 us with the producer warp and a second MMA for the remainders, 41 us with rings of
-// the warps' own, 38 us (4.0 TB/s) with the cut and the warps chosen as in `attention_launch`.
+// 512 to 2048 tokens, 153 MB per call, in a stream of calls: 57.6 us with the producer warp and a second MMA for the remainders,
+// 39.7 us (3.9 TB/s) with rings of the warps' own and their number as in attention_plan.h.
 constexpr int ATT_ERR_FULL = 0x0A000001;
 
 __device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const CUtensorMap* tmap, int c0, int c1, int c2, uint32_t bar) {

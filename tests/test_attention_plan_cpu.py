@@ -38,3 +38,13 @@ def test_as_many_warps_as_fit(plan, d, block, g, batch, heads):
         assert p.warps * p.stages * 2 * block * d * 2 <= room
         assert p.warps >= 4 or not two(4), (tokens, p.warps)
         assert p.stages >= 2 or not two(2)
+
+
+@pytest.mark.parametrize("block", [16, 32, 48, 256])
+def test_the_width_of_the_table_cuts_no_sequence(plan, block):
+    """The table's width is a capacity (a server captures its step once): the cut follows the number of sequences alone."""
+    for batch in range(1, 130):
+        fits = [n for n in (8, 4, 2, 1) if batch * 8 * n <= 2 * SMS or n == 1][0]
+        for tokens in (256, 1024, 1536, 2048, 5000, 32768):
+            p = plan(128, 3, batch, 8, block, -(-tokens // block))
+            assert p.nsplit == fits and p.table_cap >= -(-(-(-tokens // block)) // fits)
