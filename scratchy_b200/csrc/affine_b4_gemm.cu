@@ -29,7 +29,7 @@
 
 bool affine_b4_gemm_tc_enabled() { return true; }
 // Defined in affine_b4_gemm_pair.cu
-float affine_b4_gemm_pair_us(int M, int N, int K, int sms);
+bool affine_b4_gemm_pair_applies(int M, int N, int K, int sms);
 int32_t affine_b4_gemm_pair_launch(scr_ctx* ctx, const CUtensorMap& x_map, const uint8_t* packed, uint16_t* y, int M, int N, int K,
                                    int gs, int out_f32, const uint16_t* bias, cudaStream_t stream, bool* launched);
 // Defined in affine_b4_skinny.cu
@@ -383,9 +383,7 @@ int32_t affine_b4_gemm_tc_launch(scr_ctx* ctx, const uint8_t* packed, const uint
     if (!enc) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled entry point not available");
     CUtensorMap map;
     const AffineGemmPlan plan = affine_gemm_plan(M, N, K, ctx->sm_count);
-    // Pairs (affine_b4_gemm_pair.cu) where their rounds come out clearly shorter: 2048 tokens of 3072 -> 16384 166 us against 205;
-    // 2048 of 3072 -> 8192, estimates 2 % apart, 110 against 107.
-    if (affine_b4_gemm_pair_us(M, N, K, ctx->sm_count) < 0.9f * plan.us) {
+    if (affine_b4_gemm_pair_applies(M, N, K, ctx->sm_count)) {
         bool launched = false;
         if (!affine_gemm_x_map(&map, enc, x, M, K, 128)) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled failed");
         const int32_t st = affine_b4_gemm_pair_launch(ctx, map, packed, y, M, N, K, gs, out_f32, bias, stream, &launched);

@@ -2,22 +2,20 @@
 //
 //   y[m,n] = bf16( sum_k x[m,k] * w[n,k] (+ bias[n]) ),  w = the bit-exact bf16 dequantisation of the codes
 //
-// Why a pair.  The one-CTA kernel (affine_b4_gemm.cu: 256 tokens x 128 channels per CTA) pulls 64 KB of activations per
-// 128-k chunk for 256 x 128 x 128 MACs, about what one SM can take from L2 at the rate the tensor core wants them, and
-// its two 32 KB stages of dequantised weights are too shallow for the dequantise -> MMA hand-off: an instrumented build
-// showed the MMA thread waiting 430 cycles per chunk for activations and 375 for dequantised weights beside 1040 of MMA.
+// Why a pair.  One CTA that takes a tile of 256 tokens x 128 channels with its dequantised weights in shared memory pulls 64 KB of
+// activations per 128-k chunk for 256 x 128 x 128 MACs, about what one SM can take from L2 at the rate the tensor core wants
+// them, and two 32 KB stages of weights, all that fits, are too shallow for the dequantise -> MMA hand-off: an instrumented
+// build showed the MMA thread waiting 430 cycles per chunk for activations and 375 for weights beside 1040 of MMA.
 // In a pair each CTA loads the activations of ITS 128 tokens (32 KB per chunk) and dequantises ITS 128 of the tile's 256
 // channels; one `tcgen05.mma.cta_group::2` of shape 256 x 256 x 16, issued by the pair's leader CTA, reads the token rows
 // and the channel rows from both SMs' shared memory and leaves each CTA's 128 accumulator rows in that CTA's own TMEM.
 // Same MACs and the same dequantise work per SM and chunk, 44 % less L2 traffic, and room for three stages of each ring.
-// What bounds it: the shared-memory data pipe (operand reads, dequantised tile, activations), near the MMAs' own rate.  2048 tokens of
-// 3072 -> 16384: 166 us (1243 TFLOP/s) against 205 us on one CTA per tile with the weights in TMEM; issued from a divergent thread
-// the MMAs had held it to the one-CTA kernel's speed.
+// Measured: the same bits as the one-CTA kernel at its speed or below (see `affine_b4_gemm_pair_applies`), so it is opt-in.
 //
 // Per CTA (704 threads), both CTAs of a pair run the same code:
 //   warp 0       producer: per chunk 2 tiled TMA loads of this CTA's activations (`.cta_group::2`, completing on the
 //                LEADER's barrier; no multicast) and 8 bulk copies of this CTA's packed weight blocks
-//   warp 1       leader CTA only: one thread waits for both CTAs' activations and dequantised weights, issues 8 MMAs
+//   warp 1       leader CTA only: waits for both CTAs' activations and dequantised weights; one elected lane issues 8 MMAs
 //                (2 atoms of 64 k x 4 steps of K = 16) and commits to the stages' `empty` barriers of both CTAs
 //   warps 2-17   dequantise this CTA's 128 channels into the K-major 128-byte-swizzled operand image; lane 0 of each warp
 //                arrives on the leader's `dfull` barrier (the peer's warps with a remote arrive)
@@ -359,18 +357,22 @@ affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const uint
 }  // namespace
 
 
-// What this GEMM would take on pairs, in us (rounds of 256 x 256 tiles at 1.02 us per 128-k chunk, measured); more than anything
-// where it does not go there: whole 256-channel pair tiles only.  `SCR_AFFINE_GEMM_PAIR=0` in the environment switches the pair
-// kernel off (read once).
-float affine_b4_gemm_pair_us(int M, int N, int K, int sms) {
+// Whether the pair kernel takes this GEMM.  It is OFF unless `SCR_AFFINE_GEMM_PAIR=1` is in the environment (read once): the one-CTA
+// kernel is as fast or faster at every size measured (2048 tokens of 3072 -> 16384 169 us against 168, of 3072 -> 8192 84 against 95;
+// 1500 of 4096 -> 4096 43 against 65).  When on: whole 256-channel pair tiles, at least one full round of pairs, and rounds that
+// are at least 85 % full (the one-CTA kernel splits its tail along k instead).
+bool affine_b4_gemm_pair_applies(int M, int N, int K, int sms) {
     static const bool enabled = [] {
         const char* e = std::getenv("SCR_AFFINE_GEMM_PAIR");
-        return !(e && e[0] == '0');
+        return e && e[0] == '1';
     }();
+    if (!enabled) return false;
     const AffineGeom g = affine_geom(N, K, 64);
+    if ((g.RB % 16) != 0 || g.KC < 1 || M <= 128) return false;
     const int pairs = sms / 2, tiles = scr_ceil_div(M, 256) * (g.RB / 16);
-    if (!enabled || (g.RB % 16) != 0 || g.KC < 1 || M <= 128 || pairs < 1) return 1e30f;
-    return 1.02f * (float)g.KC * (float)scr_ceil_div(tiles, pairs);
+    if (pairs < 1 || tiles < pairs) return false;
+    const int rounds = (tiles + pairs - 1) / pairs;
+    return (float)tiles >= 0.85f * (float)(rounds * pairs);
 }
 
 int32_t affine_b4_gemm_pair_launch(scr_ctx* ctx, const CUtensorMap& x_map, const uint8_t* packed, uint16_t* y, int M, int N, int K,
