@@ -17,9 +17,10 @@
 // TMEM holds two accumulators of 192 columns (the epilogue of a tile overlaps the main loop of the next) and two stages of 64
 // columns of dequantised weights.  No multicast: every CTA issues its own loads.
 //
-// What bounds it: the MMAs themselves.  With A in TMEM one of 128 x N x 16 took about 110 + N / 2 cycles (measured: 125 at 32 columns,
-// 150 at 128, 195 at 192), so wide tiles pay, and 192 is what fits twice beside the stages: 1560 cycles per chunk.  128 tokens with
-// four stages took 1200 (a sixth slower per token), pairs of SMs (cta_group::2) 1900 per 256 channels.
+// What bounds it: a 128-k chunk takes about 1250 cycles, whether its MMAs have 128 columns or 192.  With two stages of dequantised weights
+// a chunk's way round (expansion, hand-over, eight MMAs, release) can be that bound as well as the MMAs with A in TMEM can; the
+// two have not been told apart.  Wide tiles pay, since a chunk is expanded once for all of a tile's tokens: 2048 tokens of 3072 -> 8192
+// 84 us (1.23 PFLOP/s) at 192, 104 us at 128.
 #include <cuda.h>
 
 #include <algorithm>
@@ -318,8 +319,9 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_
 }
 
 // ---- host --------------------------------------------------------------------------------
-// The tokens of a tile and how the tiles are cut into work units (tc_plan_units).  A 128-k chunk of a tile was measured at 0.65 us
-// for 128 tokens and 0.83 us for 192; the width whose rounds fill the GPU best wins.
+// The tokens of a tile and how the tiles are cut into work units (tc_plan_units).  A 128-k chunk takes about 0.655 us whatever the
+// width (3072 -> 3072 in one round 18.4 us at 144 to 192 tokens a tile, in two 32.5 at 128 and 33.7 at 192), and a tile's drain at
+// the end 6.5 ns a token; the width whose rounds fill the GPU best wins.
 struct AffineGemmPlan {
     int width, mt, tiles, full, ks_tail;
     float us;                                            // estimate
@@ -335,8 +337,8 @@ static AffineGemmPlan affine_gemm_plan(int M, int N, int K, int sms) {
         p.width = width;
         p.mt = scr_ceil_div(M, width);
         p.tiles = p.mt * (g.RB * 16 / A4G_BN);
-        const float us = 0.28f + 0.00286f * width;
-        p.us = tc_plan_units(p.tiles, g.KC, sms, us, &p.full, &p.ks_tail) * g.KC * us;
+        const float us = 0.655f;
+        p.us = tc_plan_units(p.tiles, g.KC, sms, us, &p.full, &p.ks_tail) * g.KC * us + 0.0065f * width;
         if (p.us < least * 0.99f) {
             least = p.us;
             best = p;
