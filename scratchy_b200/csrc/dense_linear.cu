@@ -1,8 +1,9 @@
 // Full-precision linears of the sequence models: y = x W^T with the ends of `scr_dense`.
 //
-//   M <= 16, bf16   dense_matvec_kernel   weights streamed once from HBM straight into mma.sync fragments (decode)
-//   M <= 128, bf16  dense_skinny.cu       tcgen05 GEMM, the weights as the rows of the MMA
-//   M > 128, bf16   dense_gemm.cu         tcgen05 GEMM
+//   M <= 16, bf16   dense_matvec_kernel   weights streamed once from HBM straight into mma.sync fragments (decode), unless
+//                                         each SM has much to stream
+//   M <= 128, bf16  dense_skinny.cu       tcgen05 GEMM, the weights as the rows of the MMA, unless W is wide for the rows
+//   other bf16      dense_gemm.cu         tcgen05 GEMM
 //   otherwise       dense_plain_kernel    f32 arithmetic on any sizes (the f32 data type; bf16 rows that are not a
 //                                         multiple of 16 bytes)
 #include "seq_common.cuh"
@@ -11,7 +12,7 @@
 
 size_t dense_gemm_workspace(int M, int N, int K, int groups);
 int32_t dense_gemm_launch(scr_ctx* ctx, const scr_dense& d, void* workspace, size_t workspace_bytes, cudaStream_t stream);
-bool dense_skinny_applies(int M);
+bool dense_skinny_applies(int M, int N, int K, int groups);
 int32_t dense_skinny_launch(scr_ctx* ctx, const scr_dense& d, cudaStream_t stream);
 
 namespace {
@@ -231,7 +232,7 @@ bool rows_of_16_bytes(const scr_dense& d) {
 extern "C" int32_t scr_dense_workspace_size(int32_t dtype, int32_t M, int32_t N, int32_t K, int32_t groups, size_t* bytes) {
     if (!bytes) return SCR_E_ARG;
     if (M <= 0 || N <= 0 || K <= 0 || groups <= 0) return SCR_E_SHAPE;
-    *bytes = (dtype == SCR_DTYPE_BF16 && !dense_skinny_applies(M)) ? dense_gemm_workspace(M, N, K, groups) : 0;
+    *bytes = (dtype == SCR_DTYPE_BF16 && !dense_skinny_applies(M, N, K, groups)) ? dense_gemm_workspace(M, N, K, groups) : 0;
     return SCR_OK;
 }
 
@@ -263,6 +264,6 @@ extern "C" int32_t scr_dense_linear(scr_ctx* ctx, int32_t dtype, const scr_dense
     // against 12.3 us, 183 MB of 29720 x 3072: 41.0 against 31.6, 788 MB of 128256 x 3072: 151 against 121).
     if (d.M <= 16 && (long long)scr_ceil_div(d.N, 128) * scr_ceil_div(d.K, 64) * d.groups < 16ll * ctx->sm_count)
         return d.residual ? matvec_launch<END_RESIDUAL>(ctx, d, st) : d.n_parts ? matvec_launch<END_PARTS>(ctx, d, st) : matvec_launch<END_OWN>(ctx, d, st);
-    if (dense_skinny_applies(d.M)) return dense_skinny_launch(ctx, d, st);
+    if (dense_skinny_applies(d.M, d.N, d.K, d.groups)) return dense_skinny_launch(ctx, d, st);
     return dense_gemm_launch(ctx, d, workspace, workspace_bytes, st);
 }
