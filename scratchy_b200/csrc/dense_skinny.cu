@@ -172,7 +172,8 @@ bool dense_skinny_applies(int M, int N, int K, int groups) {
 int32_t dense_skinny_launch(scr_ctx* ctx, const scr_dense& d, cudaStream_t stream) {
     CUtensorMap x_map, w_map;
     const uint64_t xg = d.groups > 1 ? (uint64_t)d.x_group * 2 : (uint64_t)d.K * 2;
-    if (!dense_tensor_map(&x_map, d.x, d.K, d.groups, d.M, xg, (uint64_t)d.ldx * 2, 1, (d.M + 15) & ~15) ||
+    const uint64_t row = (uint64_t)(d.M > 1 ? d.ldx : d.K) * 2;          // (a single row has no use for its stride)
+    if (!dense_tensor_map(&x_map, d.x, d.K, d.groups, d.M, xg, row, 1, (d.M + 15) & ~15) ||
         !dense_tensor_map(&w_map, d.w, d.K, d.N, d.groups, (uint64_t)d.K * 2, (uint64_t)d.N * d.K * 2, SKINNY_ROWS, 1))
         return scr_fail(ctx, SCR_E_CUDA, "dense_skinny: tensor map (M %d N %d K %d groups %d)", d.M, d.N, d.K, d.groups);
     switch (dense_end(d)) {

@@ -122,3 +122,22 @@ def test_no_unit_of_a_cut_is_left_without_steps(K):
 def test_dense_on_both_sides_of_the_wide_tiles(N, K, M):
     """17 to 128 rows where W's width or a short k decides for the tiles of 128 rows, and just before."""
     test_dense(N, K, M)
+
+
+@pytest.mark.parametrize("form", ["one row for all", "rows that overlap", "one x for all groups", "a row of any stride"])
+def test_rows_of_x_that_are_not_apart(form):
+    """Up to 16 rows at a size that goes to the GEMM where x is an ordinary matrix: what has no tensor map runs all the same."""
+    import torch
+    from scratchy_b200.dense import Arena, DenseLinear
+    rng = np.random.default_rng(len(form))
+    draw = lambda *shape: torch.from_numpy(rng.standard_normal(shape).astype(np.float32)).cuda().bfloat16()
+    N, K, M, groups = (6400, 1032, 5, 3) if "groups" in form else (18952, 1032, 1 if "any stride" in form else 5, 1)
+    w, a = draw(groups * N, K), Arena("cuda")
+    flat = draw(M * K)
+    x = {"one row for all": lambda: flat[:K].expand(M, K), "rows that overlap": lambda: flat.as_strided((M, K), (8, 1)),
+         "one x for all groups": lambda: flat.view(M, K), "a row of any stride": lambda: flat.as_strided((1, K), (0, 1))}[form]()
+    y = torch.full((M, groups * N), float("nan"), device="cuda")
+    DenseLinear(w, groups)(a, x, y, y_group=N)
+    torch.cuda.synchronize()
+    want = x.double() @ w.double().T
+    assert float((y.double() - want).norm() / want.norm()) < 1e-5
