@@ -6,7 +6,7 @@
 //   warp 8       producer of the weights (one tiled TMA load of 128 rows x 64 k per slice, 128-byte swizzle), load-time
 //                constants: it starts before the preceding kernel of the stream has finished
 //   warp 9       producer of x (one tiled TMA load per slice, zeros outside)
-//   warp 10      owns TMEM; one thread issues 4 tcgen05.mma (128 x rows of x x 16) per slice
+//   warp 10      owns TMEM; one elected lane issues 4 tcgen05.mma (128 x rows of x x 16) per slice
 //
 // What bounds it: the weights from HBM; for the small linears the start and end of a launch.  16384 x 3072 (100 MB) at 32 rows
 // 28.0 us with the MMAs issued from a divergent thread, 23.2 us (4.3 TB/s) from a whole warp; 128256 x 3072 139 and 132 us (6.0

@@ -24,6 +24,7 @@ int32_t fp8_gemm_pair_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* 
 // Defined in fp8_skinny.cu
 int32_t fp8_skinny_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint16_t* y, int M, int N, int K, const LinearEnds& ends,
                           cudaStream_t stream);
+float fp8_skinny_us(const scr_ctx* ctx, int M, int N, int K);
 // Channel-tile width and work units.  Wide (256-channel) tiles reuse every activation tile twice and are preferred;
 // a 128-channel tile does half the work in about three quarters of the time (measured), which can still win
 // when it quantises better over the SMs.  Units as in `tc_plan_units`.
@@ -329,10 +330,15 @@ int32_t fp8_gemm_tc_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* ac
         const int32_t st = fp8_gemm_pair_launch(ctx, wpack, act, y, M, N, K, ends, stream, &launched);
         if (st || launched) return st;
     }
-    // what one accumulator holds, where the pair kernel's tiles do not fill the GPU.  (It needs no slabs; the size query keeps what
-    // the tiles above would want, so that no caller's scratch limit moves.)
-    if (M <= 256) return fp8_skinny_launch(ctx, wpack, act, y, M, N, K, ends, stream);
+    // What one accumulator of fp8_skinny.cu holds, where the pair kernel's tiles do not fill the GPU.  Its end grows with the tokens, so beyond
+    // 64 of them the tiles below stay ahead where they need no cut (and no second launch) and k is short or W wide: 250 tokens of
+    // 1024 -> 8192 15.0 us there and 9.7 here, 2048 -> 2048 13.7 and 11.6, 3584 -> 9472 19.9 and 16.5, 128 of 3584 -> 18944 21.2 and 18.7,
+    // but 250 of 18944 -> 3584 27.4 and 30.4, 192 of 3584 -> 9472 17.1 and 16.4.  (It needs no slabs; the size query keeps what the tiles
+    // would want, so that no caller's scratch limit moves.)
     const Fp8GemmPlan plan = fp8_gemm_plan(M, N, K, ctx->sm_count);
+    const float tiles_us = 4.5f + 0.43f * (plan.bn == 256 ? 1.0f : 0.75f) * (float)(scr_ceil_div(K, FP8_TILE) * scr_ceil_div(plan.tiles, ctx->sm_count));
+    if (M <= 64 || (M <= 256 && (plan.ks_tail > 1 || fp8_skinny_us(ctx, M, N, K) < tiles_us + 0.5f)))
+        return fp8_skinny_launch(ctx, wpack, act, y, M, N, K, ends, stream);
     float* slabs = reinterpret_cast<float*>(workspace);
     if (plan.ks_tail > 1 && (!slabs || !scr_aligned16(slabs))) return scr_fail(ctx, SCR_E_WORKSPACE, "split-K needs an aligned workspace");
     if (plan.bn == 256) return fp8_gemm_launch_bn<256>(ctx, wpack, act, y, M, N, K, ends, plan, slabs, stream);

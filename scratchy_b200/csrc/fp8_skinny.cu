@@ -9,10 +9,10 @@
 //                starts before the quantisation of the activations has finished
 //   warp 9       producer of the quantised activations, which lie in the same image: the tokens' rows of a k-tile are one
 //                contiguous run (rows past the last token hold whatever the pack held; their columns are never stored)
-//   warp 10      owns TMEM; one thread issues 4 tcgen05.mma (128 x tokens x 32) per step
+//   warp 10      owns TMEM; one elected lane issues 4 tcgen05.mma (128 x tokens x 32) per step
 //
 // What bounds it: the copies into shared memory, 16 KB of weights and 128 bytes per token and step.  250 tokens of 18944 -> 3584
-// (with the quantisation) 46.4 us on the 128-token tiles of fp8_gemm.cu and their finishing launch, 36.0 us here.
+// (with the quantisation) 46.4 us on the 128-token tiles of fp8_gemm.cu and their finishing launch, 33 us here.
 #include "fp8.cuh"
 #include "skinny.cuh"
 
@@ -147,12 +147,17 @@ fp8_skinny_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ w
 }
 
 template <int TN>
+int f8s_split(const scr_ctx* ctx, const Fp8Geom& g) {
+    static SkinnyResident resident;
+    return skinny_split(resident, fp8_skinny_kernel<TN>, ctx->device, ctx->sm_count, g.NT, g.KT, F8S_THREADS, F8SCfg<TN>::kTotal, 4.0f);
+}
+
+template <int TN>
 int32_t f8s_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint16_t* y, int M, int N, int K, const LinearEnds& ends, cudaStream_t stream) {
     using C = F8SCfg<TN>;
     static_assert(C::kBarOff >= skinny_sum_bytes(TN), "the sums fit the rings");
     const Fp8Geom g = fp8_geom(N, K);
-    static SkinnyResident resident;
-    const int split = skinny_split(resident, fp8_skinny_kernel<TN>, ctx->device, ctx->sm_count, g.NT, g.KT, F8S_THREADS, C::kTotal, 4.0f);
+    const int split = f8s_split<TN>(ctx, g);
     const float* w_scale = reinterpret_cast<const float*>(wpack + (size_t)g.NT * g.KT * FP8_TILE_BYTES);
     const cudaError_t e = skinny_launch(fp8_skinny_kernel<TN>, g.NT, split, F8S_THREADS, C::kTotal, stream, wpack, w_scale, act + fp8_act_scale_bytes(M),
                                         reinterpret_cast<const float*>(act), y, M, N, g.KT, scr_ceil_div(M, FP8_TILE) * FP8_TILE, split, ends.out_f32,
@@ -162,6 +167,15 @@ int32_t f8s_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint1
 }
 
 }  // namespace
+
+// About what a call of 65 to 256 tokens takes here, in us: a k-tile of a unit 0.40 and 0.0006 a token, and start and end of a launch 2.3 and
+// 0.0335 a token (fitted to streams of calls: 3584 x 18944 at 256 tokens 27.4, 3584 x 3584 15.3, 8192 x 1024 15.2, 512 x 512 11.2).
+float fp8_skinny_us(const scr_ctx* ctx, int M, int N, int K) {
+    const Fp8Geom g = fp8_geom(N, K);
+    const int split = M <= 128 ? f8s_split<128>(ctx, g) : f8s_split<256>(ctx, g);
+    const int rounds = scr_ceil_div(g.NT * split, ctx->sm_count);
+    return 2.3f + 0.0335f * M + (float)(rounds * scr_ceil_div(g.KT, split)) * (0.40f + 0.0006f * M);
+}
 
 int32_t fp8_skinny_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint16_t* y, int M, int N, int K, const LinearEnds& ends,
                           cudaStream_t stream) {

@@ -141,3 +141,9 @@ def test_rows_of_x_that_are_not_apart(form):
     torch.cuda.synchronize()
     want = x.double() @ w.double().T
     assert float((y.double() - want).norm() / want.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("N,K,M", [(512, 512, 90), (512, 512, 128), (1000, 1000, 129), (1000, 1000, 200), (2056, 2048, 250), (8200, 1024, 140), (9480, 1536, 256)])
+def test_fp8_on_both_sides_of_the_tiles(N, K, M):
+    """65 to 256 tokens where k, the channels and the tokens decide between the GEMM for few tokens and the tiles of 128."""
+    test_fp8(N, K, M)
