@@ -5,8 +5,8 @@
 //   o = S'^T q / (max(|n'.q|, e^(-m')) + 1e-6),   q scaled by dim^(-1/2)
 // State and everything about it is f32.
 //
-//   mlstm_step_kernel    token by token: decoding, short portions, dim up to 256, both data types
-//   mlstm_recur_kernel   the same for larger dim
+//   mlstm_step_kernel    token by token: decoding, short portions, both data types; up to dim 128, and to 256 where few CTAs run
+//   mlstm_recur_kernel   the same for the others
 //   mlstm_chunk.cu       bf16 prompts, 64 tokens at a time on the tensor cores
 //   mlstm_finish_kernel  each head's output over its root mean square, the norm's weight and the output gate
 #include "seq_common.cuh"
@@ -141,8 +141,9 @@ __global__ void __launch_bounds__(RC_T) mlstm_recur_kernel(MemoryArgs a) {
 // The slice of S (and this slice's copy of n) in registers: 8 threads with 4 columns each cover a row, a thread has RPT rows, 32
 // apart.  The state's lines start for L2 before the wait for the preceding kernels and are read after it (one of those kernels may be
 // the call that leaves this one its state), and a token takes one barrier: the normaliser's n.q goes round with the outputs.
-// What bounds it: HBM, the state read and written once a step.  32 sequences of 12 heads of 128 x 256 (101 MB), alone and cold: 34.0 us
-// with the state in shared memory, asked for after the wait, and two barriers a token; 29.9 us here.
+// What bounds it: HBM, the state read and written once a step.  32 sequences of 12 heads of 128 x 256 (101 MB), alone and cold: 43.0 us
+// with the state in shared memory, asked for after the wait, and two barriers a token; 37.8 us here (both with about 4 us of the
+// measurement's own).
 template <typename T, int RPT>
 __global__ void __launch_bounds__(RC_T) mlstm_step_kernel(MemoryArgs a) {
     __shared__ float4 part[2][RC_T / 32][8];
@@ -345,7 +346,10 @@ cudaError_t step_launch(const MemoryArgs& a, cudaStream_t stream) {
 template <typename T>
 int32_t recur_launch(scr_ctx* ctx, const MemoryArgs& a, cudaStream_t stream) {
     const int dim = a.s.dim;
-    if (dim <= 8 * RC_ROWS) {                                // 8 rows of a thread fit its registers
+    // Up to 8 rows of a thread fit its registers, 8 of them at two CTAs an SM: beyond one such round the state in shared memory wins (8
+    // heads of 256 x 256, cold: 4 sequences 12.3 us against 16.4, 8 of them 18.4 both, 32 50.2 against 43.0).
+    const bool one_round = (long long)scr_ceil_div(a.s.vdim, RC_COLS) * a.s.heads * a.st.batch <= 2ll * ctx->sm_count;
+    if (dim <= 4 * RC_ROWS || (dim <= 8 * RC_ROWS && one_round)) {
         const cudaError_t e = dim <= RC_ROWS ? step_launch<T, 1>(a, stream) : dim <= 2 * RC_ROWS ? step_launch<T, 2>(a, stream)
                             : dim <= 4 * RC_ROWS ? step_launch<T, 4>(a, stream) : step_launch<T, 8>(a, stream);
         if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "mlstm_step: %s", cudaGetErrorString(e));

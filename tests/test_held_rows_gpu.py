@@ -75,3 +75,17 @@ def test_decode_attention_at_every_cut_and_number_of_warps(longest, hq, hkv, d, 
 def test_decode_attention_with_warps_that_do_not_all_fit(longest, hq, hkv, d, bs, batch):
     """Four or two warps where the query heads, the table or the blocks leave no room for six."""
     test_decode_attention_at_every_cut_and_number_of_warps(longest, hq, hkv, d, bs, batch)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,dim,vdim,batch", [(2, 129, 40, 3), (5, 256, 64, 29), (5, 256, 64, 30), (2, 260, 72, 4), (1, 512, 33, 2)])
+def test_memory_step_of_large_heads(heads, dim, vdim, batch, dtype):
+    """Keys of more than 128 values: in registers while a round of CTAs holds them, in shared memory beyond (and beyond 256)."""
+    from tests.test_sequence_ops_gpu import draw_memory, head_rows, plain_memory, run_memory
+    m = su.memory_spec(heads, dim, vdim)["mixer"]
+    rng = np.random.default_rng(dim + batch)
+    seqs = [(draw_memory(rng, 5, m, dtype), (2.0 * rng.standard_normal((5, 2 * heads))).astype(np.float32)) for _ in range(batch)]
+    bi, bf = np.zeros(heads, np.float32), np.full(heads, 2.0, np.float32)
+    got, _ = run_memory(m, dtype, [p for p, _ in seqs], [g for _, g in seqs], bi, bf, [[3] * batch, [1] * batch, [1] * batch], list(range(batch)))
+    for o, (p, g) in zip(got, seqs):
+        assert su.rel(head_rows(o, heads), head_rows(plain_memory(m, p, g, bi, bf), heads)) < (2e-5 if dtype == "float32" else 5e-4)
