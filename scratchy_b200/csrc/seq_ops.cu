@@ -369,7 +369,11 @@ extern "C" int32_t scr_seq_norm(scr_ctx* ctx, int32_t dtype, const scr_seq_norm_
     if (smem > 200 * 1024) return scr_fail(ctx, SCR_E_UNSUPPORTED, "width %d", a.width);
     const bool vec = a.width % 4 == 0 && a.ld_out % 4 == 0 && scr_aligned16(a.x) && scr_aligned16(a.delta) && scr_aligned16(a.w_delta) &&
                      scr_aligned16(a.bias) && scr_aligned16(a.w_out) && scr_aligned16(a.b_out) && scr_aligned16(a.out);
-    if (vec && a.width <= 4 * 4 * NORM_T) {
+    // Held rows cost registers (38 to 101 a thread against 32), so fewer CTAs run at once: they win while all rows are there in one round,
+    // and beyond it where the row's two sums make a chain worth cutting (cold, held / not: 8192 rows of 3072 with a sublayer's output
+    // 65.5 / 67.6 us, of 4096 92.2 / 80.7, of 88 30.7 / 22.5, of 4096 without 61.5 / 42.2; 200 rows of 3072 8.2 / 12.3).
+    const bool one_round = a.rows <= 2 * ctx->sm_count, chain = a.delta && a.width >= 4 * NORM_T && a.width <= 12 * NORM_T;
+    if (vec && a.width <= 16 * NORM_T && (one_round || chain)) {
         const int keep = scr_ceil_div(a.width, 4 * NORM_T);
         auto held = dtype == SCR_DTYPE_F32 ? (keep == 1 ? seq_norm_held_kernel<float, 1> : keep == 2 ? seq_norm_held_kernel<float, 2> : keep == 3 ? seq_norm_held_kernel<float, 3> : seq_norm_held_kernel<float, 4>)
                                            : (keep == 1 ? seq_norm_held_kernel<bf16, 1> : keep == 2 ? seq_norm_held_kernel<bf16, 2> : keep == 3 ? seq_norm_held_kernel<bf16, 3> : seq_norm_held_kernel<bf16, 4>);

@@ -89,3 +89,19 @@ def test_memory_step_of_large_heads(heads, dim, vdim, batch, dtype):
     got, _ = run_memory(m, dtype, [p for p, _ in seqs], [g for _, g in seqs], bi, bf, [[3] * batch, [1] * batch, [1] * batch], list(range(batch)))
     for o, (p, g) in zip(got, seqs):
         assert su.rel(head_rows(o, heads), head_rows(plain_memory(m, p, g, bi, bf), heads)) < (2e-5 if dtype == "float32" else 5e-4)
+
+
+@pytest.mark.parametrize("W,T,delta", [(88, 296, True), (88, 297, True), (1020, 300, True), (1024, 300, True), (3072, 300, True), (3076, 300, True), (1024, 300, False),
+                                       (4096, 296, False), (4096, 297, False)])
+def test_norm_of_many_rows(W, T, delta):
+    """Both kernels on both sides of the rule between them: one round of rows, and widths with a sublayer's output beyond it."""
+    from scratchy_b200.dense import seq_norm
+    torch = torch_()
+    rng = np.random.default_rng(W + T)
+    x, d = rng.standard_normal((T, W)).astype(np.float32), 3 * rng.standard_normal((T, W)).astype(np.float32)
+    wd, wo = (0.5 * rng.standard_normal(W).astype(np.float32) for _ in range(2))
+    xd, out = dev(x), torch.full((T, W), float("nan"), dtype=torch.bfloat16, device="cuda")
+    seq_norm(xd, 0.01, **(dict(delta=dev(d), w_delta=dev(wd)) if delta else {}), out=out, w_out=dev(wo))
+    want = x.astype(np.float64) + (plain.norm_around_zero(d.astype(np.float64), wd, 0.01) if delta else 0.0)
+    assert su.rel(host(xd), want) < 1e-6 and su.rel(host(out), plain.norm_around_zero(want, wo, 0.01)) < TOL["bfloat16"]
+    healthy()
