@@ -249,21 +249,11 @@ __global__ void __launch_bounds__(ARGMAX_THREADS) argmax_kernel(const uint16_t* 
     float best = -INFINITY;
     uint32_t best_i = 0;
     const int nv = width >> 3;
-    constexpr int AHEAD = 8;                           // one SM reads the row: eight requests a thread in flight
-    for (int v0 = threadIdx.x; v0 < nv; v0 += AHEAD * ARGMAX_THREADS) {
-        uint4 q[AHEAD];
+    for (int v = threadIdx.x; v < nv; v += ARGMAX_THREADS) {
+        float f[8];
+        unpack8(*reinterpret_cast<const uint4*>(row + v * 8), f);
 #pragma unroll
-        for (int u = 0; u < AHEAD; ++u)
-            if (v0 + u * ARGMAX_THREADS < nv) q[u] = *reinterpret_cast<const uint4*>(row + (v0 + u * ARGMAX_THREADS) * 8);
-#pragma unroll
-        for (int u = 0; u < AHEAD; ++u) {
-            const int v = v0 + u * ARGMAX_THREADS;
-            if (v >= nv) break;
-            float f[8];
-            unpack8(q[u], f);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) argmax_take(f[j], uint32_t(v * 8 + j), best, best_i);
-        }
+        for (int j = 0; j < 8; ++j) argmax_take(f[j], uint32_t(v * 8 + j), best, best_i);
     }
     for (int i = (nv << 3) + threadIdx.x; i < width; i += ARGMAX_THREADS)
         argmax_take(bf16_bits_to_f32(row[i]), uint32_t(i), best, best_i);

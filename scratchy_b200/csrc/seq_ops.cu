@@ -204,6 +204,10 @@ __device__ __forceinline__ void amax_take(float v, int i, float& best, int& best
         best_i = i;
     }
 }
+// AHEAD: requests of 16 bytes a thread has in flight.  One SM reads a row, so a wide one wants eight (32 rows of 128256, cold: 16.4 us, 22.5
+// with one of 4 bytes); they cost the registers of the SM's second CTA, and narrow rows only carry them along (200 rows of 32000 16.4 us
+// with eight, 14.4 with one of 4 bytes; 32 of 1000 8.2 and 6.6).
+template <int AHEAD>
 __global__ void __launch_bounds__(AMAX_T) seq_argmax_kernel(const float* __restrict__ logits, long long ld, int width, int* __restrict__ out) {
     __shared__ float sb[AMAX_T / 32];
     __shared__ int si[AMAX_T / 32];
@@ -213,7 +217,6 @@ __global__ void __launch_bounds__(AMAX_T) seq_argmax_kernel(const float* __restr
     float best = -INFINITY;
     int best_i = 0x7FFFFFFF;
     const int nv = (reinterpret_cast<uintptr_t>(row) & 15) == 0 ? width / 4 : 0;
-    constexpr int AHEAD = 8;                               // one SM reads the row: eight requests of 16 bytes a thread in flight
     for (int i0 = threadIdx.x; i0 < nv; i0 += AHEAD * AMAX_T) {
         float4 q[AHEAD];
 #pragma unroll
@@ -389,7 +392,8 @@ extern "C" int32_t scr_seq_argmax(scr_ctx* ctx, const float* logits, int64_t ld,
     SCR_REQUIRE_CTX(ctx);
     if (!logits || !out) return scr_fail(ctx, SCR_E_ARG, "null pointer");
     if (rows <= 0 || width <= 0) return scr_fail(ctx, SCR_E_SHAPE, "empty argmax");
-    SEQ_LAUNCH("seq_argmax", launch_pdl(seq_argmax_kernel, dim3(rows), dim3(AMAX_T), 0, (cudaStream_t)stream, logits, (long long)ld, width, out));
+    auto kernel = width >= 8 * AMAX_T && rows <= ctx->sm_count ? seq_argmax_kernel<8> : seq_argmax_kernel<1>;
+    SEQ_LAUNCH("seq_argmax", launch_pdl(kernel, dim3(rows), dim3(AMAX_T), 0, (cudaStream_t)stream, logits, (long long)ld, width, out));
 }
 
 extern "C" int32_t scr_latent_prepare(scr_ctx* ctx, int32_t dtype, const scr_latent_shape* s, const scr_step* st, const float* d, int64_t ld_d,

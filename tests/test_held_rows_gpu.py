@@ -105,3 +105,18 @@ def test_norm_of_many_rows(W, T, delta):
     want = x.astype(np.float64) + (plain.norm_around_zero(d.astype(np.float64), wd, 0.01) if delta else 0.0)
     assert su.rel(host(xd), want) < 1e-6 and su.rel(host(out), plain.norm_around_zero(want, wo, 0.01)) < TOL["bfloat16"]
     healthy()
+
+
+@pytest.mark.parametrize("rows,width,ld", [(148, 8192, 8192), (149, 8192, 8192), (5, 8191, 8192), (3, 12289, 12289), (200, 50000, 50000)])
+def test_greedy_with_one_and_eight_requests_in_flight(rows, width, ld):
+    """Rows and widths on both sides of the rule; the largest value at the ends of a thread's run, and NaN never."""
+    from scratchy_b200.dense import greedy
+    torch = torch_()
+    g = torch.Generator().manual_seed(width + rows)
+    x = torch.randint(-50, 50, (rows, ld), generator=g).float()
+    for r in range(rows):
+        x[r, (0, width - 1, width // 2, 4095, 4096)[r % 5]] = 60.0
+    x[-1] = float("nan")
+    x[-1, 7] = -1.0
+    want = torch.nan_to_num(x[:, :width], nan=-1e9).numpy().argmax(axis=1)
+    assert greedy(x.cuda()[:, :width]).cpu().numpy().tolist() == want.tolist()
