@@ -1,4 +1,4 @@
-// MLX affine int4 (groups of 32, 64, 128): prefill GEMM on tcgen05 tensor cores, M > 128.
+// MLX affine int4 (groups of 32, 64, 128): prefill GEMM on tcgen05 tensor cores, M > 128 (from 97 on where k is short).
 //
 //   y[m,n] = bf16( sum_k x[m,k] * w[n,k] (+ bias[n]) ),  w = the bit-exact bf16 dequantisation of the codes
 //
@@ -34,7 +34,7 @@ bool affine_b4_gemm_pair_applies(int M, int N, int K, int sms);
 int32_t affine_b4_gemm_pair_launch(scr_ctx* ctx, const CUtensorMap& x_map, const uint8_t* packed, uint16_t* y, int M, int N, int K,
                                    int gs, int out_f32, const uint16_t* bias, cudaStream_t stream, bool* launched);
 // Defined in affine_b4_skinny.cu
-bool affine_b4_skinny_applies(int M);
+bool affine_b4_skinny_applies(int M, int K);
 int32_t affine_b4_skinny_launch(scr_ctx* ctx, const uint8_t* packed, const uint16_t* x, uint16_t* y, int M, int N, int K, int gs, int out_f32,
                                 const uint16_t* bias, cudaStream_t stream);
 size_t affine_b4_gemm_tc_workspace_plan(int M, int N, int K);
@@ -347,7 +347,7 @@ static AffineGemmPlan affine_gemm_plan(int M, int N, int K, int sms) {
     return best;
 }
 size_t affine_b4_gemm_tc_workspace_plan(int M, int N, int K) {
-    if (affine_b4_skinny_applies(M)) return 0;
+    if (affine_b4_skinny_applies(M, K)) return 0;
     return affine_gemm_plan(M, N, K, tc_sm_count()).slab_floats() * sizeof(float);
 }
 
@@ -380,7 +380,7 @@ int32_t affine_b4_gemm_tc_launch(scr_ctx* ctx, const uint8_t* packed, const uint
                                  int gs, int out_f32, const uint16_t* bias, void* workspace, size_t, cudaStream_t stream) {
     if (((uintptr_t)packed & 127u) != 0) return scr_fail(ctx, SCR_E_ALIGN, "packed weights must be 128-byte aligned for the GEMM path");
     if (!scr_aligned16(y)) return scr_fail(ctx, SCR_E_ALIGN, "y must be 16-byte aligned");
-    if (affine_b4_skinny_applies(M)) return affine_b4_skinny_launch(ctx, packed, x, y, M, N, K, gs, out_f32, bias, stream);
+    if (affine_b4_skinny_applies(M, K)) return affine_b4_skinny_launch(ctx, packed, x, y, M, N, K, gs, out_f32, bias, stream);
     tc_encode_tiled_fn enc = tc_tensor_map_encoder();
     if (!enc) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled entry point not available");
     CUtensorMap map;

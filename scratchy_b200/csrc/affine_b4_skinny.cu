@@ -246,8 +246,10 @@ int32_t a4s_launch(scr_ctx* ctx, const CUtensorMap& map, const uint8_t* packed, 
 }  // namespace
 
 // Whether the GEMM for few tokens takes this call: above the matvec's 16 tokens, up to the 128 that one accumulator and three
-// or four activation stages hold beside the weights.  (Beyond, a second token tile would expand every weight a second time.)
-bool affine_b4_skinny_applies(int M) { return M > 16 && M <= 128; }
+// or four activation stages hold beside the weights.  (Beyond, a second token tile would expand every weight a second time.)  Its
+// end grows with the tokens, and where k is short that is most of a call: 128 tokens of 512 -> 8192 8.5 us against 5.9 on the prompt
+// kernel's tiles, of 1280 -> 4096 10.8 and 8.0, of 1536 -> 6144 10.3 and 9.9, but of 2048 -> 2048 9.0 and 9.9.
+bool affine_b4_skinny_applies(int M, int K) { return M > 16 && (M <= 96 || (M <= 128 && K > 1536)); }
 
 int32_t affine_b4_skinny_launch(scr_ctx* ctx, const uint8_t* packed, const uint16_t* x, uint16_t* y, int M, int N, int K, int gs, int out_f32,
                                 const uint16_t* bias, cudaStream_t stream) {

@@ -147,3 +147,9 @@ def test_rows_of_x_that_are_not_apart(form):
 def test_fp8_on_both_sides_of_the_tiles(N, K, M):
     """65 to 256 tokens where k, the channels and the tokens decide between the GEMM for few tokens and the tiles of 128."""
     test_fp8(N, K, M)
+
+
+@pytest.mark.parametrize("N,K,M", [(8200, 512, 96), (8200, 512, 97), (136, 128, 128), (1000, 1536, 128), (1000, 1600, 128)])
+def test_int4_of_a_short_k_on_both_sides_of_the_prompt_tiles(N, K, M):
+    """97 to 128 tokens: the prompt kernel up to a k of 1536 (tiles that are not full, cut or whole), and just beyond it."""
+    test_int4(N, K, M, 64)
