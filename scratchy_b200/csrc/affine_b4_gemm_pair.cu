@@ -128,8 +128,8 @@ affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const uint
         fence_mbar_init();
     }
     if (warp == 1) {
-        tmem_alloc_pair(smem_u32((const void*)tmem_slot), 2 * A4P_BN);    // the pair's columns: the same in both CTAs
-        tmem_relinquish_pair();
+        tmem_alloc(smem_u32((const void*)tmem_slot), 2 * A4P_BN);    // each CTA allocates its own columns; both get the same base
+        tmem_relinquish();
     }
     __syncwarp();
     tc_fence_before();
@@ -350,7 +350,7 @@ affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const uint
     a4p_pair_sync();                                      // nobody frees TMEM or leaves while the other may still signal it
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc_pair(tmem_base, 2 * A4P_BN);
+        tmem_dealloc(tmem_base, 2 * A4P_BN);
     }
 }
 

@@ -403,8 +403,8 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_c
         fence_mbar_init();
     }
     if (warp == 1) {
-        tmem_alloc_pair(smem_u32((const void*)tmem_slot), 2 * DP_BN);
-        tmem_relinquish_pair();
+        tmem_alloc(smem_u32((const void*)tmem_slot), 2 * DP_BN);
+        tmem_relinquish();
     }
     __syncwarp();
     tc_fence_before();
@@ -493,7 +493,7 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_c
     dp_pair_sync();                                    // nobody frees TMEM or leaves while the other may still signal it
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc_pair(tmem_base, 2 * DP_BN);
+        tmem_dealloc(tmem_base, 2 * DP_BN);
     }
 }
 

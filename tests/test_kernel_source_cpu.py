@@ -40,17 +40,6 @@ def kernels():
             yield name, m.group(1), body, body + called
 
 
-def test_a_kernel_names_one_cta_group():
-    """All tcgen05 instructions of a kernel have the same cta_group: a pair's MMAs go with a pair's allocation."""
-    seen = {}
-    for _, kernel, _, text in kernels():
-        groups = set(re.findall(r"tcgen05\.(?:alloc|dealloc|relinquish_alloc_permit|mma|commit|cp)\.[^\"]*?cta_group::(\d)", text))
-        if groups:
-            seen[kernel] = groups
-    assert {k for k, g in seen.items() if g == {"2"}} == {"affine_b4_gemm_pair_kernel", "fp8_gemm_pair_kernel", "dense_gemm_pair_kernel"}
-    assert len(seen) >= 8 and all(len(g) == 1 for g in seen.values()), seen
-
-
 def test_warps_are_whole_at_aligned_barriers():
     """`barrier.cluster.*.aligned` and tcgen05's `.sync.aligned` forms are executed by a whole warp: where single lanes had roles
     of their own before, a __syncwarp, or a barrier of the CTA, comes first."""
