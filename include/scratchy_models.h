@@ -39,6 +39,8 @@ extern "C" {
  *          writes them by its kind to its own y (row stride ld), column n - start of the part; y, y2, gate and act are unused
  *   residual (may be NULL): residual[m * ld_residual + n] += sum (f32); with tanh_w, y gets the norm of the new residual,
  *          tanh(tanh_alpha * residual) * tanh_w[n] + tanh_b[n] (dtype), otherwise y is unused
+ *   w_fresh: w comes from a preceding kernel of the stream.  Otherwise it is a load-time constant that may be read while
+ *          those still run
  * `workspace` (f32 slabs of a k-split) may be NULL when `scr_dense_workspace_size` reports 0. */
 #define SCR_PART_STORE 0            /* dtype */
 #define SCR_PART_F32 1              /* f32 */
@@ -67,6 +69,7 @@ typedef struct scr_dense {
     float tanh_alpha;
     int32_t n_parts;
     scr_dense_part parts[SCR_DENSE_PARTS];
+    int32_t w_fresh;
 } scr_dense;
 int32_t scr_dense_workspace_size(int32_t dtype, int32_t M, int32_t N, int32_t K, int32_t groups, size_t* bytes);
 int32_t scr_dense_linear(scr_ctx* ctx, int32_t dtype, const scr_dense* d, void* workspace, size_t workspace_bytes,

@@ -150,7 +150,7 @@ class Dense(ctypes.Structure):
                 ("y_group", _i64), ("ldy2", _i64), ("ldg", _i64), ("M", _i32), ("N", _i32), ("K", _i32), ("groups", _i32),
                 ("n_main", _i32), ("y_f32", _i32), ("act", _i32), ("limit", ctypes.c_float), ("alpha", ctypes.c_float),
                 ("residual", _vp), ("ld_residual", _i64), ("tanh_w", _vp), ("tanh_b", _vp), ("tanh_alpha", ctypes.c_float), ("n_parts", _i32),
-                ("parts", DensePart * DENSE_PARTS)]
+                ("parts", DensePart * DENSE_PARTS), ("w_fresh", _i32)]
 
 
 class SeqNorm(ctypes.Structure):

@@ -258,14 +258,15 @@ extern "C" int32_t scr_dense_linear(scr_ctx* ctx, int32_t dtype, const scr_dense
     cudaStream_t st = (cudaStream_t)stream;
     if (dtype == SCR_DTYPE_F32) return plain_launch<float>(ctx, d, st);
     if (dtype != SCR_DTYPE_BF16) return scr_fail(ctx, SCR_E_DTYPE, "dtype %d", dtype);
-    if (!rows_of_16_bytes(d)) return plain_launch<bf16>(ctx, d, st);
+    const bool rows_apart = (d.M == 1 || d.ldx >= d.K) && (d.groups == 1 || d.x_group >= d.K);
+    // (the matvec reads W ahead of the preceding kernels, so one that comes from them goes elsewhere)
+    if (!rows_of_16_bytes(d) || (d.w_fresh && d.M <= 16 && !rows_apart)) return plain_launch<bf16>(ctx, d, st);
     // Up to 16 rows: the matvec starts sooner and wins where an SM has little to stream (19 MB of 3072 x 3072 at 8 rows: 7.2 us
     // against 7.6); from 16 slices of 16 KB per SM on, the GEMM's bulk loads keep more bytes in flight (50 MB of 3072 x 8192: 14.5
     // against 12.3 us, 183 MB of 29720 x 3072: 41.0 against 31.6, 788 MB of 128256 x 3072: 151 against 121).  Rows of x that repeat or
     // overlap (one row for all, one x for all groups) have no tensor map and stay with the matvec at any size.
-    const bool rows_apart = (d.M == 1 || d.ldx >= d.K) && (d.groups == 1 || d.x_group >= d.K);
     const bool streams = (long long)scr_ceil_div(d.N, 128) * scr_ceil_div(d.K, 64) * d.groups >= 16ll * ctx->sm_count;
-    if (d.M <= 16 && !(streams && rows_apart))
+    if (d.M <= 16 && !d.w_fresh && !(streams && rows_apart))
         return d.residual ? matvec_launch<END_RESIDUAL>(ctx, d, st) : d.n_parts ? matvec_launch<END_PARTS>(ctx, d, st) : matvec_launch<END_OWN>(ctx, d, st);
     if (dense_skinny_applies(d.M, d.N, d.K, d.groups)) return dense_skinny_launch(ctx, d, st);
     return dense_gemm_launch(ctx, d, workspace, workspace_bytes, st);

@@ -35,7 +35,7 @@ struct DsCfg {
 template <int TN, DenseEnd END>
 __global__ void __launch_bounds__(DS_THREADS, DsCfg<TN>::kCtasPerSm)
 dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, int M, int N, int KT, int NT, int split,
-                    DenseEnds ends, int* __restrict__ status) {
+                    int w_fresh, DenseEnds ends, int* __restrict__ status) {
     using C = DsCfg<TN>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -77,6 +77,7 @@ dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_cons
     // griddepcontrol.wait, so that its bound does not run against that kernel.
     if (warp == 8) {
         if (lane == 0) {
+            if (w_fresh) pdl_wait();
             for (int i = 0; i < steps; ++i) {
                 const int s = i % C::kSW;
                 if (i == C::kSW) pdl_wait();
@@ -140,7 +141,7 @@ int32_t ds_launch(scr_ctx* ctx, const scr_dense& d, const CUtensorMap& x_map, co
     static SkinnyResident resident;
     const int split = skinny_split(resident, dense_skinny_kernel<TN, END>, ctx->device, ctx->sm_count, nt * d.groups, kt, DS_THREADS, C::kTotal, 4.0f);
     const cudaError_t e = skinny_launch(dense_skinny_kernel<TN, END>, nt * d.groups, split, DS_THREADS, C::kTotal, stream, x_map, w_map, d.M, d.N, kt, nt,
-                                        split, dense_ends(d), ctx->dev_status);
+                                        split, (int)(d.w_fresh != 0), dense_ends(d), ctx->dev_status);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "dense_skinny: %s", cudaGetErrorString(e));
     return scr_check_launch(ctx, "dense_skinny");
 }

@@ -106,6 +106,7 @@ class DenseLinear:
     groups: int = 1
     glu_limit: Optional[float] = None        # set: a fused gate/up matrix (`interleave8`) with the clamped activation
     glu_alpha: float = 1.702
+    fresh: bool = False                      # the weight is another kernel's output: not to be read ahead of it
 
     def __post_init__(self):
         self.weight = self.weight.contiguous()
@@ -132,6 +133,7 @@ class DenseLinear:
                        self.in_features, self.groups, self.out_features if n_main is None else n_main,
                        int(y.dtype == torch.float32 and w.dtype != torch.float32), int(self.glu_limit is not None),
                        self.glu_limit if self.glu_limit is not None else 0.0, self.glu_alpha)
+        d.w_fresh = int(self.fresh)
         self._launch(arena, code, d)
         return y
 

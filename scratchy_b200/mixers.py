@@ -127,7 +127,7 @@ class LatentAttention:
             k = a.get("la.keys", (kv, H * self.dim), dt)
             self.uk_rows(a, lat, k)
             v_t = a.get("la.values_t", (H * self.vdim, ld_v), dt)
-            DenseLinear(lat)(a, self.uv.weight, v_t)
+            DenseLinear(lat, fresh=True)(a, self.uv.weight, v_t)
             c.check(lib.scr_latent_prefill(c.handle, ps, _ptr(qf[row:]), _ptr(k), _ptr(rot), _ptr(v_t), ld_v, _ptr(gate[row:]),
                                            int(gate.stride(0)), count, seq.length, _ptr(heads[row:]), int(heads.stride(0)), stream))
             row += count

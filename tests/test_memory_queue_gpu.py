@@ -141,3 +141,29 @@ def test_latent_cache(start, tokens, heads, kv_rank, rot_dim, captured):
         queued(calls, captured and not synchronised)
         results.append(out.float().cpu().numpy())
     assert np.isfinite(results[0]).all() and np.array_equal(*results)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("M,N,K", [(5, 200, 512), (16, 18952, 1032), (120, 1024, 512), (40, 3072, 3072), (200, 512, 512)])
+def test_a_linear_whose_matrix_the_call_before_it_writes(M, N, K, captured):
+    """`w_fresh`: the latents of a prompt are the matrix of the linear that expands its values, at row counts of every kernel."""
+    from scratchy_b200.dense import Arena, DenseLinear
+    torch = torch_()
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    draw = lambda *s: torch.randn(s, device="cuda", generator=g).bfloat16()
+    a, b, x = draw(N, 2048), draw(K, 2048), draw(M, K)
+    arena, results = Arena("cuda"), []
+    for synchronised in (True, False):
+        w, y = torch.zeros((N, K), dtype=torch.bfloat16, device="cuda"), torch.full((M, N), float("nan"), device="cuda")
+        first, second = DenseLinear(b), DenseLinear(w, fresh=True)
+        calls = [lambda: first(arena, a, w), lambda: second(arena, x, y)]
+        for _ in range(2):                                                   # (the buffers have their sizes before a capture)
+            w.zero_()
+            if synchronised:
+                for call in calls:
+                    call()
+                    torch.cuda.synchronize()
+            else:
+                queued(calls, captured)
+        results.append(y)
+    assert torch.equal(*results)
