@@ -30,7 +30,7 @@
 
 bool affine_b4_gemm_tc_enabled() { return true; }
 // Defined in affine_b4_gemm_pair.cu
-bool affine_b4_gemm_pair_applies(int M, int N, int K, int sms);
+bool affine_b4_gemm_pair_applies(int M, int N, int K, int sms, float one_cta_us);
 int32_t affine_b4_gemm_pair_launch(scr_ctx* ctx, const CUtensorMap& x_map, const uint8_t* packed, uint16_t* y, int M, int N, int K,
                                    int gs, int out_f32, const uint16_t* bias, cudaStream_t stream, bool* launched);
 // Defined in affine_b4_skinny.cu
@@ -385,7 +385,7 @@ int32_t affine_b4_gemm_tc_launch(scr_ctx* ctx, const uint8_t* packed, const uint
     if (!enc) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled entry point not available");
     CUtensorMap map;
     const AffineGemmPlan plan = affine_gemm_plan(M, N, K, ctx->sm_count);
-    if (affine_b4_gemm_pair_applies(M, N, K, ctx->sm_count)) {
+    if (affine_b4_gemm_pair_applies(M, N, K, ctx->sm_count, plan.us)) {
         bool launched = false;
         if (!affine_gemm_x_map(&map, enc, x, M, K, 128)) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled failed");
         const int32_t st = affine_b4_gemm_pair_launch(ctx, map, packed, y, M, N, K, gs, out_f32, bias, stream, &launched);

@@ -490,9 +490,10 @@ def test_group_sizes_fused_ends_and_refusals(group):
 
 
 def test_two_cta_gemm_gives_the_bits_of_the_one_cta_kernel(tmp_path):
-    """The CTA-pair int4 GEMM (`tcgen05.mma.cta_group::2`, each CTA dequantising half of the pair's channels) is opt-in
-    through the environment, read once per process: a child process runs it on a shape it takes (whole 256 x 256 tiles,
-    two full rounds of 74 pairs), this process runs the one-CTA kernel; same bits, and the oracle's bound on sampled rows."""
+    """The CTA-pair int4 GEMM (`tcgen05.mma.cta_group::2`, each CTA dequantising half of the pair's channels) is given every full
+    round of pairs through the environment, read once per process: a child process runs it on such a shape (two full rounds
+    of 74 pairs), this process, which would not choose it there, the one-CTA kernel; same bits, and the oracle's bound on
+    sampled rows."""
     import subprocess
     import sys
     import torch

@@ -1,4 +1,4 @@
-"""The int4 GEMM on CTA pairs (opt-in through the environment, read once per process) in the forms that a whole-tile shape does not
+"""The int4 GEMM on CTA pairs (given every full round of them through the environment, read once per process) in the forms that a whole-tile shape does not
 show: ragged tokens and channels, every group size, f32 partial sums, several tiles per pair over rings that go round."""
 import os
 import subprocess
@@ -66,3 +66,10 @@ def test_forms(results, i):
     assert rel_l2(got["y"].reshape(M, N)[rows], want) <= REL_L2_TOL
     assert np.isfinite(part).all() and np.array_equal(synth.f32_to_bf16_bits(part), got["y"].reshape(M, N))
     assert np.array_equal(synth.f32_to_bf16_bits(part + f32(bias)[None, :]), got["biased"].reshape(M, N))
+
+
+@pytest.mark.parametrize("N,M", [(14336, 256), (14210, 193)])
+def test_where_it_is_chosen(N, M):
+    """Without the environment: a second token tile that would start a round of its own, up to its edges (192 tokens are one tile)."""
+    from test_few_tokens_gpu import test_int4
+    test_int4(N, 3072, M, 64)
