@@ -12,11 +12,11 @@
 //   warp 10      owns TMEM; one elected lane issues 8 tcgen05.mma (128 x tokens x 16) per chunk
 //
 // What bounds it: for the short k extents of a layer's linears the start of the pipeline and the two cluster barriers at its end
-// (4 of the 7 us of a 3072 x 3072), for long ones the MMAs, which with A in TMEM take about 125 cycles each however few the columns
-// (1000 cycles per chunk and SM; a chunk's 9.2 KB from HBM would take 400).  Against the 128-token tile of the prefill GEMM that it
+// (4 of the 7 us of a 3072 x 3072), for long ones about 1000 cycles per chunk and SM however few the columns (a chunk's 9.2 KB from HBM
+// would take 400): eight MMAs with A in TMEM, or a chunk's way round the stages; not told apart.  Against the 128-token tile of the prefill GEMM that it
 // replaced, whose rows were mostly padding and whose split sums took a second launch: 45 rows of 8192 -> 3072 16.1 us, here 11.5;
 // the decode step of Llama-3.2-3B at 32 sequences 3.95 -> 3.33 ms, with whole-warp issue, the counted cut, sums sent 16 bytes at
-// a time and the warp index broadcast 2.60 ms (together with the decode attention's step).
+// a time and the warp index broadcast 2.67 ms (together with the decode attention's rings).
 #include <cuda.h>
 
 #include "affine_b4.cuh"

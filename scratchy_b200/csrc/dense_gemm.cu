@@ -1,4 +1,4 @@
-// bf16 GEMM on tcgen05 tensor cores for more than 16 rows: y = x W^T, f32 accumulators in TMEM, the ends of `scr_dense`
+// bf16 GEMM on tcgen05 tensor cores for more than 128 rows, and from 17 on where W is wide: y = x W^T, f32 accumulators in TMEM, the ends of `scr_dense`
 // in the epilogue.
 //
 // Persistent, warp-specialised CTA (192 threads), one per SM; a tile is 128 rows of x by BN (128 or 256) rows of W:

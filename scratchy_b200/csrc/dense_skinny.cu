@@ -8,9 +8,8 @@
 //   warp 9       producer of x (one tiled TMA load per slice, zeros outside)
 //   warp 10      owns TMEM; one elected lane issues 4 tcgen05.mma (128 x rows of x x 16) per slice
 //
-// What bounds it: the weights from HBM; for the small linears the start and end of a launch.  16384 x 3072 (100 MB) at 32 rows
-// 28.0 us with the MMAs issued from a divergent thread, 23.2 us (4.3 TB/s) from a whole warp; 128256 x 3072 139 and 132 us (6.0
-// TB/s).  Against the 128-row tile of dense_gemm.cu and its finishing launch: a decode step of the 3B Vumipel at 32 sequences
+// What bounds it: the weights from HBM; for the small linears the start and end of a launch.  10240 x 3072 (63 MB) at 32 rows
+// 14.9 us (4.2 TB/s), 3072 x 8192 13.3 us, 128256 x 3072 at 8 rows 120 us (6.5 TB/s), in streams of calls.  Against the 128-row tile of dense_gemm.cu and its finishing launch: a decode step of the 3B Vumipel at 32 sequences
 // 4.22 -> 3.59 ms, with that issue 3.31 -> 3.09 ms.
 #include "seq_common.cuh"
 #include "skinny.cuh"
