@@ -158,15 +158,16 @@ int32_t ds_launch_rows(scr_ctx* ctx, const scr_dense& d, const CUtensorMap& x_ma
 // Whether the GEMM for few rows takes this call (up to 128 rows of x, what one accumulator holds), or the tiles of 128 rows by up to 256
 // columns of dense_gemm.cu.  Those read x once for two of this kernel's tiles and pay for 128 rows whatever there are: they are ahead
 // where W is wide enough that they need no cut of k, and its long ends count where k is short.  Streams of calls, us, few rows / tiles:
-//   3072 -> 16384, 24 rows 22.3 / 20.3, 64 27.6 / 20.5, 128 30.7 / 21.4;  3072 -> 128256, 32 rows 132 / 130, 128 220 / 140
-//   2048 -> 12288, 32 rows 14.5 / 12.3;  3072 -> 10240, 64 rows 16.7 / 16.6, 65 21.8 / 16.5;  3072 -> 8192, 65 rows 14.2 / 15.4
+//   3072 -> 16384, 33 rows 24.1 / 20.5, 64 27.6 / 20.5, 128 30.7 / 21.4;  3072 -> 128256, 64 rows 154 / 134, 128 220 / 140
+//   2048 -> 12288, 33 rows 14.8 / 12.3;  3072 -> 10240, 64 rows 16.7 / 16.6, 65 21.8 / 16.5;  3072 -> 8192, 65 rows 14.2 / 15.4
 //   512 -> 3072, 64 rows 6.0 / 5.5, 128 8.0 / 6.5;  3072 -> 3072, 128 rows 11.1 / 13.7;  8192 -> 8192, 128 rows 35.0 / 40.0
-// (An x of less than 128 KB slows the tiles down: 3072 -> 16384 at 20 rows 22.2 / 28.2.)
+// Up to 32 rows, a decode batch, the two are close (3072 -> 16384, 32 rows 22.9 / 20.3, 20 rows 22.2 / 28.2), and only this kernel
+// fetches W while the norm before it runs, which a stream of linears alone does not show.
 bool dense_skinny_applies(int M, int N, int K, int groups) {
     const long long tiles = (long long)scr_ceil_div(N, SKINNY_ROWS) * groups;
     if (M <= 16) return true;
     if (M > 128) return false;
-    return !(tiles >= 96 && (long long)M * K >= 65536) && !(M > 64 && (tiles >= 80 || K <= 512));
+    return M <= 32 || (tiles < 96 && (M <= 64 || (tiles < 80 && K > 512)));
 }
 
 int32_t dense_skinny_launch(scr_ctx* ctx, const scr_dense& d, cudaStream_t stream) {

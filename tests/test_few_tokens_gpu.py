@@ -118,7 +118,7 @@ def test_no_unit_of_a_cut_is_left_without_steps(K):
     test_dense(300, K // 2 + 32, 200)
 
 
-@pytest.mark.parametrize("N,K,M", [(12296, 1032, 64), (12288, 1032, 63), (10250, 520, 65), (10100, 520, 65), (300, 512, 70), (300, 520, 70), (24584, 4104, 17)])
+@pytest.mark.parametrize("N,K,M", [(12296, 1032, 32), (12296, 1032, 33), (12160, 1032, 64), (10250, 520, 65), (10100, 520, 65), (300, 512, 70), (300, 520, 70), (24584, 4104, 17)])
 def test_dense_on_both_sides_of_the_wide_tiles(N, K, M):
     """17 to 128 rows where W's width or a short k decides for the tiles of 128 rows, and just before."""
     test_dense(N, K, M)
