@@ -162,7 +162,7 @@ int32_t ds_launch_rows(scr_ctx* ctx, const scr_dense& d, const CUtensorMap& x_ma
 //   2048 -> 12288, 33 rows 14.8 / 12.3;  3072 -> 10240, 64 rows 16.7 / 16.6, 65 21.8 / 16.5;  3072 -> 8192, 65 rows 14.2 / 15.4
 //   512 -> 3072, 64 rows 6.0 / 5.5, 128 8.0 / 6.5;  3072 -> 3072, 128 rows 11.1 / 13.7;  8192 -> 8192, 128 rows 35.0 / 40.0
 // Up to 32 rows, a decode batch, the two are close (3072 -> 16384, 32 rows 22.9 / 20.3, 20 rows 22.2 / 28.2), and only this kernel
-// fetches W while the norm before it runs, which a stream of linears alone does not show.
+// fetches W while the norm before it runs: with the tiles a decode step of the 3B Vumipel at 32 sequences took 3.23 ms, here 3.09.
 bool dense_skinny_applies(int M, int N, int K, int groups) {
     const long long tiles = (long long)scr_ceil_div(N, SKINNY_ROWS) * groups;
     if (M <= 16) return true;

@@ -141,9 +141,8 @@ __global__ void __launch_bounds__(RC_T) mlstm_recur_kernel(MemoryArgs a) {
 // The slice of S (and this slice's copy of n) in registers: 8 threads with 4 columns each cover a row, a thread has RPT rows, 32
 // apart.  The state's lines start for L2 before the wait for the preceding kernels and are read after it (one of those kernels may be
 // the call that leaves this one its state), and a token takes one barrier: the normaliser's n.q goes round with the outputs.
-// What bounds it: HBM, the state read and written once a step.  32 sequences of 12 heads of 128 x 256 (101 MB), alone and cold: 43.0 us
-// with the state in shared memory, asked for after the wait, and two barriers a token; 37.8 us here (both with about 4 us of the
-// measurement's own).
+// What bounds it: HBM, the state read and written once a step.  32 sequences of 12 heads of 128 x 256 (101 MB): 28.8 us (3.5 TB/s) a call in
+// the benchmark, 38 with the state in shared memory, asked for after the wait, and two barriers a token.
 template <typename T, int RPT>
 __global__ void __launch_bounds__(RC_T) mlstm_step_kernel(MemoryArgs a) {
     __shared__ float4 part[2][RC_T / 32][8];
