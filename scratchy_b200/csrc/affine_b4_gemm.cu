@@ -4,12 +4,12 @@
 //
 // Persistent, warp-specialised CTA (736 threads), one per SM.  A tile is 128 channels (the rows of the MMA) by `width` tokens (its
 // columns, 128 to 192):
-//   warps 0-15   dequantise: two groups of eight warps take alternate 128-k chunks; a thread expands 64 codes of one channel and
-//                writes them to TMEM with tcgen05.st, where the MMA reads its A operand: no swizzled shared-memory image and no
-//                proxy fence, and the shared memory holds activations in flight instead
+//   warps 0-15   dequantise: four groups of four warps take the halves (64 k) of alternate 128-k chunks; a thread expands 64 codes of
+//                one channel and writes them to TMEM with tcgen05.st, where the MMA reads its A operand: no swizzled shared-memory
+//                image and no proxy fence, and the shared memory holds activations in flight instead
 //   warps 16-19  epilogue: tcgen05.ld (lane = channel, column = token), one rounding to bf16 (or f32 partials), stores of 32
 //                consecutive channels of a token per warp
-//   warp 20      producer of the packed weights: one bulk copy per row-block and chunk, ahead of the preceding kernel
+//   warp 20      producer of the packed weights: one tiled copy per chunk (affine_b4_tc.cuh), ahead of the preceding kernel
 //   warp 21      producer of the activations: tiled TMA loads of 64 k x the tokens (128-byte swizzle, zeros outside)
 //   warp 22      owns TMEM; one elected lane issues 8 tcgen05.mma (128 x width x 16) per chunk and commits the barriers; the warp
 //                goes round as a whole so that the descriptors stay in uniform registers (a divergent thread spends about 55
@@ -17,15 +17,16 @@
 // TMEM holds two accumulators of 192 columns (the epilogue of a tile overlaps the main loop of the next) and two stages of 64
 // columns of dequantised weights.  No multicast: every CTA issues its own loads.
 //
-// What bounds it: a 128-k chunk takes about 1250 cycles, whether its MMAs have 128 columns or 192.  With two stages of dequantised weights
-// a chunk's way round (expansion, hand-over, eight MMAs, release) can be that bound as well as the MMAs with A in TMEM can; the
-// two have not been told apart.  Wide tiles pay, since a chunk is expanded once for all of a tile's tokens: 2048 tokens of 3072 -> 8192
-// 84 us (1.23 PFLOP/s) at 192, 104 us at 128.
+// What bounds it: the MMAs, 64 cycles for 128 columns and 96 for 192 (alone in a loop, A in TMEM: the tensor core's full rate), 768 a chunk
+// at 192, and for large calls the clock that the power limit leaves: 2048 tokens of 3072 -> 8192 73.7 us (1.40 PFLOP/s, what cuBLAS
+// sustains) in a stream of calls.  It was 83.7 us, 1250 cycles a chunk whatever the width, while one lane issued eight bulk copies a chunk
+// and the dequantised weights were handed over in stages of a whole chunk.  Wide tiles pay, since a chunk is expanded once for all of a
+// tile's tokens.
 #include <cuda.h>
 
 #include <algorithm>
 
-#include "affine_b4.cuh"
+#include "affine_b4_tc.cuh"
 #include "skinny.cuh"
 
 bool affine_b4_gemm_tc_enabled() { return true; }
@@ -43,11 +44,12 @@ size_t affine_b4_gemm_tc_workspace(int M, int N, int K) { return affine_b4_gemm_
 #define A4G_BN 128            // channels of a tile
 constexpr int A4G_THREADS = 736, A4G_DQ_WARPS = 16;
 constexpr int A4G_WIDTH = 192;                                  // tokens of a tile at most (a multiple of 16)
-// Activation stages of 64 k; packed-weight and dequantised stages, even in number: a stage always belongs to one of the two
-// groups, whose waits take its phases in order
+// Activation stages of 64 k; packed-weight and dequantised stages of 128 k, even in number: a stage always belongs to the same
+// groups, whose waits take its phases in order.  A dequantised stage is handed over and freed in halves of 64 k
 constexpr int A4G_SX = 7, A4G_SP = 4, A4G_SA = 2;
 constexpr uint32_t A4G_XSTAGE = A4G_WIDTH * 128u;
 constexpr uint32_t A4G_POFF = A4G_SX * A4G_XSTAGE;
+constexpr uint32_t A4G_BARS = 320;
 constexpr uint32_t A4G_TMEM = 512, A4G_ACOL = 2 * A4G_WIDTH;    // columns; where the dequantised stages start
 
 static __device__ __forceinline__ void a4g_tma_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
@@ -101,8 +103,8 @@ __global__ void __launch_bounds__(256) affine_b4_gemm_tail_finish_kernel(const f
 
 template <int GS>
 __global__ void __launch_bounds__(A4G_THREADS, 1)
-affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t* __restrict__ packed, uint16_t* __restrict__ y, int M, int N, int RB,
-                         int KC, int width, int MT, int out_f32, const uint16_t* __restrict__ bias, int full, int ks_tail, float* __restrict__ slabs,
+affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const uint8_t* __restrict__ packed,
+                         uint16_t* __restrict__ y, int M, int N, int RB, int KC, int width, int MT, int out_f32, const uint16_t* __restrict__ bias, int full, int ks_tail, float* __restrict__ slabs,
                          int* __restrict__ status) {
     constexpr uint32_t kBlock = aff_block_bytes(GS), kPStage = 8u * kBlock, kBarOff = A4G_POFF + A4G_SP * kPStage;
     extern __shared__ uint8_t smem_raw[];
@@ -114,11 +116,11 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_
     auto pfull = [&](int s) { return bar + 8u * (2 * A4G_SX + s); };
     auto pempty = [&](int s) { return bar + 8u * (2 * A4G_SX + A4G_SP + s); };
     auto afull = [&](int s) { return bar + 8u * (2 * A4G_SX + 2 * A4G_SP + s); };
-    auto aempty = [&](int s) { return bar + 8u * (2 * A4G_SX + 2 * A4G_SP + A4G_SA + s); };
-    constexpr int kAccSlot = 2 * A4G_SX + 2 * A4G_SP + 2 * A4G_SA;
+    auto aempty = [&](int s) { return bar + 8u * (2 * A4G_SX + 2 * A4G_SP + 2 * A4G_SA + s); };
+    constexpr int kAccSlot = 2 * A4G_SX + 2 * A4G_SP + 4 * A4G_SA;
     auto accf = [&](int b) { return bar + 8u * (kAccSlot + b); };
     auto acce = [&](int b) { return bar + 8u * (kAccSlot + 2 + b); };
-    static_assert(8 * (kAccSlot + 5) <= 256, "barriers");
+    static_assert(8 * (kAccSlot + 5) <= A4G_BARS, "barriers");
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kBarOff + 8 * (kAccSlot + 4));
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
@@ -129,7 +131,7 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_
     if (threadIdx.x == 0) {
         for (int s = 0; s < A4G_SX; ++s) { mbar_init(xfull(s), 1); mbar_init(xempty(s), 1); }
         for (int s = 0; s < A4G_SP; ++s) { mbar_init(pfull(s), 1); mbar_init(pempty(s), A4G_DQ_WARPS / 2); }
-        for (int s = 0; s < A4G_SA; ++s) { mbar_init(afull(s), A4G_DQ_WARPS / 2); mbar_init(aempty(s), 1); }
+        for (int s = 0; s < 2 * A4G_SA; ++s) { mbar_init(afull(s), A4G_DQ_WARPS / 4); mbar_init(aempty(s), 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(accf(b), 1); mbar_init(acce(b), 4); }
         fence_mbar_init();
     }
@@ -155,8 +157,7 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_
                     if (c == A4G_SP) skinny_pdl_wait();        // only the weights may be touched before the preceding kernel has finished
                     mbar_wait(pempty(s), ((uint32_t)(c / A4G_SP) & 1u) ^ 1u, status, TC_ERR_EMPTY_WAIT);
                     mbar_arrive_expect_tx(pfull(s), kPStage);
-                    for (int j = 0; j < 8; ++j)
-                        bulk_g2s(smem_base + A4G_POFF + s * kPStage + j * kBlock, packed + ((size_t)(rb0 + j) * KC + kc) * kBlock, kBlock, pfull(s));
+                    affine_load_chunk(smem_base + A4G_POFF + s * kPStage, &w_map, kc, rb0, pfull(s));
                 }
             }
         }
@@ -190,19 +191,19 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_
             mbar_wait(acce(buf), ((uint32_t)(it >> 1) & 1u) ^ 1u, status, TC_ERR_ACC_EMPTY);
             const uint32_t d = tmem + (uint32_t)(buf * A4G_WIDTH);
             for (int kc = kc_lo; kc < kc_hi; ++kc, ++c) {
-                const int a = c % A4G_SA;
-                const uint32_t ac = tmem + A4G_ACOL + (uint32_t)(64 * a);
-                mbar_wait(afull(a), (uint32_t)(c / A4G_SA) & 1u, status, TC_ERR_DEQ_WAIT);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
+                    const int a = 2 * (c % A4G_SA) + h;
+                    const uint32_t ac = tmem + A4G_ACOL + (uint32_t)(32 * a);
                     const uint64_t bdesc = umma_desc_k_sw128(smem_base + s * A4G_XSTAGE);
                     mbar_wait(xfull(s), ph, status, TC_ERR_FULL_WAIT);
+                    mbar_wait(afull(a), (uint32_t)(c / A4G_SA) & 1u, status, TC_ERR_DEQ_WAIT);
                     tc_fence_after();
                     if (lead) {
 #pragma unroll
                         for (int k4 = 0; k4 < 4; ++k4)
-                            umma_f16_ta(d, ac + (uint32_t)(32 * h + 8 * k4), bdesc + (uint64_t)(2 * k4), idesc, kc > kc_lo || h > 0 || k4 > 0);
-                        if (h == 1) umma_commit(aempty(a));
+                            umma_f16_ta(d, ac + (uint32_t)(8 * k4), bdesc + (uint64_t)(2 * k4), idesc, kc > kc_lo || h > 0 || k4 > 0);
+                        umma_commit(aempty(a));
                         umma_commit(xempty(s));
                     }
                     __syncwarp();
@@ -214,8 +215,8 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_
         }
     } else if (warp < A4G_DQ_WARPS) {
         const bool check = *reinterpret_cast<const unsigned int*>(packed + (size_t)RB * KC * kBlock) != 0;
-        const int grp = warp >> 3, kh = (warp >> 2) & 1, row = (warp & 3) * 32 + lane, half = (row >> 3) & 1, g = row & 7;
-        const uint32_t dst0 = tmem + A4G_ACOL + (uint32_t)(32 * kh) + ((uint32_t)((warp & 3) * 32) << 16);
+        const int grp = warp >> 2, kh = grp & 1, row = (warp & 3) * 32 + lane, half = (row >> 3) & 1, g = row & 7;
+        const uint32_t dst0 = tmem + A4G_ACOL + (uint32_t)(32 * grp) + ((uint32_t)((warp & 3) * 32) << 16);
         const uint32_t src0 = smem_base + A4G_POFF + (uint32_t)((row >> 4) * kBlock);
         int c = 0;
         bool waited = false;
@@ -223,7 +224,7 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_
             int tile, ks, kc_lo, kc_hi;
             tc_unit(unit, full, ks_tail, KC, tile, ks, kc_lo, kc_hi);
             for (int kc = kc_lo; kc < kc_hi; ++kc, ++c) {
-                if ((c & 1) != grp) continue;
+                if ((c & 1) != grp >> 1) continue;
                 const int s = c % A4G_SP;
                 if (c >= A4G_SA && !waited) {
                     skinny_pdl_wait();                 // from here on a wait depends on the activations
@@ -252,7 +253,7 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_
                         affine_dequant_word_scaled(piece[t].z, cs, w + 8);
                         affine_dequant_word_scaled(piece[t].w, cs, w + 12);
                     }
-                    tmem_st_32x16(dst0 + (uint32_t)(64 * grp + 16 * t), w);
+                    tmem_st_32x16(dst0 + (uint32_t)(16 * t), w);
                 }
                 tmem_st_wait();
                 tc_fence_before();
@@ -352,12 +353,14 @@ size_t affine_b4_gemm_tc_workspace_plan(int M, int N, int K) {
 }
 
 template <int GS>
-static int32_t affine_gemm_launch(scr_ctx* ctx, const CUtensorMap& map, const uint8_t* packed, uint16_t* y, int M, int N, int K, int out_f32,
+static int32_t affine_gemm_launch(scr_ctx* ctx, tc_encode_tiled_fn enc, const CUtensorMap& map, const uint8_t* packed, uint16_t* y, int M, int N, int K, int out_f32,
                                   const uint16_t* bias, const AffineGemmPlan& p, float* slabs, cudaStream_t stream) {
     const AffineGeom g = affine_geom(N, K, 64);
     const int units = p.full + p.n_tail() * p.ks_tail;
-    constexpr size_t smem = A4G_POFF + A4G_SP * 8u * aff_block_bytes(GS) + 256 + 1024;
-    const cudaError_t e = skinny_launch(affine_b4_gemm_tc_kernel<GS>, std::min(units, ctx->sm_count), 1, A4G_THREADS, smem, stream, map, packed, y, M, N, g.RB,
+    CUtensorMap w_map;
+    if (!affine_w_map(&w_map, enc, packed, g.RB, g.KC, GS)) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled failed");
+    constexpr size_t smem = A4G_POFF + A4G_SP * 8u * aff_block_bytes(GS) + A4G_BARS + 1024;
+    const cudaError_t e = skinny_launch(affine_b4_gemm_tc_kernel<GS>, std::min(units, ctx->sm_count), 1, A4G_THREADS, smem, stream, map, w_map, packed, y, M, N, g.RB,
                                         g.KC, p.width, p.mt, out_f32, bias, p.full, p.ks_tail, slabs, ctx->dev_status);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "affine_b4_gemm_tc: %s", cudaGetErrorString(e));
     const int32_t st = scr_check_launch(ctx, "affine_b4_gemm_tc");
@@ -394,6 +397,6 @@ int32_t affine_b4_gemm_tc_launch(scr_ctx* ctx, const uint8_t* packed, const uint
     float* slabs = reinterpret_cast<float*>(workspace);
     if (plan.ks_tail > 1 && (!slabs || !scr_aligned16(slabs))) return scr_fail(ctx, SCR_E_WORKSPACE, "split-K needs an aligned workspace");
     if (!affine_gemm_x_map(&map, enc, x, M, K, plan.width)) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled failed");
-    return gs == 2 ? affine_gemm_launch<2>(ctx, map, packed, y, M, N, K, out_f32, bias, plan, slabs, stream)
-                   : affine_gemm_launch<1>(ctx, map, packed, y, M, N, K, out_f32, bias, plan, slabs, stream);
+    return gs == 2 ? affine_gemm_launch<2>(ctx, enc, map, packed, y, M, N, K, out_f32, bias, plan, slabs, stream)
+                   : affine_gemm_launch<1>(ctx, enc, map, packed, y, M, N, K, out_f32, bias, plan, slabs, stream);
 }

@@ -14,7 +14,7 @@
 //
 // Per CTA (704 threads), both CTAs of a pair run the same code:
 //   warp 0       producer: per chunk 2 tiled TMA loads of this CTA's activations (`.cta_group::2`, completing on the
-//                LEADER's barrier; no multicast) and 8 bulk copies of this CTA's packed weight blocks
+//                LEADER's barrier; no multicast) and one of this CTA's packed weight blocks
 //   warp 1       leader CTA only: waits for both CTAs' activations and dequantised weights; one elected lane issues 8 MMAs
 //                (2 atoms of 64 k x 4 steps of K = 16) and commits to the stages' `empty` barriers of both CTAs
 //   warps 2-17   dequantise this CTA's 128 channels into the K-major 128-byte-swizzled operand image; lane 0 of each warp
@@ -25,8 +25,7 @@
 
 #include <cstdlib>
 
-#include "affine_b4.cuh"
-#include "tc_common.cuh"
+#include "affine_b4_tc.cuh"
 
 namespace {
 
@@ -94,8 +93,8 @@ __device__ __forceinline__ uint32_t a4p_ld_shared_u32(uint32_t addr) {
 }
 
 __global__ void __launch_bounds__(A4P_THREADS, 1)
-affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t* __restrict__ packed, uint16_t* __restrict__ y,
-                           int M, int N, int RB, int KC, int gs, int MTP, int out_f32, const uint16_t* __restrict__ bias,
+affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const uint8_t* __restrict__ packed,
+                           uint16_t* __restrict__ y, int M, int N, int RB, int KC, int gs, int MTP, int out_f32, const uint16_t* __restrict__ bias,
                            int* __restrict__ status) {
     const uint32_t block_bytes = (uint32_t)aff_block_bytes(gs);       // 1152 (groups of 64, 128) or 1280 (groups of 32)
     extern __shared__ uint8_t smem_raw[];
@@ -150,9 +149,7 @@ affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const uint
                 for (int kc = 0; kc < KC; ++kc) {
                     mbar_wait(pempty(sp), php ^ 1u, status, TC_ERR_EMPTY_WAIT);
                     mbar_arrive_expect_tx(pfull(sp), 8u * block_bytes);
-                    for (int j = 0; j < 8; ++j)
-                        bulk_g2s(smem_base + A4P_POFF + sp * A4P_PSTAGE + j * block_bytes,
-                                 packed + ((size_t)(rb0 + j) * KC + kc) * block_bytes, block_bytes, pfull(sp));
+                    affine_load_chunk(smem_base + A4P_POFF + sp * A4P_PSTAGE, &w_map, kc, rb0, pfull(sp));
                     if (++sp == A4P_SP) { sp = 0; php ^= 1u; }
                 }
             }
@@ -409,8 +406,11 @@ int32_t affine_b4_gemm_pair_launch(scr_ctx* ctx, const CUtensorMap& x_map, const
     if (max_pairs < 1) return SCR_OK;                     // not launched: the caller runs the one-CTA kernel
     const int MTP = scr_ceil_div(M, 256);
     const int tiles = MTP * (g.RB / 16);
+    CUtensorMap w_map;
+    tc_encode_tiled_fn enc = tc_tensor_map_encoder();
+    if (!enc || !affine_w_map(&w_map, enc, packed, g.RB, g.KC, gs)) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled failed");
     cfg.gridDim = dim3(2 * std::min(tiles, max_pairs));
-    e = cudaLaunchKernelEx(&cfg, affine_b4_gemm_pair_kernel, x_map, packed, y, M, N, g.RB, g.KC, gs, MTP, out_f32, bias,
+    e = cudaLaunchKernelEx(&cfg, affine_b4_gemm_pair_kernel, x_map, w_map, packed, y, M, N, g.RB, g.KC, gs, MTP, out_f32, bias,
                            ctx->dev_status);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "affine gemm pair launch: %s", cudaGetErrorString(e));
     *launched = true;

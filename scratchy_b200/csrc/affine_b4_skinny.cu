@@ -6,20 +6,21 @@
 //   warps 0-7    dequantise: two groups of four warps take alternate chunks; a thread expands the 128 codes of ONE channel
 //                and writes them to TMEM with tcgen05.st, where the MMA reads its A operand: no swizzled shared-memory
 //                image, no proxy fence.  Afterwards they drain the accumulator.
-//   warp 8       producer of the packed weights (8 bulk copies of a block per chunk), which are load-time constants: it
-//                starts before the preceding kernel of the stream has finished
+//   warp 8       producer of the packed weights (one tiled copy of 8 blocks per chunk, affine_b4_tc.cuh), which are load-time
+//                constants: it starts before the preceding kernel of the stream has finished
 //   warp 9       producer of the activations (2 tiled TMA loads of 64 k x the tokens, 128-byte swizzle, zeros outside)
 //   warp 10      owns TMEM; one elected lane issues 8 tcgen05.mma (128 x tokens x 16) per chunk
 //
 // What bounds it: for the short k extents of a layer's linears the start of the pipeline and the two cluster barriers at its end
-// (4 of the 7 us of a 3072 x 3072), for long ones about 1000 cycles per chunk and SM however few the columns (a chunk's 9.2 KB from HBM
-// would take 400): eight MMAs with A in TMEM, or a chunk's way round the stages; not told apart.  Against the 128-token tile of the prefill GEMM that it
+// (4 of the 7 us of a 3072 x 3072), for long ones HBM and the way of a chunk round the stages, about 500 cycles a chunk and SM (its 9.2 KB take
+// 400 from HBM, its eight MMAs 16 a column of 32: 128 at 32 tokens, 512 at 128).  It was 1000 cycles while one lane issued eight bulk copies a
+// chunk.  Against the 128-token tile of the prefill GEMM that it
 // replaced, whose rows were mostly padding and whose split sums took a second launch: 45 rows of 8192 -> 3072 16.1 us, here 11.5;
 // the decode step of Llama-3.2-3B at 32 sequences 3.95 -> 3.33 ms, with whole-warp issue, the counted cut, sums sent 16 bytes at
 // a time and the warp index broadcast 2.67 ms (together with the decode attention's rings).
 #include <cuda.h>
 
-#include "affine_b4.cuh"
+#include "affine_b4_tc.cuh"
 #include "skinny.cuh"
 
 namespace {
@@ -85,8 +86,8 @@ __device__ __forceinline__ void a4s_expand(uint32_t stage, int row, uint32_t dst
 
 template <int TN, int GS>
 __global__ void __launch_bounds__(A4S_THREADS, A4SCfg<TN>::kCtasPerSm)
-affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t* __restrict__ packed, uint16_t* __restrict__ y, int M, int N, int RB,
-                        int KC, int split, int out_f32, const uint16_t* __restrict__ bias, int* __restrict__ status) {
+affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const uint8_t* __restrict__ packed,
+                        uint16_t* __restrict__ y, int M, int N, int RB, int KC, int split, int out_f32, const uint16_t* __restrict__ bias, int* __restrict__ status) {
     using C = A4SCfg<TN>;
     constexpr uint32_t kBlock = aff_block_bytes(GS), kPStage = 8u * kBlock, kBarOff = C::kPOff + C::kSP * kPStage;
     extern __shared__ uint8_t smem_raw[];
@@ -136,8 +137,7 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t
                 if (i == C::kSP) skinny_pdl_wait();
                 mbar_wait(pempty(s), ((uint32_t)(i / C::kSP) & 1u) ^ 1u, status, TC_ERR_EMPTY_WAIT);
                 mbar_arrive_expect_tx(pfull(s), kPStage);
-                for (int j = 0; j < 8; ++j)
-                    bulk_g2s(smem_base + C::kPOff + s * kPStage + j * kBlock, packed + ((size_t)(tile * 8 + j) * KC + kc_lo + i) * kBlock, kBlock, pfull(s));
+                affine_load_chunk(smem_base + C::kPOff + s * kPStage, &w_map, kc_lo + i, tile * 8, pfull(s));
             }
         }
     } else if (warp == 9) {
@@ -228,16 +228,18 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t
 }
 
 template <int TN, int GS>
-int32_t a4s_launch(scr_ctx* ctx, const CUtensorMap& map, const uint8_t* packed, uint16_t* y, int M, int N, int K, int out_f32, const uint16_t* bias,
+int32_t a4s_launch(scr_ctx* ctx, tc_encode_tiled_fn enc, const CUtensorMap& map, const uint8_t* packed, uint16_t* y, int M, int N, int K, int out_f32, const uint16_t* bias,
                    cudaStream_t stream) {
     using C = A4SCfg<TN>;
     const AffineGeom g = affine_geom(N, K, 64);          // RB / KC only: the same for every group size
     constexpr size_t smem = C::kPOff + C::kSP * 8u * aff_block_bytes(GS) + 512 + 1024;
     static_assert(C::kPOff + C::kSP * 8u * aff_block_bytes(GS) >= skinny_sum_bytes(TN), "the sums fit the rings");
+    CUtensorMap w_map;
+    if (!affine_w_map(&w_map, enc, packed, g.RB, g.KC, GS)) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled failed");
     static SkinnyResident resident;
     const int tiles = g.RB / 8;
     const int split = skinny_split(resident, affine_b4_skinny_kernel<TN, GS>, ctx->device, ctx->sm_count, tiles, g.KC, A4S_THREADS, smem, 3.0f);
-    const cudaError_t e = skinny_launch(affine_b4_skinny_kernel<TN, GS>, tiles, split, A4S_THREADS, smem, stream, map, packed, y, M, N, g.RB, g.KC, split,
+    const cudaError_t e = skinny_launch(affine_b4_skinny_kernel<TN, GS>, tiles, split, A4S_THREADS, smem, stream, map, w_map, packed, y, M, N, g.RB, g.KC, split,
                                         out_f32, bias, ctx->dev_status);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "affine_b4_skinny: %s", cudaGetErrorString(e));
     return scr_check_launch(ctx, "affine_b4_skinny");
@@ -263,8 +265,8 @@ int32_t affine_b4_skinny_launch(scr_ctx* ctx, const uint8_t* packed, const uint1
     const CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t*>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-#define A4S_CASE(TN) (gs == 2 ? a4s_launch<TN, 2>(ctx, map, packed, y, M, N, K, out_f32, bias, stream) \
-                              : a4s_launch<TN, 1>(ctx, map, packed, y, M, N, K, out_f32, bias, stream))
+#define A4S_CASE(TN) (gs == 2 ? a4s_launch<TN, 2>(ctx, enc, map, packed, y, M, N, K, out_f32, bias, stream) \
+                              : a4s_launch<TN, 1>(ctx, enc, map, packed, y, M, N, K, out_f32, bias, stream))
     if (M <= 32) return A4S_CASE(32);
     if (M <= 64) return A4S_CASE(64);
     return A4S_CASE(128);

@@ -47,6 +47,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 }
 // Bounded wait.  Returns false (and records `code`) when the limit ran out.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status, int code) {
+    if (mbar_try_wait(bar, parity)) return true;       // (ahead of the counting loop: a passing wait 69 cycles instead of 89)
     for (uint32_t i = 0; i < TC_WAIT_LIMIT; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         // once any wait anywhere in the grid has run out, every later wait gives up at once
