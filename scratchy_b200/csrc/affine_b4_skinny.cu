@@ -11,13 +11,11 @@
 //   warp 9       producer of the activations (2 tiled TMA loads of 64 k x the tokens, 128-byte swizzle, zeros outside)
 //   warp 10      owns TMEM; one elected lane issues 8 tcgen05.mma (128 x tokens x 16) per chunk
 //
-// What bounds it: for the short k extents of a layer's linears the start of the pipeline and the two cluster barriers at its end
-// (4 of the 7 us of a 3072 x 3072), for long ones HBM and the way of a chunk round the stages, about 500 cycles a chunk and SM (its 9.2 KB take
-// 400 from HBM, its eight MMAs 16 a column of 32: 128 at 32 tokens, 512 at 128).  It was 1000 cycles while one lane issued eight bulk copies a
-// chunk.  Against the 128-token tile of the prefill GEMM that it
-// replaced, whose rows were mostly padding and whose split sums took a second launch: 45 rows of 8192 -> 3072 16.1 us, here 11.5;
-// the decode step of Llama-3.2-3B at 32 sequences 3.95 -> 3.33 ms, with whole-warp issue, the counted cut, sums sent 16 bytes at
-// a time and the warp index broadcast 2.67 ms (together with the decode attention's rings).
+// What bounds it: 1.0 us from the end of the kernel before to the release of the wait and 0.4 to the first activations, then HBM and the way of
+// a chunk round the stages, about 0.31 us a chunk and SM (its 9.2 KB take 0.21 from HBM, its eight MMAs 0.07 at 32 tokens, 0.26 at 128), then
+// about 2 us for the sums and the stores.  45 tokens of 8192 -> 3072 8.6 us in a stream of calls: 16.1 on the 128-token tiles of the
+// prefill GEMM, 11.4 with a bulk copy for every block, two CTAs to an SM and two cluster barriers at the end.  The decode step of
+// Llama-3.2-3B at 32 sequences 2.66 -> 2.31 ms by the last three.
 #include <cuda.h>
 
 #include "affine_b4_tc.cuh"
@@ -87,9 +85,10 @@ __device__ __forceinline__ void a4s_expand(uint32_t stage, int row, uint32_t dst
 template <int TN, int GS>
 __global__ void __launch_bounds__(A4S_THREADS, A4SCfg<TN>::kCtasPerSm)
 affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const uint8_t* __restrict__ packed,
-                        uint16_t* __restrict__ y, int M, int N, int RB, int KC, int split, int out_f32, const uint16_t* __restrict__ bias, int* __restrict__ status) {
+                        uint16_t* __restrict__ y, int M, int N, int RB, int KC, int split, int over_rings,
+                        int out_f32, const uint16_t* __restrict__ bias, int* __restrict__ status) {
     using C = A4SCfg<TN>;
-    constexpr uint32_t kBlock = aff_block_bytes(GS), kPStage = 8u * kBlock, kBarOff = C::kPOff + C::kSP * kPStage;
+    constexpr uint32_t kBlock = aff_block_bytes(GS), kPStage = 8u * kBlock, kBarOff = C::kPOff + C::kSP * kPStage, kSumOff = kBarOff + 512u;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -101,8 +100,9 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_
     auto afull = [&](int s) { return bar + 8u * (2 * C::kSX + 2 * C::kSP + s); };
     auto aempty = [&](int s) { return bar + 8u * (2 * C::kSX + 2 * C::kSP + C::kSA + s); };
     constexpr int kSlots = 2 * C::kSX + 2 * C::kSP + 2 * C::kSA;
-    const uint32_t accf = bar + 8u * kSlots;
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kBarOff + 8 * (kSlots + 1));
+    const uint32_t accf = bar + 8u * kSlots, rbar = accf + 8u;
+    static_assert(8 * (kSlots + 3) <= 512, "barriers");
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kBarOff + 8 * (kSlots + 2));
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int tile = blockIdx.x / split, rank = blockIdx.x - tile * split;
@@ -115,6 +115,7 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_
         for (int s = 0; s < C::kSP; ++s) { mbar_init(pfull(s), 1); mbar_init(pempty(s), 4); }
         for (int s = 0; s < C::kSA; ++s) { mbar_init(afull(s), 4); mbar_init(aempty(s), 1); }
         mbar_init(accf, 1);
+        skinny_expect(rbar, M, split, rank, over_rings);
         fence_mbar_init();
     }
     if (warp == 10) {
@@ -125,6 +126,7 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if (split > 1 && !over_rings) skinny_cluster_arrive();
     skinny_pdl_trigger();                              // not before this CTA has its TMEM: the next kernel's CTAs could take it first
     auto a_col = [&](int s) { return tmem + (uint32_t)(TN + 64 * s); };
 
@@ -206,7 +208,9 @@ affine_b4_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_
     __syncwarp();
     const float factor = (*reinterpret_cast<const unsigned int*>(packed + (size_t)RB * KC * kBlock) != 0) ? 1.0f : AFF_SCALED_FACTOR;
     skinny_pdl_wait();
-    skinny_finish(tmem, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, tile * SKINNY_ROWS, N, [&](int m, int n, float a, float b) {
+    const uint32_t sums = over_rings ? 0 : kSumOff;
+    skinny_finish<true>(tmem, smem_base + sums, reinterpret_cast<const float*>(smem_gen + sums), over_rings != 0, rbar, M, split, rank, tile * SKINNY_ROWS, N, status,
+                  [&](int m, int n, float a, float b) {
         const float v[2] = {a * factor, b * factor};
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
@@ -238,9 +242,9 @@ int32_t a4s_launch(scr_ctx* ctx, tc_encode_tiled_fn enc, const CUtensorMap& map,
     if (!affine_w_map(&w_map, enc, packed, g.RB, g.KC, GS)) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled failed");
     static SkinnyResident resident;
     const int tiles = g.RB / 8;
-    const int split = skinny_split(resident, affine_b4_skinny_kernel<TN, GS>, ctx->device, ctx->sm_count, tiles, g.KC, A4S_THREADS, smem, 3.0f);
-    const cudaError_t e = skinny_launch(affine_b4_skinny_kernel<TN, GS>, tiles, split, A4S_THREADS, smem, stream, map, w_map, packed, y, M, N, g.RB, g.KC, split,
-                                        out_f32, bias, ctx->dev_status);
+    const SkinnyPlan p = skinny_plan(resident, affine_b4_skinny_kernel<TN, GS>, ctx->device, ctx->sm_count, tiles, g.KC, A4S_THREADS, smem, TN, 3.0f);
+    const cudaError_t e = skinny_launch(affine_b4_skinny_kernel<TN, GS>, tiles, p.split, A4S_THREADS, p.smem, stream, map, w_map, packed, y, M, N, g.RB, g.KC, p.split,
+                                        p.over_rings, out_f32, bias, ctx->dev_status);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "affine_b4_skinny: %s", cudaGetErrorString(e));
     return scr_check_launch(ctx, "affine_b4_skinny");
 }

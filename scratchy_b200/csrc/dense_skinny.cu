@@ -34,7 +34,7 @@ struct DsCfg {
 template <int TN, DenseEnd END>
 __global__ void __launch_bounds__(DS_THREADS, DsCfg<TN>::kCtasPerSm)
 dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, int M, int N, int KT, int NT, int split,
-                    int w_fresh, DenseEnds ends, int* __restrict__ status) {
+                    int over_rings, int w_fresh, DenseEnds ends, int* __restrict__ status) {
     using C = DsCfg<TN>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -45,9 +45,9 @@ dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_cons
     auto xfull = [&](int s) { return bar + 8u * (2 * C::kSW + s); };
     auto xempty = [&](int s) { return bar + 8u * (2 * C::kSW + C::kSX + s); };
     constexpr int kSlots = 2 * C::kSW + 2 * C::kSX;
-    static_assert(8 * (kSlots + 2) <= 256, "barriers");
-    const uint32_t accf = bar + 8u * kSlots;
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + C::kBarOff + 8 * (kSlots + 1));
+    static_assert(8 * (kSlots + 3) <= 256, "barriers");
+    const uint32_t accf = bar + 8u * kSlots, rbar = accf + 8u;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + C::kBarOff + 8 * (kSlots + 2));
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int tile = blockIdx.x / split, rank = blockIdx.x - tile * split;
@@ -60,6 +60,7 @@ dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_cons
         for (int s = 0; s < C::kSW; ++s) { mbar_init(wfull(s), 1); mbar_init(wempty(s), 1); }
         for (int s = 0; s < C::kSX; ++s) { mbar_init(xfull(s), 1); mbar_init(xempty(s), 1); }
         mbar_init(accf, 1);
+        skinny_expect(rbar, M, split, rank, over_rings);
         fence_mbar_init();
     }
     if (warp == 10) {
@@ -70,6 +71,7 @@ dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if (split > 1 && !over_rings) skinny_cluster_arrive();
     pdl_trigger();                                     // not before this CTA has its TMEM: the next kernel's CTAs could take it first
 
     // Only the weights may be touched before the preceding kernel has finished.  A wait that depends on x comes after
@@ -123,7 +125,8 @@ dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_cons
     }
     __syncwarp();
     pdl_wait();
-    skinny_finish(tmem, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, n0, N,
+    const uint32_t sums = over_rings ? 0 : C::kBarOff + 256u;
+    skinny_finish<(TN <= 64)>(tmem, smem_base + sums, reinterpret_cast<const float*>(smem_gen + sums), over_rings != 0, rbar, M, split, rank, n0, N, status,
                   [&](int m, int n, float a, float b) { dense_put_two<bf16, END>(ends, m, g, n, N, a, b); });
     __syncthreads();
     if (warp == 10) {
@@ -138,9 +141,9 @@ int32_t ds_launch(scr_ctx* ctx, const scr_dense& d, const CUtensorMap& x_map, co
     static_assert(C::kBarOff >= skinny_sum_bytes(TN), "the sums fit the rings");
     const int nt = scr_ceil_div(d.N, SKINNY_ROWS), kt = scr_ceil_div(d.K, 64);
     static SkinnyResident resident;
-    const int split = skinny_split(resident, dense_skinny_kernel<TN, END>, ctx->device, ctx->sm_count, nt * d.groups, kt, DS_THREADS, C::kTotal, 4.0f);
-    const cudaError_t e = skinny_launch(dense_skinny_kernel<TN, END>, nt * d.groups, split, DS_THREADS, C::kTotal, stream, x_map, w_map, d.M, d.N, kt, nt,
-                                        split, (int)(d.w_fresh != 0), dense_ends(d), ctx->dev_status);
+    const SkinnyPlan p = skinny_plan(resident, dense_skinny_kernel<TN, END>, ctx->device, ctx->sm_count, nt * d.groups, kt, DS_THREADS, C::kTotal, TN, 4.0f);
+    const cudaError_t e = skinny_launch(dense_skinny_kernel<TN, END>, nt * d.groups, p.split, DS_THREADS, p.smem, stream, x_map, w_map, d.M, d.N, kt, nt,
+                                        p.split, p.over_rings, (int)(d.w_fresh != 0), dense_ends(d), ctx->dev_status);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "dense_skinny: %s", cudaGetErrorString(e));
     return scr_check_launch(ctx, "dense_skinny");
 }

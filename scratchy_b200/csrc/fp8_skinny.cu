@@ -12,7 +12,7 @@
 //   warp 10      owns TMEM; one elected lane issues 4 tcgen05.mma (128 x tokens x 32) per step
 //
 // What bounds it: the copies into shared memory, 16 KB of weights and 128 bytes per token and step.  250 tokens of 18944 -> 3584
-// (with the quantisation) 46.4 us on the 128-token tiles of fp8_gemm.cu and their finishing launch, 33 us here.
+// (with the quantisation) 46.4 us on the 128-token tiles of fp8_gemm.cu and their finishing launch, 32.5 us here.
 #include "fp8.cuh"
 #include "skinny.cuh"
 
@@ -35,7 +35,7 @@ struct F8SCfg {
 template <int TN>
 __global__ void __launch_bounds__(F8S_THREADS, F8SCfg<TN>::kCtasPerSm)
 fp8_skinny_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ w_scale, const uint8_t* __restrict__ xq, const float* __restrict__ a_scale,
-                  uint16_t* __restrict__ y, int M, int N, int KT, int M_pad, int split, int out_f32, const uint16_t* __restrict__ bias,
+                  uint16_t* __restrict__ y, int M, int N, int KT, int M_pad, int split, int over_rings, int out_f32, const uint16_t* __restrict__ bias,
                   int* __restrict__ status) {
     using C = F8SCfg<TN>;
     extern __shared__ uint8_t smem_raw[];
@@ -47,9 +47,9 @@ fp8_skinny_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ w
     auto xfull = [&](int s) { return bar + 8u * (2 * C::kSW + s); };
     auto xempty = [&](int s) { return bar + 8u * (2 * C::kSW + C::kSX + s); };
     constexpr int kSlots = 2 * C::kSW + 2 * C::kSX;
-    static_assert(8 * (kSlots + 2) <= 256, "barriers");
-    const uint32_t accf = bar + 8u * kSlots;
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + C::kBarOff + 8 * (kSlots + 1));
+    static_assert(8 * (kSlots + 3) <= 256, "barriers");
+    const uint32_t accf = bar + 8u * kSlots, rbar = accf + 8u;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + C::kBarOff + 8 * (kSlots + 2));
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int tile = blockIdx.x / split, rank = blockIdx.x - tile * split;
@@ -62,6 +62,7 @@ fp8_skinny_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ w
         for (int s = 0; s < C::kSW; ++s) { mbar_init(wfull(s), 1); mbar_init(wempty(s), 1); }
         for (int s = 0; s < C::kSX; ++s) { mbar_init(xfull(s), 1); mbar_init(xempty(s), 1); }
         mbar_init(accf, 1);
+        skinny_expect(rbar, M, split, rank, over_rings);
         fence_mbar_init();
     }
     if (warp == 10) {
@@ -72,6 +73,7 @@ fp8_skinny_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ w
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if (split > 1 && !over_rings) skinny_cluster_arrive();
     skinny_pdl_trigger();                              // not before this CTA has its TMEM: the next kernel's CTAs could take it first
 
     // Only the weights may be touched before the preceding kernel has finished.  A wait that depends on the activations
@@ -123,7 +125,8 @@ fp8_skinny_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ w
     }
     __syncwarp();
     skinny_pdl_wait();
-    skinny_finish(tmem, smem_base, reinterpret_cast<const float*>(smem_gen), M, split, rank, tile * SKINNY_ROWS, N,
+    const uint32_t sums = over_rings ? 0 : C::kBarOff + 256u;
+    skinny_finish<true>(tmem, smem_base + sums, reinterpret_cast<const float*>(smem_gen + sums), over_rings != 0, rbar, M, split, rank, tile * SKINNY_ROWS, N, status,
                          [&](int m, int n, float a, float b) {
         const float as = a_scale[m], v[2] = {a, b};
 #pragma unroll
@@ -147,9 +150,9 @@ fp8_skinny_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ w
 }
 
 template <int TN>
-int f8s_split(const scr_ctx* ctx, const Fp8Geom& g) {
+SkinnyPlan f8s_plan(const scr_ctx* ctx, const Fp8Geom& g) {
     static SkinnyResident resident;
-    return skinny_split(resident, fp8_skinny_kernel<TN>, ctx->device, ctx->sm_count, g.NT, g.KT, F8S_THREADS, F8SCfg<TN>::kTotal, 4.0f);
+    return skinny_plan(resident, fp8_skinny_kernel<TN>, ctx->device, ctx->sm_count, g.NT, g.KT, F8S_THREADS, F8SCfg<TN>::kTotal, TN, 4.0f);
 }
 
 template <int TN>
@@ -157,10 +160,10 @@ int32_t f8s_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint1
     using C = F8SCfg<TN>;
     static_assert(C::kBarOff >= skinny_sum_bytes(TN), "the sums fit the rings");
     const Fp8Geom g = fp8_geom(N, K);
-    const int split = f8s_split<TN>(ctx, g);
+    const SkinnyPlan p = f8s_plan<TN>(ctx, g);
     const float* w_scale = reinterpret_cast<const float*>(wpack + (size_t)g.NT * g.KT * FP8_TILE_BYTES);
-    const cudaError_t e = skinny_launch(fp8_skinny_kernel<TN>, g.NT, split, F8S_THREADS, C::kTotal, stream, wpack, w_scale, act + fp8_act_scale_bytes(M),
-                                        reinterpret_cast<const float*>(act), y, M, N, g.KT, scr_ceil_div(M, FP8_TILE) * FP8_TILE, split, ends.out_f32,
+    const cudaError_t e = skinny_launch(fp8_skinny_kernel<TN>, g.NT, p.split, F8S_THREADS, p.smem, stream, wpack, w_scale, act + fp8_act_scale_bytes(M),
+                                        reinterpret_cast<const float*>(act), y, M, N, g.KT, scr_ceil_div(M, FP8_TILE) * FP8_TILE, p.split, p.over_rings, ends.out_f32,
                                         ends.bias, ctx->dev_status);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "fp8_skinny: %s", cudaGetErrorString(e));
     return scr_check_launch(ctx, "fp8_skinny");
@@ -172,7 +175,7 @@ int32_t f8s_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint1
 // 0.0335 a token (fitted to streams of calls: 3584 x 18944 at 256 tokens 27.4, 3584 x 3584 15.3, 8192 x 1024 15.2, 512 x 512 11.2).
 float fp8_skinny_us(const scr_ctx* ctx, int M, int N, int K) {
     const Fp8Geom g = fp8_geom(N, K);
-    const int split = M <= 128 ? f8s_split<128>(ctx, g) : f8s_split<256>(ctx, g);
+    const int split = M <= 128 ? f8s_plan<128>(ctx, g).split : f8s_plan<256>(ctx, g).split;
     const int rounds = scr_ceil_div(g.NT * split, ctx->sm_count);
     return 2.3f + 0.0335f * M + (float)(rounds * scr_ceil_div(g.KT, split)) * (0.40f + 0.0006f * M);
 }

@@ -91,6 +91,17 @@ def test_fp8(N, K, M):
     assert torch.equal((part + bias.float()).bfloat16().view(torch.int16), yb.view(torch.int16))
 
 
+@pytest.mark.parametrize("tiles", [147, 148, 149, 300])
+def test_calls_whose_clusters_do_not_all_run_at_once(tiles):
+    """As many tiles of 128 channels as SMs, where every CTA has its SM and memory for the sums to itself, and more, where two share an
+    SM and the sums lie over the rings; runs of tokens that are added four at a time and one at a time."""
+    N = 128 * tiles - 8
+    test_int4(N, 384, 33, 64)
+    test_fp8(N, 200, 45)
+    test_dense(N, 200, 16)
+    test_dense(128 * tiles // 8 + 8, 1096, 33)
+
+
 @pytest.mark.parametrize("K", [1024, 4096, 8200, 12296, 20480, 20488])
 def test_quantisation_of_every_code_and_tie(K):
     """Every bf16 value in [-448, 448] at a scale of one (half-way cases of every binade and of the subnormal grid among them),
