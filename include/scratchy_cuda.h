@@ -171,6 +171,13 @@ int32_t scr_linear_affine_b4_ends(scr_ctx* ctx, const void* packed, const uint16
                                   int32_t N, int32_t K, int32_t group, const scr_qmv_ends* ends,
                                   uint16_t* y_bf16, void* stream);
 
+/* The residual end or the gate/up pairing above the matvec's tokens: 17 to 64 of them (SCR_E_UNSUPPORTED otherwise), one launch, the bits of
+ * `scr_linear_affine_b4` followed by the separate operator.  residual: y [M,N] <- bf16(y + bf16(x @ W^T + bias)); silu_pairs: y [M,N/2] as
+ * `scr_linear_affine_b4_silu_mul` leaves it, without a bias.  packed 128-byte aligned. */
+int32_t scr_linear_affine_b4_few_ends(scr_ctx* ctx, const void* packed, const uint16_t* x_bf16, int32_t M, int32_t N, int32_t K,
+                                      int32_t group, const uint16_t* bias, int32_t residual, int32_t silu_pairs, uint16_t* y_bf16,
+                                      void* stream);
+
 /* The o / down projection with the residual add and the following RMSNorm folded in (the reference's
  * `QmvEnds` residual end, step.rs:472-482, and `fused_add_rmsnorm`, cpu_golden.rs:171-200), one launch:
  *   residual[M,N] <- bf16(residual + bf16(x @ W^T));  normed[M,N] <- rmsnorm(residual, gain, eps)

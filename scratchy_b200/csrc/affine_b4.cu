@@ -197,8 +197,6 @@ __global__ void affine_b4_embed_kernel(const uint8_t* __restrict__ packed, const
 // ticket, and the CTA that draws the last ticket adds the partial sums in CTA order (deterministic),
 // and normalises the rows.  `scratch` = the ticket counter (16 floats reserved), then [gridDim.x][16] f32; the
 // counter must be zero before the first call and is left zero.
-#define GEMV_OUT_RESIDUAL_NORM 3
-#define GEMV_OUT_RESIDUAL_ADD 4
 struct GemvEnds {
     uint16_t* residual;
     const uint16_t* gain;
@@ -965,14 +963,33 @@ int32_t affine_b4_gemm_tc_launch(scr_ctx* ctx, const uint8_t* packed, const uint
                                  cudaStream_t stream);
 size_t affine_b4_gemm_tc_workspace(int M, int N, int K);
 bool affine_b4_gemm_tc_enabled();
+// Defined in affine_b4_skinny.cu
+bool affine_b4_skinny_applies(int M, int N, int K, int sms);
+int32_t affine_b4_skinny_launch(scr_ctx* ctx, const uint8_t* packed, const uint16_t* x, uint16_t* y, int M, int N, int K, int gs, int out,
+                                const uint16_t* bias, float scale, cudaStream_t stream);
+// Tokens up to which the GEMM for few tokens takes every matrix and has the residual and gate/up ends.
+constexpr int AFFINE_FEW_ENDS = 64;
+// Whether a call of up to 16 tokens goes to the GEMM for few tokens, whose time hardly grows with them, or to the matvec, which has the shorter
+// launch.  us in streams of calls, matvec / GEMM:
+//   1024 x 1024, 16 tokens 2.7 / 3.1;  2048 x 2048, 9 tokens 3.9 / 3.7, 16 4.4 / 3.8;  4096 x 1280, 9 tokens 3.6 / 4.0, 16 4.3 / 4.1
+//   3072 x 3072, 9 tokens 5.3 / 4.9;  5120 x 3072, 8 tokens 4.9 / 5.4, 9 7.7 / 5.6;  3072 x 8192, 16 tokens 12.5 / 7.0
+//   16384 x 3072, 4 tokens 10.8 / 10.3, 5 10.0 / 9.8, 8 12.0 / 10.0, 16 20.1 / 9.9;  24576 x 3072 (more tiles than SMs), 5 tokens 13.7 / 16.2,
+//   8 15.9 / 16.2, 9 21.9 / 16.5;  128256 x 3072, 2 tokens 54.2 / 51, 4 59.2 / 51.4, 8 67.1 / 51.8
+static bool affine_few_tokens(int M, int N, int K, int sms) {
+    const long long weights = (long long)N * K;
+    const int tiles = affine_geom(N, K, 64).RB / 8;
+    if (M > 8) return weights >= 4 << 20;
+    if (tiles >= 4 * sms) return M > 2;
+    return M > 4 && weights >= 40 << 20 && tiles <= sms;
+}
 
 size_t affine_workspace_bytes(int M, int N, int K) {
     if (M <= 16 || !affine_b4_gemm_tc_enabled()) return 0;
     return affine_b4_gemm_tc_workspace(M, N, K);
 }
 
-// The forward dispatch every int4 entry point goes through: the balanced matvec up to 8 tokens, the
-// two-tile matvec up to 16, the tensor-core GEMM above.
+// The forward dispatch every int4 entry point goes through: up to 16 tokens the matvec (balanced up to 8, two tiles above) or the GEMM for few
+// tokens (`affine_few_tokens`), the tensor-core GEMMs above.
 static int32_t affine_forward(scr_ctx* ctx, const void* packed, const uint16_t* x, int M, int N, int K, int group, void* y_,
                               const AffineFwd& f_in, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
     if (!packed || !x || !y_) return scr_fail(ctx, SCR_E_ARG, "null pointer");
@@ -984,13 +1001,28 @@ static int32_t affine_forward(scr_ctx* ctx, const void* packed, const uint16_t* 
     if (!scr_aligned16(packed) || !scr_aligned16(x)) return scr_fail(ctx, SCR_E_ALIGN, "packed/x must be 16-byte aligned");
     if ((f.bias || f.scale != 1.0f) && (f.out_mode == GEMV_OUT_SILU_PAIRS || f.out_mode == GEMV_OUT_RESIDUAL_NORM))
         return scr_fail(ctx, SCR_E_UNSUPPORTED, "a bias or a scale cannot be combined with this fused epilogue");
-    if (M > 16 && (f.norm_gain || f.scale != 1.0f || f.out_mode == GEMV_OUT_RESIDUAL_ADD))
+    const bool few_ends = M > 16 && M <= AFFINE_FEW_ENDS && !f.norm_gain && f.scale == 1.0f && (f.out_mode == GEMV_OUT_RESIDUAL_ADD || f.out_mode == GEMV_OUT_SILU_PAIRS);
+    if (M > 16 && !few_ends && (f.norm_gain || f.scale != 1.0f || f.out_mode == GEMV_OUT_RESIDUAL_ADD))
         return scr_fail(ctx, SCR_E_UNSUPPORTED, "the norm-in, scale and residual ends exist on the matvec path only (M <= 16)");
     if (f.norm_gain && !scr_aligned16(f.norm_gain)) return scr_fail(ctx, SCR_E_ALIGN, "the norm gain must be 16-byte aligned");
     const uint8_t* pk = (const uint8_t*)packed;
     uint16_t* y = static_cast<uint16_t*>(y_);
+    if (M <= 16 && !f.norm_gain && affine_few_tokens(M, N, K, ctx->sm_count) && ((uintptr_t)pk & 127u) == 0 && scr_aligned16(y)) {
+        if (affine_b4_skinny_applies(M, N, K, ctx->sm_count)) {
+            const int out = f.out_mode == GEMV_OUT_RESIDUAL_NORM ? GEMV_OUT_RESIDUAL_ADD : f.out_mode;
+            st = affine_b4_skinny_launch(ctx, pk, x, y, M, N, K, f.gs, out, f.bias, f.scale, stream);
+            if (st || out == f.out_mode) return st;
+            return scr_rmsnorm_bf16(ctx, f.ends->residual, f.ends->gain, f.ends->normed, M, N, f.ends->eps, stream);
+        }
+        if ((f.out_mode == GEMV_OUT_BF16 || f.out_mode == GEMV_OUT_F32) && f.scale == 1.0f)
+            return affine_b4_gemm_tc_launch(ctx, pk, x, y, M, N, K, f.gs, f.out_mode == GEMV_OUT_F32, f.bias, nullptr, 0, stream);
+    }
     if (M <= 8) return affine_gemv_launch<1>(ctx, pk, x, y, M, N, K, f, stream);
     if (M <= 16) return affine_gemv_launch<2>(ctx, pk, x, y, M, N, K, f, stream);
+    if (few_ends) {
+        if (((uintptr_t)pk & 127u) != 0 || !scr_aligned16(y)) return scr_fail(ctx, SCR_E_ALIGN, "packed must be 128-byte aligned, y 16-byte aligned");
+        return affine_b4_skinny_launch(ctx, pk, x, y, M, N, K, f.gs, f.out_mode, f.bias, 1.0f, stream);
+    }
     if (f.out_mode != GEMV_OUT_BF16 && f.out_mode != GEMV_OUT_F32)
         return scr_fail(ctx, SCR_E_UNSUPPORTED, "this fused epilogue exists on the matvec path only (M <= 16)");
     if (affine_b4_gemm_tc_enabled()) {
@@ -1092,6 +1124,18 @@ extern "C" int32_t scr_linear_affine_b4_ends(scr_ctx* ctx, const void* packed, c
     f.out_mode = ends->residual ? GEMV_OUT_RESIDUAL_ADD : (ends->silu_pairs ? GEMV_OUT_SILU_PAIRS : GEMV_OUT_BF16);
     if (ends->silu_pairs && (N <= 0 || N % 16 != 0)) return scr_fail(ctx, SCR_E_SHAPE, "gate/up pairing: %d fused rows (8 gate + 8 up per block)", N);
     if (M > 16) return scr_fail(ctx, SCR_E_UNSUPPORTED, "the matvec ends exist up to 16 tokens (M=%d): run the operators separately", M);
+    return affine_forward(ctx, packed, x, M, N, K, group, y, f, nullptr, 0, (cudaStream_t)stream_);
+}
+
+extern "C" int32_t scr_linear_affine_b4_few_ends(scr_ctx* ctx, const void* packed, const uint16_t* x, int32_t M, int32_t N, int32_t K, int32_t group,
+                                                 const uint16_t* bias, int32_t residual, int32_t silu_pairs, uint16_t* y, void* stream_) {
+    SCR_REQUIRE_CTX(ctx);
+    if ((residual != 0) == (silu_pairs != 0)) return scr_fail(ctx, SCR_E_ARG, "either the residual end or the gate/up pairing");
+    if (silu_pairs && (N <= 0 || N % 16 != 0)) return scr_fail(ctx, SCR_E_SHAPE, "gate/up pairing: %d fused rows (8 gate + 8 up per block)", N);
+    if (M <= 16 || M > AFFINE_FEW_ENDS) return scr_fail(ctx, SCR_E_UNSUPPORTED, "these ends exist for 17 to %d tokens (M=%d)", AFFINE_FEW_ENDS, M);
+    AffineFwd f;
+    f.bias = bias;
+    f.out_mode = residual ? GEMV_OUT_RESIDUAL_ADD : GEMV_OUT_SILU_PAIRS;
     return affine_forward(ctx, packed, x, M, N, K, group, y, f, nullptr, 0, (cudaStream_t)stream_);
 }
 

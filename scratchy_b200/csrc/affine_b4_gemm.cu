@@ -11,15 +11,14 @@
 //                consecutive channels of a token per warp
 //   warp 20      producer of the packed weights: one tiled copy per chunk (affine_b4_tc.cuh), ahead of the preceding kernel
 //   warp 21      producer of the activations: tiled TMA loads of 64 k x the tokens (128-byte swizzle, zeros outside)
-//   warp 22      owns TMEM; one elected lane issues 8 tcgen05.mma (128 x width x 16) per chunk and commits the barriers; the warp
-//                goes round as a whole so that the descriptors stay in uniform registers (a divergent thread spends about 55
-//                cycles on each MMA it issues)
+//   warp 22      owns TMEM; the warp issues 8 tcgen05.mma (128 x width x 16) per chunk and commits the barriers, a lane elected
+//                inside each: 3072 -> 16384 at 4096 tokens 284 us, 297 with the lane elected once and branches around the issue
 // TMEM holds two accumulators of 192 columns (the epilogue of a tile overlaps the main loop of the next) and two stages of 64
 // columns of dequantised weights.  No multicast: every CTA issues its own loads.
 //
 // What bounds it: the MMAs, 64 cycles for 128 columns and 96 for 192 (alone in a loop, A in TMEM: the tensor core's full rate), 768 a chunk
 // at 192, and for large calls the clock that the power limit leaves: 2048 tokens of 3072 -> 8192 73.7 us (1.40 PFLOP/s, what cuBLAS
-// sustains) in a stream of calls.  It was 83.7 us, 1250 cycles a chunk whatever the width, while one lane issued eight bulk copies a chunk
+// sustains) in a stream of calls, 72.4 with the election inside.  It was 83.7 us, 1250 cycles a chunk whatever the width, while one lane issued eight bulk copies a chunk
 // and the dequantised weights were handed over in stages of a whole chunk.  Wide tiles pay, since a chunk is expanded once for all of a
 // tile's tokens.
 #include <cuda.h>
@@ -27,6 +26,7 @@
 #include <algorithm>
 
 #include "affine_b4_tc.cuh"
+#include "gemv_common.cuh"
 #include "skinny.cuh"
 
 bool affine_b4_gemm_tc_enabled() { return true; }
@@ -35,9 +35,9 @@ bool affine_b4_gemm_pair_applies(int M, int N, int K, int sms, float one_cta_us)
 int32_t affine_b4_gemm_pair_launch(scr_ctx* ctx, const CUtensorMap& x_map, const uint8_t* packed, uint16_t* y, int M, int N, int K,
                                    int gs, int out_f32, const uint16_t* bias, cudaStream_t stream, bool* launched);
 // Defined in affine_b4_skinny.cu
-bool affine_b4_skinny_applies(int M, int K);
-int32_t affine_b4_skinny_launch(scr_ctx* ctx, const uint8_t* packed, const uint16_t* x, uint16_t* y, int M, int N, int K, int gs, int out_f32,
-                                const uint16_t* bias, cudaStream_t stream);
+bool affine_b4_skinny_applies(int M, int N, int K, int sms);
+int32_t affine_b4_skinny_launch(scr_ctx* ctx, const uint8_t* packed, const uint16_t* x, uint16_t* y, int M, int N, int K, int gs, int out,
+                                const uint16_t* bias, float scale, cudaStream_t stream);
 size_t affine_b4_gemm_tc_workspace_plan(int M, int N, int K);
 size_t affine_b4_gemm_tc_workspace(int M, int N, int K) { return affine_b4_gemm_tc_workspace_plan(M, N, K); }
 
@@ -180,7 +180,6 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
         }
     } else if (warp == 22) {
         skinny_pdl_wait();
-        const bool lead = elect_one();
         const uint32_t idesc = umma_idesc(1, 1, A4G_BN, (uint32_t)width);
         int s = 0, c = 0, it = 0;
         uint32_t ph = 0;
@@ -199,19 +198,15 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
                     mbar_wait(xfull(s), ph, status, TC_ERR_FULL_WAIT);
                     mbar_wait(afull(a), (uint32_t)(c / A4G_SA) & 1u, status, TC_ERR_DEQ_WAIT);
                     tc_fence_after();
-                    if (lead) {
 #pragma unroll
-                        for (int k4 = 0; k4 < 4; ++k4)
-                            umma_f16_ta(d, ac + (uint32_t)(8 * k4), bdesc + (uint64_t)(2 * k4), idesc, kc > kc_lo || h > 0 || k4 > 0);
-                        umma_commit(aempty(a));
-                        umma_commit(xempty(s));
-                    }
-                    __syncwarp();
+                    for (int k4 = 0; k4 < 4; ++k4)
+                        umma_f16_ta_warp(d, ac + (uint32_t)(8 * k4), bdesc + (uint64_t)(2 * k4), idesc, kc > kc_lo || h > 0 || k4 > 0);
+                    umma_commit_warp(aempty(a));
+                    umma_commit_warp(xempty(s));
                     if (++s == A4G_SX) { s = 0; ph ^= 1u; }
                 }
             }
-            if (lead) umma_commit(accf(buf));
-            __syncwarp();
+            umma_commit_warp(accf(buf));
         }
     } else if (warp < A4G_DQ_WARPS) {
         const bool check = *reinterpret_cast<const unsigned int*>(packed + (size_t)RB * KC * kBlock) != 0;
@@ -333,6 +328,14 @@ static AffineGemmPlan affine_gemm_plan(int M, int N, int K, int sms) {
     const AffineGeom g = affine_geom(N, K, 64);
     AffineGemmPlan best{};
     float least = 1e30f;
+    if (M <= 96 || (M <= 128 && K > 1536)) {
+        // few tokens of a matrix of more tiles than SMs: whole tiles of just these tokens, no workspace
+        best.width = (M + 15) & ~15;
+        best.mt = 1;
+        best.tiles = best.full = g.RB * 16 / A4G_BN;
+        best.ks_tail = 1;
+        return best;
+    }
     for (int width = A4G_WIDTH; width >= 128; width -= 16) {
         AffineGemmPlan p;
         p.width = width;
@@ -348,7 +351,7 @@ static AffineGemmPlan affine_gemm_plan(int M, int N, int K, int sms) {
     return best;
 }
 size_t affine_b4_gemm_tc_workspace_plan(int M, int N, int K) {
-    if (affine_b4_skinny_applies(M, K)) return 0;
+    if (affine_b4_skinny_applies(M, N, K, tc_sm_count())) return 0;
     return affine_gemm_plan(M, N, K, tc_sm_count()).slab_floats() * sizeof(float);
 }
 
@@ -383,7 +386,8 @@ int32_t affine_b4_gemm_tc_launch(scr_ctx* ctx, const uint8_t* packed, const uint
                                  int gs, int out_f32, const uint16_t* bias, void* workspace, size_t, cudaStream_t stream) {
     if (((uintptr_t)packed & 127u) != 0) return scr_fail(ctx, SCR_E_ALIGN, "packed weights must be 128-byte aligned for the GEMM path");
     if (!scr_aligned16(y)) return scr_fail(ctx, SCR_E_ALIGN, "y must be 16-byte aligned");
-    if (affine_b4_skinny_applies(M, K)) return affine_b4_skinny_launch(ctx, packed, x, y, M, N, K, gs, out_f32, bias, stream);
+    if (affine_b4_skinny_applies(M, N, K, ctx->sm_count))
+        return affine_b4_skinny_launch(ctx, packed, x, y, M, N, K, gs, out_f32 ? GEMV_OUT_F32 : GEMV_OUT_BF16, bias, 1.0f, stream);
     tc_encode_tiled_fn enc = tc_tensor_map_encoder();
     if (!enc) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled entry point not available");
     CUtensorMap map;

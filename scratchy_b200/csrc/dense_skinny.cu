@@ -126,7 +126,7 @@ dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_cons
     __syncwarp();
     pdl_wait();
     const uint32_t sums = over_rings ? 0 : C::kBarOff + 256u;
-    skinny_finish<(TN <= 64)>(tmem, smem_base + sums, reinterpret_cast<const float*>(smem_gen + sums), over_rings != 0, rbar, M, split, rank, n0, N, status,
+    skinny_finish<8, (TN <= 64)>(tmem, smem_base + sums, reinterpret_cast<const float*>(smem_gen + sums), over_rings != 0, rbar, M, split, rank, n0, N, status,
                   [&](int m, int n, float a, float b) { dense_put_two<bf16, END>(ends, m, g, n, N, a, b); });
     __syncthreads();
     if (warp == 10) {

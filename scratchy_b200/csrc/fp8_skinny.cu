@@ -126,7 +126,7 @@ fp8_skinny_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ w
     __syncwarp();
     skinny_pdl_wait();
     const uint32_t sums = over_rings ? 0 : C::kBarOff + 256u;
-    skinny_finish<true>(tmem, smem_base + sums, reinterpret_cast<const float*>(smem_gen + sums), over_rings != 0, rbar, M, split, rank, tile * SKINNY_ROWS, N, status,
+    skinny_finish<8, true>(tmem, smem_base + sums, reinterpret_cast<const float*>(smem_gen + sums), over_rings != 0, rbar, M, split, rank, tile * SKINNY_ROWS, N, status,
                          [&](int m, int n, float a, float b) {
         const float as = a_scale[m], v[2] = {a, b};
 #pragma unroll

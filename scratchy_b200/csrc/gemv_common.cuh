@@ -132,6 +132,8 @@ __device__ __forceinline__ void gemv_block_compute(uint32_t blk, float acc[2][MT
 #define GEMV_OUT_BF16 0
 #define GEMV_OUT_F32 1
 #define GEMV_OUT_SILU_PAIRS 2
+#define GEMV_OUT_RESIDUAL_NORM 3
+#define GEMV_OUT_RESIDUAL_ADD 4
 
 // Called by all 32 lanes of a warp.  `total` is this lane's (row, token) sum; bit 1 of `idx` says
 // whether the row is a gate row (0) or the up row 8 below it (1).

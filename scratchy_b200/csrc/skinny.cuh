@@ -11,7 +11,6 @@
 
 constexpr int SKINNY_ROWS = 128;                 // output channels of a tile
 constexpr int SKINNY_MAX_SPLIT = 8;              // portable cluster size
-constexpr int SKINNY_EPI_WARPS = 8;              // warps 0..7 drain the accumulator
 
 __device__ __forceinline__ void skinny_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void skinny_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -19,7 +18,7 @@ __device__ __forceinline__ void skinny_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // The same in two parts: after a CTA's barriers are initialised, and before it touches another CTA's.
-__device__ __forceinline__ void skinny_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void skinny_cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void skinny_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
@@ -62,8 +61,8 @@ __device__ __forceinline__ void skinny_wait_sums(uint32_t rbar, int* status) {
     atomicCAS(status, 0, TC_ERR_ACC_FULL);
 }
 
-// The end of a unit, called by every thread of every CTA of the cluster once its role is done; warps 0..7 have seen the
-// accumulator complete.  `d` = the accumulator (lane = channel, column = token), `sums` = where the cluster's sums go (shared and generic
+// The end of a unit, called by every thread of every CTA of the cluster once its role is done; warps 0 .. EPI_WARPS - 1 have
+// seen the accumulator complete.  `d` = the accumulator (lane = channel, column = token), `sums` = where the cluster's sums go (shared and generic
 // address).  A CTA sends every run to its owner, which adds the `split` sums of a value in rank order and passes the channels n and n + 8
 // (n % 16 < 8: a gate and its up, where they are interleaved) to put(token, n, sum, sum8).
 // Where the sums have memory of their own they travel by asynchronous stores that count on the owner's `rbar`: no barrier of the cluster in the
@@ -73,7 +72,7 @@ __device__ __forceinline__ void skinny_wait_sums(uint32_t rbar, int* status) {
 // From SKINNY_QUAD_TOKENS on a run has work for every thread four tokens at a time (QUADS; 250 fp8 tokens of 18944 -> 3584 31.4 -> 29.8 us, but the
 // bf16 linears of 65 to 128 rows, whose put is longer, lost 2 to 8 %).
 constexpr int SKINNY_QUAD_TOKENS = 12;
-template <bool QUADS, typename Put>
+template <int EPI_WARPS, bool QUADS, typename Put>
 __device__ __forceinline__ void skinny_finish(uint32_t d, uint32_t sums, const float* sums_gen, bool over_rings, uint32_t rbar, int M, int split, int rank,
                                               int n0, int N, int* status, Put put) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -81,13 +80,13 @@ __device__ __forceinline__ void skinny_finish(uint32_t d, uint32_t sums, const f
     const bool async = split > 1 && !over_rings;
     if (async) skinny_cluster_wait();            // the others' barriers are set up (they arrived when theirs were)
     else if (split > 1) skinny_cluster_sync();
-    if (warp < SKINNY_EPI_WARPS) {
+    if (warp < EPI_WARPS) {
         tc_fence_after();
         const int row = (warp & 3) * 32 + lane;
         // [sender][4 tokens][channel][token of the 4]
         int owner = 0, at = (warp >> 2) * 16;
         while (at >= per) { at -= per; ++owner; }
-        for (int c = (warp >> 2) * 16; c < M; c += 32) {
+        for (int c = (warp >> 2) * 16; c < M; c += EPI_WARPS * 4) {
             uint32_t r[16], dst[4], bar[4];
             tmem_ld_32x16(d + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c, r);
             int o = owner, t = at;
@@ -113,7 +112,7 @@ __device__ __forceinline__ void skinny_finish(uint32_t d, uint32_t sums, const f
                 else
                     asm volatile("st.shared::cluster.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst[j]), "r"(r[4 * j]), "r"(r[4 * j + 1]), "r"(r[4 * j + 2]), "r"(r[4 * j + 3]) : "memory");
             }
-            at += 32;
+            at += EPI_WARPS * 4;
             while (at >= per) { at -= per; ++owner; }
         }
         tc_fence_before();

@@ -342,7 +342,7 @@ class LlamaDecoder:
         residual adds keep the bits of the separate operator; the norm-in end runs the reference matvec's own arithmetic
         (the dot over `x * gain`, the row scaled by `1 / rms(x)`: as close to the exact product as norm-then-matvec, not
         its bits) unless `exact_norm_in` asks for the rounded normalised row of the separate RMSNorm (slower: every
-        CTA then finishes the row's sum of squares before its first product).  `fuse_residual` (up to 16 tokens, when
+        CTA then finishes the row's sum of squares before its first product).  `fuse_residual` (up to 64 tokens, when
         `fuse_ends` is off): the o and down projections add into the residual stream themselves (the residual end alone,
         the bits of the separate add) and the norms run as plain RMSNorm launches — the same number of launches as with
         `fused_add_rmsnorm`, each norm reading one row instead of two and no intermediate projection output."""
@@ -429,7 +429,7 @@ class LlamaDecoder:
         ends = (self.fuse_ends and not self.fuse_residual_norm and
                 AffineQuantLinear.norm_in_supported(buf.batch, cfg.hidden))
         row_scale = not self.exact_norm_in
-        resid_end = self.fuse_residual and not ends and not self.fuse_residual_norm and buf.batch <= 16
+        resid_end = self.fuse_residual and not ends and not self.fuse_residual_norm and buf.batch <= AffineQuantLinear.FEW_ENDS
         if not ends:
             rmsnorm(buf.residual, self.layers[0].input_norm, cfg.rms_eps, out=buf.normed)
         for i, layer in enumerate(self.layers):
@@ -456,10 +456,10 @@ class LlamaDecoder:
                                            norm_row_scale=row_scale)
                 layer.down.forward_ends(buf.act, buf.residual, residual=True)
             elif resid_end:
-                layer.o.forward_ends(buf.attn, buf.residual, residual=True)
+                layer.o.forward_add(buf.attn, buf.residual)
                 rmsnorm(buf.residual, layer.post_norm, cfg.rms_eps, out=buf.normed)
                 layer.gate_up.forward_silu_mul(buf.normed, out=buf.act, scratch=buf.gate_up, workspace=buf.workspace)
-                layer.down.forward_ends(buf.act, buf.residual, residual=True)
+                layer.down.forward_add(buf.act, buf.residual)
                 rmsnorm(buf.residual, nxt, cfg.rms_eps, out=buf.normed)
             elif self.fuse_residual_norm:
                 layer.o.forward_residual_rmsnorm(buf.attn, buf.residual, layer.post_norm, cfg.rms_eps, buf.normed,

@@ -210,8 +210,9 @@ class AffineQuantLinear:
 
     def forward_silu_mul(self, x: torch.Tensor, out: Optional[torch.Tensor] = None,
                          scratch: Optional[torch.Tensor] = None, workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """`silu(x @ gate^T) * (x @ up^T)` on a matrix built by `load_rows_interleave8`: one launch up to 16
-        tokens (`scr_linear_affine_b4_silu_mul`), the linear into `scratch` plus `scr_silu_mul_pairs8_bf16` above."""
+        """`silu(x @ gate^T) * (x @ up^T)` on a matrix built by `load_rows_interleave8`: one launch up to 64
+        tokens (`scr_linear_affine_b4_silu_mul`, `scr_linear_affine_b4_few_ends`), the linear into `scratch` plus
+        `scr_silu_mul_pairs8_bf16` above."""
         if not getattr(self, "pairs8", False):
             raise ValueError("forward_silu_mul needs a gate/up matrix built by load_rows_interleave8")
         if self.linear_bias is not None:
@@ -225,6 +226,10 @@ class AffineQuantLinear:
         if M <= 16:
             ctx.check(_lib.lib().scr_linear_affine_b4_silu_mul(ctx.handle, _ptr(self.packed), _ptr(x2), M, self.out_features,
                                                                self.in_features, self.group_size, _ptr(out), _stream(dev)))
+            return out
+        if M <= self.FEW_ENDS:
+            ctx.check(_lib.lib().scr_linear_affine_b4_few_ends(ctx.handle, _ptr(self.packed), _ptr(x2), M, self.out_features, self.in_features,
+                                                               self.group_size, None, 0, 1, _ptr(out), _stream(dev)))
             return out
         if scratch is None:
             scratch = torch.empty((M, self.out_features), dtype=torch.bfloat16, device=dev)
@@ -340,6 +345,19 @@ class AffineQuantLinear:
         ctx.check(_lib.lib().scr_linear_affine_b4_ends(ctx.handle, _ptr(self.packed), _ptr(x2), M, self.out_features, self.in_features,
                                                        self.group_size, ctypes.byref(ends), _ptr(out), _stream(dev)))
         return out
+
+    FEW_ENDS = 64                   # tokens up to which the residual end is one launch (`forward_add`)
+
+    def forward_add(self, x: torch.Tensor, residual: torch.Tensor) -> torch.Tensor:
+        """`residual <- bf16(residual + bf16(x @ W^T + bias))` in place, the bits of `forward` and a separate add; up to FEW_ENDS rows."""
+        x2 = x.reshape(-1, self.in_features).contiguous()
+        M = int(x2.shape[0])
+        if M <= 16:
+            return self.forward_ends(x2, residual, residual=True)
+        ctx = _lib.context(_dev_index(x2.device))
+        ctx.check(_lib.lib().scr_linear_affine_b4_few_ends(ctx.handle, _ptr(self.packed), _ptr(x2), M, self.out_features, self.in_features,
+                                                           self.group_size, _ptr(self.linear_bias), 1, 0, _ptr(residual), _stream(x2.device)))
+        return residual
 
     @staticmethod
     def norm_in_supported(M: int, K: int) -> bool:

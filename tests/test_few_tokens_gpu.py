@@ -91,6 +91,43 @@ def test_fp8(N, K, M):
     assert torch.equal((part + bias.float()).bfloat16().view(torch.int16), yb.view(torch.int16))
 
 
+@pytest.mark.parametrize("M", [5, 8, 9, 16, 17, 33, 64])
+@pytest.mark.parametrize("N,K,group", [(2064, 2048, 64), (4160, 1024, 32), (16400, 2560, 128)])
+def test_int4_ends_of_few_tokens(N, K, group, M):
+    """The ends of the GEMM for few tokens on both sides of the matvec's sizes: bias and scale, the residual add and the gate/up pairing
+    give the bits of the plain linear followed by the operator; the plain linear is held to the oracle."""
+    import torch
+    from scratchy_b200 import AffineQuantLinear, _lib
+    seed = synth.seed_for("few-ends", N, K, M, group)
+    w, s, b = synth.affine_int4_weights(N, K, group, seed)
+    x = synth.activations_bf16(M, K, seed + 1)
+    layer = AffineQuantLinear.from_tensors(u32_dev(w), bf16_dev(s), bf16_dev(b), group, 4)
+    xd, new = bf16_dev(x).reshape(M, K), lambda n=N: torch.full((M, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+    y = layer.forward(xd, out=new())
+    rows = np.unique(np.random.default_rng(M).integers(0, M, 8))
+    want = oracle.affine_qmm_t_b4(w.view(np.uint8).reshape(-1), s, b, x[rows], len(rows), N, K, group)
+    assert rel_l2(bits_of(y).reshape(M, N)[rows], want) <= REL_L2_TOL
+    res = bf16_dev(synth.activations_bf16(M, N, seed + 2)).reshape(M, N)
+    added = layer.forward_add(xd, res.clone())
+    assert torch.equal(added.view(torch.int16), (res.float() + y.float()).bfloat16().view(torch.int16))
+    layer.pairs8 = True
+    act, two = layer.forward_silu_mul(xd, out=new(N // 2)), new(N // 2)
+    ctx = _lib.context(0)
+    ctx.check(_lib.lib().scr_silu_mul_pairs8_bf16(ctx.handle, y.data_ptr(), N, two.data_ptr(), M, N // 2, None))
+    assert torch.equal(act.view(torch.int16), two.view(torch.int16))
+    layer.linear_bias = bf16_dev(synth.activations_bf16(1, N, seed + 3)).reshape(N)
+    part = layer.forward_partial(xd)
+    assert torch.equal(part.bfloat16().view(torch.int16), y.view(torch.int16))
+    biased = (part + layer.linear_bias.float()).bfloat16()
+    assert torch.equal(layer.forward(xd).view(torch.int16), biased.view(torch.int16))
+    added = layer.forward_add(xd, res.clone())
+    assert torch.equal(added.view(torch.int16), (res.float() + biased.float()).bfloat16().view(torch.int16))
+    if M <= 16:
+        scaled = layer.forward_ends(xd, new(), scale=0.125)
+        assert torch.equal(scaled.view(torch.int16), ((part + layer.linear_bias.float()) * 0.125).bfloat16().view(torch.int16))
+    torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize("tiles", [147, 148, 149, 300])
 def test_calls_whose_clusters_do_not_all_run_at_once(tiles):
     """As many tiles of 128 channels as SMs, where every CTA has its SM and memory for the sums to itself, and more, where two share an
