@@ -5,13 +5,18 @@
 // A CTA takes one head and 256 query rows as two tiles of 128 that run in turn: while the tensor core works on one tile,
 // the softmax warps of the other work.  320 threads:
 //   warp 0       TMA: the query tiles once, then key tiles (64 keys) and value tiles through two rings
-//   warp 1       owns TMEM; one thread issues, per key tile and query tile, O += P V of the previous key tile and then
-//                S = Q K^T of this one
+//   warp 1       owns TMEM; the warp issues, per key tile, S = Q K^T of both query tiles and then O += P V of the previous key tile,
+//                a lane elected inside each instruction
 //   warps 2-5, 6-9   softmax of tile 0, tile 1 (thread = query row): S from TMEM, f32 softmax, P back to TMEM as a bf16
 //                head and remainder (two products: the weights keep about 16 bits), O rescaled in TMEM only when the
 //                row maximum has grown by more than 2^8 over the reference the sums are kept in
 // The end divides by the row sum and multiplies by the sigmoid of the output gate.
-// TMEM per tile: S 64 columns, P 32 + 32, O 128.  Every wait is bounded (tc_common.cuh).
+// TMEM per tile: two S of 64 columns, whose P (32 + 32) takes their place, O 128.  Every wait is bounded (tc_common.cuh).
+//
+// What bounds it: per key tile and query tile the tensor core works 1088 cycles (12 MMAs of 64 columns from shared memory at 48, eight of 128 from
+// TMEM at 64), and a tile's softmax, one thread to a row, about twice that; the two tiles take turns.  8192 tokens of 24 heads of 192 + 128:
+// 758 us.  1059 with the MMAs issued by lane 0 of a divergent warp and S in a buffer that waited for the P V before it; 1074 with two threads to a
+// row, which exchange their maxima over a barrier.
 #include "seq_common.cuh"
 
 #include <algorithm>
@@ -65,11 +70,11 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     auto k_empty = [&](int s) { return bars + 8u * (4 + s); };
     auto v_full = [&](int s) { return bars + 8u * (7 + s); };
     auto v_empty = [&](int s) { return bars + 8u * (10 + s); };
-    auto s_full = [&](int t) { return bars + 8u * (13 + t); };
-    auto p_full = [&](int t) { return bars + 8u * (15 + t); };
-    auto o_full = [&](int t) { return bars + 8u * (17 + t); };
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L.bars + 8 * 19);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto s_full = [&](int t, int j) { return bars + 8u * (13 + 2 * t + (j & 1)); };
+    auto p_full = [&](int t, int j) { return bars + 8u * (17 + 2 * t + (j & 1)); };
+    auto pv_done = [&](int t) { return bars + 8u * (21 + t); };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L.bars + 8 * 23);
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int head = blockIdx.x, q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * 256;      // the longest tiles first
     int n[2];                                                                          // key tiles of the two query tiles
 #pragma unroll
@@ -82,7 +87,10 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     if (threadIdx.x == 0) {
         mbar_init(q_full(), 1);
         for (int s = 0; s < 3; ++s) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 1); mbar_init(v_full(s), 1); mbar_init(v_empty(s), 1); }
-        for (int t = 0; t < 2; ++t) { mbar_init(s_full(t), 1); mbar_init(p_full(t), 128); mbar_init(o_full(t), 1); }
+        for (int t = 0; t < 2; ++t) {
+            for (int j = 0; j < 2; ++j) { mbar_init(s_full(t, j), 1); mbar_init(p_full(t, j), 4); }
+            mbar_init(pv_done(t), 1);
+        }
         fence_mbar_init();
     }
     if (warp == 1) {
@@ -94,9 +102,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     pdl_trigger();                                     // not before this CTA has its TMEM: the next kernel's CTAs could take it first
-    auto s_col = [&](int t) { return tmem + 256u * t; };
-    auto ph_col = [&](int t) { return tmem + 256u * t + 64u; };
-    auto pl_col = [&](int t) { return tmem + 256u * t + 96u; };
+    auto s_col = [&](int t, int j) { return tmem + 256u * t + 64u * (j & 1); };        // S, then P: 32 columns of heads, 32 of remainders
     auto o_col = [&](int t) { return tmem + 256u * t + 128u; };
     pdl_wait();
 
@@ -125,44 +131,44 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t s_desc = umma_idesc(1, 1, 128, LF_KEYS), o_desc = umma_idesc(1, 1, 128, (uint32_t)L.vp);
-            mbar_wait(q_full(), 0, a.status, TC_ERR_FULL_WAIT);
-            int ks = 0, vs = 0;
-            uint32_t kp = 0, vp = 0;
-            for (int j = 0; j <= nmax; ++j) {
-                if (j < nmax) mbar_wait(k_full(ks), kp, a.status, TC_ERR_FULL_WAIT);
-                if (j > 0) mbar_wait(v_full(vs), vp, a.status, TC_ERR_FULL_WAIT);
+        const uint32_t s_desc = umma_idesc(1, 1, 128, LF_KEYS), o_desc = umma_idesc(1, 1, 128, (uint32_t)L.vp);
+        mbar_wait(q_full(), 0, a.status, TC_ERR_FULL_WAIT);
+        int ks = 0, vs = 0;
+        uint32_t kp = 0, vp = 0;
+        for (int j = 0; j <= nmax; ++j) {
+            if (j < nmax) {                                                          // S(j) = Q K(j): P V of two tiles before, whose S it takes, is issued
+                mbar_wait(k_full(ks), kp, a.status, TC_ERR_FULL_WAIT);
                 tc_fence_after();
                 for (int t = 0; t < 2; ++t) {
-                    if (j > 0 && j <= n[t]) {                                        // O += P(j - 1) V(j - 1)
-                        mbar_wait(p_full(t), (uint32_t)(j - 1) & 1u, a.status, TC_ERR_DEQ_WAIT);
-                        tc_fence_after();
-                        const uint64_t vd = umma_desc_k_sw128(base + L.v + vs * L.v_bytes());
+                    if (j >= n[t]) continue;
+                    const uint32_t col = s_col(t, j);
+                    for (int c = 0; c < L.chunks; ++c) {
+                        const uint64_t qd = umma_desc_k_sw128(base + (t * L.chunks + c) * LF_Q_CHUNK);
+                        const uint64_t kd = umma_desc_k_sw128(base + L.k + ks * L.k_bytes() + c * LF_K_CHUNK);
 #pragma unroll
-                        for (int k4 = 0; k4 < 4; ++k4) umma_f16_ta(o_col(t), ph_col(t) + 8u * k4, vd + (uint64_t)(2 * k4), o_desc, (j > 1) || k4 > 0);
-#pragma unroll
-                        for (int k4 = 0; k4 < 4; ++k4) umma_f16_ta(o_col(t), pl_col(t) + 8u * k4, vd + (uint64_t)(2 * k4), o_desc, 1);
-                        if (j == n[t]) umma_commit(o_full(t));
+                        for (int k4 = 0; k4 < 4; ++k4) umma_f16_warp(col, qd + (uint64_t)(2 * k4), kd + (uint64_t)(2 * k4), s_desc, (c | k4) != 0);
                     }
-                    if (j < n[t]) {
-                        for (int c = 0; c < L.chunks; ++c) {
-                            const uint64_t qd = umma_desc_k_sw128(base + (t * L.chunks + c) * LF_Q_CHUNK);
-                            const uint64_t kd = umma_desc_k_sw128(base + L.k + ks * L.k_bytes() + c * LF_K_CHUNK);
+                    umma_commit_warp(s_full(t, j));
+                }
+                umma_commit_warp(k_empty(ks));
+                if (++ks == L.k_stages) { ks = 0; kp ^= 1u; }
+            }
+            if (j > 0) {                                                             // O += P(j - 1) V(j - 1)
+                mbar_wait(v_full(vs), vp, a.status, TC_ERR_FULL_WAIT);
+                const uint64_t vd = umma_desc_k_sw128(base + L.v + vs * L.v_bytes());
+                for (int t = 0; t < 2; ++t) {
+                    if (j > n[t]) continue;
+                    mbar_wait(p_full(t, j - 1), (uint32_t)((j - 1) >> 1) & 1u, a.status, TC_ERR_DEQ_WAIT);
+                    tc_fence_after();
+                    const uint32_t col = s_col(t, j - 1);
 #pragma unroll
-                            for (int k4 = 0; k4 < 4; ++k4) umma_f16(s_col(t), qd + (uint64_t)(2 * k4), kd + (uint64_t)(2 * k4), s_desc, (c | k4) != 0);
-                        }
-                        umma_commit(s_full(t));
-                    }
+                    for (int k4 = 0; k4 < 4; ++k4) umma_f16_ta_warp(o_col(t), col + 8u * k4, vd + (uint64_t)(2 * k4), o_desc, (j > 1) || k4 > 0);
+#pragma unroll
+                    for (int k4 = 0; k4 < 4; ++k4) umma_f16_ta_warp(o_col(t), col + 32u + 8u * k4, vd + (uint64_t)(2 * k4), o_desc, 1);
+                    umma_commit_warp(pv_done(t));
                 }
-                if (j < nmax) {
-                    umma_commit(k_empty(ks));
-                    if (++ks == L.k_stages) { ks = 0; kp ^= 1u; }
-                }
-                if (j > 0) {
-                    umma_commit(v_empty(vs));
-                    if (++vs == L.v_stages) { vs = 0; vp ^= 1u; }
-                }
+                umma_commit_warp(v_empty(vs));
+                if (++vs == L.v_stages) { vs = 0; vp ^= 1u; }
             }
         }
     } else {
@@ -171,13 +177,13 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
         const int row = q0 + t * 128 + q * 32 + lane, pos = a.pos0 + row;
         float m_ref = -INFINITY, l = 0.0f;
         for (int j = 0; j < n[t]; ++j) {
-            mbar_wait(s_full(t), (uint32_t)j & 1u, a.status, TC_ERR_ACC_FULL);
+            mbar_wait(s_full(t, j), (uint32_t)(j >> 1) & 1u, a.status, TC_ERR_ACC_FULL);
             tc_fence_after();
             float v[64];
             {
                 uint32_t r0[32], r1[32];
-                tmem_ld_32x32(s_col(t) + lanes, r0);
-                tmem_ld_32x32(s_col(t) + lanes + 32, r1);
+                tmem_ld_32x32(s_col(t, j) + lanes, r0);
+                tmem_ld_32x32(s_col(t, j) + lanes + 32, r1);
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
@@ -199,7 +205,9 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                 m_ref = mx;
             } else {
                 const bool grow = mx > m_ref + 8.0f;
-                if (__any_sync(0xffffffffu, grow)) {                                 // PV of the tiles before is complete (s_full)
+                if (__any_sync(0xffffffffu, grow)) {
+                    mbar_wait(pv_done(t), (uint32_t)(j - 1) & 1u, a.status, TC_ERR_ACC_FULL);        // (that of j - 2 is: S(j) came after it)
+                    tc_fence_after();
                     const float c = grow ? exp2_fast(m_ref - mx) : 1.0f;
                     if (grow) m_ref = mx;
                     l *= c;
@@ -223,14 +231,15 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                 lo[i] = pack_bf16x2(p0 - bf16_lo(hi[i]), p1 - bf16_hi(hi[i]));
             }
             l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
-            tmem_st_32x32(ph_col(t) + lanes, hi);
-            tmem_st_32x32(pl_col(t) + lanes, lo);
+            tmem_st_32x32(s_col(t, j) + lanes, hi);
+            tmem_st_32x32(s_col(t, j) + lanes + 32, lo);
             tmem_st_wait();
             tc_fence_before();
-            mbar_arrive(p_full(t));
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_full(t, j));
         }
         if (n[t] > 0) {
-            mbar_wait(o_full(t), 0, a.status, TC_ERR_ACC_FULL);
+            mbar_wait(pv_done(t), (uint32_t)(n[t] - 1) & 1u, a.status, TC_ERR_ACC_FULL);
             tc_fence_after();
             const float inv = 1.0f / l;
             for (int c0 = 0; c0 < L.vp; c0 += 32) {

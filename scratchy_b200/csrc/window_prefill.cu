@@ -157,7 +157,6 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
             }
         }
     } else if (warp == 1) {
-        const bool issuer = elect_one();
         const uint32_t s_desc = umma_idesc(1, 1, 128, WF_KEYS), o_desc = umma_idesc(1, 1, 128, (uint32_t)L.vp) | UMMA_B_MN_MAJOR;
         const Own own[2] = {own_tiles(0), own_tiles(1)};
         uint64_t qd[2][CHUNKS];
@@ -180,15 +179,12 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                 if (!has[t]) continue;
                 const uint32_t col = s_col(t, started[t]), full = s_full(t, started[t]);
                 const uint64_t kd = umma_desc_k_sw128(base + L.k + ks * K_BYTES);
-                if (issuer) {
 #pragma unroll
-                    for (int c = 0; c < CHUNKS; ++c)
+                for (int c = 0; c < CHUNKS; ++c)
 #pragma unroll
-                        for (int k4 = 0; k4 < 4; ++k4)
-                            umma_f16(col, qd[t][c] + (uint64_t)(2 * k4), kd + (uint64_t)(c * (WF_K_CHUNK >> 4) + 2 * k4), s_desc, (c | k4) != 0);
-                    umma_commit(full);
-                }
-                __syncwarp();
+                    for (int k4 = 0; k4 < 4; ++k4)
+                        umma_f16_warp(col, qd[t][c] + (uint64_t)(2 * k4), kd + (uint64_t)(c * (WF_K_CHUNK >> 4) + 2 * k4), s_desc, (c | k4) != 0);
+                umma_commit_warp(full);
                 ++started[t];
             }
             const uint64_t vd = umma_desc_mn_sw128(base + L.k + prev * K_BYTES, WF_K_CHUNK);
@@ -199,19 +195,15 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                     mbar_wait(p_full(t, i), (uint32_t)(i >> 1) & 1u, a.status, TC_ERR_DEQ_WAIT);
                     tc_fence_after();
                     const uint32_t col = s_col(t, i), o = o_col(t), pv = pv_done(t);
-                    if (issuer) {
 #pragma unroll
-                        for (int k4 = 0; k4 < 4; ++k4) umma_f16_ta(o, col + 8u * k4, vd + (uint64_t)(128 * k4), o_desc, i > 0 || k4 > 0);
+                    for (int k4 = 0; k4 < 4; ++k4) umma_f16_ta_warp(o, col + 8u * k4, vd + (uint64_t)(128 * k4), o_desc, i > 0 || k4 > 0);
 #pragma unroll
-                        for (int k4 = 0; k4 < 4; ++k4) umma_f16_ta(o, col + 32u + 8u * k4, vd + (uint64_t)(128 * k4), o_desc, 1);
-                        umma_commit(pv);
-                    }
-                    __syncwarp();
+                    for (int k4 = 0; k4 < 4; ++k4) umma_f16_ta_warp(o, col + 32u + 8u * k4, vd + (uint64_t)(128 * k4), o_desc, 1);
+                    umma_commit_warp(pv);
                 }
                 before[t] = has[t];
             }
-            if (j > 0 && issuer) umma_commit(k_empty(prev));                         // both products of the tile before are issued
-            __syncwarp();
+            if (j > 0) umma_commit_warp(k_empty(prev));                              // both products of the tile before are issued
             prev = ks;
             if (++ks == L.stages) { ks = 0; kp ^= 1u; }
         }
