@@ -5,6 +5,7 @@
 
 #include <initializer_list>
 
+constexpr int ATT_MAX_WARPS = 12;                      // of a CTA
 constexpr int ATT_SPLITS = 8;                          // CTAs of a cluster at most
 constexpr int ATT_MAX_STAGES = 24;
 // Bytes of dynamic shared memory one CTA may take so that two CTAs fit on an SM; alone on its SM.
@@ -47,6 +48,37 @@ static inline AttPlan att_plan(int D, int G, int batch, int num_kv_heads, int bl
         p.warps = w;
         p.stages_per_warp = fit < 3 ? int(fit) : 3;
         if (p.stages_per_warp >= 2) break;
+    }
+    return p;
+}
+
+// More sequences than a kv head has SMs: every CTA takes whole sequences, alone on its SM, `bins` CTAs per kv head.  Dealt back and forth by falling
+// length (rank r goes to CTA r % bins in even rounds, from the other end in odd ones) the longest CTA has little more than the mean or than the longest
+// sequence.
+constexpr int ATT_MAX_ITEMS = 4;
+constexpr size_t ATT_SMEM_PACKED = 226 * 1024;
+struct AttBins {
+    int bins, items;                                   // CTAs per kv head; sequences a CTA takes at most (0: not this way)
+    int warps, stages, table_cap;
+    size_t smem;
+};
+static inline AttBins att_bins(int D, int G, int batch, int num_kv_heads, int block_size, int max_blocks_per_seq, int sm_count, int nsplit) {
+    AttBins p{};
+    p.bins = sm_count / num_kv_heads;
+    if (nsplit > 1 || p.bins < 1 || batch <= p.bins || (batch + p.bins - 1) / p.bins > ATT_MAX_ITEMS) return p;
+    const int items = (batch + p.bins - 1) / p.bins;
+    const size_t stage = size_t(block_size) * D * 4;
+    p.table_cap = items * max_blocks_per_seq;
+    for (int w : {12, 8}) {                            // two stages each, more warps before more stages
+        const size_t fixed = size_t(items) * w * G * (D + 2) * sizeof(float) + size_t((p.table_cap + 1) & ~1) * 4 + size_t(batch) * 4 + ATT_MAX_STAGES * 8 +
+                             1024 + 128;
+        const size_t fit = ATT_SMEM_PACKED > fixed ? (ATT_SMEM_PACKED - fixed) / (stage * w) : 0;
+        if (fit < 2) continue;
+        p.warps = w;
+        p.stages = w * 2;
+        p.smem = size_t(p.stages) * stage + fixed;
+        p.items = items;
+        break;
     }
     return p;
 }

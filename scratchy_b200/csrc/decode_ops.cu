@@ -311,7 +311,7 @@ template <int D>
 __device__ __forceinline__ void att_cta_merge(int G, int nwarps, const float* warp_part, float* cl_part, int split, int nsplit,
                                               int q_head0, int b, uint16_t* __restrict__ out, long long ld_o) {
     constexpr int STATE = D + 2;
-    __shared__ float wgt[8][ATT_WARPS + 2];          // per query head: the warps' weights, the merged maximum and sum
+    __shared__ float wgt[8][ATT_MAX_WARPS + 2];      // per query head: the warps' weights, the merged maximum and sum
     const int nthreads = nwarps * 32;
     asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
     if (threadIdx.x < G) {
@@ -324,8 +324,8 @@ __device__ __forceinline__ void att_cta_merge(int G, int nwarps, const float* wa
             wgt[g][w] = c;
             lt += warp_part[(w * G + g) * STATE + D + 1] * c;
         }
-        wgt[g][ATT_WARPS] = mt;
-        wgt[g][ATT_WARPS + 1] = lt;
+        wgt[g][ATT_MAX_WARPS] = mt;
+        wgt[g][ATT_MAX_WARPS + 1] = lt;
     }
     asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
     for (int idx = threadIdx.x; idx < G * D; idx += nthreads) {
@@ -333,13 +333,13 @@ __device__ __forceinline__ void att_cta_merge(int G, int nwarps, const float* wa
         float a = 0.0f;
         for (int w = 0; w < nwarps; ++w) a += warp_part[(w * G + g) * STATE + d] * wgt[g][w];
         if (nsplit == 1) {
-            out[b * ld_o + (q_head0 + g) * D + d] = uint16_t(f32_to_bf16_bits(a * __fdiv_rn(1.0f, wgt[g][ATT_WARPS + 1] + 1e-6f)));
+            out[b * ld_o + (q_head0 + g) * D + d] = uint16_t(f32_to_bf16_bits(a * __fdiv_rn(1.0f, wgt[g][ATT_MAX_WARPS + 1] + 1e-6f)));
         } else {
             float* dst = cl_part + (split * G + g) * STATE;
             att_store_rank0(dst + d, a);
             if (d == 0) {
-                att_store_rank0(dst + D, wgt[g][ATT_WARPS]);
-                att_store_rank0(dst + D + 1, wgt[g][ATT_WARPS + 1]);
+                att_store_rank0(dst + D, wgt[g][ATT_MAX_WARPS]);
+                att_store_rank0(dst + D + 1, wgt[g][ATT_MAX_WARPS + 1]);
             }
         }
     }
@@ -543,8 +543,8 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_kernel(
 
 // ---- the streaming variant: TMA tiles + tensor cores -------------------------------------------
 // In the paged layout one (block, kv head) is a contiguous run of block_size tokens x D bf16.  A run
-// (K and V) comes into shared memory with a few 3-D TMA tile loads (tensor map over the cache viewed
-// as [token][D/64][64], 128-byte swizzle), one stage per cache block, completion counted in bytes on
+// (K and V) comes into shared memory with two 3-D TMA tile loads (tensor map over the cache viewed
+// as [D/64][token][64], 128-byte swizzle; a copy costs the lane that issues it about 130 cycles), one stage per cache block, completion counted in bytes on
 // the stage's mbarrier.  Every warp has its own ring of stages, takes blocks warp, warp + warps, ..
 // and refills a stage itself once its lanes are done with it, so no warp waits for another: a producer
 // warp whose lanes fed one stage each went round in lockstep with the slowest of them.  Blocks run
@@ -557,7 +557,9 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_kernel(
 //
 // What bounds it: HBM (8 KB per block of 16 tokens and kv head), and the longest sequence's CTA.  Llama-3.2-3B at 32 sequences of
 // 512 to 2048 tokens, 153 MB per call, in a stream of calls: 57.6 us with the producer warp and a second MMA for the remainders,
-// 39.7 us (3.9 TB/s) with rings of the warps' own and their number as in attention_plan.h.
+// 39.9 us with rings of the warps' own and a CTA for every sequence and kv head, 32.9 us (4.7 TB/s) with whole sequences dealt to one CTA
+// per SM (PACKED; their blocks in even shares to the warps, 36.8 us with the sequences one after the other over all of eight warps).
+// 20 sequences 39.2 -> 26.0 us, 48 61.8 -> 46.3; 32 of 100 to 400 tokens 11.3 -> 12.9 us, 32 of 2048 45.1 -> 47.5, what it costs.
 constexpr int ATT_ERR_FULL = 0x0A000001;
 
 __device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const CUtensorMap* tmap, int c0, int c1, int c2, uint32_t bar) {
@@ -617,13 +619,16 @@ __device__ __forceinline__ uint32_t att_rope_pair(uint32_t x0w, uint32_t x1w, co
     return pack_bf16x2(rl, rh);
 }
 
-template <int D>
-__global__ void __launch_bounds__(ATT_THREADS) attention_decode_tc_kernel(
+// PACKED: a CTA has its SM to itself and takes one to `items` whole sequences of a kv head, so that all CTAs have about as much to read
+// (attention_plan.h): the sequences, ranked by their lengths on the device, are dealt to the gridDim.z CTAs back and forth.  The warps' rings run on
+// from one sequence into the next, and the sequences' partial sums meet at the end.  Registers: at most 168 (ATT_MAX_WARPS in the bounds), so that two
+// half-SM CTAs of six warps fit; at 173 8 sequences took 21.2 us for 13.0.
+template <int D, bool PACKED>
+__global__ void __launch_bounds__(ATT_MAX_WARPS * 32) attention_decode_tc_kernel(
     const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, const uint16_t* __restrict__ q,
     long long ld_q, const uint32_t* __restrict__ block_table, const uint32_t* __restrict__ seq_used_k,
     uint16_t* __restrict__ out, long long ld_o, int G, int num_kv_heads, int block_size, int max_blocks_per_seq,
-    uint32_t num_blocks, int table_cap, int stages, float scale, int* status, AttRope rope) {
-    constexpr int NH = D / 64;                       // 128-byte rows per token
+    uint32_t num_blocks, int table_cap, int stages, float scale, int* status, AttRope rope, int batch, int items) {
     constexpr int STATE = D + 2;
     constexpr int KSTEPS = D / 16;
     constexpr int NTILES = D / 8;
@@ -633,72 +638,153 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_tc_kernel(
     const uint32_t half_bytes = uint32_t(block_size) * 128;                // one 64-dim half of it: [token][128 bytes], swizzled
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(att_smem) + 1023) & ~uintptr_t(1023));
     float* warp_part = reinterpret_cast<float*>(ring);                     // aliases the ring once it is drained
-    const size_t ring_bytes = max(size_t(stages) * 2 * chunk, size_t(nwarps) * G * STATE * sizeof(float));
+    const size_t ring_bytes = PACKED ? size_t(stages) * 2 * chunk : max(size_t(stages) * 2 * chunk, size_t(nwarps) * G * STATE * sizeof(float));
     float* cl_part = reinterpret_cast<float*>(ring + ((ring_bytes + 127) & ~size_t(127)));        // [nsplit<=8][G][STATE]
     uint32_t* blocks = reinterpret_cast<uint32_t*>(cl_part + ATT_SPLITS * G * STATE);
+    if (PACKED) {                                                          // sums of their own: [item][warp][G][STATE]
+        warp_part = cl_part;
+        blocks = reinterpret_cast<uint32_t*>(warp_part + size_t(items) * nwarps * G * STATE);
+    }
     uint64_t* bars = reinterpret_cast<uint64_t*>(blocks + ((table_cap + 1) & ~1));                // full[stages]
+    int* lens = reinterpret_cast<int*>(bars + stages);                                            // PACKED: [batch]
+    __shared__ int item_seq[ATT_MAX_ITEMS], item_len[ATT_MAX_ITEMS];
+    __shared__ float rope_rows[PACKED ? ATT_MAX_ITEMS : 1][2][D / 2];        // cos and sin of the sequences' positions
 
     pdl_trigger();
     uint32_t nsplit;
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(nsplit));
     const int split = int(att_cluster_rank());
-    const int kvh = blockIdx.y, b = blockIdx.z;
+    const int kvh = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    long long kv_len_raw = seq_used_k[b];
     const long long kv_cap = (long long)max_blocks_per_seq * block_size;
-    if (kv_len_raw > kv_cap) {
-        if (threadIdx.x == 0) atomicCAS(status, 0, DEV_BAD_BLOCK);
-        kv_len_raw = kv_cap;
-    }
-    const int kv_len = int(kv_len_raw);
-    const int total_blk = (kv_len + block_size - 1) / block_size;
-    const int per = (total_blk + int(nsplit) - 1) / int(nsplit);
-    const int first_blk = min(split * per, total_blk);
-    int nblk = min(per, total_blk - first_blk);
-    if (nblk > table_cap) {
-        if (threadIdx.x == 0) atomicCAS(status, 0, DEV_BAD_BLOCK);
-        nblk = 0;
-    }
-    for (int i = threadIdx.x; i < nblk; i += int(blockDim.x)) {
-        uint32_t pb = block_table[size_t(b) * max_blocks_per_seq + first_blk + i];
-        if (pb >= num_blocks) {                                            // never copy from outside the cache
-            atomicCAS(status, 0, DEV_BAD_BLOCK);
-            pb = 0;
+    auto used = [&](int seq) {
+        const long long raw = seq_used_k[seq];
+        if (raw > kv_cap) atomicCAS(status, 0, DEV_BAD_BLOCK);
+        return int(raw > kv_cap ? kv_cap : raw);
+    };
+    auto look_up = [&](int seq, int first, int count, int at) {            // blocks[at ..]: the sequence's blocks from `first` on
+        for (int i = threadIdx.x; i < count; i += int(blockDim.x)) {
+            uint32_t pb = block_table[size_t(seq) * max_blocks_per_seq + first + i];
+            if (pb >= num_blocks) {                                        // never copy from outside the cache
+                atomicCAS(status, 0, DEV_BAD_BLOCK);
+                pb = 0;
+            }
+            blocks[at + i] = pb;
         }
-        blocks[i] = pb;
-    }
+    };
+    auto blocks_of = [&](int len) { return (len + block_size - 1) / block_size; };
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) mbar_init(smem_u32(&bars[s]), 1);
         fence_mbar_init();
+    }
+    int b = blockIdx.z, kv_len = 0, total_blk = 0, first_blk = 0, nblk = 0;
+    if (PACKED) {
+        if (threadIdx.x < ATT_MAX_ITEMS) {
+            item_seq[threadIdx.x] = -1;
+            item_len[threadIdx.x] = 0;
+        }
+        for (int i = threadIdx.x; i < batch; i += int(blockDim.x)) lens[i] = used(i);
+        __syncthreads();
+        const int bins = int(gridDim.z);
+        for (int i = threadIdx.x; i < batch; i += int(blockDim.x)) {
+            const int mine = lens[i];
+            int rank = 0;
+            for (int k = 0; k < batch; ++k) rank += lens[k] > mine || (lens[k] == mine && k < i);
+            const int g = rank / bins, at = rank - g * bins;
+            if ((g & 1 ? bins - 1 - at : at) == int(blockIdx.z)) {
+                item_seq[g] = i;
+                item_len[g] = mine;
+            }
+        }
+        __syncthreads();
+        int at = 0;
+        for (int g = 0; g < items; ++g) {
+            const int count = blocks_of(item_len[g]);
+            if (item_seq[g] >= 0) look_up(item_seq[g], 0, count, at);
+            at += count;
+        }
+    } else {
+        kv_len = used(b);
+        total_blk = blocks_of(kv_len);
+        const int per = (total_blk + int(nsplit) - 1) / int(nsplit);
+        first_blk = min(split * per, total_blk);
+        nblk = min(per, total_blk - first_blk);
+        if (nblk > table_cap) {
+            if (threadIdx.x == 0) atomicCAS(status, 0, DEV_BAD_BLOCK);
+            nblk = 0;
+        }
+        look_up(b, first_blk, nblk, 0);
     }
     __syncthreads();
     // What the previous kernels of the stream produce for this one is q and the cache slot of the newest token
     // (position kv_len - 1, in the sequence's last block).  Every other cache block was written in earlier steps, so a warp
     // fills its ring at once and only the last block and q wait (with the append folded in, no preceding kernel writes the
     // cache at all).
-    const int newest_blk = total_blk - 1;
     const int spw = stages / nwarps;
-    auto load = [&](int n) {                           // (one lane) the warp's n-th block
-        const int i = warp + n * nwarps;
-        if (i >= nblk) return;
+    // A warp's n-th block as an index of `blocks`: every nwarps-th one of a sequence; of several (PACKED) an even share of all of them in a row, so
+    // that most warps work on one sequence and all end together.
+    const int ng = PACKED ? items : 1;
+    int w_lo = warp, w_hi = nblk;
+    if (PACKED) {
+        int all = 0;
+        for (int g = 0; g < ng; ++g) all += blocks_of(item_len[g]);
+        w_lo = all * warp / nwarps;
+        w_hi = all * (warp + 1) / nwarps;
+    }
+    auto index_of = [&](int n) { return PACKED ? w_lo + n : w_lo + n * nwarps; };
+    auto is_newest = [&](int f) {
+        bool last = !PACKED && first_blk + f >= total_blk - 1;
+        for (int g = 0; PACKED && g < ng; ++g) {
+            f -= blocks_of(item_len[g]);
+            last |= f == -1;
+        }
+        return last;
+    };
+    auto load = [&](int n) {                           // (one lane) the warp's n-th block into its stage
+        const int f = index_of(n);
+        if (f >= w_hi) return;
         const int s = warp * spw + n % spw;
         const uint32_t full = smem_u32(&bars[s]), dst = smem_u32(ring + size_t(s) * 2 * chunk);
-        const int token0 = int((blocks[i] * uint32_t(num_kv_heads) + uint32_t(kvh)) * uint32_t(block_size));
+        const int token0 = int((blocks[f] * uint32_t(num_kv_heads) + uint32_t(kvh)) * uint32_t(block_size));
         mbar_arrive_expect_tx(full, 2 * chunk);
-#pragma unroll
-        for (int h = 0; h < NH; ++h) {                 // [half][token][128 bytes]: ldmatrix rows 8 tokens apart never share a bank
-            tma_load_3d(dst + h * half_bytes, &k_map, 0, h, token0, full);
-            tma_load_3d(dst + chunk + h * half_bytes, &v_map, 0, h, token0, full);
-        }
+        tma_load_3d(dst, &k_map, 0, token0, 0, full);  // [half][token][128 bytes]: ldmatrix rows 8 tokens apart never share a bank
+        tma_load_3d(dst + chunk, &v_map, 0, token0, 0, full);
     };
     {
         // lane n fills stage n: the lanes issue side by side, and q's loads below are not held up behind them
-        const bool waits = !rope.enabled && first_blk + warp + lane * nwarps >= newest_blk;
+        const bool waits = !rope.enabled && index_of(lane) < w_hi && is_newest(index_of(lane));
         if (lane < spw && !waits) load(lane);
+        // The rotation's rows, which follow from what the host wrote for the step, come in while the kernel before runs (two loads one after the
+        // other; one sequence of 2048 tokens 7.8 -> 7.5 us, 8 13.7 -> 13.0).
+        if (rope.enabled)
+            for (int i = threadIdx.x; i < ng * (D / 2); i += int(blockDim.x)) {
+                const int g = i / (D / 2), d = i - g * (D / 2), seq = PACKED ? item_seq[g] : b;
+                const uint32_t pos = seq >= 0 ? rope.positions[seq] : rope.max_pos;
+                rope_rows[g][0][d] = pos < rope.max_pos ? rope.cos_table[size_t(pos) * D + d] : 0.0f;
+                rope_rows[g][1][d] = pos < rope.max_pos ? rope.sin_table[size_t(pos) * D + d] : 0.0f;
+            }
         pdl_wait();
         if (lane < spw && waits) load(lane);
-        __syncwarp();
+        __syncthreads();
+        int j = 0, at = 0;                             // the warp's blocks so far; where this sequence's blocks start
+        for (int g = 0; g < ng; ++g) {
+        int i0 = warp, i1 = nblk;                      // the warp's blocks of this sequence
+        if (PACKED) {
+            b = item_seq[g];
+            if (b < 0) continue;
+            kv_len = item_len[g];
+            total_blk = blocks_of(kv_len);
+            i0 = max(w_lo - at, 0);
+            i1 = min(w_hi - at, total_blk);
+            at += total_blk;
+            if (i0 >= i1) {                            // none
+                for (int x = lane; x < G * STATE; x += 32) warp_part[(g * nwarps + warp) * G * STATE + x] = x % STATE == D ? -INFINITY : 0.0f;
+                continue;
+            }
+        }
+        const int table0 = PACKED ? at - total_blk : 0;
+        const int newest_blk = total_blk - 1;
         const int row = lane >> 2, quad = lane & 3;
         uint32_t qa0[KSTEPS], qa2[KSTEPS];             // A fragments of Q: row = query head (zero beyond G), 16 dims per step
 #pragma unroll
@@ -715,16 +801,21 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_tc_kernel(
             if (pos >= rope.max_pos) {
                 if (lane == 0) atomicCAS(status, 0, DEV_BAD_POSITION);
             } else if (row < G) {
-                const float* cs = rope.cos_table + size_t(pos) * D;
-                const float* sn = rope.sin_table + size_t(pos) * D;
+                const uint32_t rows = smem_u32(&rope_rows[g][0][0]);
 #pragma unroll
                 for (int kk = 0; kk < KSTEPS / 2; ++kk) {
                     const int d = kk * 16 + quad * 2;                      // < D/2; partner dim d + D/2 sits KSTEPS/2 steps on
+                    float cs[2][2], sn[2][2];                              // (volatile: all of a row's at once would cost 34 registers)
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(cs[x][0]), "=f"(cs[x][1]) : "r"(rows + 4u * (d + 8 * x)));
+                        asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(sn[x][0]), "=f"(sn[x][1]) : "r"(rows + 4u * (D / 2 + d + 8 * x)));
+                    }
                     const uint32_t a0 = qa0[kk], b0 = qa0[kk + KSTEPS / 2], a2 = qa2[kk], b2 = qa2[kk + KSTEPS / 2];
-                    qa0[kk] = att_rope_pair(a0, b0, cs + d, sn + d, true);
-                    qa0[kk + KSTEPS / 2] = att_rope_pair(a0, b0, cs + d, sn + d, false);
-                    qa2[kk] = att_rope_pair(a2, b2, cs + d + 8, sn + d + 8, true);
-                    qa2[kk + KSTEPS / 2] = att_rope_pair(a2, b2, cs + d + 8, sn + d + 8, false);
+                    qa0[kk] = att_rope_pair(a0, b0, cs[0], sn[0], true);
+                    qa0[kk + KSTEPS / 2] = att_rope_pair(a0, b0, cs[0], sn[0], false);
+                    qa2[kk] = att_rope_pair(a2, b2, cs[1], sn[1], true);
+                    qa2[kk + KSTEPS / 2] = att_rope_pair(a2, b2, cs[1], sn[1], false);
                 }
             }
         }
@@ -736,7 +827,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_tc_kernel(
         // ldmatrix lane roles: lane supplies the row address of matrix lane/8, row lane%8
         const int lm = lane >> 3, lr = lane & 7;
         bool alive = true;
-        for (int i = warp, j = 0; i < nblk && alive; i += nwarps, ++j) {
+        for (int i = i0; i < i1 && alive; i += PACKED ? 1 : nwarps, ++j) {
             const int s = warp * spw + j % spw;
             alive = mbar_wait(smem_u32(&bars[s]), uint32_t((j / spw) & 1), status, ATT_ERR_FULL);
             if (!alive) break;
@@ -747,7 +838,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_tc_kernel(
                 // the newest token: rotate k_new, write it and v_new to the cache slot and into this tile
                 const int slot = kv_len - 1 - t0;
                 const uint32_t pos = rope.positions[b];
-                const size_t cache_off = ((size_t(blocks[i]) * num_kv_heads + kvh) * block_size + slot) * D;
+                const size_t cache_off = ((size_t(blocks[table0 + i]) * num_kv_heads + kvh) * block_size + slot) * D;
                 unsigned char* ktile = ring + size_t(s) * 2 * chunk;
                 // a block id outside the cache was replaced by 0 for the loads (and reported): never append there
                 const bool slot_ok = pos < rope.max_pos && block_table[size_t(b) * max_blocks_per_seq + newest_blk] < num_blocks;
@@ -755,8 +846,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_tc_kernel(
                     const int d = lane * 8;                                // dims d..d+7 pair with d + D/2 ..
                     const uint16_t* kp = rope.k_new + b * rope.ld_k + size_t(kvh) * D;
                     const uint4 x0 = *reinterpret_cast<const uint4*>(kp + d), x1 = *reinterpret_cast<const uint4*>(kp + d + D / 2);
-                    const float* cs = rope.cos_table + size_t(pos) * D + d;
-                    const float* sn = rope.sin_table + size_t(pos) * D + d;
+                    const float *cs = rope_rows[g][0] + d, *sn = rope_rows[g][1] + d;
                     const uint32_t xw0[4] = {x0.x, x0.y, x0.z, x0.w}, xw1[4] = {x1.x, x1.y, x1.z, x1.w};
                     uint32_t r0[4], r1[4];
 #pragma unroll
@@ -847,9 +937,9 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_tc_kernel(
         lsum += __shfl_xor_sync(0xffffffffu, lsum, 2);
         // every warp is past its last ring read before warp_part (which aliases the ring) is written;
         // the blocks another warp still waits for are that warp's own
-        asm volatile("bar.sync 1, %0;" ::"r"(nwarps * 32) : "memory");
+        if (!PACKED) asm volatile("bar.sync 1, %0;" ::"r"(nwarps * 32) : "memory");
         if (row < G) {
-            float* st = warp_part + (warp * G + row) * STATE;
+            float* st = warp_part + ((g * nwarps + warp) * G + row) * STATE;
 #pragma unroll
             for (int nt = 0; nt < NTILES; ++nt) {
                 st[nt * 8 + quad * 2] = o[nt][0] + o[nt][2];
@@ -860,9 +950,13 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_tc_kernel(
                 st[D + 1] = lsum;
             }
         }
-        att_cta_merge<D>(G, nwarps, warp_part, cl_part, split, int(nsplit), kvh * G, b, out, ld_o);
+        if (!PACKED) att_cta_merge<D>(G, nwarps, warp_part, cl_part, split, int(nsplit), kvh * G, b, out, ld_o);
+        }
+        if (PACKED)
+            for (int g = 0; g < ng; ++g)
+                if (item_seq[g] >= 0) att_cta_merge<D>(G, nwarps, warp_part + size_t(g) * nwarps * G * STATE, cl_part, 0, 1, kvh * G, item_seq[g], out, ld_o);
     }
-    if (nsplit > 1) {
+    if (!PACKED && nsplit > 1) {
         att_cluster_sync();
         if (split == 0) att_cluster_finish<D>(G, cl_part, int(nsplit), kvh * G, b, out, ld_o, int(blockDim.x));
     }
@@ -893,13 +987,15 @@ cudaError_t attention_launch(const uint16_t* q, long long ld_q, const uint16_t* 
     const unsigned long long total_tokens = (unsigned long long)num_blocks * num_kv_heads * block_size;
     tc_encode_tiled_fn enc = tc_tensor_map_encoder();
     if (enc && block_size % 16 == 0 && block_size <= 256 && total_tokens < (1ull << 31) && spw >= 1) {
-        const int stages = spw * nwarps;
+        const AttBins bins = att_bins(D, G, batch, num_kv_heads, block_size, max_blocks_per_seq, sm_count, nsplit);
+        const bool packed = bins.items > 0;
+        const int stages = packed ? bins.stages : spw * nwarps;
         const size_t ring = std::max(size_t(stages) * 2 * chunk, size_t(nwarps) * G * (D + 2) * sizeof(float));
-        const size_t smem = ((ring + 127) & ~size_t(127)) + plan.fixed;
+        const size_t smem = packed ? bins.smem : ((ring + 127) & ~size_t(127)) + plan.fixed;
         CUtensorMap maps[2];
-        const cuuint64_t dims[3] = {64, cuuint64_t(D / 64), cuuint64_t(total_tokens)};
-        const cuuint64_t strides[2] = {128, cuuint64_t(D) * 2};
-        const cuuint32_t box[3] = {64, 1, cuuint32_t(block_size)};
+        const cuuint64_t dims[3] = {64, cuuint64_t(total_tokens), cuuint64_t(D / 64)};     // a box: every 64-dim half of a block's tokens
+        const cuuint64_t strides[2] = {cuuint64_t(D) * 2, 128};
+        const cuuint32_t box[3] = {64, cuuint32_t(block_size), cuuint32_t(D / 64)};
         const cuuint32_t estr[3] = {1, 1, 1};
         const void* bases[2] = {cache_k, cache_v};
         for (int i = 0; i < 2; ++i) {
@@ -908,15 +1004,15 @@ cudaError_t attention_launch(const uint16_t* q, long long ld_q, const uint16_t* 
                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
         }
-        auto kernel = attention_decode_tc_kernel<D>;
+        auto kernel = packed ? attention_decode_tc_kernel<D, true> : attention_decode_tc_kernel<D, false>;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
-        cfg.gridDim = dim3(nsplit, num_kv_heads, batch);
-        cfg.blockDim = dim3(nwarps * 32);
+        cfg.gridDim = packed ? dim3(1, num_kv_heads, bins.bins) : dim3(nsplit, num_kv_heads, batch);
+        cfg.blockDim = dim3(packed ? bins.warps * 32 : nwarps * 32);
         cfg.dynamicSmemBytes = smem;
-        attr[0].val.clusterDim.x = nsplit;
+        attr[0].val.clusterDim.x = packed ? 1 : nsplit;
         return cudaLaunchKernelEx(&cfg, kernel, maps[0], maps[1], q, ld_q, block_table, seq_used_k, out, ld_o, G, num_kv_heads,
-                                  block_size, max_blocks_per_seq, num_blocks, table_cap, stages, scale, status, rope);
+                                  block_size, max_blocks_per_seq, num_blocks, packed ? bins.table_cap : table_cap, stages, scale, status, rope, batch, bins.items);
     }
     if (rope.enabled) return cudaErrorNotSupported;  // the rotation and the append are folded into the streaming variant only
     // small or odd blocks: per-token loads

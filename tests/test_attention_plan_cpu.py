@@ -48,3 +48,32 @@ def test_the_width_of_the_table_cuts_no_sequence(plan, block):
         for tokens in (256, 1024, 1536, 2048, 5000, 32768):
             p = plan(128, 3, batch, 8, block, -(-tokens // block))
             assert p.nsplit == fits and p.table_cap >= -(-(-(-tokens // block)) // fits)
+
+
+def test_sequences_are_dealt_evenly_to_bins_that_fit(tmp_path):
+    """The packed layout: every sequence has a place, the shared memory of a CTA suffices, and falling lengths dealt back and forth leave no CTA
+    with more than the mean, the longest sequence and the spread of one round allow."""
+    source, library = tmp_path / "bins.cpp", tmp_path / "bins.so"
+    source.write_text('#include "attention_plan.h"\nextern "C" AttBins bins(int d, int g, int b, int h, int bs, int mb, int split) '
+                      f'{{ return att_bins(d, g, b, h, bs, mb, {SMS}, split); }}\n')
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, "-o", library, source], check=True)
+
+    class Bins(ctypes.Structure):
+        _fields_ = [(n, ctypes.c_int) for n in ("bins", "items", "warps", "stages", "table_cap")] + [("smem", ctypes.c_size_t)]
+    call = ctypes.CDLL(str(library)).bins
+    call.restype = Bins
+    for batch in range(1, 80):
+        for g in range(1, 9):
+            for block, blocks in ((16, 128), (32, 64), (16, 2048), (128, 16)):
+                p = call(128, g, batch, 8, block, blocks, 1)
+                if not p.items:
+                    continue
+                assert p.bins * 8 <= SMS and p.bins < batch <= p.bins * p.items and p.items <= 4
+                assert p.stages >= 2 * p.warps and p.smem <= 227 * 1024 and p.table_cap >= p.items * blocks
+                lens = sorted(((7919 * (i + g)) % 1500 + 500 for i in range(batch)), reverse=True)
+                load, rounds = [0] * p.bins, -(-batch // p.bins)
+                for r, n in enumerate(lens):
+                    at = r % p.bins
+                    load[p.bins - 1 - at if (r // p.bins) & 1 else at] += n
+                assert max(load) <= max(lens[0], sum(load) / p.bins) + lens[0] - lens[-1]
+    assert not call(128, 3, 32, 8, 16, 128, 2).items and not call(128, 3, 18, 8, 16, 128, 1).items and not call(128, 3, 73, 8, 16, 128, 1).items

@@ -260,6 +260,24 @@ def test_rope_attention_one_launch_equals_the_two_operators(lens, hq, hkv, d, bs
     assert rel_l2(bits_of(one), rbits(want)) <= REL_L2_TOL
 
 
+@pytest.mark.parametrize("lens,hq,hkv,d,bs", [
+    ([16 * (i % 5) + 1 for i in range(19)], 24, 8, 128, 16),                      # one sequence more than CTAs of a kv head
+    ([1 + (97 * i) % 800 for i in range(36)], 24, 8, 128, 16),                    # two for each
+    ([700] * 37, 16, 8, 128, 16),                                                 # equal lengths, three rounds
+    ([1 + (131 * i) % 300 for i in range(72)], 8, 8, 64, 16),                     # four for each, head_dim 64
+    ([1 + (131 * i) % 300 for i in range(73)], 8, 8, 64, 16),                     # one too many: a CTA per pair
+    ([40 + (53 * i) % 500 for i in range(40)], 32, 4, 128, 16),                   # 8 query heads per kv head, 37 CTAs of a head
+    ([1 + (211 * i) % 900 for i in range(30)], 24, 8, 128, 32),                   # 32-token blocks
+    ([5000] + [3] * 21, 16, 8, 128, 16),                                          # one long sequence among short ones
+])
+def test_attention_of_more_sequences_than_ctas(lens, hq, hkv, d, bs):
+    """Whole sequences dealt to CTAs by their lengths: rings that run on from one sequence into the next, appended tokens of several
+    sequences in a CTA, CTAs with fewer sequences than others."""
+    test_rope_attention_one_launch_equals_the_two_operators(lens, hq, hkv, d, bs)
+    if bs == 16 and len(lens) < 40:
+        test_attention_via_cache(lens[:-2] + [0, 1], hq, hkv, d, bs)
+
+
 def test_rope_attention_refuses_what_it_cannot_stream():
     """Blocks that are not a multiple of 16 tokens have no one-launch form: the call says so and touches nothing."""
     import torch
