@@ -18,6 +18,11 @@
 // chunks: a first launch runs only the state updates of every group (the first from the sequence's state, the others from
 // nothing), a second one lets every group put together the state it starts from (S' = e^(F+m-m') S + e^(M-m') U over the
 // groups before it) and compute its outputs; its last group leaves the sequence's state.
+//
+// What bounds it: mma.sync, about 14 cycles for a 16x8x16 product and SM quarter: 10,000 of the 15,500 cycles that a chunk of 128 columns takes, and the
+// latencies around it.  So the slices are as wide as an SM's shared memory takes (128 columns at up to 128 dimensions): the products of queries and keys
+// are computed once for a slice.  8192 tokens, 12 heads of 128 x 256: 468 us in slices of 128, 541 in slices of 64; 2000 tokens with a constant decay 130
+// and 139 us.  Loading by warps of their own instead of the computing ones was slower (524 us).
 #pragma once
 
 #include "memory.cuh"
@@ -327,10 +332,32 @@ __global__ void __launch_bounds__(CH_THREADS, 1) memory_chunk_kernel(MemoryArgs 
                     if (t4 == 0) psum[quarter * CH_L + t] = sum;
                 }
             }
-            for (int i = tid; i < CH_L * COLS / 2; i += CH_T) {     // values weighted for the state's update, and the ones
-                const int r = i / (COLS / 2), x = (i - r * (COLS / 2)) * 2;
-                const uint32_t w = *reinterpret_cast<const uint32_t*>(Vc + (size_t)r * LDV + x);
-                split_store(wv_hi, wv_lo, (size_t)r * LDV + x, bf16_lo(w) * w_up[r], bf16_hi(w) * w_up[r]);
+            // Values weighted for the state's update, and the ones: 8 values a thread and round, all rounds read before any is written (two values
+            // at a time, one round behind the other's stores, this took 3500 of a chunk's 16000 cycles)
+            constexpr int WV = (CH_L * COLS / 8 + CH_T - 1) / CH_T;
+            uint4 wv[WV];
+            float up[WV];
+#pragma unroll
+            for (int j = 0; j < WV; ++j) {
+                const int i = min(tid + j * CH_T, CH_L * COLS / 8 - 1), r = i / (COLS / 8);
+                wv[j] = *reinterpret_cast<const uint4*>(Vc + (size_t)r * LDV + (i - r * (COLS / 8)) * 8);
+                up[j] = w_up[r];
+            }
+#pragma unroll
+            for (int j = 0; j < WV; ++j) {
+                const int i = tid + j * CH_T, r = i / (COLS / 8);
+                if (i >= CH_L * COLS / 8) break;
+                const uint32_t w[4] = {wv[j].x, wv[j].y, wv[j].z, wv[j].w};
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float x = bf16_lo(w[k]) * up[j], y = bf16_hi(w[k]) * up[j];
+                    hi[k] = pack_bf16x2(x, y);
+                    lo[k] = pack_bf16x2(x - bf16_lo(hi[k]), y - bf16_hi(hi[k]));
+                }
+                const size_t at = (size_t)r * LDV + (i - r * (COLS / 8)) * 8;
+                *reinterpret_cast<uint4*>(wv_hi + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(wv_lo + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             }
             if (!DECAY && tid < CH_L) split_store(wv_hi, wv_lo, (size_t)tid * LDV + COLS, w_up[tid], 0.0f);
             asm volatile("bar.sync 1, %0;" ::"n"(CH_T) : "memory");         // (the gate warp has the whole chunk for its work)
@@ -459,16 +486,17 @@ ChPlan ch_plan(const scr_mlstm_shape& s, const scr_step& st, int sms) {
     const int chains = s.heads * st.batch, chunks = scr_ceil_div(st.max_count, CH_L);
     // narrow slices where the wide ones do not fit an SM, or where even all of them leave SMs idle on a short sequence
     p.cols = s.dim > 128 || s.vdim <= 32 || (scr_ceil_div(s.vdim, 32) * chains <= sms && chunks < 8) ? 32 : 64;
+    if (p.cols == 64 && s.vdim % 128 == 0 && chunks >= 8) p.cols = 128;
     const int ctas = scr_ceil_div(s.vdim, p.cols) * chains;
     p.groups = 1;
     p.chunks = chunks;
     if (chunks >= 8 && 2 * ctas <= sms * 3) {
         // the second pass costs one chunk's update again: cut to about two rounds of CTAs, groups of at least two chunks
-        p.groups = std::min(std::max(2, 2 * sms / ctas), chunks / 2);
+        p.groups = std::min(std::max(2, (p.cols == 128 ? 1 : 2) * sms / ctas), chunks / 2);
         p.chunks = scr_ceil_div(chunks, p.groups);
         p.groups = scr_ceil_div(chunks, p.chunks);
     }
-    const size_t entry = p.cols == 64 ? ChShape<64, 8>::kEntryFloats : s.dim > 128 ? ChShape<32, 16>::kEntryFloats : ChShape<32, 8>::kEntryFloats;
+    const size_t entry = p.cols == 128 ? ChShape<128, 8>::kEntryFloats : p.cols == 64 ? ChShape<64, 8>::kEntryFloats : s.dim > 128 ? ChShape<32, 16>::kEntryFloats : ChShape<32, 8>::kEntryFloats;
     p.bytes = p.groups > 1 ? (size_t)ctas * (p.groups + 1) * entry * sizeof(float) : 0;
     return p;
 }
@@ -509,6 +537,7 @@ int32_t ch_run(scr_ctx* ctx, const MemoryArgs& a, void* workspace, size_t worksp
     if (p.bytes > workspace_bytes || (p.bytes && !workspace)) return scr_fail(ctx, SCR_E_WORKSPACE, "matrix memory in %d groups needs %zu bytes", p.groups, p.bytes);
     float* ws = (float*)workspace;
     if (a.s.dim > 128) return ch_launch<32, 16, DECAY>(ctx, a, p, ws, stream);
+    if (p.cols == 128) return ch_launch<128, 8, DECAY>(ctx, a, p, ws, stream);
     return p.cols == 64 ? ch_launch<64, 8, DECAY>(ctx, a, p, ws, stream) : ch_launch<32, 8, DECAY>(ctx, a, p, ws, stream);
 }
 
