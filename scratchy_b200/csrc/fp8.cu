@@ -640,14 +640,12 @@ extern "C" int32_t scr_fp8_act_size(int32_t M, int32_t K, size_t* bytes) {
     return SCR_OK;
 }
 
-extern "C" int32_t scr_fp8_quant_per_token(scr_ctx* ctx, const uint16_t* x, int32_t M, int32_t K, void* act, void* stream) {
-    SCR_REQUIRE_CTX(ctx);
+// `tiled`: rows of `M_pad` tokens a k-tile in the swizzled image, else row after row.
+static int32_t fp8_quant_launch(scr_ctx* ctx, const uint16_t* x, int32_t M, int32_t K, int tiled, int M_pad, void* act, void* stream) {
     if (!x || !act) return scr_fail(ctx, SCR_E_ARG, "null pointer");
     if (M <= 0 || K <= 0) return scr_fail(ctx, SCR_E_SHAPE, "M=%d K=%d must be positive", M, K);
     if (K % 8 != 0) return scr_fail(ctx, SCR_E_SHAPE, "K=%d must be a multiple of 8", K);
     if (!scr_aligned16(x) || !scr_aligned16(act)) return scr_fail(ctx, SCR_E_ALIGN, "x/act must be 16-byte aligned");
-    const int tiled = fp8_act_tiled(M) ? 1 : 0;
-    const int M_pad = scr_ceil_div(M, FP8_TILE) * FP8_TILE;
     const int u = scr_ceil_div(scr_ceil_div(K, FP8_TILE) * (FP8_TILE / 16), QUANT_THREADS);
     auto kernel = u <= 1 ? fp8_quant_per_token_kernel<1> : u <= 2 ? fp8_quant_per_token_kernel<2> : u <= 3 ? fp8_quant_per_token_kernel<3>
                 : u <= 5 ? fp8_quant_per_token_kernel<5> : fp8_quant_per_token_kernel<0>;
@@ -663,6 +661,11 @@ extern "C" int32_t scr_fp8_quant_per_token(scr_ctx* ctx, const uint16_t* x, int3
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, x, (int)M, (int)K, tiled, M_pad, (uint8_t*)act);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "fp8_quant_per_token: %s", cudaGetErrorString(e));
     return scr_check_launch(ctx, "fp8_quant_per_token");
+}
+
+extern "C" int32_t scr_fp8_quant_per_token(scr_ctx* ctx, const uint16_t* x, int32_t M, int32_t K, void* act, void* stream) {
+    SCR_REQUIRE_CTX(ctx);
+    return fp8_quant_launch(ctx, x, M, K, fp8_act_tiled(M) ? 1 : 0, scr_ceil_div(M, FP8_TILE) * FP8_TILE, act, stream);
 }
 
 extern "C" int32_t scr_rmsnorm_fp8_quant(scr_ctx* ctx, const uint16_t* x, const uint16_t* gain, float eps, int32_t M, int32_t K,
@@ -785,9 +788,29 @@ static int32_t fp8_gemv_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t
     return scr_check_launch(ctx, "fp8_gemv");
 }
 
+// Defined in fp8_skinny.cu
+int32_t fp8_skinny16_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint16_t* y, int M, int N, int K, const LinearEnds& ends, cudaStream_t stream);
+// Whether a dynamic linear of up to 16 tokens is quantised for, and goes to, the GEMM for few tokens, whose time does not grow with them.  (A pack that the
+// caller holds is the matvec's.)  us in streams of calls with the quantisation, matvec / GEMM:
+//   one launch that quantises by itself (M <= 4, 14 KB of codes): 2048 x 2048, 4 tokens 6.2 / 4.6;  3584 x 3584, 1 token 5.9 / 5.7, 4 10.2 / 5.8;
+//   18944 x 3584, 1 token 14.5 / 14.0, 4 19.0 / 14.3;  16384 x 1024, 4 tokens 8.2 / 6.5;  1 token of a long k, whose codes every CTA makes for itself:
+//   4096 x 14336 19.2 / 13.2;  8192 x 8192 17.3 / 14.6.  (Partial sums stay with the matvec, whose bits the
+//   matvec with the exchange in its end has.)
+//   quantised beforehand: 1024 x 16384, 8 tokens 7.3 / 8.7;  5120 x 5120, 8 tokens 8.1 / 8.0;  2048 x 16384, 1 token 10.5 / 10.4, 8 12.1 / 10.7;
+//   8192 x 8192, 1 token 17.3 / 14.6;  3584 x 18944, 1 token 22.0 / 15.3
+//   9 to 16 tokens, two tiles of the matvec: 1024 x 8192, 16 tokens 6.1 / 6.2;  3584 x 3584, 9 tokens 6.5 / 6.0;  8192 x 2048 8.4 / 6.8;
+//   18944 x 3584 22.2 / 14.7
+static bool fp8_few_tokens(int M, int N, int K, bool partial) {
+    const long long weights = (long long)N * K;
+    if (M > 16) return false;
+    if (fp8_gemv_fuses_quant(M, K)) return !partial && (M > 2 ? weights >= 4 << 20 : weights >= 48 << 20 && K >= 8192);
+    return weights >= (M > 8 ? 12 << 20 : 30 << 20);
+}
+
 size_t fp8_workspace_bytes(int M, int N, int K) {
     // the dynamic entry point keeps its activation pack in the workspace
     size_t b = (fp8_act_bytes(M, K) + 127) / 128 * 128;
+    if (fp8_few_tokens(M, N, K, false)) b = std::max(b, fp8_few_bytes(M, K));
     if (fp8_act_tiled(M)) b += fp8_gemm_tc_workspace(M, N, K);
     return (b + 127) / 128 * 128;
 }
@@ -839,12 +862,18 @@ static int32_t fp8_linear_dynamic(scr_ctx* ctx, const void* packed, const uint16
     if (M <= 0) return scr_fail(ctx, SCR_E_SHAPE, "M=%d must be positive", M);
     if (!scr_aligned16(packed) || !scr_aligned16(x)) return scr_fail(ctx, SCR_E_ALIGN, "packed/x must be 16-byte aligned");
     if (ends.bias && ends.out_f32) return scr_fail(ctx, SCR_E_ARG, "a bias is added after the partial sums have been reduced, not to a partial");
+    if (fp8_few_tokens(M, N, K, ends.out_f32 != 0) && workspace && scr_aligned16(workspace) && workspace_bytes >= fp8_few_bytes(M, K)) {
+        st = fp8_quant_launch(ctx, x, M, K, 1, FP8_FEW_ROWS, workspace, stream);
+        if (st) return st;
+        return fp8_skinny16_launch(ctx, (const uint8_t*)packed, (const uint8_t*)workspace, static_cast<uint16_t*>(y), M, N, K, ends, (cudaStream_t)stream);
+    }
     if (fp8_gemv_fuses_quant(M, K)) {
         // few tokens: the matvec quantises the activations itself, no pack and no second launch
         return fp8_gemv_launch<1>(ctx, (const uint8_t*)packed, nullptr, nullptr, static_cast<uint16_t*>(y), M, N, K, ends,
                                   (cudaStream_t)stream, x);
     }
-    const size_t need = fp8_workspace_bytes(M, N, K);
+    size_t need = (fp8_act_bytes(M, K) + 127) / 128 * 128;         // (the GEMM's part follows the pack)
+    if (fp8_act_tiled(M)) need = fp8_workspace_bytes(M, N, K);
     if (!workspace || workspace_bytes < need)
         return scr_fail(ctx, SCR_E_WORKSPACE, "workspace %zu bytes < required %zu", workspace_bytes, need);
     if (!scr_aligned16(workspace)) return scr_fail(ctx, SCR_E_ALIGN, "workspace must be 16-byte aligned");

@@ -35,7 +35,10 @@ static inline size_t fp8_weight_bytes(int N, int K) {
 
 bool fp8_gemm_tc_enabled();
 static inline bool fp8_act_tiled(int M) { return M > 16 && fp8_gemm_tc_enabled(); }
+// The tiled pack of up to 16 tokens for the GEMM for few tokens: k-tiles of 16 rows.
+#define FP8_FEW_ROWS 16
 static inline size_t fp8_act_scale_bytes(int M) { return ((size_t)M * 4 + 127) / 128 * 128; }
+static inline size_t fp8_few_bytes(int M, int K) { return fp8_act_scale_bytes(M) + (size_t)scr_ceil_div(K, FP8_TILE) * FP8_FEW_ROWS * FP8_TILE; }
 static inline size_t fp8_act_bytes(int M, int K) {
     if (fp8_act_tiled(M))
         return fp8_act_scale_bytes(M) + (size_t)scr_ceil_div(K, FP8_TILE) * scr_ceil_div(M, FP8_TILE) * FP8_TILE_BYTES;

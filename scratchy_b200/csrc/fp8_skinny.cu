@@ -1,4 +1,4 @@
-// fp8-dynamic-per-channel: GEMM for 17 to 256 tokens on tcgen05 tensor cores (kind::f8f6f4), weights as the rows of the MMA
+// fp8-dynamic-per-channel: GEMM for few tokens (up to 256; from how many on, fp8.cu) on tcgen05 tensor cores (kind::f8f6f4), weights as the rows of the MMA
 // (skinny.cuh).
 //
 //   y[m,n] = bf16( (sum_k x_q[m,k] * w_q[n,k]) * a_scale[m] * w_scale[n] (+ bias[n]) )
@@ -13,6 +13,7 @@
 //
 // What bounds it: the copies into shared memory, 16 KB of weights and 128 bytes per token and step.  250 tokens of 18944 -> 3584
 // (with the quantisation) 46.4 us on the 128-token tiles of fp8_gemm.cu and their finishing launch, 32.5 us here.
+// One token of 3584 -> 18944 14.0 us, of 18944 -> 3584 15.3 (22.0 in the matvec, which quantises in a launch of its own there).
 #include "fp8.cuh"
 #include "skinny.cuh"
 
@@ -23,13 +24,14 @@ constexpr uint32_t F8S_W_STAGE = FP8_TILE_BYTES;
 
 template <int TN>
 struct F8SCfg {
-    static constexpr int kSW = TN == 256 ? 4 : TN == 128 ? 6 : 5;                 // weight stages
+    static constexpr int kSW = TN == 256 ? 4 : TN == 128 || TN == 16 ? 6 : 5;                 // weight stages
     static constexpr int kSX = TN == 64 ? 3 : kSW;                                // activation stages
     static constexpr uint32_t kXStage = TN * 128u;
     static constexpr uint32_t kXOff = kSW * F8S_W_STAGE;
     static constexpr uint32_t kBarOff = kXOff + kSX * kXStage;
     static constexpr uint32_t kTotal = kBarOff + 256u + 1024u;
     static constexpr int kCtasPerSm = TN >= 128 ? 1 : 2;
+    static constexpr uint32_t kTmemCols = TN < 32 ? 32 : TN;
 };
 
 template <int TN>
@@ -66,7 +68,7 @@ fp8_skinny_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ w
         fence_mbar_init();
     }
     if (warp == 10) {
-        tmem_alloc(smem_u32((const void*)tmem_slot), TN);
+        tmem_alloc(smem_u32((const void*)tmem_slot), C::kTmemCols);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -145,7 +147,7 @@ fp8_skinny_kernel(const uint8_t* __restrict__ wpack, const float* __restrict__ w
     __syncthreads();
     if (warp == 10) {
         tc_fence_after();
-        tmem_dealloc(tmem, TN);
+        tmem_dealloc(tmem, C::kTmemCols);
     }
 }
 
@@ -156,14 +158,15 @@ SkinnyPlan f8s_plan(const scr_ctx* ctx, const Fp8Geom& g) {
 }
 
 template <int TN>
-int32_t f8s_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint16_t* y, int M, int N, int K, const LinearEnds& ends, cudaStream_t stream) {
+int32_t f8s_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, int rows, uint16_t* y, int M, int N, int K, const LinearEnds& ends,
+                   cudaStream_t stream) {
     using C = F8SCfg<TN>;
     static_assert(C::kBarOff >= skinny_sum_bytes(TN), "the sums fit the rings");
     const Fp8Geom g = fp8_geom(N, K);
     const SkinnyPlan p = f8s_plan<TN>(ctx, g);
     const float* w_scale = reinterpret_cast<const float*>(wpack + (size_t)g.NT * g.KT * FP8_TILE_BYTES);
     const cudaError_t e = skinny_launch(fp8_skinny_kernel<TN>, g.NT, p.split, F8S_THREADS, p.smem, stream, wpack, w_scale, act + fp8_act_scale_bytes(M),
-                                        reinterpret_cast<const float*>(act), y, M, N, g.KT, scr_ceil_div(M, FP8_TILE) * FP8_TILE, p.split, p.over_rings, ends.out_f32,
+                                        reinterpret_cast<const float*>(act), y, M, N, g.KT, rows, p.split, p.over_rings, ends.out_f32,
                                         ends.bias, ctx->dev_status);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "fp8_skinny: %s", cudaGetErrorString(e));
     return scr_check_launch(ctx, "fp8_skinny");
@@ -182,8 +185,15 @@ float fp8_skinny_us(const scr_ctx* ctx, int M, int N, int K) {
 
 int32_t fp8_skinny_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint16_t* y, int M, int N, int K, const LinearEnds& ends,
                           cudaStream_t stream) {
-    if (M <= 32) return f8s_launch<32>(ctx, wpack, act, y, M, N, K, ends, stream);
-    if (M <= 64) return f8s_launch<64>(ctx, wpack, act, y, M, N, K, ends, stream);
-    if (M <= 128) return f8s_launch<128>(ctx, wpack, act, y, M, N, K, ends, stream);
-    return f8s_launch<256>(ctx, wpack, act, y, M, N, K, ends, stream);
+    const int rows = scr_ceil_div(M, FP8_TILE) * FP8_TILE;
+    if (M <= 32) return f8s_launch<32>(ctx, wpack, act, rows, y, M, N, K, ends, stream);
+    if (M <= 64) return f8s_launch<64>(ctx, wpack, act, rows, y, M, N, K, ends, stream);
+    if (M <= 128) return f8s_launch<128>(ctx, wpack, act, rows, y, M, N, K, ends, stream);
+    return f8s_launch<256>(ctx, wpack, act, rows, y, M, N, K, ends, stream);
+}
+
+// Up to 16 tokens, whose pack (`rows` = FP8_FEW_ROWS of a k-tile) only `scr_linear_fp8_dynamic` makes, for itself.
+int32_t fp8_skinny16_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint16_t* y, int M, int N, int K, const LinearEnds& ends,
+                            cudaStream_t stream) {
+    return f8s_launch<16>(ctx, wpack, act, FP8_FEW_ROWS, y, M, N, K, ends, stream);
 }

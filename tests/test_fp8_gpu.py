@@ -221,6 +221,30 @@ def test_matvec_quantises_by_itself_with_the_same_bits(N, K, M):
     assert rel_l2(bits_of(fused).reshape(M, N), want) <= REL_L2_TOL
 
 
+@pytest.mark.parametrize("N,K,M", [(2056, 2048, 3), (1224, 3432, 4), (8200, 3840, 1), (2048, 15368, 5), (8192, 3848, 8), (4104, 3080, 9), (12296, 1032, 16)])
+def test_few_tokens_that_the_call_quantises_for_the_gemm(N, K, M):
+    """Dynamic linears of up to 16 tokens whose matrix is large enough for the GEMM for few tokens, in a workspace of the size that the query
+    names, at both kinds of row ends; without the workspace for it the matvec runs.  Against the oracle, bias and partial sums as well."""
+    import torch
+    from scratchy_b200 import Fp8Linear
+    seed = synth.seed_for("few16", N, K, M)
+    wq, ws = oracle.fp8_quantize_weight_per_channel(synth.fp8_weights_f32(N, K, seed))
+    layer, x = make_layer(wq, ws), synth.activations_bf16(M, K, seed + 1)
+    xd = bf16_dev(x).reshape(M, K)
+    want = oracle.fp8_dynamic_linear(x, wq, ws, M, N, K)
+    work = torch.full((layer.workspace_bytes(M),), 0x7F, dtype=torch.uint8, device="cuda")         # NaN codes in the rows past the last token
+    y = layer.forward(xd, workspace=work)
+    part = layer.forward_partial(xd)
+    bias = bf16_dev(synth.activations_bf16(1, N, seed + 2)).reshape(N)
+    layer.linear_bias = bias
+    yb = layer.forward(xd, workspace=work)
+    torch.cuda.synchronize()
+    assert rel_l2(bits_of(y).reshape(M, N), want) <= REL_L2_TOL
+    assert rel_l2(bits_of(part.bfloat16()).reshape(M, N), want) <= REL_L2_TOL
+    f = lambda t: t.float()
+    assert float((f(yb) - (part + f(bias))).norm() / (part + f(bias)).norm()) < 4e-3                  # one bf16 rounding
+
+
 @pytest.mark.parametrize("M,K", [(1, 3584), (16, 8192), (40, 3584), (300, 256), (3, 72)])
 def test_rmsnorm_fused_with_the_quantisation(M, K):
     """The W8A8 activation producer straight from the residual stream (norm-side quantisation,
