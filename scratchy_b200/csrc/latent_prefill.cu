@@ -73,7 +73,8 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     auto s_full = [&](int t, int j) { return bars + 8u * (13 + 2 * t + (j & 1)); };
     auto p_full = [&](int t, int j) { return bars + 8u * (17 + 2 * t + (j & 1)); };
     auto pv_done = [&](int t) { return bars + 8u * (21 + t); };
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L.bars + 8 * 23);
+    auto o_full = [&](int t) { return bars + 8u * (23 + t); };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L.bars + 8 * 25);
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int head = blockIdx.x, q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * 256;      // the longest tiles first
     int n[2];                                                                          // key tiles of the two query tiles
@@ -90,6 +91,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
         for (int t = 0; t < 2; ++t) {
             for (int j = 0; j < 2; ++j) { mbar_init(s_full(t, j), 1); mbar_init(p_full(t, j), 4); }
             mbar_init(pv_done(t), 1);
+            mbar_init(o_full(t), 1);
         }
         fence_mbar_init();
     }
@@ -165,7 +167,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
                     for (int k4 = 0; k4 < 4; ++k4) umma_f16_ta_warp(o_col(t), col + 8u * k4, vd + (uint64_t)(2 * k4), o_desc, (j > 1) || k4 > 0);
 #pragma unroll
                     for (int k4 = 0; k4 < 4; ++k4) umma_f16_ta_warp(o_col(t), col + 32u + 8u * k4, vd + (uint64_t)(2 * k4), o_desc, 1);
-                    umma_commit_warp(pv_done(t));
+                    umma_commit_warp(j == n[t] ? o_full(t) : pv_done(t));
                 }
                 umma_commit_warp(v_empty(vs));
                 if (++vs == L.v_stages) { vs = 0; vp ^= 1u; }
@@ -239,7 +241,9 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
             if (lane == 0) mbar_arrive(p_full(t, j));
         }
         if (n[t] > 0) {
-            mbar_wait(pv_done(t), (uint32_t)(n[t] - 1) & 1u, a.status, TC_ERR_ACC_FULL);
+            // (a barrier of its own: the last S says that P V of two tiles before it is complete, not that of one, whose phase the parity of the
+            // last one would also be met by)
+            mbar_wait(o_full(t), 0, a.status, TC_ERR_ACC_FULL);
             tc_fence_after();
             const float inv = 1.0f / l;
             for (int c0 = 0; c0 < L.vp; c0 += 32) {

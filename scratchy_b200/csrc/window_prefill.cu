@@ -72,7 +72,8 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     auto s_full = [&](int t, int i) { return bars + 8u * (1 + 2 * WF_MAX_STAGES + 2 * t + (i & 1)); };        // i: the tile's i-th S
     auto p_full = [&](int t, int i) { return bars + 8u * (5 + 2 * WF_MAX_STAGES + 2 * t + (i & 1)); };
     auto pv_done = [&](int t) { return bars + 8u * (9 + 2 * WF_MAX_STAGES + t); };
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L.bars + 8 * (11 + 2 * WF_MAX_STAGES));
+    auto o_full = [&]() { return bars + 8u * (11 + 2 * WF_MAX_STAGES); };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L.bars + 8 * (12 + 2 * WF_MAX_STAGES));
     // (the broadcast lets the compiler see that a warp takes one way through the roles, and keep descriptors in uniform registers)
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int head = blockIdx.x, q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * 256, b = blockIdx.z;      // the longest first
@@ -102,6 +103,7 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
             for (int i = 0; i < 2; ++i) { mbar_init(s_full(t, i), 1); mbar_init(p_full(t, i), 8); }
             mbar_init(pv_done(t), 1);
         }
+        mbar_init(o_full(), 1);
         fence_mbar_init();
     }
     if (warp == 1) {
@@ -207,6 +209,7 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
             prev = ks;
             if (++ks == L.stages) { ks = 0; kp ^= 1u; }
         }
+        umma_commit_warp(o_full());
     } else {
         const int t = warp >= 10, half = ((warp - 2) >> 2) & 1, q = warp & 3;        // half: keys 0..31 or 32..63 of a tile
         const uint32_t lanes = (uint32_t)(q * 32) << 16;
@@ -314,7 +317,9 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
             mine[half * 128] = l;
             asm volatile("bar.sync %0, 256;" ::"r"(1 + t) : "memory");
             l += mine[(half ^ 1) * 128];
-            mbar_wait(pv_done(t), (uint32_t)(seen - 1) & 1u, a.status, TC_ERR_ACC_FULL);
+            // (a barrier of its own: the last S says that P V of two tiles before it is complete, not that of one, whose phase the parity of the
+            // last one would also be met by)
+            mbar_wait(o_full(), 0, a.status, TC_ERR_ACC_FULL);
             tc_fence_after();
             const float f = row < count ? sigmoid_f32(a.gate[(first + row) * a.ld_gate + head]) * s.out_scale / l : 0.0f;
             for (int c0 = half * 32; c0 < L.vp; c0 += 64) {

@@ -317,6 +317,31 @@ def test_expanded_prompt_attention(dim, rot_dim, vdim, heads, kv_rank, pos0, row
     assert np.abs(host(out) - want).max() < 0.03 * np.abs(want).max()
 
 
+@pytest.mark.parametrize("rows", [4096, 4000])
+def test_long_prompt_attention_repeats_itself(rows):
+    """The sums that a tile's end reads contain its last two key tiles however the other query tile of the CTA is delayed: the same
+    bits on every call."""
+    torch = torch_()
+    L, c = lib()
+    heads, dim, rot, vdim = 24, 128, 64, 128
+    m = su.attention_spec(heads=heads, dim=dim, rot_dim=rot, vdim=vdim, kv_rank=512)["mixer"]
+    lt = Latents(m, [0], [8], "bfloat16", seed=rows)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(rows)
+    new = lambda *s: torch.randn(s, device="cuda", generator=g).bfloat16()
+    q, k, r, vt, gate = new(rows, heads, dim + rot), new(rows, heads, dim), new(rows, rot), new(heads * vdim, rows), new(rows, heads * vdim)
+    outs = [torch.full((rows, heads * vdim), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(8)]
+    for out in outs:
+        c.check(L.scr_latent_prefill(c.handle, ctypes.byref(lt.shape), ptr(q), ptr(k), ptr(r), ptr(vt), rows, ptr(gate), heads * vdim, rows, 0, ptr(out),
+                                     heads * vdim, stream()))
+    healthy()
+    assert all(torch.equal(out.view(torch.int16), outs[0].view(torch.int16)) for out in outs)
+    scores = torch.einsum("hd,thd->ht", q[-1, :, :dim].double(), k.double()) + q[-1, :, dim:].double() @ r.double().T
+    p = torch.softmax(scores * m["scale"], dim=1)
+    want = torch.einsum("ht,hvt->hv", p, vt.view(heads, vdim, rows).double()).reshape(-1) * torch.sigmoid(gate[-1].double())
+    assert float((outs[0][-1].double() - want).norm() / want.norm()) < TOL["bfloat16"]
+
+
 def test_scores_that_climb_along_the_sequence_rescale_the_sums():
     """Keys ordered so that the running maximum grows at every tile by more than the kernels let it grow unscaled."""
     torch = torch_()
