@@ -4,12 +4,12 @@
 // A unit is 128 rows of W by one CTA's share of the 64-wide k slices; 352 threads:
 //   warps 0-7    drain the accumulator and store
 //   warp 8       producer of the weights (one tiled TMA load of 128 rows x 64 k per slice, 128-byte swizzle), load-time
-//                constants: it starts before the preceding kernel of the stream has finished
+//                constants: it starts before the preceding kernel of the stream has finished, and ahead of this kernel's own setting up
 //   warp 9       producer of x (one tiled TMA load per slice, zeros outside)
 //   warp 10      owns TMEM; one elected lane issues 4 tcgen05.mma (128 x rows of x x 16) per slice
 //
 // What bounds it: the weights from HBM; for the small linears the start and end of a launch.  10240 x 3072 (63 MB) at 32 rows
-// 14.9 us (4.2 TB/s), 3072 x 8192 13.3 us, 128256 x 3072 at 8 rows 120 us (6.5 TB/s), in streams of calls.  Against the 128-row tile of dense_gemm.cu and its finishing launch: a decode step of the 3B Vumipel at 32 sequences
+// 14.9 us (4.2 TB/s), 3072 x 8192 11.9 us (13.3 with two CTAs to an SM and cluster barriers, 12.3 with the first weights after the setting up), 128256 x 3072 at 8 rows 120 us (6.5 TB/s), in streams of calls.  Against the 128-row tile of dense_gemm.cu and its finishing launch: a decode step of the 3B Vumipel at 32 sequences
 // 4.22 -> 3.59 ms, with that issue 3.31 -> 3.09 ms.
 #include "seq_common.cuh"
 #include "skinny.cuh"
@@ -56,14 +56,31 @@ dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_cons
     skinny_range(KT, rank, split, k_lo, k_hi);
     const int steps = k_hi - k_lo;
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < C::kSW; ++s) { mbar_init(wfull(s), 1); mbar_init(wempty(s), 1); }
-        for (int s = 0; s < C::kSX; ++s) { mbar_init(xfull(s), 1); mbar_init(xempty(s), 1); }
-        mbar_init(accf, 1);
-        skinny_expect(rbar, M, split, rank, over_rings);
-        fence_mbar_init();
-    }
-    if (warp == 10) {
+    // The first weights are on their way before anything else is set up (unless another kernel writes them): their copy needs only its own
+    // barriers.
+    auto load = [&](int i) {
+        const int s = i % C::kSW;
+        mbar_arrive_expect_tx(wfull(s), DS_W_STAGE);
+        tma_load_3d(smem_base + s * DS_W_STAGE, &w_map, (k_lo + i) * 64, n0, g, wfull(s));
+    };
+    const int early = w_fresh ? 0 : min(steps, 2);
+    if (warp == 8) {
+        if (lane == 0) {
+            for (int s = 0; s < C::kSW; ++s) { mbar_init(wfull(s), 1); mbar_init(wempty(s), 1); }
+            fence_mbar_init();
+            for (int i = 0; i < early; ++i) load(i);
+        }
+        __syncwarp();
+    } else if (warp == 9) {
+        if (lane == 0) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&x_map) : "memory");
+            for (int s = 0; s < C::kSX; ++s) { mbar_init(xfull(s), 1); mbar_init(xempty(s), 1); }
+            mbar_init(accf, 1);
+            skinny_expect(rbar, M, split, rank, over_rings);
+            fence_mbar_init();
+        }
+        __syncwarp();
+    } else if (warp == 10) {
         tmem_alloc(smem_u32((const void*)tmem_slot), C::kTmemCols);
         tmem_relinquish();
     }
@@ -79,12 +96,10 @@ dense_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_cons
     if (warp == 8) {
         if (lane == 0) {
             if (w_fresh) pdl_wait();
-            for (int i = 0; i < steps; ++i) {
-                const int s = i % C::kSW;
+            for (int i = early; i < steps; ++i) {
                 if (i == C::kSW) pdl_wait();
-                mbar_wait(wempty(s), ((uint32_t)(i / C::kSW) & 1u) ^ 1u, status, TC_ERR_EMPTY_WAIT);
-                mbar_arrive_expect_tx(wfull(s), DS_W_STAGE);
-                tma_load_3d(smem_base + s * DS_W_STAGE, &w_map, (k_lo + i) * 64, n0, g, wfull(s));
+                mbar_wait(wempty(i % C::kSW), ((uint32_t)(i / C::kSW) & 1u) ^ 1u, status, TC_ERR_EMPTY_WAIT);
+                load(i);
             }
         }
     } else if (warp == 9) {
