@@ -3,7 +3,7 @@
 //   y[m,n] = bf16( sum_k x[m,k] * w[n,k] (+ bias[n]) ),  w = the bit-exact bf16 dequantisation of the codes
 //
 // Persistent, warp-specialised CTA (736 threads), one per SM.  A tile is 128 channels (the rows of the MMA) by `width` tokens (its
-// columns, 128 to 192):
+// columns, 96 to 192):
 //   warps 0-15   dequantise: four groups of four warps take the halves (64 k) of alternate 128-k chunks; a thread expands 64 codes of
 //                one channel and writes them to TMEM with tcgen05.st, where the MMA reads its A operand: no swizzled shared-memory
 //                image and no proxy fence, and the shared memory holds activations in flight instead
@@ -31,7 +31,7 @@
 
 bool affine_b4_gemm_tc_enabled() { return true; }
 // Defined in affine_b4_gemm_pair.cu
-bool affine_b4_gemm_pair_applies(int M, int N, int K, int sms, float one_cta_us);
+bool affine_b4_gemm_pair_applies(int M, int N, int K, int sms);
 int32_t affine_b4_gemm_pair_launch(scr_ctx* ctx, const CUtensorMap& x_map, const uint8_t* packed, uint16_t* y, int M, int N, int K,
                                    int gs, int out_f32, const uint16_t* bias, cudaStream_t stream, bool* launched);
 // Defined in affine_b4_skinny.cu
@@ -315,9 +315,10 @@ affine_b4_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid
 }
 
 // ---- host --------------------------------------------------------------------------------
-// The tokens of a tile and how the tiles are cut into work units (tc_plan_units).  A 128-k chunk takes about 0.655 us whatever the
-// width (3072 -> 3072 in one round 18.4 us at 144 to 192 tokens a tile, in two 32.5 at 128 and 33.7 at 192), and a tile's drain at
-// the end 6.5 ns a token; the width whose rounds fill the GPU best wins.
+// The tokens of a tile and how the tiles are cut into work units (tc_plan_units).  A 128-k chunk takes about 0.26 us and 1.23 ns a token (148
+// tiles of 24 chunks a round: further rounds 9.0 us at 112 tokens, 10.0 at 128, 10.6 at 144, 10.9 at 160, 11.3 at 176, 11.9 at 192), and a tile's drain at
+// the end 6.5 ns a token; the width whose rounds fill the GPU best wins.  512 tokens of 3072 -> 8192 26.6 us at 192, 23.1 at 128; 777 of 8192 -> 3072
+// 35.4 and at 144 30.1; 200 of 3072 -> 3072 13.0 and at 112 11.1.  A cut costs about 5 us in all.
 struct AffineGemmPlan {
     int width, mt, tiles, full, ks_tail;
     float us;                                            // estimate
@@ -336,13 +337,13 @@ static AffineGemmPlan affine_gemm_plan(int M, int N, int K, int sms) {
         best.ks_tail = 1;
         return best;
     }
-    for (int width = A4G_WIDTH; width >= 128; width -= 16) {
+    for (int width = A4G_WIDTH; width >= 96; width -= 16) {
         AffineGemmPlan p;
         p.width = width;
         p.mt = scr_ceil_div(M, width);
         p.tiles = p.mt * (g.RB * 16 / A4G_BN);
-        const float us = 0.655f;
-        p.us = tc_plan_units(p.tiles, g.KC, sms, us, &p.full, &p.ks_tail) * g.KC * us + 0.0065f * width;
+        const float us = 0.26f + 0.00123f * width;
+        p.us = tc_plan_units(p.tiles, g.KC, sms, us, &p.full, &p.ks_tail, 1.6f, 3.4f) * g.KC * us + 0.0065f * width;
         if (p.us < least * 0.99f) {
             least = p.us;
             best = p;
@@ -392,7 +393,7 @@ int32_t affine_b4_gemm_tc_launch(scr_ctx* ctx, const uint8_t* packed, const uint
     if (!enc) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled entry point not available");
     CUtensorMap map;
     const AffineGemmPlan plan = affine_gemm_plan(M, N, K, ctx->sm_count);
-    if (affine_b4_gemm_pair_applies(M, N, K, ctx->sm_count, plan.us)) {
+    if (affine_b4_gemm_pair_applies(M, N, K, ctx->sm_count)) {
         bool launched = false;
         if (!affine_gemm_x_map(&map, enc, x, M, K, 128)) return scr_fail(ctx, SCR_E_CUDA, "cuTensorMapEncodeTiled failed");
         const int32_t st = affine_b4_gemm_pair_launch(ctx, map, packed, y, M, N, K, gs, out_f32, bias, stream, &launched);

@@ -10,7 +10,7 @@
 // channels; one `tcgen05.mma.cta_group::2` of shape 256 x 256 x 16, issued by the pair's leader CTA, reads the token rows
 // and the channel rows from both SMs' shared memory and leaves each CTA's 128 accumulator rows in that CTA's own TMEM.
 // Same MACs and the same dequantise work per SM and chunk, 44 % less L2 traffic, and room for three stages of each ring.
-// Measured: the same bits as the one-CTA kernel, at its speed or below but for one range of sizes (`affine_b4_gemm_pair_applies`).
+// Measured: the same bits as the one-CTA kernel, below its speed: opt-in (`affine_b4_gemm_pair_applies`).
 //
 // Per CTA (704 threads), both CTAs of a pair run the same code:
 //   warp 0       producer: per chunk 2 tiled TMA loads of this CTA's activations (`.cta_group::2`, completing on the
@@ -354,24 +354,19 @@ affine_b4_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __gr
 }  // namespace
 
 
-// Whether the pair kernel takes this GEMM, whose one-CTA plan is estimated at `one_cta_us`: whole 256-channel pair tiles, where they come out
-// a good part shorter.  A round of 256 x 256 tiles takes 0.92 us per 128-k chunk and 5.5 us at least, the launch 7 us around them
-// (measured).  In practice that is a second token tile that the one-CTA kernel would start a round for: 193 to 256 tokens of 3072 ->
-// 16384 30.5 us against 32.8; elsewhere it is level (2048 tokens of 3072 -> 16384 168 against 169) or behind (of 3072 -> 8192 95 against 84).
-// `SCR_AFFINE_GEMM_PAIR` in the environment (read once): 0 switches the pair kernel off, 1 gives it every GEMM of at least one full round
-// of pairs whose rounds are at least 85 % full.
-bool affine_b4_gemm_pair_applies(int M, int N, int K, int sms, float one_cta_us) {
-    static const int asked = [] {
+// Whether the pair kernel takes this GEMM: only where `SCR_AFFINE_GEMM_PAIR=1` in the environment (read once) asks for it, and then every GEMM of at
+// least one full round of 256 x 256 pair tiles whose rounds are at least 85 % full.  A round of pairs takes 0.92 us per 128-k chunk, the same tokens and
+// channels in the one-CTA kernel 0.83 (affine_b4_gemm.cu), and the launch 7 us around them: 256 tokens of 3072 -> 16384 30.5 and 23.3 us.
+bool affine_b4_gemm_pair_applies(int M, int N, int K, int sms) {
+    static const bool asked = [] {
         const char* e = std::getenv("SCR_AFFINE_GEMM_PAIR");
-        return e && (e[0] == '0' || e[0] == '1') ? e[0] - '0' : -1;
+        return e && e[0] == '1';
     }();
     const AffineGeom g = affine_geom(N, K, 64);
     const int pairs = sms / 2, tiles = scr_ceil_div(M, 256) * (g.RB / 16);
-    if (asked == 0 || (g.RB % 16) != 0 || g.KC < 1 || M <= 128 || pairs < 1) return false;
+    if (!asked || (g.RB % 16) != 0 || g.KC < 1 || M <= 128 || pairs < 1) return false;
     const int rounds = (tiles + pairs - 1) / pairs;
-    if (asked == 1) return tiles >= pairs && (float)tiles >= 0.85f * (float)(rounds * pairs);
-    const float chunk = 0.92f * (float)g.KC;
-    return 7.0f + (float)rounds * (chunk > 5.5f ? chunk : 5.5f) < 0.92f * one_cta_us;
+    return tiles >= pairs && (float)tiles >= 0.85f * (float)(rounds * pairs);
 }
 
 int32_t affine_b4_gemm_pair_launch(scr_ctx* ctx, const CUtensorMap& x_map, const uint8_t* packed, uint16_t* y, int M, int N, int K,

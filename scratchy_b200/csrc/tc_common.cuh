@@ -186,15 +186,15 @@ __host__ __device__ __forceinline__ uint32_t umma_idesc(uint32_t a_fmt, uint32_t
 // Work units of a persistent GEMM with `tiles` output tiles of `k_steps` k-steps on `sms` SMs.  Candidates: whole
 // tiles only; every tile split ks ways along k; or whole tiles round by round with only the last, partial round
 // split (units [0, full) are whole tiles, the other tiles - full are split ks_tail ways).  The estimate is in
-// tile-times.  A split unit costs 1/ks of a tile plus a fixed ~3 us (its own accumulator drain and f32 slab
-// write), and split work needs the finishing kernel (~4 us); `us_per_kstep` (how long one k-step of one tile
+// tile-times.  A split unit costs 1/ks of a tile plus a fixed `unit_us` (its own accumulator drain and f32 slab
+// write), and split work needs the finishing kernel (`finish_us`); `us_per_kstep` (how long one k-step of one tile
 // takes, measured per kernel) turns those into tile-times.  Returns the estimate.
-static inline float tc_plan_units(int tiles, int k_steps, int sms, float us_per_kstep, int* full, int* ks_tail) {
+static inline float tc_plan_units(int tiles, int k_steps, int sms, float us_per_kstep, int* full, int* ks_tail, float unit_us = 3.0f, float finish_us = 4.0f) {
     *full = tiles;
     *ks_tail = 1;
     const int max_ks = k_steps / 4 < 8 ? k_steps / 4 : 8;
     const float tile_us = k_steps * us_per_kstep;
-    const float unit_ovh = 3.0f / tile_us, finish = 4.0f / tile_us;
+    const float unit_ovh = unit_us / tile_us, finish = finish_us / tile_us;
     float best = (float)((tiles + sms - 1) / sms);
     for (int ks = 2; ks <= max_ks; ++ks) {
         const float all = (float)((tiles * ks + sms - 1) / sms) * (1.0f / ks + unit_ovh) + finish;
