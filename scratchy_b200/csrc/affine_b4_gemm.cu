@@ -18,7 +18,7 @@
 //
 // What bounds it: the MMAs, 64 cycles for 128 columns and 96 for 192 (alone in a loop, A in TMEM: the tensor core's full rate), 768 a chunk
 // at 192, and for large calls the clock that the power limit leaves: 2048 tokens of 3072 -> 8192 73.7 us (1.40 PFLOP/s, what cuBLAS
-// sustains) in a stream of calls, 72.4 with the election inside.  It was 83.7 us, 1250 cycles a chunk whatever the width, while one lane issued eight bulk copies a chunk
+// sustains) in a stream of calls, 72.4 with the election inside (70.2 with the plan below).  It was 83.7 us, 1250 cycles a chunk whatever the width, while one lane issued eight bulk copies a chunk
 // and the dequantised weights were handed over in stages of a whole chunk.  Wide tiles pay, since a chunk is expanded once for all of a
 // tile's tokens.
 #include <cuda.h>

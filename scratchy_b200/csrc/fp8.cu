@@ -793,7 +793,7 @@ int32_t fp8_skinny16_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* a
 // Whether a dynamic linear of up to 16 tokens is quantised for, and goes to, the GEMM for few tokens, whose time does not grow with them.  (A pack that the
 // caller holds is the matvec's.)  us in streams of calls with the quantisation, matvec / GEMM:
 //   one launch that quantises by itself (M <= 4, 14 KB of codes): 2048 x 2048, 4 tokens 6.2 / 4.6;  3584 x 3584, 1 token 5.9 / 5.7, 4 10.2 / 5.8;
-//   18944 x 3584, 1 token 14.5 / 14.0, 4 19.0 / 14.3;  16384 x 1024, 4 tokens 8.2 / 6.5;  1 token of a long k, whose codes every CTA makes for itself:
+//   18944 x 3584, 1 token 14.5 / 14.0 (called one by one 14.5 / 15.1), 4 19.0 / 14.3;  16384 x 1024, 4 tokens 8.2 / 6.5;  1 token of a long k, whose codes every CTA makes for itself:
 //   4096 x 14336 19.2 / 13.2;  8192 x 8192 17.3 / 14.6.  (Partial sums stay with the matvec, whose bits the
 //   matvec with the exchange in its end has.)
 //   quantised beforehand: 1024 x 16384, 8 tokens 7.3 / 8.7;  5120 x 5120, 8 tokens 8.1 / 8.0;  2048 x 16384, 1 token 10.5 / 10.4, 8 12.1 / 10.7;

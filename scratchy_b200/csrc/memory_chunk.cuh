@@ -19,8 +19,8 @@
 // nothing), a second one lets every group put together the state it starts from (S' = e^(F+m-m') S + e^(M-m') U over the
 // groups before it) and compute its outputs; its last group leaves the sequence's state.
 //
-// What bounds it: mma.sync, about 14 cycles for a 16x8x16 product and SM quarter: 10,000 of the 15,500 cycles that a chunk of 128 columns takes, and the
-// latencies around it.  So the slices are as wide as an SM's shared memory takes (128 columns at up to 128 dimensions): the products of queries and keys
+// What bounds it: the products with the ldmatrix loads that feed them, about 14 cycles for a 16x8x16 product and SM quarter in these loops (mma.sync alone
+// sustains 8.6): 10,000 of the 15,500 cycles that a chunk of 128 columns takes, and the latencies around them.  So the slices are as wide as an SM's shared memory takes (128 columns at up to 128 dimensions): the products of queries and keys
 // are computed once for a slice.  8192 tokens, 12 heads of 128 x 256: 468 us in slices of 128, 541 in slices of 64; 2000 tokens with a constant decay 130
 // and 139 us.  Loading by warps of their own instead of the computing ones was slower (524 us).
 #pragma once
