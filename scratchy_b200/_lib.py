@@ -118,6 +118,7 @@ MODELS_SIGNATURES = {
     "scr_window_attention": (_i32, [_vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _vp]),
     "scr_lightning_workspace": (_i32, [_i32, _vp, _vp, _psz]),
     "scr_lightning_run": (_i32, [_vp, _i32, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _sz, _vp]),
+    "scr_lightning_beside": (_i32, [_vp, _i32, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _sz, _vp]),
     "scr_lightning_finish": (_i32, [_vp, _i32, _vp, _vp, _vp, _vp, _i64, _i32, _vp, _i64, _vp]),
 }
 

@@ -413,8 +413,8 @@ __global__ void __launch_bounds__(WA_WARPS * 32) window_attention_plain_kernel(s
     float* qs = wa_smem;                                     // [dim]
     float* part = qs + s.dim;                                // [WA_WARPS][dim]
     float* ml = part + WA_WARPS * s.dim;                     // [WA_WARPS][2]
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();                                           // (after the wait: scr_lightning_beside)
     const int r = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = h / (s.heads / s.kv_heads);
     const int pos = st.tok_pos[r], seg = st.tok_seg[r];
     const T* qp = q + ((size_t)r * s.heads + h) * s.dim;

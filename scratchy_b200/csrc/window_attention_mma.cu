@@ -60,7 +60,6 @@ __global__ void __launch_bounds__(WM_THREADS) window_attention_mma_kernel(const 
     uint8_t* gen = wm_smem + (base - smem_u32(wm_smem));
     const scr_window_shape& s = a.s;
     const int dim = s.dim, G = s.kv_heads, group = s.heads / G;
-    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, t4 = lane & 3, lm = lane >> 3, lr = lane & 7;
     const int split = blockIdx.x % a.splits, g = blockIdx.x / a.splits % G, tile = blockIdx.x / a.splits / G, b = blockIdx.y;
     const int first = a.st.segs[b * 4], count = a.st.segs[b * 4 + 1], pos0 = a.st.segs[b * 4 + 2];
@@ -101,6 +100,7 @@ __global__ void __launch_bounds__(WM_THREADS) window_attention_mma_kernel(const 
         fence_mbar_init();
     }
     pdl_wait();
+    pdl_trigger();                                           // after the wait: a memory beside this attention runs from here on (scr_lightning_beside)
     if (lane == 0) {
 #pragma unroll
         for (int n = 0; n < STAGES; ++n) load(n, look_up(n));

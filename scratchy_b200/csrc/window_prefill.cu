@@ -80,8 +80,8 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     const int first = a.st.segs[b * 4], count = a.st.segs[b * 4 + 1], pos0 = a.st.segs[b * 4 + 2];
 
     if (q0 >= count || first < 0 || first + count > a.st.rows) {
-        pdl_trigger();
         pdl_wait();
+        pdl_trigger();
         return;
     }
     // the CTA's key tiles, and of those each query tile's: its kept ones and those from its own first one to its last
@@ -121,10 +121,12 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    pdl_trigger();                                           // not before this CTA has its TMEM: the next kernel's CTAs could take it first
     auto s_col = [&](int t, int i) { return tmem + 256u * t + 64u * (i & 1); };        // S, then P: 32 columns of heads, 32 of remainders
     auto o_col = [&](int t) { return tmem + 256u * t + 128u; };
     pdl_wait();
+    // Not before this CTA has its TMEM, which the next kernel's CTAs could take first, and after the wait: a memory beside this attention runs from here
+    // on (scr_lightning_beside).
+    pdl_trigger();
 
     if (warp == 0) {
         if (lane == 0) {

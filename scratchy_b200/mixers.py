@@ -326,7 +326,8 @@ class LightningAttention:
     def memory(self, cache_rows: int, slots: int, device) -> torch.Tensor:
         return torch.zeros((slots, self.heads, self.dim, self.vdim), dtype=torch.float32, device=device)
 
-    def run(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], memory: torch.Tensor, out: torch.Tensor) -> None:
+    def run(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], memory: torch.Tensor, out: torch.Tensor, beside: bool = False) -> None:
+        """`beside`: the call directly before is a window attention's, which the memory may run beside."""
         qkv, gate = bufs[f"{self.prefix}.qkv"], bufs[f"{self.prefix}.g"]
         lib, c = _lib.models_lib(), _lib.models_context(_dev_index(qkv.device))
         code, stream = dtype_code(self.dtype), _stream(qkv.device)
@@ -335,8 +336,9 @@ class LightningAttention:
         need = ctypes.c_size_t(0)
         c.check(lib.scr_lightning_workspace(code, ctypes.byref(shape), ctypes.byref(ctx.step), ctypes.byref(need)))
         ws = ctx.arena.get("li.workspace", (need.value,), torch.uint8) if need.value else None
-        c.check(lib.scr_lightning_run(c.handle, code, ctypes.byref(shape), ctypes.byref(ctx.step), _ptr(qkv), int(qkv.stride(0)), _ptr(self.powers), _ptr(memory),
-                                      _ptr(o), _ptr(ws), need, stream))
+        run = lib.scr_lightning_beside if beside else lib.scr_lightning_run
+        c.check(run(c.handle, code, ctypes.byref(shape), ctypes.byref(ctx.step), _ptr(qkv), int(qkv.stride(0)), _ptr(self.powers), _ptr(memory),
+                    _ptr(o), _ptr(ws), need, stream))
         c.check(lib.scr_lightning_finish(c.handle, code, ctypes.byref(shape), _ptr(o), _ptr(self.norm), _ptr(gate), int(gate.stride(0)), ctx.rows, _ptr(out),
                                          int(out.stride(0)), stream))
 
@@ -394,6 +396,9 @@ class SideBySide:
             lo, hi = self.columns[-1]
             bufs[f"{self.mlp.prefix}.act"] = rows[:, lo:hi]
         self.inp.run(a, h, bufs)
+        before = None
         for m, mem, (lo, hi) in zip(self.mixers, memory, self.columns):
-            m.run(ctx, bufs, mem, rows[:, lo:hi])
+            beside = {"beside": True} if isinstance(m, LightningAttention) and isinstance(before, WindowAttention) else {}
+            m.run(ctx, bufs, mem, rows[:, lo:hi], **beside)
+            before = m
         self.out.add_to(a, rows, residual, norm, h)

@@ -6,8 +6,8 @@ import numpy as np
 import pytest
 
 from tests import seq_util as su
-from tests.test_side_ops_gpu import per_head, plain_lightning, run_lightning
-from tests.test_sequence_ops_gpu import DTYPES, Latents, dev, draw_memory, healthy, head_rows, lib, plain_memory, ptr, run_memory, stream, torch_
+from tests.test_side_ops_gpu import Window, per_head, plain_lightning, run_lightning
+from tests.test_sequence_ops_gpu import DTYPES, Latents, arena, dev, draw, draw_memory, healthy, head_rows, lib, plain_memory, ptr, run_memory, stream, torch_
 
 pytestmark = pytest.mark.gpu
 
@@ -101,6 +101,51 @@ def test_decaying_memory(heads, dim, vdim, portions, dtype, captured):
     got = out.cpu().numpy()
     assert np.array_equal(got, want.astype(np.float32))
     assert per_head(got, plain_lightning(m, proj), heads) < (4e-6 if dtype == "float32" else 1e-4)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,dim,vdim", [(3, 48, 72), (8, 128, 128), (1, 300, 20)])
+@pytest.mark.parametrize("rows,attention", [(1, (4, 2, 64)), (3, (5, 1, 10)), (70, (2, 1, 128))])
+def test_decaying_memory_beside_an_attention(rows, attention, heads, dim, vdim, dtype, captured):
+    """The memory beside each kernel of the window attention, its input by the linear before that, in the buffer that the step before has read."""
+    from scratchy_b200 import _lib
+    from scratchy_b200.dense import DenseLinear, dtype_code
+    from scratchy_b200.mixers import decay_powers
+    torch = torch_()
+    L, c = lib()
+    steps, W, past = 8, heads * (2 * dim + vdim), 200
+    rng = np.random.default_rng(rows + dim)
+    w = Window(*attention, 90, 5, 40, [past + rows], dtype, seed=rows)
+    w.cache.copy_(dev(draw(rng, tuple(w.cache.shape), dtype), dtype))
+    w.key_scale.fill_(0.1)
+    st, sh, nq, bias = w.step([rows], [past], [1]), w.shape(), attention[0] * attention[2], w.padded_bias()
+    q, gate = dev(draw(rng, (rows, nq), dtype), dtype), dev(rng.standard_normal((rows, attention[0])))
+    x, a, lin = dev(draw(rng, (steps, rows, 64), dtype), dtype), arena(), DenseLinear(dev(draw(rng, (W, 64), dtype, 0.125), dtype))
+    shape, powers, code = _lib.LightningShape(heads, dim, vdim, 1e-5, 1.0), decay_powers(np.asarray(([0.999, 0.6, 0.97] * 3)[:heads], np.float64)).cuda(), dtype_code(q.dtype)
+    need = ctypes.c_size_t(0)
+    c.check(L.scr_lightning_workspace(code, ctypes.byref(shape), ctypes.byref(st), ctypes.byref(need)))
+    ws, results = torch.empty(max(16, need.value), dtype=torch.uint8, device="cuda"), []
+    for beside in (False, True):
+        nan = lambda *n, t=torch.float32: torch.full(n, float("nan"), dtype=t, device="cuda")
+        proj, state, out, y = nan(rows, W, t=q.dtype), torch.zeros((2, heads, dim, vdim), device="cuda"), nan(steps, rows, heads * vdim), nan(steps, rows, nq + 8, t=q.dtype)
+        memory = L.scr_lightning_beside if beside else L.scr_lightning_run
+
+        def step(t, memory=memory, proj=proj, state=state, out=out, y=y):
+            lin(a, x[t], proj)
+            c.check(L.scr_window_attention(c.handle, code, ctypes.byref(sh), ctypes.byref(st), ptr(q), ptr(w.cache), ptr(w.key_scale), ptr(bias), ptr(gate), attention[0],
+                                           ptr(y[t]), nq + 8, stream()))
+            c.check(memory(c.handle, code, ctypes.byref(shape), ctypes.byref(st), ptr(proj), W, ptr(powers), ptr(state), ptr(out[t]), ptr(ws), need, stream()))
+
+        if beside:
+            queued([lambda t=t: step(t) for t in range(steps)], captured)
+        else:
+            for t in range(steps):
+                step(t)
+                healthy()
+        results.append((out, state[1], y[:, :, :nq]))
+    for one, other in zip(*results):
+        assert torch.equal(one, other) and torch.isfinite(one).all()
 
 
 @pytest.mark.parametrize("captured", [False, True])
