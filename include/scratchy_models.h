@@ -216,13 +216,16 @@ typedef struct scr_lightning_shape {
 int32_t scr_lightning_workspace(int32_t dtype, const scr_lightning_shape* s, const scr_step* st, size_t* bytes);
 int32_t scr_lightning_run(scr_ctx* ctx, int32_t dtype, const scr_lightning_shape* s, const scr_step* st, const void* proj, int64_t ld,
                           const float* powers, float* state, float* out, void* workspace, size_t workspace_bytes, void* stream);
-/* The same directly after `scr_window_attention` on the stream, whose kernel has nothing that the memory needs (`proj` and `state` come from the calls
- * before it, `out` is not read by it): token by token the memory runs beside the attention, and what follows waits for both. */
+/* The same directly after `scr_window_prepare` or `scr_window_attention` on the stream, whose kernels have nothing that the memory needs (`proj` and
+ * `state` come from the calls before them, `out` is not read by them): token by token the memory runs beside them, and what follows waits for both. */
 int32_t scr_lightning_beside(scr_ctx* ctx, int32_t dtype, const scr_lightning_shape* s, const scr_step* st, const void* proj, int64_t ld,
                              const float* powers, float* state, float* out, void* workspace, size_t workspace_bytes, void* stream);
 /* y[t, :] (dtype, row stride ld_y) = out / rms(out over all heads) * norm * sigmoid(gate[t, :]) * out_scale */
 int32_t scr_lightning_finish(scr_ctx* ctx, int32_t dtype, const scr_lightning_shape* s, const float* out, const float* norm,
                              const void* gate, int64_t ld_gate, int32_t rows, void* y, int64_t ld_y, void* stream);
+/* The same directly after `scr_window_attention`, with `out` and `gate` from the calls before that: it runs beside the attention. */
+int32_t scr_lightning_finish_beside(scr_ctx* ctx, int32_t dtype, const scr_lightning_shape* s, const float* out, const float* norm,
+                                    const void* gate, int64_t ld_gate, int32_t rows, void* y, int64_t ld_y, void* stream);
 
 #ifdef __cplusplus
 }

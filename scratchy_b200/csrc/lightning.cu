@@ -17,14 +17,16 @@ namespace {
 // kernels and are read after it: one of those kernels may be the call that leaves this one its state.
 constexpr int LR_T = 256, LR_COLS = 32, LR_ROWS = LR_T / 8;
 
-// BESIDE: the kernel directly before (an attention over the same input) has nothing that this one needs and lets its dependents start only once the
-// kernels before it are complete, so this one runs beside it and waits for it at its end, where its own dependents count on both.  It reads past L1, which
-// no wait has cleared.  An attention over few sequences leaves most of HBM idle (0.37 of it at 8 sequences of 2048 tokens) and the memory is state in and out:
-// a step of 8 such sequences takes 2,193 µs instead of 2,288 (28 layers).
+// BESIDE: the kernel directly before (an attention's preparation, or the attention, over the same input) has nothing that this one needs and lets its
+// dependents start only once the kernels before it are complete, so this one runs beside it and waits for it at its end, where its own dependents count on
+// both.  It reads past L1, which no wait has cleared.  The preparation has one CTA per row; the attention then follows both, with the readout norm beside it.
+// Its dependents start at the end: an attention whose CTAs are placed while this kernel still fills the SMs is spread unevenly (24 sequences with heads of 64:
+// 1,416 µs a step against 1,319).  Steps at context 2048, 28 layers of the larger design: 8 sequences 2,229 µs one after the other, 2,217 beside the
+// attention, 2,139 beside the preparation; 32: 3,431, 3,297, 3,098; 16 layers of the smaller one: 8: 971, 957, 931; 32: 1,465, 1,464, 1,400.
 template <typename T, int RPT, bool BESIDE>
 __global__ void __launch_bounds__(LR_T) lightning_recur_kernel(MemoryArgs a) {
     __shared__ float4 part[2][LR_T / 32][8];
-    pdl_trigger();
+    if (!BESIDE) pdl_trigger();
     const scr_mlstm_shape& s = a.s;
     const int dim = s.dim, vdim = s.vdim;
     const int h = blockIdx.y, b = blockIdx.z, c0 = blockIdx.x * LR_COLS;
@@ -119,28 +121,32 @@ __global__ void __launch_bounds__(LR_T) lightning_recur_kernel(MemoryArgs a) {
             if (cols > 3) p[3] = S[i].w;
         }
     }
-    if (BESIDE) pdl_wait();
+    if (BESIDE) {
+        pdl_trigger();
+        pdl_wait();
+    }
 }
 
 constexpr int LN_T = 512;
 __device__ __forceinline__ void ln_gate(const bf16* p, float (&g)[4]) {
-    const uint2 w = *reinterpret_cast<const uint2*>(p);
+    const uint2 w = __ldcg(reinterpret_cast<const uint2*>(p));
     g[0] = bf16_lo(w.x); g[1] = bf16_hi(w.x); g[2] = bf16_lo(w.y); g[3] = bf16_hi(w.y);
 }
 __device__ __forceinline__ void ln_gate(const float* p, float (&g)[4]) {
-    const float4 w = *reinterpret_cast<const float4*>(p);
+    const float4 w = __ldcg(reinterpret_cast<const float4*>(p));
     g[0] = w.x; g[1] = w.y; g[2] = w.z; g[3] = w.w;
 }
 __device__ __forceinline__ void ln_put(bf16* p, const float (&v)[4]) { *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3])); }
 __device__ __forceinline__ void ln_put(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
 
 // One CTA per row.  KEEP: runs of 4 values a thread holds in registers between the sum and the product (0: any sizes).
+// beside: as for the memory; the attention between the two hides all of it.
 template <typename T, int KEEP>
-__global__ void __launch_bounds__(LN_T) lightning_finish_kernel(scr_lightning_shape s, const float* __restrict__ out, const float* __restrict__ norm,
-                                                                const T* __restrict__ gate, long long ld_gate, T* __restrict__ y, long long ld_y) {
+__global__ void __launch_bounds__(LN_T) lightning_finish_kernel(scr_lightning_shape s, const float* out, const float* __restrict__ norm, const T* gate,
+                                                                long long ld_gate, T* __restrict__ y, long long ld_y, bool beside) {
     __shared__ float red[LN_T / 32];
     pdl_trigger();
-    pdl_wait();
+    if (!beside) pdl_wait();
     const int n = s.heads * s.vdim, tid = threadIdx.x;
     const size_t r = blockIdx.x;
     const float* o = out + r * n;
@@ -168,20 +174,21 @@ __global__ void __launch_bounds__(LN_T) lightning_finish_kernel(scr_lightning_sh
             ln_put(y + r * ld_y + i, v[k]);
         }
     } else {
-        for (int i = tid; i < n; i += LN_T) ss = fmaf(o[i], o[i], ss);
+        for (int i = tid; i < n; i += LN_T) ss = fmaf(__ldcg(o + i), __ldcg(o + i), ss);
         const float inv = s.out_scale / sqrtf(cta_sum<LN_T>(ss, red) / float(n) + s.eps);
-        for (int i = tid; i < n; i += LN_T) y[r * ld_y + i] = from_f32<T>(o[i] * inv * norm[i] * sigmoid_f32(to_f32(gate[r * ld_gate + i])));
+        for (int i = tid; i < n; i += LN_T) y[r * ld_y + i] = from_f32<T>(__ldcg(o + i) * inv * norm[i] * sigmoid_f32(to_f32(__ldcg(gate + r * ld_gate + i))));
     }
+    if (beside) pdl_wait();
 }
 
 template <typename T>
 int32_t finish(scr_ctx* ctx, const scr_lightning_shape& s, const float* out, const float* norm, const void* gate, int64_t ld_gate, int32_t rows, void* y,
-               int64_t ld_y, cudaStream_t stream) {
+               int64_t ld_y, bool beside, cudaStream_t stream) {
     const int n = s.heads * s.vdim;
     const bool vec = n % 4 == 0 && ld_gate % 4 == 0 && ld_y % 4 == 0 && scr_aligned16(out) && scr_aligned16(norm) && scr_aligned16(gate) && scr_aligned16(y);
     auto kernel = !vec || n > 16 * LN_T ? lightning_finish_kernel<T, 0> : n > 8 * LN_T ? lightning_finish_kernel<T, 4>
                 : n > 4 * LN_T ? lightning_finish_kernel<T, 2> : lightning_finish_kernel<T, 1>;
-    const cudaError_t e = launch_pdl(kernel, dim3(rows), dim3(LN_T), 0, stream, s, out, norm, (const T*)gate, (long long)ld_gate, (T*)y, (long long)ld_y);
+    const cudaError_t e = launch_pdl(kernel, dim3(rows), dim3(LN_T), 0, stream, s, out, norm, (const T*)gate, (long long)ld_gate, (T*)y, (long long)ld_y, beside);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "lightning_finish: %s", cudaGetErrorString(e));
     return scr_check_launch(ctx, "lightning_finish");
 }
@@ -234,12 +241,22 @@ extern "C" int32_t scr_lightning_beside(scr_ctx* ctx, int32_t dtype, const scr_l
     return lightning_run(ctx, dtype, s, st, proj, ld, powers, state, out, workspace, workspace_bytes, true, stream);
 }
 
-extern "C" int32_t scr_lightning_finish(scr_ctx* ctx, int32_t dtype, const scr_lightning_shape* s, const float* out, const float* norm,
-                                        const void* gate, int64_t ld_gate, int32_t rows, void* y, int64_t ld_y, void* stream) {
+static int32_t lightning_finish(scr_ctx* ctx, int32_t dtype, const scr_lightning_shape* s, const float* out, const float* norm, const void* gate,
+                                int64_t ld_gate, int32_t rows, void* y, int64_t ld_y, bool beside, void* stream) {
     SCR_REQUIRE_CTX(ctx);
     if (!s || !out || !norm || !gate || !y) return scr_fail(ctx, SCR_E_ARG, "null pointer");
     if (rows <= 0 || s->heads <= 0 || s->vdim <= 0) return scr_fail(ctx, SCR_E_SHAPE, "%d rows", rows);
     if (dtype != SCR_DTYPE_F32 && dtype != SCR_DTYPE_BF16) return scr_fail(ctx, SCR_E_DTYPE, "dtype %d", dtype);
-    return dtype == SCR_DTYPE_F32 ? finish<float>(ctx, *s, out, norm, gate, ld_gate, rows, y, ld_y, (cudaStream_t)stream)
-                                  : finish<bf16>(ctx, *s, out, norm, gate, ld_gate, rows, y, ld_y, (cudaStream_t)stream);
+    return dtype == SCR_DTYPE_F32 ? finish<float>(ctx, *s, out, norm, gate, ld_gate, rows, y, ld_y, beside, (cudaStream_t)stream)
+                                  : finish<bf16>(ctx, *s, out, norm, gate, ld_gate, rows, y, ld_y, beside, (cudaStream_t)stream);
+}
+
+extern "C" int32_t scr_lightning_finish(scr_ctx* ctx, int32_t dtype, const scr_lightning_shape* s, const float* out, const float* norm,
+                                        const void* gate, int64_t ld_gate, int32_t rows, void* y, int64_t ld_y, void* stream) {
+    return lightning_finish(ctx, dtype, s, out, norm, gate, ld_gate, rows, y, ld_y, false, stream);
+}
+
+extern "C" int32_t scr_lightning_finish_beside(scr_ctx* ctx, int32_t dtype, const scr_lightning_shape* s, const float* out, const float* norm,
+                                               const void* gate, int64_t ld_gate, int32_t rows, void* y, int64_t ld_y, void* stream) {
+    return lightning_finish(ctx, dtype, s, out, norm, gate, ld_gate, rows, y, ld_y, true, stream);
 }

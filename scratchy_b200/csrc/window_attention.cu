@@ -81,8 +81,8 @@ __global__ void __launch_bounds__(WP_T) window_prepare_any_kernel(scr_window_sha
                                                                   T* __restrict__ q, T* __restrict__ cache, float* __restrict__ key_scale, int* status) {
     extern __shared__ float y[];                             // [channels]
     __shared__ float red_q[WP_T / 32], red_k[WP_T / 32];
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();                                           // after the wait, as in all kernels here: a memory beside them (scr_lightning_beside)
     const int r = blockIdx.x, tid = threadIdx.x, nq = s.heads * s.dim, C = nq + s.kv_heads * s.dim, hist = s.taps - 1;
     const PrepRow p = prep_row(s, st, r, status);
     if (p.at < 0) return;
@@ -118,14 +118,16 @@ __global__ void __launch_bounds__(512) window_prepare_kernel(scr_window_shape s,
     constexpr int N = ROWS + TAPS - 1;
     __shared__ float red[16][2 * ROWS];
     __shared__ PrepRow rows[ROWS];
-    pdl_trigger();
     const int r0 = blockIdx.x * ROWS, tid = threadIdx.x, nq = s.heads * s.dim, C = nq + s.kv_heads * s.dim, hist = s.taps - 1;
     if (tid < ROWS) rows[tid] = prep_row(s, st, r0 + tid, status);
     __syncthreads();
     float sq[ROWS], sk[ROWS], y[PER][ROWS][8];
 #pragma unroll
     for (int i = 0; i < ROWS; ++i) sq[i] = sk[i] = 0.0f;
-    if (PER > 1) pdl_wait();
+    if (PER > 1) {
+        pdl_wait();
+        pdl_trigger();
+    }
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
         const int c = (k * blockDim.x + tid) * 8;
@@ -140,7 +142,10 @@ __global__ void __launch_bounds__(512) window_prepare_kernel(scr_window_shape s,
                 for (int j = 0; j < 8; ++j) w[o][j] = 0.0f;
             }
         }
-        if (PER == 1) pdl_wait();
+        if (PER == 1) {
+            pdl_wait();
+            pdl_trigger();
+        }
         if (!in) continue;
         // what came before the first row: rows of the step, or the state of its sequence
         float u[N][8];
@@ -276,7 +281,6 @@ __global__ void __launch_bounds__(512) window_prepare_walk_kernel(scr_window_sha
     constexpr int PAST = TAPS - 1;
     __shared__ __align__(16) float red[2][16][2][WP_STEP];
     __shared__ PrepRow rows[WP_WALK];
-    pdl_trigger();
     const int r0 = blockIdx.x * per, n = min(per, st.rows - r0), tid = threadIdx.x, nq = s.heads * s.dim, C = nq + s.kv_heads * s.dim, hist = s.taps - 1;
     for (int i = tid; i < n; i += blockDim.x) rows[i] = prep_row(s, st, r0 + i, status);
     const int c = tid * 8;
@@ -293,6 +297,7 @@ __global__ void __launch_bounds__(512) window_prepare_walk_kernel(scr_window_sha
     for (int i = 0; i < PAST + WP_STEP; ++i) u[i].zero();
     __syncthreads();
     pdl_wait();
+    pdl_trigger();
 #pragma unroll
     for (int o = 1; o < TAPS; ++o)                           // the rows before the first one, where they are of this step
         if (in && o <= hist && o <= rows[0].at) u[PAST - o].load(proj + (r0 - o) * ld + c);
@@ -381,8 +386,8 @@ __global__ void __launch_bounds__(512) window_prepare_walk_kernel(scr_window_sha
 template <typename T>
 __global__ void __launch_bounds__(256) window_conv_state_kernel(scr_window_shape s, scr_step st, const T* __restrict__ proj, long long ld, T* state,
                                                                 int* status) {
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     const int b = blockIdx.y, c = blockIdx.x * 256 + threadIdx.x, C = (s.heads + s.kv_heads) * s.dim, hist = s.taps - 1;
     const int first = st.segs[b * 4], count = st.segs[b * 4 + 1], pos0 = st.segs[b * 4 + 2], slot = st.segs[b * 4 + 3];
     if (count <= 1 || c >= C) return;                        // (one token: done by the prepare kernel)
@@ -414,7 +419,7 @@ __global__ void __launch_bounds__(WA_WARPS * 32) window_attention_plain_kernel(s
     float* part = qs + s.dim;                                // [WA_WARPS][dim]
     float* ml = part + WA_WARPS * s.dim;                     // [WA_WARPS][2]
     pdl_wait();
-    pdl_trigger();                                           // (after the wait: scr_lightning_beside)
+    pdl_trigger();                                           // (after the wait: scr_lightning_finish_beside)
     const int r = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = h / (s.heads / s.kv_heads);
     const int pos = st.tok_pos[r], seg = st.tok_seg[r];
     const T* qp = q + ((size_t)r * s.heads + h) * s.dim;

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(WM_THREADS) window_attention_mma_kernel(const 
         fence_mbar_init();
     }
     pdl_wait();
-    pdl_trigger();                                           // after the wait: a memory beside this attention runs from here on (scr_lightning_beside)
+    pdl_trigger();                                           // after the wait: what runs beside this attention starts here (scr_lightning_finish_beside)
     if (lane == 0) {
 #pragma unroll
         for (int n = 0; n < STAGES; ++n) load(n, look_up(n));

@@ -124,8 +124,8 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_co
     auto s_col = [&](int t, int i) { return tmem + 256u * t + 64u * (i & 1); };        // S, then P: 32 columns of heads, 32 of remainders
     auto o_col = [&](int t) { return tmem + 256u * t + 128u; };
     pdl_wait();
-    // Not before this CTA has its TMEM, which the next kernel's CTAs could take first, and after the wait: a memory beside this attention runs from here
-    // on (scr_lightning_beside).
+    // Not before this CTA has its TMEM, which the next kernel's CTAs could take first, and after the wait: what runs beside this attention starts
+    // here (scr_lightning_finish_beside).
     pdl_trigger();
 
     if (warp == 0) {

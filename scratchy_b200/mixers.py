@@ -279,13 +279,25 @@ class WindowAttention:
 
     def run(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], memory, out: torch.Tensor) -> None:
         """`out`: the gated heads [rows, heads * dim], dense rows of any stride."""
-        qk, gate = bufs[f"{self.prefix}.qk"], bufs[f"{self.prefix}.g"]
-        cache, inv, rows = memory
-        lib, c = _lib.models_lib(), _lib.models_context(_dev_index(qk.device))
-        code, stream, ps, pt = dtype_code(self.dtype), _stream(qk.device), ctypes.byref(self.shape(ctx)), ctypes.byref(ctx.step)
+        self.prepare(ctx, bufs, memory)
+        self.attend(ctx, bufs, memory, out)
+
+    def _call(self, ctx: StepContext, bufs: Dict[str, torch.Tensor]):
+        qk = bufs[f"{self.prefix}.qk"]
         q = ctx.arena.get("wa.q", (ctx.rows, self.heads * self.dim), self.dtype)
+        return (_lib.models_lib(), _lib.models_context(_dev_index(qk.device)), dtype_code(self.dtype), ctypes.byref(self.shape(ctx)), ctypes.byref(ctx.step),
+                _stream(qk.device), q)
+
+    def prepare(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], memory) -> None:
+        """Queries, and the step's rows in the cache."""
+        qk, (cache, inv, rows) = bufs[f"{self.prefix}.qk"], memory
+        lib, c, code, ps, pt, stream, q = self._call(ctx, bufs)
         c.check(lib.scr_window_prepare(c.handle, code, ps, pt, _ptr(qk), int(qk.stride(0)), _ptr(self.conv), _ptr(self.norm), _ptr(rows), _ptr(q), _ptr(cache),
                                        _ptr(inv), stream))
+
+    def attend(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], memory, out: torch.Tensor) -> None:
+        gate, (cache, inv, _) = bufs[f"{self.prefix}.g"], memory
+        lib, c, code, ps, pt, stream, q = self._call(ctx, bufs)
         c.check(lib.scr_window_attention(c.handle, code, ps, pt, _ptr(q), _ptr(cache), _ptr(inv), _ptr(self.bias), _ptr(gate), int(gate.stride(0)), _ptr(out),
                                          int(out.stride(0)), stream))
 
@@ -326,9 +338,13 @@ class LightningAttention:
     def memory(self, cache_rows: int, slots: int, device) -> torch.Tensor:
         return torch.zeros((slots, self.heads, self.dim, self.vdim), dtype=torch.float32, device=device)
 
-    def run(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], memory: torch.Tensor, out: torch.Tensor, beside: bool = False) -> None:
-        """`beside`: the call directly before is a window attention's, which the memory may run beside."""
-        qkv, gate = bufs[f"{self.prefix}.qkv"], bufs[f"{self.prefix}.g"]
+    def run(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], memory: torch.Tensor, out: torch.Tensor) -> None:
+        self.remember(ctx, bufs, memory)
+        self.read(ctx, bufs, out)
+
+    def remember(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], memory: torch.Tensor, beside: bool = False) -> None:
+        """The memory's step.  `beside`: the call directly before is a window attention's `prepare`, which it may run beside."""
+        qkv = bufs[f"{self.prefix}.qkv"]
         lib, c = _lib.models_lib(), _lib.models_context(_dev_index(qkv.device))
         code, stream = dtype_code(self.dtype), _stream(qkv.device)
         shape = _lib.LightningShape(self.heads, self.dim, self.vdim, self.eps, self.out_scale)
@@ -339,8 +355,16 @@ class LightningAttention:
         run = lib.scr_lightning_beside if beside else lib.scr_lightning_run
         c.check(run(c.handle, code, ctypes.byref(shape), ctypes.byref(ctx.step), _ptr(qkv), int(qkv.stride(0)), _ptr(self.powers), _ptr(memory),
                     _ptr(o), _ptr(ws), need, stream))
-        c.check(lib.scr_lightning_finish(c.handle, code, ctypes.byref(shape), _ptr(o), _ptr(self.norm), _ptr(gate), int(gate.stride(0)), ctx.rows, _ptr(out),
-                                         int(out.stride(0)), stream))
+
+    def read(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], out: torch.Tensor, beside: bool = False) -> None:
+        """The readouts' norm and gate.  `beside`: the call directly before is a window attention's `attend`."""
+        gate = bufs[f"{self.prefix}.g"]
+        lib, c = _lib.models_lib(), _lib.models_context(_dev_index(gate.device))
+        shape = _lib.LightningShape(self.heads, self.dim, self.vdim, self.eps, self.out_scale)
+        o = ctx.arena.get("li.out", (ctx.rows, self.out_features), torch.float32)
+        finish = lib.scr_lightning_finish_beside if beside else lib.scr_lightning_finish
+        c.check(finish(c.handle, dtype_code(self.dtype), ctypes.byref(shape), _ptr(o), _ptr(self.norm), _ptr(gate), int(gate.stride(0)), ctx.rows, _ptr(out),
+                       int(out.stride(0)), _stream(gate.device)))
 
 
 class GeluGlu:
@@ -396,9 +420,14 @@ class SideBySide:
             lo, hi = self.columns[-1]
             bufs[f"{self.mlp.prefix}.act"] = rows[:, lo:hi]
         self.inp.run(a, h, bufs)
-        before = None
-        for m, mem, (lo, hi) in zip(self.mixers, memory, self.columns):
-            beside = {"beside": True} if isinstance(m, LightningAttention) and isinstance(before, WindowAttention) else {}
-            m.run(ctx, bufs, mem, rows[:, lo:hi], **beside)
-            before = m
+        outs = [rows[:, lo:hi] for lo, hi in self.columns]
+        if [type(m) for m in self.mixers] == [WindowAttention, LightningAttention]:
+            (window, lightning), (cache, state) = self.mixers, memory
+            window.prepare(ctx, bufs, cache)                  # a CTA per row: the memory runs beside it
+            lightning.remember(ctx, bufs, state, beside=True)
+            window.attend(ctx, bufs, cache, outs[0])          # and its readouts' norm beside this
+            lightning.read(ctx, bufs, outs[1], beside=True)
+        else:
+            for m, mem, out in zip(self.mixers, memory, outs):
+                m.run(ctx, bufs, mem, out)
         self.out.add_to(a, rows, residual, norm, h)

@@ -106,36 +106,51 @@ def test_decaying_memory(heads, dim, vdim, portions, dtype, captured):
 @pytest.mark.parametrize("captured", [False, True])
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads,dim,vdim", [(3, 48, 72), (8, 128, 128), (1, 300, 20)])
-@pytest.mark.parametrize("rows,attention", [(1, (4, 2, 64)), (3, (5, 1, 10)), (70, (2, 1, 128))])
-def test_decaying_memory_beside_an_attention(rows, attention, heads, dim, vdim, dtype, captured):
-    """The memory beside each kernel of the window attention, its input by the linear before that, in the buffer that the step before has read."""
+@pytest.mark.parametrize("rows,attention", [(1, (4, 2, 64)), (1, (5, 1, 10)), (3, (40, 8, 128)), (70, (2, 1, 128)), (300, (2, 1, 64))])
+@pytest.mark.parametrize("order", ["attention", "preparation"])
+def test_decaying_memory_beside_an_attention(order, rows, attention, heads, dim, vdim, dtype, captured):
+    """The memory beside each kernel of the window attention or of its preparation and, after the latter, the readout norm beside the attention; the
+    inputs by the linear before them, in the buffers that the step before has read."""
     from scratchy_b200 import _lib
     from scratchy_b200.dense import DenseLinear, dtype_code
     from scratchy_b200.mixers import decay_powers
     torch = torch_()
     L, c = lib()
-    steps, W, past = 8, heads * (2 * dim + vdim), 200
+    steps, W, past, C = 8, heads * (2 * dim + vdim), 200, (attention[0] + attention[1]) * attention[2]
     rng = np.random.default_rng(rows + dim)
     w = Window(*attention, 90, 5, 40, [past + rows], dtype, seed=rows)
-    w.cache.copy_(dev(draw(rng, tuple(w.cache.shape), dtype), dtype))
-    w.key_scale.fill_(0.1)
+    cache, taps, ones = dev(draw(rng, tuple(w.cache.shape), dtype), dtype), dev(rng.standard_normal((3, C))), torch.ones(C, device="cuda")
     st, sh, nq, bias = w.step([rows], [past], [1]), w.shape(), attention[0] * attention[2], w.padded_bias()
     q, gate = dev(draw(rng, (rows, nq), dtype), dtype), dev(rng.standard_normal((rows, attention[0])))
-    x, a, lin = dev(draw(rng, (steps, rows, 64), dtype), dtype), arena(), DenseLinear(dev(draw(rng, (W, 64), dtype, 0.125), dtype))
+    x, a, lin = dev(draw(rng, (steps, rows, 64), dtype), dtype), arena(), DenseLinear(dev(draw(rng, (W + C + heads * vdim, 64), dtype, 0.125), dtype))
     shape, powers, code = _lib.LightningShape(heads, dim, vdim, 1e-5, 1.0), decay_powers(np.asarray(([0.999, 0.6, 0.97] * 3)[:heads], np.float64)).cuda(), dtype_code(q.dtype)
     need = ctypes.c_size_t(0)
     c.check(L.scr_lightning_workspace(code, ctypes.byref(shape), ctypes.byref(st), ctypes.byref(need)))
     ws, results = torch.empty(max(16, need.value), dtype=torch.uint8, device="cuda"), []
+    ones_v = torch.ones(heads * vdim, device="cuda")
     for beside in (False, True):
         nan = lambda *n, t=torch.float32: torch.full(n, float("nan"), dtype=t, device="cuda")
-        proj, state, out, y = nan(rows, W, t=q.dtype), torch.zeros((2, heads, dim, vdim), device="cuda"), nan(steps, rows, heads * vdim), nan(steps, rows, nq + 8, t=q.dtype)
-        memory = L.scr_lightning_beside if beside else L.scr_lightning_run
+        proj, state, out, y = nan(rows, W + C + heads * vdim, t=q.dtype), torch.zeros((2, heads, dim, vdim), device="cuda"), nan(rows, heads * vdim), nan(steps, rows, nq + 8, t=q.dtype)
+        z, kept, inv, last = nan(steps, rows, heads * vdim, t=q.dtype), cache.clone(), torch.full_like(w.key_scale, 0.1), torch.zeros((2, 2, C), dtype=q.dtype, device="cuda")
+        ld, qs = proj.shape[1], q.clone()
+        common = (c.handle, code, ctypes.byref(sh), ctypes.byref(st))
 
-        def step(t, memory=memory, proj=proj, state=state, out=out, y=y):
+        def step(t, beside=beside, proj=proj, state=state, out=out, y=y, z=z, kept=kept, inv=inv, last=last, ld=ld, qs=qs, common=common):
             lin(a, x[t], proj)
-            c.check(L.scr_window_attention(c.handle, code, ctypes.byref(sh), ctypes.byref(st), ptr(q), ptr(w.cache), ptr(w.key_scale), ptr(bias), ptr(gate), attention[0],
-                                           ptr(y[t]), nq + 8, stream()))
-            c.check(memory(c.handle, code, ctypes.byref(shape), ctypes.byref(st), ptr(proj), W, ptr(powers), ptr(state), ptr(out[t]), ptr(ws), need, stream()))
+            prepare = lambda: c.check(L.scr_window_prepare(*common, ptr(proj, W), ld, ptr(taps), ptr(ones), ptr(last), ptr(qs), ptr(kept), ptr(inv), stream()))
+            attend = lambda: c.check(L.scr_window_attention(*common, ptr(qs), ptr(kept), ptr(inv), ptr(bias), ptr(gate), attention[0], ptr(y[t]), nq + 8, stream()))
+            remember = lambda: c.check((L.scr_lightning_beside if beside else L.scr_lightning_run)(
+                c.handle, code, ctypes.byref(shape), ctypes.byref(st), ptr(proj), ld, ptr(powers), ptr(state), ptr(out), ptr(ws), need, stream()))
+            read = lambda finish: c.check(finish(c.handle, code, ctypes.byref(shape), ptr(out), ptr(ones_v), ptr(proj, W + C), ld, rows, ptr(z[t]), heads * vdim, stream()))
+            prepare()
+            if order == "attention":
+                attend()
+                remember()
+                read(L.scr_lightning_finish)
+            else:
+                remember()
+                attend()
+                read(L.scr_lightning_finish_beside if beside else L.scr_lightning_finish)
 
         if beside:
             queued([lambda t=t: step(t) for t in range(steps)], captured)
@@ -143,7 +158,7 @@ def test_decaying_memory_beside_an_attention(rows, attention, heads, dim, vdim, 
             for t in range(steps):
                 step(t)
                 healthy()
-        results.append((out, state[1], y[:, :, :nq]))
+        results.append((z, state[1], y[:, :, :nq], last, kept))
     for one, other in zip(*results):
         assert torch.equal(one, other) and torch.isfinite(one).all()
 
