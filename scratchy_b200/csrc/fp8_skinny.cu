@@ -193,6 +193,13 @@ int32_t fp8_skinny_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act
 }
 
 // Up to 16 tokens, whose pack (`rows` = FP8_FEW_ROWS of a k-tile) only `scr_linear_fp8_dynamic` makes, for itself.
+bool fp8_skinny16_even(scr_ctx* ctx, int N, int K) {
+    const Fp8Geom g = fp8_geom(N, K);
+    const float share = (float)g.NT * g.KT / ctx->sm_count;
+    const int rounds = (g.NT + ctx->sm_count - 1) / ctx->sm_count;
+    return f8s_plan<16>(ctx, g).units <= 1.6f * share && 20 * g.NT < 19 * rounds * ctx->sm_count;
+}
+
 int32_t fp8_skinny16_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint16_t* y, int M, int N, int K, const LinearEnds& ends,
                             cudaStream_t stream) {
     return f8s_launch<16>(ctx, wpack, act, FP8_FEW_ROWS, y, M, N, K, ends, stream);

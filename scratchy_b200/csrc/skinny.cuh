@@ -196,6 +196,7 @@ struct SkinnyPlan {
     int split;
     size_t smem;
     int over_rings;
+    float units;                                 // k steps that an SM works through, and `unit_cost` for each of its units
 };
 constexpr size_t SKINNY_ALONE = 118 * 1024;      // dynamic shared memory that leaves no room for a second CTA on the SM
 
@@ -210,14 +211,14 @@ static inline SkinnyPlan skinny_plan(SkinnyResident& cache, void (*kernel)(KArgs
     const size_t sums = skinny_sum_bytes(tokens);
     const bool own = rings + sums <= 227 * 1024;
     const size_t alone_smem = own ? (rings + sums > SKINNY_ALONE ? rings + sums : SKINNY_ALONE) : rings;
-    SkinnyPlan best{1, rings, 1};
+    SkinnyPlan best{1, rings, 1, 0.0f};
     float least = 1e30f;
     for (int s = 1; s <= SKINNY_MAX_SPLIT && s <= steps; ++s) {
         if (tiles <= skinny_resident(cache, kernel, device, sms, s, true, threads, alone_smem)) {
             const float t = (float)((steps + s - 1) / s) + unit_cost;
             if (t < least * 0.999f) {
                 least = t;
-                best = {s, alone_smem, !own};
+                best = {s, alone_smem, !own, t};
             }
             continue;
         }
@@ -226,7 +227,7 @@ static inline SkinnyPlan skinny_plan(SkinnyResident& cache, void (*kernel)(KArgs
         const float t = (float)rounds * ((float)(beside * ((steps + s - 1) / s)) + unit_cost);
         if (t < least * 0.999f) {
             least = t;
-            best = {s, rings, 1};
+            best = {s, rings, 1, t};
         }
     }
     return best;
