@@ -221,7 +221,8 @@ def test_matvec_quantises_by_itself_with_the_same_bits(N, K, M):
     assert rel_l2(bits_of(fused).reshape(M, N), want) <= REL_L2_TOL
 
 
-@pytest.mark.parametrize("N,K,M", [(2056, 2048, 3), (1224, 3432, 4), (8200, 3840, 1), (2048, 15368, 5), (8192, 3848, 8), (4104, 3080, 9), (12296, 1032, 16)])
+@pytest.mark.parametrize("N,K,M", [(2056, 2048, 3), (1224, 3432, 4), (8200, 3840, 1), (2048, 15368, 5), (8192, 3848, 8), (4104, 3080, 9), (12296, 1032, 16),
+                                   (6144, 6144, 8), (6144, 8192, 1), (18944, 2048, 6)])        # (left to the matvec: an uneven cut, whole rounds of tiles)
 def test_few_tokens_that_the_call_quantises_for_the_gemm(N, K, M):
     """Dynamic linears of up to 16 tokens whose matrix is large enough for the GEMM for few tokens, in a workspace of the size that the query
     names, at both kinds of row ends; without the workspace for it the matvec runs.  Against the oracle, bias and partial sums as well."""
