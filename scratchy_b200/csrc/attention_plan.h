@@ -56,7 +56,17 @@ static inline AttPlan att_plan(int D, int G, int batch, int num_kv_heads, int bl
 // length (rank r goes to CTA r % bins in even rounds, from the other end in odd ones) the longest CTA has little more than the mean or than the longest
 // sequence.
 constexpr int ATT_MAX_ITEMS = 4;
-constexpr size_t ATT_SMEM_PACKED = 226 * 1024;
+constexpr size_t ATT_SMEM_BLOCK = 227 * 1024;          // shared memory that a CTA of sm_100a may have, dynamic and static together
+constexpr size_t ATT_SMEM_STATIC = 3 * 1024;           // of it the kernel's own arrays (AttShared, and the merge's weights) at most
+constexpr size_t ATT_SMEM_PACKED = ATT_SMEM_BLOCK - ATT_SMEM_STATIC;
+template <int D, int ITEMS>
+struct AttShared {
+    float rope_rows[ITEMS][2][D / 2];                  // cos and sin of the sequences' positions
+    int item_seq[ATT_MAX_ITEMS], item_len[ATT_MAX_ITEMS];
+};
+struct AttMergeShared {
+    float wgt[8][ATT_MAX_WARPS + 2];                   // per query head: the warps' weights, the merged maximum and sum
+};
 struct AttBins {
     int bins, items;                                   // CTAs per kv head; sequences a CTA takes at most (0: not this way)
     int warps, stages, table_cap;

@@ -311,7 +311,8 @@ template <int D>
 __device__ __forceinline__ void att_cta_merge(int G, int nwarps, const float* warp_part, float* cl_part, int split, int nsplit,
                                               int q_head0, int b, uint16_t* __restrict__ out, long long ld_o) {
     constexpr int STATE = D + 2;
-    __shared__ float wgt[8][ATT_MAX_WARPS + 2];      // per query head: the warps' weights, the merged maximum and sum
+    __shared__ AttMergeShared merge_shared;
+    auto& wgt = merge_shared.wgt;
     const int nthreads = nwarps * 32;
     asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
     if (threadIdx.x < G) {
@@ -647,8 +648,11 @@ __global__ void __launch_bounds__(ATT_MAX_WARPS * 32) attention_decode_tc_kernel
     }
     uint64_t* bars = reinterpret_cast<uint64_t*>(blocks + ((table_cap + 1) & ~1));                // full[stages]
     int* lens = reinterpret_cast<int*>(bars + stages);                                            // PACKED: [batch]
-    __shared__ int item_seq[ATT_MAX_ITEMS], item_len[ATT_MAX_ITEMS];
-    __shared__ float rope_rows[PACKED ? ATT_MAX_ITEMS : 1][2][D / 2];        // cos and sin of the sequences' positions
+    using Shared = AttShared<D, PACKED ? ATT_MAX_ITEMS : 1>;
+    static_assert(sizeof(Shared) + sizeof(AttMergeShared) + 512 <= ATT_SMEM_STATIC, "what att_bins leaves for the static arrays");
+    __shared__ Shared shared;
+    auto &item_seq = shared.item_seq, &item_len = shared.item_len;
+    auto& rope_rows = shared.rope_rows;
 
     pdl_trigger();
     uint32_t nsplit;

@@ -77,3 +77,25 @@ def test_sequences_are_dealt_evenly_to_bins_that_fit(tmp_path):
                     load[p.bins - 1 - at if (r // p.bins) & 1 else at] += n
                 assert max(load) <= max(lens[0], sum(load) / p.bins) + lens[0] - lens[-1]
     assert not call(128, 3, 32, 8, 16, 128, 2).items and not call(128, 3, 18, 8, 16, 128, 1).items and not call(128, 3, 73, 8, 16, 128, 1).items
+
+
+def test_packed_layout_leaves_room_for_the_static_arrays(tmp_path):
+    """A CTA may have 227 KB, dynamic and static together: no layout asks for more, at any width of the table."""
+    source, library = tmp_path / "bins.cpp", tmp_path / "bins.so"
+    source.write_text('#include "attention_plan.h"\nextern "C" size_t most(int d, int g, int b, int bs, int from, int to) {\n'
+                      '    size_t most = 0;\n    for (int mb = from; mb < to; ++mb) {\n'
+                      f'        const AttBins p = att_bins(d, g, b, 8, bs, mb, {SMS}, 1);\n        if (p.items && p.smem > most) most = p.smem;\n    }}\n    return most;\n}}\n'
+                      'extern "C" size_t fixed_part(int d) {\n'
+                      '    return sizeof(AttMergeShared) + (d == 128 ? sizeof(AttShared<128, ATT_MAX_ITEMS>) : sizeof(AttShared<64, ATT_MAX_ITEMS>));\n}\n')
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, "-o", library, source], check=True)
+    call = ctypes.CDLL(str(library))
+    call.most.restype = call.fixed_part.restype = ctypes.c_size_t
+    seen = 0
+    for d in (64, 128):
+        for g in range(1, 9):
+            for batch in (20, 32, 36, 40, 48, 54, 72):
+                for block in (16, 32):
+                    most = call.most(d, g, batch, block, 1, 12000)
+                    assert most + call.fixed_part(d) <= 227 * 1024, (d, g, batch, block, most)
+                    seen += most > 220 * 1024
+    assert seen > 50

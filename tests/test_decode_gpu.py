@@ -153,7 +153,7 @@ def test_rope_append_bit_exact(tokens, hq, hkv, d, bs, nblk):
     assert np.array_equal(bits_of(dk), rbits(ok)) and np.array_equal(bits_of(dv), rbits(ov))
 
 
-def _attention_case(lens, hq, hkv, d, bs, seed, scale=None):
+def _attention_case(lens, hq, hkv, d, bs, seed, scale=None, width=0):
     import torch
     from scratchy_b200 import decode
     rng = np.random.default_rng(seed)
@@ -161,6 +161,7 @@ def _attention_case(lens, hq, hkv, d, bs, seed, scale=None):
     max_blocks = max(1, max((n + bs - 1) // bs for n in lens)) + 1
     nblk = batch * max_blocks + 3
     table = rng.permutation(nblk)[:batch * max_blocks].reshape(batch, max_blocks).astype(np.uint32)
+    table = np.pad(table, ((0, 0), (0, max(0, width - max_blocks))), mode="edge")
     ck = rbits(rng.standard_normal((nblk, hkv, bs, d)))
     cv = rbits(rng.standard_normal((nblk, hkv, bs, d)))
     q = rbits(rng.standard_normal((batch, hq * d)))
@@ -276,6 +277,15 @@ def test_attention_of_more_sequences_than_ctas(lens, hq, hkv, d, bs):
     test_rope_attention_one_launch_equals_the_two_operators(lens, hq, hkv, d, bs)
     if bs == 16 and len(lens) < 40:
         test_attention_via_cache(lens[:-2] + [0, 1], hq, hkv, d, bs)
+
+
+@pytest.mark.parametrize("batch,hq,hkv,d,width", [(20, 16, 8, 128, 1024), (32, 32, 8, 128, 8192), (40, 8, 8, 128, 1100), (48, 24, 8, 128, 5000), (40, 32, 8, 64, 8192),
+                                                  (48, 24, 8, 128, 5200)])
+def test_attention_with_wide_block_tables(batch, hq, hkv, d, width):
+    """Tables of long contexts, whose block ids take what shared memory the stages and the kernel's own arrays leave, and more than that: the call
+    runs, whichever layout has room."""
+    got, want = _attention_case([1 + (53 * i) % 90 for i in range(batch)], hq, hkv, d, 16, synth.seed_for("wide", batch, hq, d, width), width=width)
+    assert rel_l2(got, want) <= REL_L2_TOL
 
 
 def test_rope_attention_refuses_what_it_cannot_stream():
