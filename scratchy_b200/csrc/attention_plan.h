@@ -61,7 +61,7 @@ constexpr size_t ATT_SMEM_STATIC = 3 * 1024;           // of it the kernel's own
 constexpr size_t ATT_SMEM_PACKED = ATT_SMEM_BLOCK - ATT_SMEM_STATIC;
 template <int D, int ITEMS>
 struct AttShared {
-    float rope_rows[ITEMS][2][D / 2];                  // cos and sin of the sequences' positions
+    alignas(16) float rope_rows[ITEMS][2][D / 2];      // cos and sin of the sequences' positions; read two at a time
     int item_seq[ATT_MAX_ITEMS], item_len[ATT_MAX_ITEMS];
 };
 struct AttMergeShared {

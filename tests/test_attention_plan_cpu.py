@@ -99,3 +99,13 @@ def test_packed_layout_leaves_room_for_the_static_arrays(tmp_path):
                     assert most + call.fixed_part(d) <= 227 * 1024, (d, g, batch, block, most)
                     seen += most > 220 * 1024
     assert seen > 50
+
+
+def test_rotation_rows_are_aligned_for_the_loads_that_read_them(tmp_path):
+    """`ld.shared.v2.f32` in inline assembly needs 8 bytes, of which the compiler knows nothing: the struct has to say so, wherever the arrays
+    beside it end."""
+    source = tmp_path / "rows.cpp"
+    source.write_text('#include <stddef.h>\n#include "attention_plan.h"\n' + "".join(
+        f"using S{d}_{n} = AttShared<{d}, {n}>;\nstatic_assert(alignof(S{d}_{n}) >= 8 && offsetof(S{d}_{n}, rope_rows) % 8 == 0, \"\");\n"
+        for d in (64, 128) for n in (1, 4)))
+    subprocess.run(["g++", "-std=c++17", "-fsyntax-only", "-I", CSRC, source], check=True)
