@@ -258,8 +258,12 @@ int32_t scr_e4m3_encode(scr_ctx* ctx, const float* v, int64_t count, uint8_t* ou
  *   y[m,n] (bf16) = ((sum_k x_q[m,k] * w_q[n,k]) * a_scale[m]) * w_scale[n],  f32 accumulation.
  * `scr_linear_fp8` consumes an activation pack; `scr_linear_fp8_dynamic` is the whole
  * generated Linear (quantise, then contract) and needs a workspace that holds the pack.  For
- * M <= 4 (and M*K <= 16 KiB of codes) the matvec quantises the activations itself — same x_q and
- * a_scale bits, one launch, the workspace is not touched.  `bias_bf16` (may be NULL) is the linear's
+ * M <= 4 (and M * K16 <= 14 KiB of codes, K16 = K rounded up to 16) the matvec quantises the activations
+ * itself — same x_q and a_scale bits, one launch, the workspace is not touched; the result has the bits of
+ * `scr_fp8_quant_per_token` and `scr_linear_fp8`.  Beyond that, up to 16 tokens, a large matrix goes to another
+ * kernel than a pack does (equal to the rounding of the f32 sums), given the workspace that
+ * `scr_linear_workspace_size` names; with one that only holds the pack (`scr_fp8_act_size`) it runs as the
+ * two calls do.  `bias_bf16` (may be NULL) is the linear's
  * own bias [N] (`{prefix}.bias`; the q/k/v projections of Qwen2.5 carry one), added in f32 to the
  * dequantised sum before the one rounding. */
 int32_t scr_linear_fp8(scr_ctx* ctx, const void* packed, const void* act, int32_t M, int32_t N,

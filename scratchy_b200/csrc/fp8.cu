@@ -790,31 +790,24 @@ static int32_t fp8_gemv_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t
 
 // Defined in fp8_skinny.cu
 int32_t fp8_skinny16_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, uint16_t* y, int M, int N, int K, const LinearEnds& ends, cudaStream_t stream);
-// Whether that GEMM beats the matvec with one tile of tokens (3 and 4 tokens of a short k, which the matvec quantises slowly, aside): not where its cut leaves an SM much more than its even share (us, matvec / GEMM, 8 tokens:
-// 12288 x 5120, 1.70 shares 14.7 / 18.5;  6144 x 6144, 1.80 10.5 / 11.6;  1 token of 6144 x 8192, 1.73 12.2 / 13.1;  5120 x 7168, 1.52 11.3 / 10.9;  14336 x 4096, 1.49 15.0 / 14.8;  8192 x 4096, 1.45
+// Whether that GEMM beats the matvec with one tile of tokens: not where its cut leaves an SM much more than its even share (us, matvec / GEMM, 8 tokens:
+// 12288 x 5120, 1.70 shares 14.7 / 18.5;  6144 x 6144, 1.80 10.5 / 11.6;  5120 x 7168, 1.52 11.3 / 10.9;  14336 x 4096, 1.49 15.0 / 14.8;  8192 x 4096, 1.45
 // 10.5 / 9.9;  9472 x 3584, 1.29 11.1 / 9.8), nor where the channel tiles fill whole rounds of SMs, which the matvec then streams (18944 x 3584 16.1 / 16.3).
 bool fp8_skinny16_even(scr_ctx* ctx, int N, int K);
 // Whether a dynamic linear of up to 16 tokens is quantised for, and goes to, the GEMM for few tokens, whose time does not grow with them.  (A pack that the
-// caller holds is the matvec's.)  us in streams of calls with the quantisation, matvec / GEMM:
-//   one launch that quantises by itself (M <= 4, 14 KB of codes): 2048 x 2048, 4 tokens 6.2 / 4.6;  3584 x 3584, 1 token 5.9 / 5.7, 4 10.2 / 5.8;
-//   18944 x 3584, 1 token 14.5 / 14.0 (called one by one 14.5 / 15.1), 4 19.0 / 14.3;  16384 x 1024, 4 tokens 8.2 / 6.5;  1 token of a long k, whose codes every CTA makes for itself:
-//   4096 x 14336 19.2 / 13.2;  8192 x 8192 17.3 / 14.6.  (Partial sums stay with the matvec, whose bits the
-//   matvec with the exchange in its end has.)
-//   quantised beforehand: 1024 x 16384, 8 tokens 7.3 / 8.7;  5120 x 5120, 8 tokens 8.1 / 8.0;  2048 x 16384, 1 token 10.5 / 10.4, 8 12.1 / 10.7;
-//   8192 x 8192, 1 token 17.3 / 14.6;  3584 x 18944, 1 token 22.0 / 15.3
+// caller holds is the matvec's.)  Not where the matvec quantises by itself: that call leaves the workspace alone and has the bits of the matvec on a
+// pack, with partial sums and with the exchange too.  us in streams of calls with the quantisation, matvec / GEMM:
+//   up to 8 tokens: 1024 x 16384, 8 tokens 7.3 / 8.7;  5120 x 5120, 8 tokens 8.1 / 8.0;  2048 x 16384, 1 token 10.5 / 10.4, 8 12.1 / 10.7;  3584 x 18944, 1 token 22.0 / 15.3
 //   9 to 16 tokens, two tiles of the matvec: 1024 x 8192, 16 tokens 6.1 / 6.2;  3584 x 3584, 9 tokens 6.5 / 6.0;  8192 x 2048 8.4 / 6.8;
 //   18944 x 3584 22.2 / 14.7
-static bool fp8_few_tokens(int M, int N, int K, bool partial) {
-    const long long weights = (long long)N * K;
-    if (M > 16) return false;
-    if (fp8_gemv_fuses_quant(M, K)) return !partial && (M > 2 ? weights >= 4 << 20 : weights >= 48 << 20 && K >= 8192);
-    return weights >= (M > 8 ? 12 << 20 : 30 << 20);
+static bool fp8_few_tokens(int M, int N, int K) {
+    return M <= 16 && !fp8_gemv_fuses_quant(M, K) && (long long)N * K >= (M > 8 ? 12 << 20 : 30 << 20);
 }
 
 size_t fp8_workspace_bytes(int M, int N, int K) {
     // the dynamic entry point keeps its activation pack in the workspace
     size_t b = (fp8_act_bytes(M, K) + 127) / 128 * 128;
-    if (fp8_few_tokens(M, N, K, false)) b = std::max(b, fp8_few_bytes(M, K));
+    if (fp8_few_tokens(M, N, K)) b = std::max(b, fp8_few_bytes(M, K));
     if (fp8_act_tiled(M)) b += fp8_gemm_tc_workspace(M, N, K);
     return (b + 127) / 128 * 128;
 }
@@ -866,8 +859,8 @@ static int32_t fp8_linear_dynamic(scr_ctx* ctx, const void* packed, const uint16
     if (M <= 0) return scr_fail(ctx, SCR_E_SHAPE, "M=%d must be positive", M);
     if (!scr_aligned16(packed) || !scr_aligned16(x)) return scr_fail(ctx, SCR_E_ALIGN, "packed/x must be 16-byte aligned");
     if (ends.bias && ends.out_f32) return scr_fail(ctx, SCR_E_ARG, "a bias is added after the partial sums have been reduced, not to a partial");
-    if (fp8_few_tokens(M, N, K, ends.out_f32 != 0) && workspace && scr_aligned16(workspace) && workspace_bytes >= fp8_few_bytes(M, K) &&
-        (M > 8 || (M > 2 && fp8_gemv_fuses_quant(M, K)) || fp8_skinny16_even(ctx, N, K))) {
+    if (fp8_few_tokens(M, N, K) && workspace && scr_aligned16(workspace) && workspace_bytes >= fp8_few_bytes(M, K) &&
+        (M > 8 || fp8_skinny16_even(ctx, N, K))) {
         st = fp8_quant_launch(ctx, x, M, K, 1, FP8_FEW_ROWS, workspace, stream);
         if (st) return st;
         return fp8_skinny16_launch(ctx, (const uint8_t*)packed, (const uint8_t*)workspace, static_cast<uint16_t*>(y), M, N, K, ends, (cudaStream_t)stream);

@@ -13,7 +13,7 @@
 //
 // What bounds it: the copies into shared memory, 16 KB of weights and 128 bytes per token and step.  250 tokens of 18944 -> 3584
 // (with the quantisation) 46.4 us on the 128-token tiles of fp8_gemm.cu and their finishing launch, 32.5 us here.
-// One token of 3584 -> 18944 14.0 us, of 18944 -> 3584 15.3 (22.0 in the matvec, which quantises in a launch of its own there).
+// One token of 18944 -> 3584 15.3 us (22.0 in the matvec, which quantises in a launch of its own there).
 #include "fp8.cuh"
 #include "skinny.cuh"
 

@@ -197,7 +197,7 @@ def test_prefill_gemm_full_size_sampled_rows(name, M):
 
 
 @pytest.mark.parametrize("N,K,M", [(3584, 3584, 1), (512, 3584, 4), (18944, 3584, 2), (130, 328, 3), (24, 200, 1),
-                                  (1280, 8192, 2), (8192, 1024, 1), (64, 16384, 1)])
+                                  (1280, 8192, 2), (8192, 1024, 1), (64, 16384, 1), (2056, 2048, 3), (3584, 3584, 4), (8192, 8192, 1), (4096, 14336, 1)])
 def test_matvec_quantises_by_itself_with_the_same_bits(N, K, M):
     """For M <= 4 (and up to 14 KiB of codes) the whole linear is one launch: the matvec computes a_scale and x_q in
     shared memory.
@@ -219,6 +219,31 @@ def test_matvec_quantises_by_itself_with_the_same_bits(N, K, M):
     assert np.array_equal(bits_of(part.to(torch.bfloat16)), bits_of(fused))
     want = oracle.fp8_dynamic_linear(bits_of(x).reshape(M, K), wq, ws, M, N, K)
     assert rel_l2(bits_of(fused).reshape(M, N), want) <= REL_L2_TOL
+
+
+def dynamic(layer, x, y, work):
+    """The C call, with a workspace of any size (the layer's `forward` takes a larger one by itself)."""
+    import ctypes
+    from scratchy_b200 import _lib
+    ctx = _lib.context(0)
+    ctx.check(_lib.lib().scr_linear_fp8_dynamic(ctx.handle, layer.packed.data_ptr(), x.data_ptr(), x.shape[0], layer.out_features, layer.in_features, None,
+                                                y.data_ptr(), work.data_ptr(), ctypes.c_size_t(work.numel()), None))
+
+
+@pytest.mark.parametrize("N,K,M", [(512, 3584, 4), (2056, 2048, 3), (3584, 3584, 4), (8192, 8192, 1)])
+def test_matvec_that_quantises_by_itself_leaves_the_workspace_alone(N, K, M):
+    """A program may hand one workspace to such calls on several streams, or none: it is not written, and the bits do not depend on it."""
+    import torch
+    wq, ws = oracle.fp8_quantize_weight_per_channel(synth.fp8_weights_f32(N, K, synth.seed_for("alone", N, K)))
+    layer, x = make_layer(wq, ws), bf16_dev(synth.activations_bf16(M, K, 9)).reshape(M, K)
+    outs = []
+    for size in (16, layer.workspace_bytes(M), 1 << 22):
+        work, y = torch.full((size,), 0x5A, dtype=torch.uint8, device="cuda"), torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+        dynamic(layer, x, y, work)
+        torch.cuda.synchronize()
+        assert bool((work == 0x5A).all())
+        outs.append(bits_of(y))
+    assert all(np.array_equal(o, outs[0]) for o in outs)
 
 
 @pytest.mark.parametrize("N,K,M", [(2056, 2048, 3), (1224, 3432, 4), (8200, 3840, 1), (2048, 15368, 5), (8192, 3848, 8), (4104, 3080, 9), (12296, 1032, 16),
