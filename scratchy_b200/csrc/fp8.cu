@@ -804,12 +804,16 @@ static bool fp8_few_tokens(int M, int N, int K) {
     return M <= 16 && !fp8_gemv_fuses_quant(M, K) && (long long)N * K >= (M > 8 ? 12 << 20 : 30 << 20);
 }
 
-size_t fp8_workspace_bytes(int M, int N, int K) {
-    // the dynamic entry point keeps its activation pack in the workspace
+// The pack of `scr_fp8_quant_per_token` and what a linear from it needs.
+static size_t fp8_pack_workspace_bytes(int M, int N, int K) {
     size_t b = (fp8_act_bytes(M, K) + 127) / 128 * 128;
-    if (fp8_few_tokens(M, N, K)) b = std::max(b, fp8_few_bytes(M, K));
     if (fp8_act_tiled(M)) b += fp8_gemm_tc_workspace(M, N, K);
     return (b + 127) / 128 * 128;
+}
+size_t fp8_workspace_bytes(int M, int N, int K) {
+    // the dynamic entry point keeps its activation pack in the workspace
+    const size_t b = fp8_pack_workspace_bytes(M, N, K);
+    return fp8_few_tokens(M, N, K) ? std::max(b, (fp8_few_bytes(M, K) + 127) / 128 * 128) : b;
 }
 
 static int32_t fp8_linear_from_pack(scr_ctx* ctx, const uint8_t* wpack, const uint8_t* act, int M, int N, int K,
@@ -870,8 +874,7 @@ static int32_t fp8_linear_dynamic(scr_ctx* ctx, const void* packed, const uint16
         return fp8_gemv_launch<1>(ctx, (const uint8_t*)packed, nullptr, nullptr, static_cast<uint16_t*>(y), M, N, K, ends,
                                   (cudaStream_t)stream, x);
     }
-    size_t need = (fp8_act_bytes(M, K) + 127) / 128 * 128;         // (the GEMM's part follows the pack)
-    if (fp8_act_tiled(M)) need = fp8_workspace_bytes(M, N, K);
+    const size_t need = fp8_pack_workspace_bytes(M, N, K);         // (the GEMM's part follows the pack)
     if (!workspace || workspace_bytes < need)
         return scr_fail(ctx, SCR_E_WORKSPACE, "workspace %zu bytes < required %zu", workspace_bytes, need);
     if (!scr_aligned16(workspace)) return scr_fail(ctx, SCR_E_ALIGN, "workspace must be 16-byte aligned");
@@ -1003,7 +1006,7 @@ extern "C" int32_t scr_linear_fp8_dynamic_static(scr_ctx* ctx, const void* packe
     if (st) return st;
     if (M <= 0) return scr_fail(ctx, SCR_E_SHAPE, "M=%d must be positive", M);
     if (!scr_aligned16(packed) || !scr_aligned16(x)) return scr_fail(ctx, SCR_E_ALIGN, "packed/x must be 16-byte aligned");
-    const size_t need = fp8_workspace_bytes(M, N, K);
+    const size_t need = fp8_pack_workspace_bytes(M, N, K);
     if (need > (size_t)SCR_STATIC_SCRATCH_BYTES)
         return scr_fail(ctx, SCR_E_WORKSPACE,
                         "M=%d K=%d needs %zu bytes of scratch, the built-in array holds %u; use scr_linear_fp8_dynamic "

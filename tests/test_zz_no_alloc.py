@@ -60,6 +60,22 @@ def test_static_scratch_matches_workspace_entry_point_twice(N, K, M1, M2):
         assert torch.equal(y, y_ref)        # the same arithmetic on the same bytes: bit-identical
 
 
+def test_a_pack_that_fits_the_array_is_taken():
+    """What counts is the pack of the call's own route (562 KB here), not a larger one that another entry point would make."""
+    import torch
+    from scratchy_b200 import Fp8Linear
+    N, K = 56, 562000
+    g = torch.Generator(device="cuda").manual_seed(8)
+    w = torch.randn((N, K), device="cuda", generator=g).mul_(0.02)
+    scale = w.abs().amax(dim=1) / 448.0
+    layer = Fp8Linear.from_tensors((w / scale[:, None]).to(torch.float8_e4m3fn), scale)
+    x = torch.randn((1, K), device="cuda", generator=g).bfloat16()
+    y, y_ref = _both(layer, x, 1, N, K)
+    assert float((y.float() - y_ref.float()).norm() / y_ref.float().norm()) < 1e-3
+    want = x.double() @ w.double().T
+    assert float((y.double() - want).norm() / want.norm()) < 0.05       # two e4m3 roundings of 2^-4 at most
+
+
 def test_requests_beyond_the_array_are_refused():
     import torch
     from scratchy_b200 import _lib
