@@ -855,6 +855,25 @@ static int32_t fp8_linear(scr_ctx* ctx, const void* packed, const void* act, int
                                 workspace_bytes, stream);
 }
 
+// Quantises into the workspace and contracts from there.
+static int32_t fp8_linear_through(scr_ctx* ctx, const void* packed, const uint16_t* x, int M, int N, int K, void* y, const LinearEnds& ends,
+                                  void* workspace, size_t workspace_bytes, void* stream) {
+    const size_t need = fp8_pack_workspace_bytes(M, N, K);         // (the GEMM's part follows the pack)
+    if (!workspace || workspace_bytes < need)
+        return scr_fail(ctx, SCR_E_WORKSPACE, "workspace %zu bytes < required %zu", workspace_bytes, need);
+    if (!scr_aligned16(workspace)) return scr_fail(ctx, SCR_E_ALIGN, "workspace must be 16-byte aligned");
+    if (fp8_few_tokens(M, N, K) && workspace_bytes >= fp8_few_bytes(M, K) && (M > 8 || fp8_skinny16_even(ctx, N, K))) {
+        const int32_t st = fp8_quant_launch(ctx, x, M, K, 1, FP8_FEW_ROWS, workspace, stream);
+        if (st) return st;
+        return fp8_skinny16_launch(ctx, (const uint8_t*)packed, (const uint8_t*)workspace, static_cast<uint16_t*>(y), M, N, K, ends, (cudaStream_t)stream);
+    }
+    const int32_t st = scr_fp8_quant_per_token(ctx, x, M, K, workspace, stream);
+    if (st) return st;
+    const size_t act_bytes = (fp8_act_bytes(M, K) + 127) / 128 * 128;
+    return fp8_linear_from_pack(ctx, (const uint8_t*)packed, (const uint8_t*)workspace, M, N, K, static_cast<uint16_t*>(y), ends,
+                                (uint8_t*)workspace + act_bytes, workspace_bytes - act_bytes, (cudaStream_t)stream);
+}
+
 static int32_t fp8_linear_dynamic(scr_ctx* ctx, const void* packed, const uint16_t* x, int M, int N, int K, void* y,
                                   const LinearEnds& ends, void* workspace, size_t workspace_bytes, void* stream) {
     if (!packed || !x || !y) return scr_fail(ctx, SCR_E_ARG, "null pointer");
@@ -863,26 +882,12 @@ static int32_t fp8_linear_dynamic(scr_ctx* ctx, const void* packed, const uint16
     if (M <= 0) return scr_fail(ctx, SCR_E_SHAPE, "M=%d must be positive", M);
     if (!scr_aligned16(packed) || !scr_aligned16(x)) return scr_fail(ctx, SCR_E_ALIGN, "packed/x must be 16-byte aligned");
     if (ends.bias && ends.out_f32) return scr_fail(ctx, SCR_E_ARG, "a bias is added after the partial sums have been reduced, not to a partial");
-    if (fp8_few_tokens(M, N, K) && workspace && scr_aligned16(workspace) && workspace_bytes >= fp8_few_bytes(M, K) &&
-        (M > 8 || fp8_skinny16_even(ctx, N, K))) {
-        st = fp8_quant_launch(ctx, x, M, K, 1, FP8_FEW_ROWS, workspace, stream);
-        if (st) return st;
-        return fp8_skinny16_launch(ctx, (const uint8_t*)packed, (const uint8_t*)workspace, static_cast<uint16_t*>(y), M, N, K, ends, (cudaStream_t)stream);
-    }
     if (fp8_gemv_fuses_quant(M, K)) {
         // few tokens: the matvec quantises the activations itself, no pack and no second launch
         return fp8_gemv_launch<1>(ctx, (const uint8_t*)packed, nullptr, nullptr, static_cast<uint16_t*>(y), M, N, K, ends,
                                   (cudaStream_t)stream, x);
     }
-    const size_t need = fp8_pack_workspace_bytes(M, N, K);         // (the GEMM's part follows the pack)
-    if (!workspace || workspace_bytes < need)
-        return scr_fail(ctx, SCR_E_WORKSPACE, "workspace %zu bytes < required %zu", workspace_bytes, need);
-    if (!scr_aligned16(workspace)) return scr_fail(ctx, SCR_E_ALIGN, "workspace must be 16-byte aligned");
-    st = scr_fp8_quant_per_token(ctx, x, M, K, workspace, stream);
-    if (st) return st;
-    const size_t act_bytes = (fp8_act_bytes(M, K) + 127) / 128 * 128;
-    return fp8_linear_from_pack(ctx, (const uint8_t*)packed, (const uint8_t*)workspace, M, N, K, static_cast<uint16_t*>(y), ends,
-                                (uint8_t*)workspace + act_bytes, workspace_bytes - act_bytes, (cudaStream_t)stream);
+    return fp8_linear_through(ctx, packed, x, M, N, K, y, ends, workspace, workspace_bytes, stream);
 }
 
 extern "C" int32_t scr_linear_fp8(scr_ctx* ctx, const void* packed, const void* act, int32_t M, int32_t N, int32_t K,
@@ -1014,9 +1019,5 @@ extern "C" int32_t scr_linear_fp8_dynamic_static(scr_ctx* ctx, const void* packe
     void* scratch = nullptr;
     st = static_scratch_for(ctx, &scratch);
     if (st) return st;
-    st = scr_fp8_quant_per_token(ctx, x, M, K, scratch, stream);
-    if (st) return st;
-    const size_t act_bytes = (fp8_act_bytes(M, K) + 127) / 128 * 128;
-    return fp8_linear_from_pack(ctx, (const uint8_t*)packed, (const uint8_t*)scratch, M, N, K, y, LinearEnds(),
-                                (uint8_t*)scratch + act_bytes, (size_t)SCR_STATIC_SCRATCH_BYTES - act_bytes, (cudaStream_t)stream);
+    return fp8_linear_through(ctx, packed, x, M, N, K, y, LinearEnds(), scratch, SCR_STATIC_SCRATCH_BYTES, stream);
 }

@@ -46,7 +46,7 @@ def _both(layer, x, M, N, K):
     return y, y_ref
 
 
-@pytest.mark.parametrize("N,K,M1,M2", [(384, 512, 3, 16), (512, 384, 200, 40), (256, 1024, 64, 2)])
+@pytest.mark.parametrize("N,K,M1,M2", [(384, 512, 3, 16), (512, 384, 200, 40), (256, 1024, 64, 2), (4104, 3080, 16, 9), (2048, 15368, 5, 8)])
 def test_static_scratch_matches_workspace_entry_point_twice(N, K, M1, M2):
     import torch
     from scratchy_b200 import Fp8Linear
