@@ -261,7 +261,7 @@ __device__ __forceinline__ bool elect_one() {
 typedef CUresult (*tc_encode_tiled_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                        const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                        CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static inline tc_encode_tiled_fn tc_tensor_map_encoder() {
+static inline tc_encode_tiled_fn tc_driver_encoder() {
     static tc_encode_tiled_fn fn = nullptr;
     if (!fn) {
         void* p = nullptr;
@@ -271,4 +271,18 @@ static inline tc_encode_tiled_fn tc_tensor_map_encoder() {
             fn = (tc_encode_tiled_fn)p;
     }
     return fn;
+}
+// The driver's function wants a context of the calling thread, which the runtime sets only at a call of its own that needs one: the encoder is the
+// first such call of a linear that a new host thread makes.
+template <typename... A>
+static CUresult tc_encode_in_context(A... a) {
+    const tc_encode_tiled_fn encode = tc_driver_encoder();
+    const CUresult r = encode(a...);
+    int device = 0;
+    if (r != CUDA_ERROR_INVALID_CONTEXT || cudaGetDevice(&device) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) return r;
+    return encode(a...);
+}
+static inline tc_encode_tiled_fn tc_tensor_map_encoder() {
+    const tc_encode_tiled_fn bound = tc_encode_in_context;
+    return tc_driver_encoder() ? bound : nullptr;
 }
