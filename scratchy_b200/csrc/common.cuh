@@ -51,6 +51,33 @@ static inline bool scr_aligned16(const void* p) { return (reinterpret_cast<uintp
 
 static inline int scr_ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// Lets `kernel` be launched with `bytes` of dynamic shared memory.  The limit is a property of the kernel on the device, which all host threads share:
+// it is always set to all that a CTA can have beside the kernel's static arrays, so that no thread lowers it between another's setting and
+// launch.  (Those arrays' size is asked for once; the limit itself is set on every call, since a reset of the device takes it back.)
+constexpr int SCR_SMEM_BLOCK = 227 * 1024;
+static inline cudaError_t scr_smem_limit(const void* kernel, size_t bytes) {
+    static std::atomic<const void*> kernels[256];
+    static std::atomic<int> rooms[256];
+    int room = 0;
+    size_t at = (reinterpret_cast<uintptr_t>(kernel) >> 4) % 256, tries = 0;
+    for (; tries < 256; ++tries, at = (at + 1) % 256) {
+        const void* there = kernels[at].load(std::memory_order_acquire);
+        if (there == kernel) room = rooms[at].load(std::memory_order_acquire);
+        if (!there || there == kernel) break;
+    }
+    if (room == 0) {
+        cudaFuncAttributes a;
+        const cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+        if (e != cudaSuccess) return e;
+        room = SCR_SMEM_BLOCK - (int)a.sharedSizeBytes;
+        const void* none = nullptr;
+        if (tries < 256 && (kernels[at].compare_exchange_strong(none, kernel, std::memory_order_acq_rel) || none == kernel))
+            rooms[at].store(room, std::memory_order_release);
+    }
+    if (bytes > (size_t)room) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, room);
+}
+
 // ---- device-side load helpers -------------------------------------------------------
 // Streaming 128-bit / 64-bit loads for weights that are read exactly once per call:
 // read-only path, no L1 allocation.

@@ -182,7 +182,7 @@ static inline int skinny_resident(SkinnyResident& cache, void (*kernel)(KArgs...
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    if (scr_smem_limit((const void*)kernel, smem) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
         (void)cudaGetLastError();
         n = sms / split > 0 ? sms / split : 1;
@@ -236,7 +236,7 @@ static inline SkinnyPlan skinny_plan(SkinnyResident& cache, void (*kernel)(KArgs
 // One launch of `split`-CTA clusters, overlapping its start with the kernel before it.
 template <typename... KArgs, typename... Args>
 static inline cudaError_t skinny_launch(void (*kernel)(KArgs...), int tiles, int split, int threads, size_t smem, cudaStream_t stream, Args... args) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = scr_smem_limit((const void*)kernel, smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(tiles * split));
