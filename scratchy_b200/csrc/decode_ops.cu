@@ -1009,7 +1009,7 @@ cudaError_t attention_launch(const uint16_t* q, long long ld_q, const uint16_t* 
             if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
         }
         auto kernel = packed ? attention_decode_tc_kernel<D, true> : attention_decode_tc_kernel<D, false>;
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        cudaError_t e = scr_smem_limit((const void*)kernel, smem);
         if (e != cudaSuccess) return e;
         cfg.gridDim = packed ? dim3(1, num_kv_heads, bins.bins) : dim3(nsplit, num_kv_heads, batch);
         cfg.blockDim = dim3(packed ? bins.warps * 32 : nwarps * 32);
@@ -1023,7 +1023,7 @@ cudaError_t attention_launch(const uint16_t* q, long long ld_q, const uint16_t* 
     const int cap1 = max_blocks_per_seq / ATT_SPLITS + 3;
     const size_t smem = warp_part + part + size_t(cap1) * sizeof(uint32_t);
     auto kernel = attention_decode_kernel<D, G>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = scr_smem_limit((const void*)kernel, smem);
     if (e != cudaSuccess) return e;
     cfg.gridDim = dim3(ATT_SPLITS, num_kv_heads, batch);
     cfg.blockDim = dim3(ATT_THREADS);
@@ -1076,12 +1076,12 @@ static int32_t norm_launch(scr_ctx* ctx, bool add, uint16_t* residual, const uin
     if (rows == 0) return SCR_OK;
     cudaError_t e = cudaSuccess;
     if (add) {
-        if (smem > 48 * 1024) e = cudaFuncSetAttribute(rmsnorm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        if (smem > 48 * 1024) e = scr_smem_limit((const void*)rmsnorm_kernel<true>, smem);
         if (e == cudaSuccess)
             e = launch_pdl(rmsnorm_kernel<true>, dim3(rows), dim3(NORM_THREADS), smem, (cudaStream_t)stream, residual, delta, weight,
                            out, hidden, eps);
     } else {
-        if (smem > 48 * 1024) e = cudaFuncSetAttribute(rmsnorm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        if (smem > 48 * 1024) e = scr_smem_limit((const void*)rmsnorm_kernel<false>, smem);
         if (e == cudaSuccess)
             e = launch_pdl(rmsnorm_kernel<false>, dim3(rows), dim3(NORM_THREADS), smem, (cudaStream_t)stream, residual,
                            (const uint16_t*)nullptr, weight, out, hidden, eps);

@@ -679,7 +679,7 @@ extern "C" int32_t scr_rmsnorm_fp8_quant(scr_ctx* ctx, const uint16_t* x, const 
     const size_t smem = (size_t)K * sizeof(float);
     if (smem > 200 * 1024) return scr_fail(ctx, SCR_E_UNSUPPORTED, "K=%d exceeds the shared-memory row buffer", K);
     if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(fp8_rmsnorm_quant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = scr_smem_limit((const void*)fp8_rmsnorm_quant_kernel, smem);
         if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "rmsnorm_fp8_quant smem attribute: %s", cudaGetErrorString(e));
     }
     const int tiled = fp8_act_tiled(M) ? 1 : 0;
@@ -752,7 +752,7 @@ static int32_t fp8_gemv_launch(scr_ctx* ctx, const uint8_t* wpack, const uint8_t
     auto kernel = exchange ? ((split == 1) ? fp8_gemv_kernel<1, 0, 1, 1> : fp8_gemv_kernel<1, 1, 1, 1>)
                   : fuse   ? ((split == 1) ? fp8_gemv_kernel<1, 0, 1, 0> : fp8_gemv_kernel<1, 1, 1, 0>)
                            : ((split == 1) ? fp8_gemv_kernel<MT, 0, 0, 0> : fp8_gemv_kernel<MT, 1, 0, 0>);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingBytes);
+    cudaError_t e = scr_smem_limit((const void*)kernel, kRingBytes);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "fp8_gemv smem attribute: %s", cudaGetErrorString(e));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid_x, split, 1);

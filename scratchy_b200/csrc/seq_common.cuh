@@ -32,10 +32,10 @@ static inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 b
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
-// Raises a kernel's dynamic shared memory limit where a launch needs more than the default 48 KB.
+// The same where a launch needs more than the default 48 KB.
 template <typename K>
 static inline cudaError_t seq_smem(K kernel, size_t bytes) {
-    return bytes > 48 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) : cudaSuccess;
+    return bytes > 48 * 1024 ? scr_smem_limit((const void*)kernel, bytes) : cudaSuccess;
 }
 
 __device__ __forceinline__ float to_f32(float v) { return v; }

@@ -125,3 +125,24 @@ def test_few_token_linears(hammer):
     torch.cuda.synchronize()
     assert failed == 0
     assert all(torch.equal(a, b) for a, b in zip(y, want))
+
+
+def test_decode_attention(hammer):
+    """One sequence, whose CTAs are alone on their SMs, beside as many as share theirs."""
+    import torch
+    from scratchy_b200 import decode
+    made, H, G, D = [], 16, 8, 128
+    for B, length in ((1, 900), (16, 100)):
+        blocks, g = (length + 15) // 16, torch.Generator(device="cuda").manual_seed(B)
+        q, k, v = (torch.randn(s, device="cuda", generator=g).bfloat16() for s in ((B, H * D), (B * blocks, G, 16, D), (B * blocks, G, 16, D)))
+        table = torch.arange(B * blocks, dtype=torch.int32, device="cuda").reshape(B, blocks)
+        used = torch.full((B,), length, dtype=torch.int32, device="cuda")
+        want = decode.attention_via_cache(q, k, v, table, used, H, G, D, 16, 0.088)
+        made.append((q, k, v, table, used, torch.empty_like(want), torch.cuda.Stream(), want, B, blocks))
+    q, k, v, table, used, y, streams, want, batch, blocks = zip(*made)
+    torch.cuda.synchronize()
+    failed = hammer.attentions(library("scr_attention_via_cache_bf16"), ROUNDS, pointers(q), pointers(k), pointers(v), pointers(table), pointers(used),
+                               pointers(y), ints(batch), ints(blocks), H, G, D, pointers(streams))
+    torch.cuda.synchronize()
+    assert failed == 0
+    assert all(torch.equal(a, b) for a, b in zip(y, want))
