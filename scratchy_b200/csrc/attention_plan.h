@@ -52,10 +52,15 @@ static inline AttPlan att_plan(int D, int G, int batch, int num_kv_heads, int bl
     return p;
 }
 
-// More sequences than a kv head has SMs: every CTA takes whole sequences, alone on its SM, `bins` CTAs per kv head.  Dealt back and forth by falling
-// length (rank r goes to CTA r % bins in even rounds, from the other end in odd ones) the longest CTA has little more than the mean or than the longest
-// sequence.
-constexpr int ATT_MAX_ITEMS = 4;
+// Whole sequences dealt to CTAs alone on their SMs, `bins` CTAs per kv head, back and forth by falling length (rank r goes to CTA r % bins in even
+// rounds, from the other end in odd ones): the longest CTA has little more than the mean or than the longest sequence.  Only where a CTA for each
+// sequence and kv head (two to an SM) would start a second round of them, up to three sequences a CTA.  With one round the small CTAs overlap the kernels
+// before and after, which a CTA of a whole SM does not, and equally long sequences make whole rounds here: steps of the 3B Llama with 8 kv heads
+// at contexts of 2000, us packed / not, equal lengths and a quarter of it to all:  19 sequences 2208 / 1836, 1680 / 1791;  24 2290 / 2033, 1844 / 1915;
+// 32 2401 / 2347, 2041 / 2030;  37 2894 / 2546, 2205 / 2160;  38 2950 / 3111, 2232 / 2266;  48 3211 / 3326, 2587 / 2713;  52 3317 / 3381, 2689 / 2762;
+// four a CTA: 56 3796 / 3408, 2897 / 2956;  72 4126 / 4025, 3242 / 3217.  Contexts of 400: 24 1488 / 1386, 1390 / 1341;  48 1876 / 1907, 1712 / 1728.
+// (Lengths are the device's; the width of the table, which the host knows, says little of them.)
+constexpr int ATT_MAX_ITEMS = 3;
 constexpr size_t ATT_SMEM_BLOCK = 227 * 1024;          // shared memory that a CTA of sm_100a may have, dynamic and static together
 constexpr size_t ATT_SMEM_STATIC = 3 * 1024;           // of it the kernel's own arrays (AttShared, and the merge's weights) at most
 constexpr size_t ATT_SMEM_PACKED = ATT_SMEM_BLOCK - ATT_SMEM_STATIC;
@@ -75,7 +80,7 @@ struct AttBins {
 static inline AttBins att_bins(int D, int G, int batch, int num_kv_heads, int block_size, int max_blocks_per_seq, int sm_count, int nsplit) {
     AttBins p{};
     p.bins = sm_count / num_kv_heads;
-    if (nsplit > 1 || p.bins < 1 || batch <= p.bins || (batch + p.bins - 1) / p.bins > ATT_MAX_ITEMS) return p;
+    if (nsplit > 1 || (long long)batch * num_kv_heads <= 2LL * sm_count || batch > ATT_MAX_ITEMS * p.bins) return p;
     const int items = (batch + p.bins - 1) / p.bins;
     const size_t stage = size_t(block_size) * D * 4;
     p.table_cap = items * max_blocks_per_seq;

@@ -93,7 +93,7 @@ def test_packed_layout_leaves_room_for_the_static_arrays(tmp_path):
     seen = 0
     for d in (64, 128):
         for g in range(1, 9):
-            for batch in (20, 32, 36, 40, 48, 54, 72):
+            for batch in (20, 36, 38, 40, 44, 48, 52, 54, 55, 72):
                 for block in (16, 32):
                     most = call.most(d, g, batch, block, 1, 12000)
                     assert most + call.fixed_part(d) <= 227 * 1024, (d, g, batch, block, most)
@@ -107,5 +107,19 @@ def test_rotation_rows_are_aligned_for_the_loads_that_read_them(tmp_path):
     source = tmp_path / "rows.cpp"
     source.write_text('#include <stddef.h>\n#include "attention_plan.h"\n' + "".join(
         f"using S{d}_{n} = AttShared<{d}, {n}>;\nstatic_assert(alignof(S{d}_{n}) >= 8 && offsetof(S{d}_{n}, rope_rows) % 8 == 0, \"\");\n"
-        for d in (64, 128) for n in (1, 4)))
+        for d in (64, 128) for n in (1, 3)))
     subprocess.run(["g++", "-std=c++17", "-fsyntax-only", "-I", CSRC, source], check=True)
+
+
+def test_packed_only_where_single_sequences_would_start_a_second_round(tmp_path):
+    source, library = tmp_path / "bins.cpp", tmp_path / "bins.so"
+    source.write_text('#include "attention_plan.h"\nextern "C" int items(int g, int b, int h, int mb) {\n'
+                      f'    return att_bins(128, g, b, h, 16, mb, {SMS}, att_plan(128, g, b, h, 16, mb, {SMS}).nsplit).items;\n}}\n')
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, "-o", library, source], check=True)
+    items = ctypes.CDLL(str(library)).items
+    for heads in (1, 2, 4, 8, 16):
+        for blocks in (8, 128, 512):
+            for batch in range(1, 500):
+                one_round, three = batch * heads <= 2 * SMS, batch <= 3 * (SMS // heads)
+                assert (items(3, batch, heads, blocks) > 0) == (three and not one_round), (heads, batch)
+    assert items(3, 37, 8, 128) == 0 and items(3, 38, 8, 128) == 3 and items(3, 54, 8, 128) == 3 and items(3, 55, 8, 128) == 0

@@ -270,12 +270,20 @@ def test_rope_attention_one_launch_equals_the_two_operators(lens, hq, hkv, d, bs
     ([40 + (53 * i) % 500 for i in range(40)], 32, 4, 128, 16),                   # 8 query heads per kv head, 37 CTAs of a head
     ([1 + (211 * i) % 900 for i in range(30)], 24, 8, 128, 32),                   # 32-token blocks
     ([5000] + [3] * 21, 16, 8, 128, 16),                                          # one long sequence among short ones
+    ([16 * (i % 5) + 1 for i in range(38)], 24, 8, 128, 16),                      # the first number that is dealt: three in some CTAs, two in others
+    ([1 + (97 * i) % 800 for i in range(39)], 24, 8, 128, 16),
+    ([300] * 54, 16, 8, 128, 16),                                                 # three for each, equal lengths
+    ([1 + (131 * i) % 300 for i in range(55)], 16, 8, 128, 16),                   # one too many: a CTA per pair
+    ([1 + (131 * i) % 300 for i in range(48)], 8, 8, 64, 16),                     # head_dim 64
+    ([1 + (53 * i) % 200 for i in range(80)], 32, 4, 128, 16),                    # 8 query heads per kv head, 37 CTAs of a head
+    ([1 + (211 * i) % 900 for i in range(44)], 16, 8, 64, 32),                    # 32-token blocks
+    ([5000] + [3] * 40, 8, 8, 128, 16),                                           # one long sequence among short ones
 ])
 def test_attention_of_more_sequences_than_ctas(lens, hq, hkv, d, bs):
     """Whole sequences dealt to CTAs by their lengths: rings that run on from one sequence into the next, appended tokens of several
     sequences in a CTA, CTAs with fewer sequences than others."""
     test_rope_attention_one_launch_equals_the_two_operators(lens, hq, hkv, d, bs)
-    if bs == 16 and len(lens) < 40:
+    if bs == 16 and len(lens) < 49:
         test_attention_via_cache(lens[:-2] + [0, 1], hq, hkv, d, bs)
 
 
