@@ -480,25 +480,41 @@ __global__ void __launch_bounds__(CH_THREADS, 1) memory_chunk_kernel(MemoryArgs 
 struct ChPlan {
     int cols, groups, chunks;
     size_t bytes;
+    float cost;                                            // rounds of CTAs x what one of them does, in chunks of 64 columns
 };
-ChPlan ch_plan(const scr_mlstm_shape& s, const scr_step& st, int sms) {
+// A prompt cut into groups with slices of `cols` columns.  A chunk of 128 columns costs about 1.3 of 64, a group as much of a chunk again for putting its
+// state together (with a constant decay that is more beside the shorter chunk), and a round that is only begun costs less than a full one.
+inline ChPlan ch_plan_of(int cols, const scr_mlstm_shape& s, const scr_step& st, int sms, bool decay) {
     ChPlan p{};
     const int chains = s.heads * st.batch, chunks = scr_ceil_div(st.max_count, CH_L);
-    // narrow slices where the wide ones do not fit an SM, or where even all of them leave SMs idle on a short sequence
-    p.cols = s.dim > 128 || s.vdim <= 32 || (scr_ceil_div(s.vdim, 32) * chains <= sms && chunks < 8) ? 32 : 64;
-    if (p.cols == 64 && s.vdim % 128 == 0 && chunks >= 8) p.cols = 128;
-    const int ctas = scr_ceil_div(s.vdim, p.cols) * chains;
+    p.cols = cols;
+    const int ctas = scr_ceil_div(s.vdim, cols) * chains;
     p.groups = 1;
     p.chunks = chunks;
     if (chunks >= 8 && 2 * ctas <= sms * 3) {
         // the second pass costs one chunk's update again: cut to about two rounds of CTAs, groups of at least two chunks
-        p.groups = std::min(std::max(2, (p.cols == 128 ? 1 : 2) * sms / ctas), chunks / 2);
+        p.groups = std::min(std::max(2, (cols == 128 ? 1 : 2) * sms / ctas), chunks / 2);
         p.chunks = scr_ceil_div(chunks, p.groups);
         p.groups = scr_ceil_div(chunks, p.chunks);
     }
-    const size_t entry = p.cols == 128 ? ChShape<128, 8>::kEntryFloats : p.cols == 64 ? ChShape<64, 8>::kEntryFloats : s.dim > 128 ? ChShape<32, 16>::kEntryFloats : ChShape<32, 8>::kEntryFloats;
+    const size_t entry = cols == 128 ? ChShape<128, 8>::kEntryFloats : cols == 64 ? ChShape<64, 8>::kEntryFloats : s.dim > 128 ? ChShape<32, 16>::kEntryFloats : ChShape<32, 8>::kEntryFloats;
     p.bytes = p.groups > 1 ? (size_t)ctas * (p.groups + 1) * entry * sizeof(float) : 0;
+    const int rounds = scr_ceil_div(ctas * p.groups, sms);
+    const float fill = (float)(ctas * p.groups) / (float)sms - (float)(rounds - 1), state = cols == 128 ? (decay ? 0.22f : 0.08f) : 0.05f;
+    p.cost = ((float)rounds - (rounds > 1 ? 0.6f * (1.0f - fill) : 0.0f)) * ((float)p.chunks * (cols == 128 ? 1.3f : 1.0f) + (p.groups > 1 ? (float)p.groups * state : 0.0f));
     return p;
+}
+inline ChPlan ch_plan(const scr_mlstm_shape& s, const scr_step& st, int sms, bool decay) {
+    const int chains = s.heads * st.batch, chunks = scr_ceil_div(st.max_count, CH_L);
+    // narrow slices where the wide ones do not fit an SM, or where even all of them leave SMs idle on a short sequence
+    if (s.dim > 128 || s.vdim <= 32 || (scr_ceil_div(s.vdim, 32) * chains <= sms && chunks < 8)) return ch_plan_of(32, s, st, sms, decay);
+    // Slices of 128 columns share the products of queries and keys, slices of 64 fill the SMs where there are few heads for the chunks (us, 64 / 128
+    // columns, mLSTM and constant decay: 8 heads of 256, 512 tokens 28 / 40, 22 / 34, 768 49 / 43, 38 / 37, 8192 265 / 210, 207 / 178;  4 of 128,
+    // 3000 tokens 42 / 62, 32 / 54, 8192 104 / 96, 77 / 82;  12 of 256, 512 tokens 43 / 41, 33 / 35, 2000 115 / 90, 89 / 76).
+    const ChPlan narrow = ch_plan_of(64, s, st, sms, decay);
+    if (s.vdim % 128 != 0 || chunks < 8) return narrow;
+    const ChPlan wide = ch_plan_of(128, s, st, sms, decay);
+    return wide.cost < narrow.cost ? wide : narrow;
 }
 
 template <int COLS, int RTILES, ChMode MODE, bool DECAY>
@@ -533,7 +549,7 @@ bool ch_applies(const scr_mlstm_shape& s, const scr_step& st) {
 // The chunks of a step, `workspace` as `ch_plan` wants it.
 template <bool DECAY>
 int32_t ch_run(scr_ctx* ctx, const MemoryArgs& a, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
-    const ChPlan p = ch_plan(a.s, a.st, ctx->sm_count);
+    const ChPlan p = ch_plan(a.s, a.st, ctx->sm_count, DECAY);
     if (p.bytes > workspace_bytes || (p.bytes && !workspace)) return scr_fail(ctx, SCR_E_WORKSPACE, "matrix memory in %d groups needs %zu bytes", p.groups, p.bytes);
     float* ws = (float*)workspace;
     if (a.s.dim > 128) return ch_launch<32, 16, DECAY>(ctx, a, p, ws, stream);

@@ -16,11 +16,11 @@ __global__ void __launch_bounds__(256) mlstm_gates_kernel(MemoryArgs a) {
 
 bool mlstm_chunk_applies(const scr_mlstm_shape& s, const scr_step& st) { return ch_applies(s, st); }
 
-size_t mlstm_chunk_workspace(const scr_mlstm_shape& s, const scr_step& st, int sms) { return ch_plan(s, st, sms).bytes; }
+size_t mlstm_chunk_workspace(const scr_mlstm_shape& s, const scr_step& st, int sms) { return ch_plan(s, st, sms, false).bytes; }
 
 int32_t mlstm_chunk_launch(scr_ctx* ctx, const MemoryArgs& a, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
     if (a.ld % 8 || !scr_aligned16(a.proj)) return scr_fail(ctx, SCR_E_ALIGN, "mlstm projections need 16-byte rows");
-    const size_t need = ch_plan(a.s, a.st, ctx->sm_count).bytes;
+    const size_t need = ch_plan(a.s, a.st, ctx->sm_count, false).bytes;
     if (need > workspace_bytes || (need && !workspace)) return scr_fail(ctx, SCR_E_WORKSPACE, "mlstm needs %zu bytes", need);
     const cudaError_t e = launch_pdl(mlstm_gates_kernel, dim3(scr_ceil_div(a.st.rows * 2 * a.s.heads, 256)), dim3(256), 0, stream, a);
     if (e != cudaSuccess) return scr_fail(ctx, SCR_E_CUDA, "mlstm_gates: %s", cudaGetErrorString(e));

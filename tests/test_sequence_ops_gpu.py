@@ -474,6 +474,21 @@ def test_recurrence_in_portions(heads, dim, vdim, portions, dtype):
     assert (err > 4 * tol).mean() < 0.04 and err.max() < 3000 * tol, (np.median(err), np.sort(err)[-5:])
 
 
+@pytest.mark.parametrize("heads,dim,vdim,lengths", [(12, 128, 256, [1000]), (24, 32, 128, [512] * 9 + [530])])
+def test_recurrence_in_wide_slices(heads, dim, vdim, lengths):
+    """Enough heads and sequences for slices of 128 columns: in groups of chunks, and every sequence whole."""
+    m = su.memory_spec(heads, dim, vdim, gate_cap=7.0)["mixer"]
+    rng = np.random.default_rng(heads)
+    make = lambda T: (draw_memory(rng, T, m, "bfloat16"), (2.5 * rng.standard_normal((T, 2 * heads))).astype(np.float32))
+    seqs = [make(n) for n in lengths]
+    bi, bf = rng.standard_normal(heads).astype(np.float32), (2.0 + rng.standard_normal(heads)).astype(np.float32)
+    got, _ = run_memory(m, "bfloat16", [p for p, _ in seqs], [g for _, g in seqs], bi, bf, [lengths], list(range(len(lengths))))
+    for i in {0, len(lengths) - 1}:
+        want = plain_memory(m, *seqs[i], bi, bf)
+        err = np.sqrt(((head_rows(got[i], heads) - head_rows(want, heads)) ** 2).mean(axis=2)).ravel()
+        assert np.isfinite(got[i]).all() and np.median(err) < 5e-5 and (err > 8e-4).mean() < 0.04, (np.median(err), np.sort(err)[-5:])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_recurrence_with_extreme_gates(dtype):
     """Gates at their caps: long memory, instant forgetting, writes far above and far below what is remembered, and the first

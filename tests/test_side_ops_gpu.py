@@ -376,6 +376,17 @@ def test_decaying_memory_in_portions(heads, dim, vdim, portions, dtype):
     assert np.isfinite(got).all() and per_head(got, plain_lightning(m, proj), heads) < (4e-6 if dtype == "float32" else 1e-4)
 
 
+@pytest.mark.parametrize("heads,dim,vdim,lengths", [(12, 128, 256, [1000]), (24, 32, 128, [512] * 9 + [530])])
+def test_decaying_memory_in_wide_slices(heads, dim, vdim, lengths):
+    """Enough heads and sequences for slices of 128 columns: in groups of chunks, and every sequence whole."""
+    m = {"heads": heads, "dim": dim, "vdim": vdim, "decay": list(np.linspace(0.6, 0.999, heads))}
+    rng = np.random.default_rng(heads)
+    seqs = [draw(rng, (n, heads * (2 * dim + vdim)), "bfloat16") for n in lengths]
+    got, _ = run_lightning(m, "bfloat16", seqs, [lengths], list(range(len(lengths))))
+    for i in {0, len(lengths) - 1}:
+        assert np.isfinite(got[i]).all() and per_head(got[i], plain_lightning(m, seqs[i]), heads) < 1e-4
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_decays_at_their_limits(dtype):
     m = {"heads": 4, "dim": 32, "vdim": 40, "decay": [0.0, 1.0, 1e-6, 0.99999]}
