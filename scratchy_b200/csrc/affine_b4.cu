@@ -1007,7 +1007,8 @@ static int32_t affine_forward(scr_ctx* ctx, const void* packed, const uint16_t* 
     if (f.norm_gain && !scr_aligned16(f.norm_gain)) return scr_fail(ctx, SCR_E_ALIGN, "the norm gain must be 16-byte aligned");
     const uint8_t* pk = (const uint8_t*)packed;
     uint16_t* y = static_cast<uint16_t*>(y_);
-    if (M <= 16 && !f.norm_gain && affine_few_tokens(M, N, K, ctx->sm_count) && ((uintptr_t)pk & 127u) == 0 && scr_aligned16(y)) {
+    const bool norm_fits = f.out_mode != GEMV_OUT_RESIDUAL_NORM || N <= SCR_NORM_MAX_HIDDEN;       // (its norm is a launch of its own beside the GEMM)
+    if (M <= 16 && !f.norm_gain && norm_fits && affine_few_tokens(M, N, K, ctx->sm_count) && ((uintptr_t)pk & 127u) == 0 && scr_aligned16(y)) {
         if (affine_b4_skinny_applies(M, N, K, ctx->sm_count)) {
             const int out = f.out_mode == GEMV_OUT_RESIDUAL_NORM ? GEMV_OUT_RESIDUAL_ADD : f.out_mode;
             st = affine_b4_skinny_launch(ctx, pk, x, y, M, N, K, f.gs, out, f.bias, f.scale, stream);

@@ -78,6 +78,8 @@ static inline cudaError_t scr_smem_limit(const void* kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, room);
 }
 
+constexpr int SCR_NORM_MAX_HIDDEN = 200 * 1024 / 4;      // features that scr_rmsnorm_bf16 holds in shared memory
+
 // ---- device-side load helpers -------------------------------------------------------
 // Streaming 128-bit / 64-bit loads for weights that are read exactly once per call:
 // read-only path, no L1 allocation.

@@ -1072,7 +1072,7 @@ static int32_t norm_launch(scr_ctx* ctx, bool add, uint16_t* residual, const uin
     DEC_REQUIRE(scr_aligned16(residual) && scr_aligned16(weight) && scr_aligned16(out) && (!add || scr_aligned16(delta)),
                 SCR_E_ALIGN, "rmsnorm: pointer not 16-byte aligned");
     const size_t smem = size_t(hidden) * sizeof(float);
-    DEC_REQUIRE(smem <= 200 * 1024, SCR_E_UNSUPPORTED, "rmsnorm: hidden=%d exceeds the shared-memory row buffer", hidden);
+    DEC_REQUIRE(hidden <= SCR_NORM_MAX_HIDDEN, SCR_E_UNSUPPORTED, "rmsnorm: hidden=%d exceeds the shared-memory row buffer", hidden);
     if (rows == 0) return SCR_OK;
     cudaError_t e = cudaSuccess;
     if (add) {

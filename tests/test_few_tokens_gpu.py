@@ -128,6 +128,25 @@ def test_int4_ends_of_few_tokens(N, K, group, M):
     torch.cuda.synchronize()
 
 
+@pytest.mark.parametrize("N", [51200, 51208])
+def test_residual_and_norm_of_rows_wider_than_a_norm_takes(N):
+    """The residual end with the norm behind it: rows up to what the stand-alone norm holds, whose launch follows the GEMM, and wider ones, which
+    only the matvec's epilogue normalises."""
+    import torch
+    from scratchy_b200 import AffineQuantLinear
+    K, M = 128, 9
+    w, s, b = synth.affine_int4_weights(N, K, 64, synth.seed_for("wide-norm", N))
+    layer = AffineQuantLinear.from_tensors(u32_dev(w), bf16_dev(s), bf16_dev(b), 64, 4)
+    x, res0 = bf16_dev(synth.activations_bf16(M, K, 1)).reshape(M, K), bf16_dev(synth.activations_bf16(M, N, 2)).reshape(M, N)
+    gain, res, normed = bf16_dev(synth.activations_bf16(1, N, 3)).reshape(N), res0.clone(), torch.full_like(res0, float("nan"))
+    layer.forward_residual_rmsnorm(x, res, gain, 1e-5, normed, torch.zeros(AffineQuantLinear.ENDS_SCRATCH_BYTES, dtype=torch.uint8, device="cuda"))
+    want = res0.double() + (x.double() @ layer.dequantize().double().T).bfloat16().double()
+    assert float((res.double() - want).norm() / want.norm()) < 4e-3                       # one bf16 rounding, a few of the product's the other way
+    r = res.double()
+    want = r / torch.sqrt((r * r).mean(dim=1, keepdim=True) + 1e-5) * gain.double()
+    assert float((normed.double() - want).norm() / want.norm()) < 4e-3
+
+
 @pytest.mark.parametrize("tiles", [147, 148, 149, 300])
 def test_calls_whose_clusters_do_not_all_run_at_once(tiles):
     """As many tiles of 128 channels as SMs, where every CTA has its SM and memory for the sums to itself, and more, where two share an
