@@ -964,7 +964,6 @@ int32_t affine_b4_gemm_tc_launch(scr_ctx* ctx, const uint8_t* packed, const uint
 size_t affine_b4_gemm_tc_workspace(int M, int N, int K);
 bool affine_b4_gemm_tc_enabled();
 // Defined in affine_b4_skinny.cu
-bool affine_b4_skinny_applies(int M, int N, int K, int sms);
 int32_t affine_b4_skinny_launch(scr_ctx* ctx, const uint8_t* packed, const uint16_t* x, uint16_t* y, int M, int N, int K, int gs, int out,
                                 const uint16_t* bias, float scale, cudaStream_t stream);
 // Tokens up to which the GEMM for few tokens takes every matrix and has the residual and gate/up ends.
@@ -1009,14 +1008,10 @@ static int32_t affine_forward(scr_ctx* ctx, const void* packed, const uint16_t* 
     uint16_t* y = static_cast<uint16_t*>(y_);
     const bool norm_fits = f.out_mode != GEMV_OUT_RESIDUAL_NORM || N <= SCR_NORM_MAX_HIDDEN;       // (its norm is a launch of its own beside the GEMM)
     if (M <= 16 && !f.norm_gain && norm_fits && affine_few_tokens(M, N, K, ctx->sm_count) && ((uintptr_t)pk & 127u) == 0 && scr_aligned16(y)) {
-        if (affine_b4_skinny_applies(M, N, K, ctx->sm_count)) {
-            const int out = f.out_mode == GEMV_OUT_RESIDUAL_NORM ? GEMV_OUT_RESIDUAL_ADD : f.out_mode;
-            st = affine_b4_skinny_launch(ctx, pk, x, y, M, N, K, f.gs, out, f.bias, f.scale, stream);
-            if (st || out == f.out_mode) return st;
-            return scr_rmsnorm_bf16(ctx, f.ends->residual, f.ends->gain, f.ends->normed, M, N, f.ends->eps, stream);
-        }
-        if ((f.out_mode == GEMV_OUT_BF16 || f.out_mode == GEMV_OUT_F32) && f.scale == 1.0f)
-            return affine_b4_gemm_tc_launch(ctx, pk, x, y, M, N, K, f.gs, f.out_mode == GEMV_OUT_F32, f.bias, nullptr, 0, stream);
+        const int out = f.out_mode == GEMV_OUT_RESIDUAL_NORM ? GEMV_OUT_RESIDUAL_ADD : f.out_mode;
+        st = affine_b4_skinny_launch(ctx, pk, x, y, M, N, K, f.gs, out, f.bias, f.scale, stream);
+        if (st || out == f.out_mode) return st;
+        return scr_rmsnorm_bf16(ctx, f.ends->residual, f.ends->gain, f.ends->normed, M, N, f.ends->eps, stream);
     }
     if (M <= 8) return affine_gemv_launch<1>(ctx, pk, x, y, M, N, K, f, stream);
     if (M <= 16) return affine_gemv_launch<2>(ctx, pk, x, y, M, N, K, f, stream);
