@@ -68,6 +68,7 @@ template <int D, int ITEMS>
 struct AttShared {
     alignas(16) float rope_rows[ITEMS][2][D / 2];      // cos and sin of the sequences' positions; read two at a time
     int item_seq[ATT_MAX_ITEMS], item_len[ATT_MAX_ITEMS];
+    unsigned item_pos[ITEMS];                          // the positions that the rows belong to
 };
 struct AttMergeShared {
     float wgt[8][ATT_MAX_WARPS + 2];                   // per query head: the warps' weights, the merged maximum and sum

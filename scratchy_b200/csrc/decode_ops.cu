@@ -759,12 +759,14 @@ __global__ void __launch_bounds__(ATT_MAX_WARPS * 32) attention_decode_tc_kernel
         // lane n fills stage n: the lanes issue side by side, and q's loads below are not held up behind them
         const bool waits = !rope.enabled && index_of(lane) < w_hi && is_newest(index_of(lane));
         if (lane < spw && !waits) load(lane);
-        // The rotation's rows, which follow from what the host wrote for the step, come in while the kernel before runs (two loads one after the
-        // other; one sequence of 2048 tokens 7.8 -> 7.5 us, 8 13.7 -> 13.0).
+        // The rotation's rows come in while the kernel before runs (two loads one after the other; one sequence of 2048 tokens 7.8 -> 7.5 us, 8
+        // 13.7 -> 13.0): their positions follow from what the host wrote for the step.  Where a kernel that is still running writes one
+        // all the same, it differs after the wait, and the rows are read again.
         if (rope.enabled)
             for (int i = threadIdx.x; i < ng * (D / 2); i += int(blockDim.x)) {
                 const int g = i / (D / 2), d = i - g * (D / 2), seq = PACKED ? item_seq[g] : b;
                 const uint32_t pos = seq >= 0 ? rope.positions[seq] : rope.max_pos;
+                if (d == 0) shared.item_pos[g] = pos;
                 rope_rows[g][0][d] = pos < rope.max_pos ? rope.cos_table[size_t(pos) * D + d] : 0.0f;
                 rope_rows[g][1][d] = pos < rope.max_pos ? rope.sin_table[size_t(pos) * D + d] : 0.0f;
             }
@@ -790,6 +792,7 @@ __global__ void __launch_bounds__(ATT_MAX_WARPS * 32) attention_decode_tc_kernel
         const int table0 = PACKED ? at - total_blk : 0;
         const int newest_blk = total_blk - 1;
         const int row = lane >> 2, quad = lane & 3;
+        const uint32_t pos = rope.enabled ? __ldcg(rope.positions + b) : 0;    // (past L1, which may hold what was there before the wait)
         uint32_t qa0[KSTEPS], qa2[KSTEPS];             // A fragments of Q: row = query head (zero beyond G), 16 dims per step
 #pragma unroll
         for (int kk = 0; kk < KSTEPS; ++kk) {
@@ -801,7 +804,13 @@ __global__ void __launch_bounds__(ATT_MAX_WARPS * 32) attention_decode_tc_kernel
             }
         }
         if (rope.enabled) {
-            const uint32_t pos = rope.positions[b];
+            if (pos != shared.item_pos[g]) {                               // (every warp for itself, with the same values)
+                for (int d = lane; d < D / 2; d += 32) {
+                    rope_rows[g][0][d] = pos < rope.max_pos ? rope.cos_table[size_t(pos) * D + d] : 0.0f;
+                    rope_rows[g][1][d] = pos < rope.max_pos ? rope.sin_table[size_t(pos) * D + d] : 0.0f;
+                }
+                __syncwarp();
+            }
             if (pos >= rope.max_pos) {
                 if (lane == 0) atomicCAS(status, 0, DEV_BAD_POSITION);
             } else if (row < G) {
@@ -841,7 +850,6 @@ __global__ void __launch_bounds__(ATT_MAX_WARPS * 32) attention_decode_tc_kernel
             if (rope.enabled && first_blk + i == newest_blk) {
                 // the newest token: rotate k_new, write it and v_new to the cache slot and into this tile
                 const int slot = kv_len - 1 - t0;
-                const uint32_t pos = rope.positions[b];
                 const size_t cache_off = ((size_t(blocks[table0 + i]) * num_kv_heads + kvh) * block_size + slot) * D;
                 unsigned char* ktile = ring + size_t(s) * 2 * chunk;
                 // a block id outside the cache was replaced by 0 for the loads (and reported): never append there

@@ -296,6 +296,42 @@ def test_attention_with_wide_block_tables(batch, hq, hkv, d, width):
     assert rel_l2(got, want) <= REL_L2_TOL
 
 
+@pytest.mark.parametrize("batch,length", [(1, 200), (6, 300), (24, 90), (40, 60)])
+def test_positions_that_the_kernel_before_writes(batch, length):
+    """The call may start while the kernel before it on the stream still runs, and reads its positions early; the ones that count are those that are
+    there when that kernel is done.  Here it is a greedy sampling over wide rows, which lets its dependents start at once and stores late."""
+    import torch
+    from scratchy_b200 import _lib, decode
+    hq, hkv, d, bs, width = 16, 8, 128, 16, 400000
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    blocks = -(-length // bs)
+    new = lambda *s: torch.randn(s, device="cuda", generator=g).bfloat16()
+    qkv, ck, cv = new(batch, (hq + 2 * hkv) * d), new(batch * blocks, hkv, bs, d), new(batch * blocks, hkv, bs, d)
+    q, k, v = qkv[:, :hq * d], qkv[:, hq * d:(hq + hkv) * d], qkv[:, (hq + hkv) * d:]
+    cos, sin = (torch.randn((512, d), device="cuda", generator=g) for _ in range(2))
+    table, used = torch.arange(batch * blocks, dtype=torch.int32, device="cuda").reshape(batch, blocks), torch.full((batch,), length, dtype=torch.int32, device="cuda")
+    want_pos = (torch.arange(batch, device="cuda") * 37 + 11) % 512
+    logits = torch.zeros((batch, width), dtype=torch.bfloat16, device="cuda")
+    logits[torch.arange(batch, device="cuda"), want_pos] = 1.0
+    call = lambda pos, a, b: decode.rope_attention_via_cache(q, k, v, pos, cos, sin, a, b, table, used, hq, hkv, d, bs, d ** -0.5)
+    a, b = ck.clone(), cv.clone()
+    want = call(want_pos.to(torch.int32), a, b)
+    positions, k2, v2, graph = torch.zeros(batch, dtype=torch.int32, device="cuda"), ck.clone(), cv.clone(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):      # (the two launches without the host between them)
+        decode.argmax(logits, out=positions)
+        got = call(positions, k2, v2)
+    for _ in range(8):
+        positions.fill_(500)
+        k2.copy_(ck)
+        v2.copy_(cv)
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16)) and torch.equal(k2, a) and torch.equal(v2, b)
+    _lib.context(0).device_status(None)
+
+
 def test_rope_attention_refuses_what_it_cannot_stream():
     """Blocks that are not a multiple of 16 tokens have no one-launch form: the call says so and touches nothing."""
     import torch
