@@ -105,7 +105,9 @@ int32_t scr_affine_b4_embed(scr_ctx* ctx, const void* packed, const uint32_t* id
  * kernel pickers (crates/targets/metal/src/tape/quantized.rs:130-157,403-426,563-595):
  *   y[M,N] (bf16) = x[M,K] (bf16) @ dequant(W)[N,K]^T, f32 accumulation, one rounding,
  * the contraction of `cpu_reference::affine_qmm_t_b4` (crates/targets/metal/src/cpu_reference.rs:107-137).
- * The kernel is chosen from M (matvec for M <= 16, tensor-core GEMM above).
+ * The kernel is chosen from M, N and K: up to 16 tokens the matvec or, where the matrix is large for them (9 tokens from 4M weights on,
+ * 5 from 40M, 3 where there are very many rows), the tensor-core GEMM for few tokens; tensor-core GEMMs above.  They add in
+ * different orders: calls on either side of a choice agree to the rounding of the f32 sums, not bit for bit.
  * `bias_bf16` (may be NULL) is the linear's own bias [N], the `{prefix}.bias` tensor the loader
  * takes (crates/targets/metal/src/layers_quant.rs:318-351): it is added in f32 before the one
  * rounding, as the reference's matvec epilogue does (the `QmvEnds.bias` end,
@@ -121,9 +123,10 @@ int32_t scr_linear_affine_b4(scr_ctx* ctx, const void* packed, const uint16_t* x
 /* Up to 4 independent linears over the SAME activations — q, k, v of a layer; gate and up — as ONE launch: what the
  * reference gets by fusing the projections at load time (`load_rows_concat`, crates/targets/metal/src/layers_quant.rs:363-450)
  * without re-laying the weights.  Every member keeps its own packed buffer (`packed[i]`, [N[i], K]) and its own output
- * (`y[i]`, [M, N[i]] bf16); all share K, the group size and x.  Same bits per member as `scr_linear_affine_b4`.  Up to
- * 16 tokens one matvec launch runs over all members' rows; above, the members run one after the other (`workspace` as
- * for `scr_linear_affine_b4` at the largest member). */
+ * (`y[i]`, [M, N[i]] bf16); all share K, the group size and x.  Up to 16 tokens one matvec launch runs over all members'
+ * rows: a member's bits are those of `scr_linear_affine_b4` where that runs the matvec too and both launches cut k alike, otherwise
+ * equal to the rounding of the f32 sums.  Above, the members run one after the other (`workspace` as for
+ * `scr_linear_affine_b4` at the largest member), with its bits. */
 int32_t scr_linear_affine_b4_group(scr_ctx* ctx, int32_t count, const void* const* packed, const uint16_t* x_bf16,
                                    int32_t M, const int32_t* N, int32_t K, int32_t group, uint16_t* const* y_bf16,
                                    void* workspace, size_t workspace_bytes, void* stream);
@@ -132,7 +135,8 @@ int32_t scr_linear_affine_b4_group(scr_ctx* ctx, int32_t count, const void* cons
  *   out[M, N2/2] (bf16) = silu(bf16(x @ gate^T)) * bf16(x @ up^T)
  * for a matrix of N2 rows that holds, per block of 16 rows, 8 gate rows then the 8 up rows of the
  * same channels (the Python mirror's `load_rows_interleave8`).  One launch; M <= 16 only
- * (SCR_E_UNSUPPORTED above: run `scr_linear_affine_b4` and `scr_silu_mul_pairs8_bf16`). */
+ * (SCR_E_UNSUPPORTED above: `scr_linear_affine_b4_few_ends` up to 64 tokens, `scr_linear_affine_b4` and
+ * `scr_silu_mul_pairs8_bf16` beyond). */
 int32_t scr_linear_affine_b4_silu_mul(scr_ctx* ctx, const void* packed, const uint16_t* x_bf16,
                                       int32_t M, int32_t N2, int32_t K, int32_t group,
                                       uint16_t* out_bf16, void* stream);
@@ -142,7 +146,8 @@ int32_t scr_linear_affine_b4_silu_mul(scr_ctx* ctx, const void* packed, const ui
  * on the output side, the gate/up pairing of `scr_linear_affine_b4_silu_mul`.  Up to 16 tokens (SCR_E_UNSUPPORTED above).
  *   norm_gain != NULL   x is the INPUT of an RMSNorm whose gain this is: every CTA normalises the rows into shared
  *                       memory as it loads them, with the arithmetic and summation order of `scr_rmsnorm_bf16`
- *                       (cpu_golden.rs:25-37), so the result is the bits of that operator followed by the plain linear
+ *                       (cpu_golden.rs:25-37), so the result is the bits of that operator followed by the matvec: by the
+ *                       plain linear, except where that takes the GEMM for few tokens (equal to the rounding of the sums then)
  *                       (the reference's fused kernel keeps x * gain in f32 instead, one rounding away from its own
  *                       unfused path).  Up to 8 tokens and M * K * 2 <= 20 KiB.
  *   bias, scale         sum + bias[n], then * scale, in f32 before the one rounding (scale 0 is read as 1)
@@ -150,7 +155,7 @@ int32_t scr_linear_affine_b4_silu_mul(scr_ctx* ctx, const void* packed, const ui
  *                       (`fused_add_rmsnorm`'s residual, cpu_golden.rs:171-200)
  *   silu_pairs          the gate/up pairing (N = fused rows, y is [M, N/2]); excludes bias, scale and residual
  *   norm_row_scale      with `norm_gain`, which arithmetic the norm-in end uses.  0: the normalised row is formed and rounded
- *                       to bf16 exactly as `scr_rmsnorm_bf16` stores it, then dotted — the bits of the two separate operators,
+ *                       to bf16 exactly as `scr_rmsnorm_bf16` stores it, then dotted — the bits of that operator and the matvec,
  *                       at the price of every CTA finishing the row's sum of squares before its first product.  Non-zero: the
  *                       reference matvec's own form (crates/targets/metal/tests/affine_qmv_ends_test.rs:6-9, "dots x (.) gain
  *                       and scales the row by 1 / rms(x), so it skips the normed row's rounding"): the dot runs over
@@ -179,12 +184,14 @@ int32_t scr_linear_affine_b4_few_ends(scr_ctx* ctx, const void* packed, const ui
                                       void* stream);
 
 /* The o / down projection with the residual add and the following RMSNorm folded in (the reference's
- * `QmvEnds` residual end, step.rs:472-482, and `fused_add_rmsnorm`, cpu_golden.rs:171-200), one launch:
+ * `QmvEnds` residual end, step.rs:472-482, and `fused_add_rmsnorm`, cpu_golden.rs:171-200), one call:
  *   residual[M,N] <- bf16(residual + bf16(x @ W^T));  normed[M,N] <- rmsnorm(residual, gain, eps)
- * The last CTA to finish normalises the rows (partial sums of squares are added in CTA order:
- * deterministic).  `scratch`: SCR_ENDS_SCRATCH_BYTES of device memory, zeroed once by the caller before
+ * In the matvec, one launch, the last CTA to finish normalises the rows (partial sums of squares are added in CTA
+ * order: deterministic); a matrix that takes the GEMM for few tokens (`scr_linear_affine_b4`) takes its residual end and
+ * `scr_rmsnorm_bf16` after it, two launches.  `scratch`: SCR_ENDS_SCRATCH_BYTES of device memory, zeroed once by the caller before
  * the first call and left zeroed; calls that may overlap on the GPU need their own.  M <= 16 only
- * (SCR_E_UNSUPPORTED above: run `scr_linear_affine_b4` and `scr_fused_add_rmsnorm_bf16`); N % 8 == 0. */
+ * (SCR_E_UNSUPPORTED above: run `scr_linear_affine_b4` and `scr_fused_add_rmsnorm_bf16`, or up to 64 tokens
+ * `scr_linear_affine_b4_few_ends` and `scr_rmsnorm_bf16`); N % 8 == 0. */
 #define SCR_ENDS_SCRATCH_BYTES 65536
 int32_t scr_linear_affine_b4_residual_rmsnorm(scr_ctx* ctx, const void* packed, const uint16_t* x_bf16,
                                               int32_t M, int32_t N, int32_t K, int32_t group,
@@ -278,7 +285,8 @@ int32_t scr_linear_fp8_dynamic(scr_ctx* ctx, const void* packed, const uint16_t*
  * (crates/compiler/subtile/src/tensor_parallel.rs:508-625): these variants write the UNROUNDED
  * f32 sums [M,N] instead of bf16, the caller all-reduces them over the ranks (the reference's
  * meaning: a sum in rank order, tensor_parallel.rs:1350-1362) and rounds once with
- * `scr_partial_to_bf16`.  Same arguments otherwise as `scr_linear_affine_b4` / `scr_linear_fp8`. */
+ * `scr_partial_to_bf16`.  Same arguments and kernels otherwise as `scr_linear_affine_b4` / `scr_linear_fp8`: the sums that those
+ * round.  (From exact ones they are 1e-7 of their norm off in the matvec and up to 1e-5 in the tensor cores' accumulators, which truncate.) */
 int32_t scr_linear_affine_b4_partial(scr_ctx* ctx, const void* packed, const uint16_t* x_bf16,
                                      int32_t M, int32_t N, int32_t K, int32_t group, float* y_f32,
                                      void* workspace, size_t workspace_bytes, void* stream);
@@ -317,7 +325,8 @@ int32_t scr_silu_mul_bf16(scr_ctx* ctx, const uint16_t* gate, const uint16_t* up
                           uint16_t* out, int32_t rows, int32_t inter, void* stream);
 /* The same on a fused gate/up output whose columns interleave gate and up in runs of 8 (8 gate
  * columns, then the 8 up columns of the same channels) — the row order `scr_linear_affine_b4_silu_mul`
- * expects of its matrix; used above 16 tokens, where that fused epilogue is not available. */
+ * expects of its matrix; used above 64 tokens, where no linear has that pairing in its epilogue (17 to 64:
+ * `scr_linear_affine_b4_few_ends`). */
 int32_t scr_silu_mul_pairs8_bf16(scr_ctx* ctx, const uint16_t* gate_up, int64_t ld_in, uint16_t* out,
                                  int32_t rows, int32_t inter, void* stream);
 /* `rope_append` (cpu_golden.rs:289-362): NeoX pairing, f32 cos/sin tables [max_pos, head_dim]
@@ -354,7 +363,9 @@ int32_t scr_attention_via_cache_bf16(scr_ctx* ctx, const uint16_t* q, int64_t ld
  * slot of token seq_used_k[b] - 1 of sequence b (block block_table[b][(seq_used_k[b]-1) /
  * block_size], i.e. the slot the reference's slot_mapping names for that token), and attends over
  * the seq_used_k[b] tokens including it.  q is left unrotated.  The cache contents and `out` are
- * the same bits as the two separate calls give.  Needs block_size a multiple of 16 (<= 256);
+ * the same bits as the two separate calls give.  The previous kernels of the stream may produce q, k, v and
+ * positions; block_table and seq_used_k are the host's as above, and so are the rotation tables.  Needs
+ * block_size a multiple of 16 (<= 256);
  * SCR_E_UNSUPPORTED otherwise — call the two operators separately then. */
 int32_t scr_rope_attention_via_cache_bf16(scr_ctx* ctx, const uint16_t* q, int64_t ld_q,
                                           const uint16_t* k, int64_t ld_k, const uint16_t* v,

@@ -35,8 +35,8 @@ struct A4SCfg {
     static constexpr int kSA = TN == 128 ? 4 : 3;                                       // stages of activations (128 k) and of dequantised weights in TMEM (64
                                                                         //   columns each beside the accumulator): one a group, and one pair
                                                                         //   of barriers for both
-    static constexpr int kSP = TN == 128 ? 8 : 6;                       // packed-weight stages, a multiple of four: a stage always belongs
-                                                                        //   to the same group, whose waits take its phases in order
+    static constexpr int kSP = TN == 128 ? 8 : 6;                       // packed-weight stages, even: a stage always belongs to the
+                                                                        //   same of the two groups, whose waits take its phases in order
     static constexpr uint32_t kACol = TN < 32 ? 32 : TN, kTmemCols = TN == 128 ? 512 : 256;
     static constexpr uint32_t kXStage = TN * 256u;                      // 2 atoms of TN rows x 128 B
     static constexpr uint32_t kPOff = kSA * kXStage;

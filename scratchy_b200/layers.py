@@ -297,7 +297,8 @@ class AffineQuantLinear:
     @staticmethod
     def forward_group(layers, x: torch.Tensor, outs=None, workspace: Optional[torch.Tensor] = None):
         """Up to 4 linears over the SAME activations (q, k, v; gate, up) as one launch (`scr_linear_affine_b4_group`): each
-        keeps its own packed buffer and gets its own output, the bits of `forward` per member.  Returns the outputs."""
+        keeps its own packed buffer and gets its own output: `forward`'s bits where that runs the matvec and both launches cut k
+        alike, else equal to the rounding of the f32 sums.  Returns the outputs."""
         layers = list(layers)
         if not 1 <= len(layers) <= 4:
             raise ValueError(f"a group holds 1 to 4 linears, got {len(layers)}")
@@ -333,7 +334,7 @@ class AffineQuantLinear:
         input as it is loaded (`norm_gain`: x is the norm's INPUT), the layer's bias, a scale, and either the add into the
         residual stream `out` (`residual`) or the gate/up pairing (`silu_pairs`, a matrix built by `load_rows_interleave8`).
         `norm_row_scale`: the reference matvec's own norm-in arithmetic (dot over `x * gain`, the row scaled by `1 / rms(x)`;
-        crates/targets/metal/tests/affine_qmv_ends_test.rs:6-9) instead of the bits of the separate RMSNorm."""
+        crates/targets/metal/tests/affine_qmv_ends_test.rs:6-9) instead of the bits of the separate RMSNorm and the matvec."""
         x2 = x.reshape(-1, self.in_features).contiguous()
         M = int(x2.shape[0])
         dev = x2.device
@@ -369,7 +370,7 @@ class AffineQuantLinear:
     def forward_residual_rmsnorm(self, x: torch.Tensor, residual: torch.Tensor, gain: torch.Tensor, eps: float,
                                  normed: torch.Tensor, scratch: torch.Tensor,
                                  delta: Optional[torch.Tensor] = None, workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """`residual += x @ W^T` (in place, bf16) and `normed = rmsnorm(residual, gain)`: one launch up to 16 tokens
+        """`residual += x @ W^T` (in place, bf16) and `normed = rmsnorm(residual, gain)`: one call up to 16 tokens
         (`scr_linear_affine_b4_residual_rmsnorm`; `scratch` = ENDS_SCRATCH_BYTES, zeroed once by the caller), the
         linear into `delta` followed by `scr_fused_add_rmsnorm_bf16` above."""
         if self.linear_bias is not None:

@@ -526,7 +526,7 @@ def test_two_cta_gemm_gives_the_bits_of_the_one_cta_kernel(tmp_path):
     assert rel_l2(pair.reshape(M, N)[rows], want) <= REL_L2_TOL
 
 
-@pytest.mark.parametrize("M", [1, 3, 8, 16, 40])
+@pytest.mark.parametrize("M", [1, 3, 8, 9, 16, 40])
 @pytest.mark.parametrize("ns,K", [((3072, 1024, 1024), 3072), ((8192, 8192), 3072), ((24, 136, 8, 40), 320), ((3072,), 8192)])
 def test_group_launch_gives_each_member_the_bits_of_its_own_launch(ns, K, M):
     """`scr_linear_affine_b4_group`: q, k, v (or gate, up) over the same activations in one launch.  A member's summation
@@ -549,6 +549,21 @@ def test_group_launch_gives_each_member_the_bits_of_its_own_launch(ns, K, M):
         assert rel_l2(got, alone) <= 1e-4 and np.mean(got == alone) > 0.98
     from scratchy_b200 import _lib
     _lib.context(0).device_status(None)
+
+
+@pytest.mark.parametrize("N,K,M", [(76008, 512, 3), (16384, 2560, 4), (41008, 1024, 6)])
+def test_norm_in_beside_the_linear_of_a_large_matrix(N, K, M):
+    """The rounded-row norm-in end is the norm and the matvec; the plain linear of such a matrix goes to the GEMM for few tokens at some of these
+    counts (many rows from 3 tokens on, 40M weights from 5).  Bits where it does not, equal to the rounding of the sums where it does."""
+    import torch
+    from scratchy_b200 import decode
+    w, s, b = synth.affine_int4_weights(N, K, 64, synth.seed_for("norm-in-large", N, K))
+    layer = make_layer(w, s, b)
+    x, gain = bf16_dev(synth.activations_bf16(M, K, 1)).reshape(M, K), bf16_dev(synth.f32_to_bf16_bits(np.linspace(0.5, 1.5, K).astype(np.float32)))
+    got = bits_of(layer.forward_ends(x, torch.empty((M, N), dtype=torch.bfloat16, device="cuda"), norm_gain=gain, norm_eps=1e-5))
+    plain = bits_of(layer.forward(decode.rmsnorm(x, gain, 1e-5)))
+    assert rel_l2(got, plain) <= 1e-4 and np.mean(got == plain) > 0.98
+    assert N != 16384 or np.array_equal(got, plain)
 
 
 def test_group_launch_refusals():

@@ -246,11 +246,13 @@ def test_matvec_that_quantises_by_itself_leaves_the_workspace_alone(N, K, M):
     assert all(np.array_equal(o, outs[0]) for o in outs)
 
 
-@pytest.mark.parametrize("N,K,M", [(2056, 2048, 3), (1224, 3432, 4), (8200, 3840, 1), (2048, 15368, 5), (8192, 3848, 8), (4104, 3080, 9), (12296, 1032, 16),
-                                   (6144, 6144, 8), (6144, 8192, 1), (18944, 2048, 6)])        # (left to the matvec: an uneven cut, whole rounds of tiles)
+@pytest.mark.parametrize("N,K,M", [(2048, 15368, 1), (2048, 15368, 5), (8192, 3848, 8), (4104, 3080, 9), (12296, 1032, 16),
+                                   (6144, 6144, 8), (18944, 2048, 6),                                              # (left to the matvec: an uneven cut, whole rounds of tiles)
+                                   (2056, 2048, 3), (1224, 3432, 4), (8200, 3840, 1), (6144, 8192, 1)])            # (and where that quantises by itself)
 def test_few_tokens_that_the_call_quantises_for_the_gemm(N, K, M):
     """Dynamic linears of up to 16 tokens whose matrix is large enough for the GEMM for few tokens, in a workspace of the size that the query
-    names, at both kinds of row ends; without the workspace for it the matvec runs.  Against the oracle, bias and partial sums as well."""
+    names, at both kinds of row ends; with a workspace that only holds the pack the matvec runs, with the bits of the two calls.  Against the oracle, bias
+    and partial sums as well."""
     import torch
     from scratchy_b200 import Fp8Linear
     seed = synth.seed_for("few16", N, K, M)
@@ -260,6 +262,10 @@ def test_few_tokens_that_the_call_quantises_for_the_gemm(N, K, M):
     want = oracle.fp8_dynamic_linear(x, wq, ws, M, N, K)
     work = torch.full((layer.workspace_bytes(M),), 0x7F, dtype=torch.uint8, device="cuda")         # NaN codes in the rows past the last token
     y = layer.forward(xd, workspace=work)
+    pack = Fp8Linear.quantize_activation(xd)
+    small, two = torch.empty_like(y), layer.forward_quantized(pack)
+    dynamic(layer, xd, small, torch.empty(-(-pack.buf.numel() // 128) * 128, dtype=torch.uint8, device="cuda"))
+    assert np.array_equal(bits_of(small), bits_of(two)) and rel_l2(bits_of(small).reshape(M, N), want) <= REL_L2_TOL
     part = layer.forward_partial(xd)
     bias = bf16_dev(synth.activations_bf16(1, N, seed + 2)).reshape(N)
     layer.linear_bias = bias
