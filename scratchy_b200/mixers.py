@@ -279,26 +279,28 @@ class WindowAttention:
 
     def run(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], memory, out: torch.Tensor) -> None:
         """`out`: the gated heads [rows, heads * dim], dense rows of any stride."""
-        self.prepare(ctx, bufs, memory)
-        self.attend(ctx, bufs, memory, out)
+        call = self.call(ctx, bufs)
+        self.prepare(call, bufs, memory)
+        self.attend(call, bufs, memory, out)
 
-    def _call(self, ctx: StepContext, bufs: Dict[str, torch.Tensor]):
-        qk = bufs[f"{self.prefix}.qk"]
+    def call(self, ctx: StepContext, bufs: Dict[str, torch.Tensor]):
+        """What a step's `prepare` and `attend` share; a short prompt's step is bound by what the host does for its launches."""
+        device = bufs[f"{self.prefix}.qk"].device
         q = ctx.arena.get("wa.q", (ctx.rows, self.heads * self.dim), self.dtype)
-        return (_lib.models_lib(), _lib.models_context(_dev_index(qk.device)), dtype_code(self.dtype), ctypes.byref(self.shape(ctx)), ctypes.byref(ctx.step),
-                _stream(qk.device), q)
+        return (_lib.models_lib(), _lib.models_context(_dev_index(device)), dtype_code(self.dtype), ctypes.byref(self.shape(ctx)), ctypes.byref(ctx.step),
+                _stream(device), _ptr(q), q)
 
-    def prepare(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], memory) -> None:
+    def prepare(self, call, bufs: Dict[str, torch.Tensor], memory) -> None:
         """Queries, and the step's rows in the cache."""
         qk, (cache, inv, rows) = bufs[f"{self.prefix}.qk"], memory
-        lib, c, code, ps, pt, stream, q = self._call(ctx, bufs)
-        c.check(lib.scr_window_prepare(c.handle, code, ps, pt, _ptr(qk), int(qk.stride(0)), _ptr(self.conv), _ptr(self.norm), _ptr(rows), _ptr(q), _ptr(cache),
+        lib, c, code, ps, pt, stream, q, _ = call
+        c.check(lib.scr_window_prepare(c.handle, code, ps, pt, _ptr(qk), int(qk.stride(0)), _ptr(self.conv), _ptr(self.norm), _ptr(rows), q, _ptr(cache),
                                        _ptr(inv), stream))
 
-    def attend(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], memory, out: torch.Tensor) -> None:
+    def attend(self, call, bufs: Dict[str, torch.Tensor], memory, out: torch.Tensor) -> None:
         gate, (cache, inv, _) = bufs[f"{self.prefix}.g"], memory
-        lib, c, code, ps, pt, stream, q = self._call(ctx, bufs)
-        c.check(lib.scr_window_attention(c.handle, code, ps, pt, _ptr(q), _ptr(cache), _ptr(inv), _ptr(self.bias), _ptr(gate), int(gate.stride(0)), _ptr(out),
+        lib, c, code, ps, pt, stream, q, _ = call
+        c.check(lib.scr_window_attention(c.handle, code, ps, pt, q, _ptr(cache), _ptr(inv), _ptr(self.bias), _ptr(gate), int(gate.stride(0)), _ptr(out),
                                          int(out.stride(0)), stream))
 
 
@@ -339,32 +341,33 @@ class LightningAttention:
         return torch.zeros((slots, self.heads, self.dim, self.vdim), dtype=torch.float32, device=device)
 
     def run(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], memory: torch.Tensor, out: torch.Tensor) -> None:
-        self.remember(ctx, bufs, memory)
-        self.read(ctx, bufs, out)
+        call = self.call(ctx, bufs)
+        self.remember(call, bufs, memory)
+        self.read(call, bufs, out)
 
-    def remember(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], memory: torch.Tensor, beside: bool = False) -> None:
+    def call(self, ctx: StepContext, bufs: Dict[str, torch.Tensor]):
+        """What a step's `remember` and `read` share."""
+        device = bufs[f"{self.prefix}.qkv"].device
+        lib, c, code = _lib.models_lib(), _lib.models_context(_dev_index(device)), dtype_code(self.dtype)
+        shape, step = ctypes.byref(_lib.LightningShape(self.heads, self.dim, self.vdim, self.eps, self.out_scale)), ctypes.byref(ctx.step)
+        o, need = ctx.arena.get("li.out", (ctx.rows, self.out_features), torch.float32), ctypes.c_size_t(0)
+        c.check(lib.scr_lightning_workspace(code, shape, step, ctypes.byref(need)))
+        ws = ctx.arena.get("li.workspace", (need.value,), torch.uint8) if need.value else None
+        return lib, c, code, shape, step, _stream(device), _ptr(o), o, _ptr(ws), ws, need
+
+    def remember(self, call, bufs: Dict[str, torch.Tensor], memory: torch.Tensor, beside: bool = False) -> None:
         """The memory's step.  `beside`: the call directly before is a window attention's `prepare`, which it may run beside."""
         qkv = bufs[f"{self.prefix}.qkv"]
-        lib, c = _lib.models_lib(), _lib.models_context(_dev_index(qkv.device))
-        code, stream = dtype_code(self.dtype), _stream(qkv.device)
-        shape = _lib.LightningShape(self.heads, self.dim, self.vdim, self.eps, self.out_scale)
-        o = ctx.arena.get("li.out", (ctx.rows, self.out_features), torch.float32)
-        need = ctypes.c_size_t(0)
-        c.check(lib.scr_lightning_workspace(code, ctypes.byref(shape), ctypes.byref(ctx.step), ctypes.byref(need)))
-        ws = ctx.arena.get("li.workspace", (need.value,), torch.uint8) if need.value else None
+        lib, c, code, shape, step, stream, o, _, ws, _, need = call
         run = lib.scr_lightning_beside if beside else lib.scr_lightning_run
-        c.check(run(c.handle, code, ctypes.byref(shape), ctypes.byref(ctx.step), _ptr(qkv), int(qkv.stride(0)), _ptr(self.powers), _ptr(memory),
-                    _ptr(o), _ptr(ws), need, stream))
+        c.check(run(c.handle, code, shape, step, _ptr(qkv), int(qkv.stride(0)), _ptr(self.powers), _ptr(memory), o, ws, need, stream))
 
-    def read(self, ctx: StepContext, bufs: Dict[str, torch.Tensor], out: torch.Tensor, beside: bool = False) -> None:
+    def read(self, call, bufs: Dict[str, torch.Tensor], out: torch.Tensor, beside: bool = False) -> None:
         """The readouts' norm and gate.  `beside`: the call directly before is a window attention's `attend`."""
         gate = bufs[f"{self.prefix}.g"]
-        lib, c = _lib.models_lib(), _lib.models_context(_dev_index(gate.device))
-        shape = _lib.LightningShape(self.heads, self.dim, self.vdim, self.eps, self.out_scale)
-        o = ctx.arena.get("li.out", (ctx.rows, self.out_features), torch.float32)
+        lib, c, code, shape, _, stream, o, kept, _, _, _ = call
         finish = lib.scr_lightning_finish_beside if beside else lib.scr_lightning_finish
-        c.check(finish(c.handle, dtype_code(self.dtype), ctypes.byref(shape), _ptr(o), _ptr(self.norm), _ptr(gate), int(gate.stride(0)), ctx.rows, _ptr(out),
-                       int(out.stride(0)), _stream(gate.device)))
+        c.check(finish(c.handle, code, shape, o, _ptr(self.norm), _ptr(gate), int(gate.stride(0)), int(kept.shape[0]), _ptr(out), int(out.stride(0)), stream))
 
 
 class GeluGlu:
@@ -420,13 +423,14 @@ class SideBySide:
             lo, hi = self.columns[-1]
             bufs[f"{self.mlp.prefix}.act"] = rows[:, lo:hi]
         self.inp.run(a, h, bufs)
-        outs = [rows[:, lo:hi] for lo, hi in self.columns]
+        outs = [rows[:, lo:hi] for lo, hi in self.columns[:len(self.mixers)]]
         if [type(m) for m in self.mixers] == [WindowAttention, LightningAttention]:
             (window, lightning), (cache, state) = self.mixers, memory
-            window.prepare(ctx, bufs, cache)                  # a CTA per row: the memory runs beside it
-            lightning.remember(ctx, bufs, state, beside=True)
-            window.attend(ctx, bufs, cache, outs[0])          # and its readouts' norm beside this
-            lightning.read(ctx, bufs, outs[1], beside=True)
+            attention, decaying = window.call(ctx, bufs), lightning.call(ctx, bufs)
+            window.prepare(attention, bufs, cache)            # a CTA per row: the memory runs beside it
+            lightning.remember(decaying, bufs, state, beside=True)
+            window.attend(attention, bufs, cache, outs[0])    # and its readouts' norm beside this
+            lightning.read(decaying, bufs, outs[1], beside=True)
         else:
             for m, mem, out in zip(self.mixers, memory, outs):
                 m.run(ctx, bufs, mem, out)

@@ -83,6 +83,30 @@ def run_cut(model, tokens, portions, name="s", close=True):
     return np.concatenate(out)
 
 
+@pytest.mark.parametrize("name", ["side_by_side", "mixed_loop"])
+def test_a_layer_sets_up_its_calls_once(name):
+    """A short prompt takes as long as the host needs for its launches: what a layer's calls share (step buffers, the library's context, shapes) is
+    looked up once for each part of the layer."""
+    from scratchy_b200 import mixers
+    cfg, _, model = built(name, "bfloat16")
+    runs, asked, contexts = len(cfg["layers"]) * (cfg.get("loop") or {"times": 1})["times"], {}, [0]
+    get, context = model.arena.get, mixers._lib.models_context
+    model.arena.get = lambda key, *a: (asked.__setitem__(key, asked.get(key, 0) + 1), get(key, *a))[1]
+
+    def counted(device):
+        contexts[0] += 1
+        return context(device)
+    mixers._lib.models_context = counted
+    try:
+        run_cut(model, su.tokens_of(cfg, 20), [20])
+    finally:
+        del model.arena.get
+        mixers._lib.models_context = context
+    mixing = {k: n for k, n in asked.items() if k.startswith(("wa.", "li.", "mm.", "la."))}
+    assert mixing and all(n <= runs for n in mixing.values()), mixing
+    assert contexts[0] <= 12 * runs + 12, contexts
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("name", sorted(CONFIGS))
 def test_whole_prompt_and_every_layer(name, dtype):
