@@ -970,7 +970,9 @@ int32_t affine_b4_skinny_launch(scr_ctx* ctx, const uint8_t* packed, const uint1
 constexpr int AFFINE_FEW_ENDS = 64;
 // Whether a call of up to 16 tokens goes to the GEMM for few tokens, whose time hardly grows with them, or to the matvec, which has the shorter
 // launch.  us in streams of calls, matvec / GEMM:
-//   1024 x 1024, 16 tokens 2.7 / 3.1;  2048 x 2048, 9 tokens 3.9 / 3.7, 16 4.4 / 3.8;  4096 x 1280, 9 tokens 3.6 / 4.0, 16 4.3 / 4.1
+//   1024 x 1024, 16 tokens 2.7 / 3.1;  2048 x 2048, 9 tokens 3.9 / 3.7, 16 4.4 / 3.8
+//   a short k whose row-blocks fit the GPU in one round, two to an SM: 4096 x 1024, 9 tokens 2.9 / 3.9, 16 3.4 / 4.0;  4096 x 1280, 9 tokens 3.6 / 4.2, 14 4.1 / 4.2;
+//   4736 x 1280, 14 tokens 4.2 / 4.3;  4800 x 1024 (a second round), 9 tokens 3.7 / 4.0, 12 4.2 / 4.0;  4096 x 1536, 9 tokens 3.7 / 4.2, 14 4.3 / 4.3;  3072 x 1536, 9 tokens 4.0 / 3.7
 //   3072 x 3072, 9 tokens 5.3 / 4.9;  5120 x 3072, 8 tokens 4.9 / 5.4, 9 7.7 / 5.6;  3072 x 8192, 16 tokens 12.5 / 7.0
 //   16384 x 3072, 4 tokens 10.8 / 10.3, 5 10.0 / 9.8, 8 12.0 / 10.0, 16 20.1 / 9.9;  24576 x 3072 (more tiles than SMs), 5 tokens 13.7 / 16.2,
 //   8 15.9 / 16.2, 9 21.9 / 16.5;  128256 x 3072, 2 tokens 54.2 / 51, 4 59.2 / 51.4, 8 67.1 / 51.8
@@ -979,7 +981,11 @@ constexpr int AFFINE_FEW_ENDS = 64;
 static bool affine_few_tokens(int M, int N, int K, int sms) {
     const long long weights = (long long)N * K;
     const int tiles = affine_geom(N, K, 64).RB / 8;
-    if (M > 8) return weights >= 4 << 20;
+    if (M > 8) {
+        const int rb = scr_ceil_div(N, 16);
+        const bool short_round = rb <= 2 * sms && (K <= 1024 || (M <= 14 && (K <= 1280 || (K <= 1536 && 2 * rb > 3 * sms))));
+        return weights >= 4 << 20 && !short_round;
+    }
     if (tiles >= 4 * sms) return M > 2;
     return M > 4 && weights >= 40 << 20 && tiles <= sms;
 }

@@ -92,7 +92,7 @@ def test_fp8(N, K, M):
 
 
 @pytest.mark.parametrize("M", [5, 8, 9, 16, 17, 33, 64])
-@pytest.mark.parametrize("N,K,group", [(2064, 2048, 64), (4160, 1024, 32), (16400, 2560, 128)])
+@pytest.mark.parametrize("N,K,group", [(2064, 2048, 64), (4160, 1024, 32), (16400, 2560, 128), (4736, 1024, 64), (3600, 1536, 64)])
 def test_int4_ends_of_few_tokens(N, K, group, M):
     """The ends of the GEMM for few tokens on both sides of the matvec's sizes: bias and scale, the residual add and the gate/up pairing
     give the bits of the plain linear followed by the operator; the plain linear is held to the oracle."""
