@@ -363,9 +363,9 @@ int32_t scr_attention_via_cache_bf16(scr_ctx* ctx, const uint16_t* q, int64_t ld
  * slot of token seq_used_k[b] - 1 of sequence b (block block_table[b][(seq_used_k[b]-1) /
  * block_size], i.e. the slot the reference's slot_mapping names for that token), and attends over
  * the seq_used_k[b] tokens including it.  q is left unrotated.  The cache contents and `out` are
- * the same bits as the two separate calls give.  The previous kernels of the stream may produce q, k, v and
- * positions; block_table and seq_used_k are the host's as above, and so are the rotation tables.  Needs
- * block_size a multiple of 16 (<= 256);
+ * the same bits as the two separate calls give.  The previous kernels of the stream may produce q, k, v,
+ * positions and the rotation tables; block_table and seq_used_k are the host's as above.  Needs block_size a
+ * multiple of 16 (<= 256);
  * SCR_E_UNSUPPORTED otherwise — call the two operators separately then. */
 int32_t scr_rope_attention_via_cache_bf16(scr_ctx* ctx, const uint16_t* q, int64_t ld_q,
                                           const uint16_t* k, int64_t ld_k, const uint16_t* v,

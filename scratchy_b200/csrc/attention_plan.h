@@ -62,13 +62,10 @@ static inline AttPlan att_plan(int D, int G, int batch, int num_kv_heads, int bl
 // (Lengths are the device's; the width of the table, which the host knows, says little of them.)
 constexpr int ATT_MAX_ITEMS = 3;
 constexpr size_t ATT_SMEM_BLOCK = 227 * 1024;          // shared memory that a CTA of sm_100a may have, dynamic and static together
-constexpr size_t ATT_SMEM_STATIC = 3 * 1024;           // of it the kernel's own arrays (AttShared, and the merge's weights) at most
+constexpr size_t ATT_SMEM_STATIC = 1024;               // of it the kernel's own arrays (AttShared, and the merge's weights) at most
 constexpr size_t ATT_SMEM_PACKED = ATT_SMEM_BLOCK - ATT_SMEM_STATIC;
-template <int D, int ITEMS>
 struct AttShared {
-    alignas(16) float rope_rows[ITEMS][2][D / 2];      // cos and sin of the sequences' positions; read two at a time
     int item_seq[ATT_MAX_ITEMS], item_len[ATT_MAX_ITEMS];
-    unsigned item_pos[ITEMS];                          // the positions that the rows belong to
 };
 struct AttMergeShared {
     float wgt[8][ATT_MAX_WARPS + 2];                   // per query head: the warps' weights, the merged maximum and sum

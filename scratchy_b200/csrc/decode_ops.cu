@@ -558,8 +558,8 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_kernel(
 //
 // What bounds it: HBM (8 KB per block of 16 tokens and kv head), and the longest sequence's CTA.  Llama-3.2-3B at 32 sequences of
 // 512 to 2048 tokens, 153 MB per call, in a stream of calls: 57.6 us with the producer warp and a second MMA for the remainders,
-// 40.9 us with rings of the warps' own and a CTA for every sequence and kv head, 37.9 (4.0 TB/s) with two copies a block and the rotation's rows
-// ahead of the wait; all of 2048 44.3 us (6.1 TB/s).  Whole sequences dealt to one CTA per SM (PACKED; their blocks in even shares to the warps)
+// 40.9 us with rings of the warps' own and a CTA for every sequence and kv head, 37.9 (4.0 TB/s) with two copies a block;
+// all of 2048 44.3 us (6.1 TB/s).  Whole sequences dealt to one CTA per SM (PACKED; their blocks in even shares to the warps)
 // are faster in such a stream, 31.6, but not between the kernels of a step (attention_plan.h): 48 sequences, which take them, 62.4 -> 48.3 us, all of 2048 81.9 -> 67.9.
 constexpr int ATT_ERR_FULL = 0x0A000001;
 
@@ -648,11 +648,9 @@ __global__ void __launch_bounds__(ATT_MAX_WARPS * 32) attention_decode_tc_kernel
     }
     uint64_t* bars = reinterpret_cast<uint64_t*>(blocks + ((table_cap + 1) & ~1));                // full[stages]
     int* lens = reinterpret_cast<int*>(bars + stages);                                            // PACKED: [batch]
-    using Shared = AttShared<D, PACKED ? ATT_MAX_ITEMS : 1>;
-    static_assert(sizeof(Shared) + sizeof(AttMergeShared) + 512 <= ATT_SMEM_STATIC, "what att_bins leaves for the static arrays");
-    __shared__ Shared shared;
+    __shared__ AttShared shared;                                           // PACKED
     auto &item_seq = shared.item_seq, &item_len = shared.item_len;
-    auto& rope_rows = shared.rope_rows;
+    static_assert(sizeof(AttShared) + sizeof(AttMergeShared) + 512 <= ATT_SMEM_STATIC, "what att_bins leaves for the static arrays");
 
     pdl_trigger();
     uint32_t nsplit;
@@ -759,20 +757,9 @@ __global__ void __launch_bounds__(ATT_MAX_WARPS * 32) attention_decode_tc_kernel
         // lane n fills stage n: the lanes issue side by side, and q's loads below are not held up behind them
         const bool waits = !rope.enabled && index_of(lane) < w_hi && is_newest(index_of(lane));
         if (lane < spw && !waits) load(lane);
-        // The rotation's rows come in while the kernel before runs (two loads one after the other; one sequence of 2048 tokens 7.8 -> 7.5 us, 8
-        // 13.7 -> 13.0): their positions follow from what the host wrote for the step.  Where a kernel that is still running writes one
-        // all the same, it differs after the wait, and the rows are read again.
-        if (rope.enabled)
-            for (int i = threadIdx.x; i < ng * (D / 2); i += int(blockDim.x)) {
-                const int g = i / (D / 2), d = i - g * (D / 2), seq = PACKED ? item_seq[g] : b;
-                const uint32_t pos = seq >= 0 ? rope.positions[seq] : rope.max_pos;
-                if (d == 0) shared.item_pos[g] = pos;
-                rope_rows[g][0][d] = pos < rope.max_pos ? rope.cos_table[size_t(pos) * D + d] : 0.0f;
-                rope_rows[g][1][d] = pos < rope.max_pos ? rope.sin_table[size_t(pos) * D + d] : 0.0f;
-            }
         pdl_wait();
         if (lane < spw && waits) load(lane);
-        __syncthreads();
+        __syncwarp();
         int j = 0, at = 0;                             // the warp's blocks so far; where this sequence's blocks start
         for (int g = 0; g < ng; ++g) {
         int i0 = warp, i1 = nblk;                      // the warp's blocks of this sequence
@@ -792,7 +779,6 @@ __global__ void __launch_bounds__(ATT_MAX_WARPS * 32) attention_decode_tc_kernel
         const int table0 = PACKED ? at - total_blk : 0;
         const int newest_blk = total_blk - 1;
         const int row = lane >> 2, quad = lane & 3;
-        const uint32_t pos = rope.enabled ? __ldcg(rope.positions + b) : 0;    // (past L1, which may hold what was there before the wait)
         uint32_t qa0[KSTEPS], qa2[KSTEPS];             // A fragments of Q: row = query head (zero beyond G), 16 dims per step
 #pragma unroll
         for (int kk = 0; kk < KSTEPS; ++kk) {
@@ -804,31 +790,20 @@ __global__ void __launch_bounds__(ATT_MAX_WARPS * 32) attention_decode_tc_kernel
             }
         }
         if (rope.enabled) {
-            if (pos != shared.item_pos[g]) {                               // (every warp for itself, with the same values)
-                for (int d = lane; d < D / 2; d += 32) {
-                    rope_rows[g][0][d] = pos < rope.max_pos ? rope.cos_table[size_t(pos) * D + d] : 0.0f;
-                    rope_rows[g][1][d] = pos < rope.max_pos ? rope.sin_table[size_t(pos) * D + d] : 0.0f;
-                }
-                __syncwarp();
-            }
+            const uint32_t pos = rope.positions[b];
             if (pos >= rope.max_pos) {
                 if (lane == 0) atomicCAS(status, 0, DEV_BAD_POSITION);
             } else if (row < G) {
-                const uint32_t rows = smem_u32(&rope_rows[g][0][0]);
+                const float* cs = rope.cos_table + size_t(pos) * D;
+                const float* sn = rope.sin_table + size_t(pos) * D;
 #pragma unroll
                 for (int kk = 0; kk < KSTEPS / 2; ++kk) {
                     const int d = kk * 16 + quad * 2;                      // < D/2; partner dim d + D/2 sits KSTEPS/2 steps on
-                    float cs[2][2], sn[2][2];                              // (volatile: all of a row's at once would cost 34 registers)
-#pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(cs[x][0]), "=f"(cs[x][1]) : "r"(rows + 4u * (d + 8 * x)));
-                        asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(sn[x][0]), "=f"(sn[x][1]) : "r"(rows + 4u * (D / 2 + d + 8 * x)));
-                    }
                     const uint32_t a0 = qa0[kk], b0 = qa0[kk + KSTEPS / 2], a2 = qa2[kk], b2 = qa2[kk + KSTEPS / 2];
-                    qa0[kk] = att_rope_pair(a0, b0, cs[0], sn[0], true);
-                    qa0[kk + KSTEPS / 2] = att_rope_pair(a0, b0, cs[0], sn[0], false);
-                    qa2[kk] = att_rope_pair(a2, b2, cs[1], sn[1], true);
-                    qa2[kk + KSTEPS / 2] = att_rope_pair(a2, b2, cs[1], sn[1], false);
+                    qa0[kk] = att_rope_pair(a0, b0, cs + d, sn + d, true);
+                    qa0[kk + KSTEPS / 2] = att_rope_pair(a0, b0, cs + d, sn + d, false);
+                    qa2[kk] = att_rope_pair(a2, b2, cs + d + 8, sn + d + 8, true);
+                    qa2[kk + KSTEPS / 2] = att_rope_pair(a2, b2, cs + d + 8, sn + d + 8, false);
                 }
             }
         }
@@ -850,6 +825,7 @@ __global__ void __launch_bounds__(ATT_MAX_WARPS * 32) attention_decode_tc_kernel
             if (rope.enabled && first_blk + i == newest_blk) {
                 // the newest token: rotate k_new, write it and v_new to the cache slot and into this tile
                 const int slot = kv_len - 1 - t0;
+                const uint32_t pos = rope.positions[b];
                 const size_t cache_off = ((size_t(blocks[table0 + i]) * num_kv_heads + kvh) * block_size + slot) * D;
                 unsigned char* ktile = ring + size_t(s) * 2 * chunk;
                 // a block id outside the cache was replaced by 0 for the loads (and reported): never append there
@@ -858,7 +834,8 @@ __global__ void __launch_bounds__(ATT_MAX_WARPS * 32) attention_decode_tc_kernel
                     const int d = lane * 8;                                // dims d..d+7 pair with d + D/2 ..
                     const uint16_t* kp = rope.k_new + b * rope.ld_k + size_t(kvh) * D;
                     const uint4 x0 = *reinterpret_cast<const uint4*>(kp + d), x1 = *reinterpret_cast<const uint4*>(kp + d + D / 2);
-                    const float *cs = rope_rows[g][0] + d, *sn = rope_rows[g][1] + d;
+                    const float* cs = rope.cos_table + size_t(pos) * D + d;
+                    const float* sn = rope.sin_table + size_t(pos) * D + d;
                     const uint32_t xw0[4] = {x0.x, x0.y, x0.z, x0.w}, xw1[4] = {x1.x, x1.y, x1.z, x1.w};
                     uint32_t r0[4], r1[4];
 #pragma unroll
