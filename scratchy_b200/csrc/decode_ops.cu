@@ -622,10 +622,11 @@ __device__ __forceinline__ uint32_t att_rope_pair(uint32_t x0w, uint32_t x1w, co
 
 // PACKED: a CTA has its SM to itself and takes one to `items` whole sequences of a kv head, so that all CTAs have about as much to read
 // (attention_plan.h): the sequences, ranked by their lengths on the device, are dealt to the gridDim.z CTAs back and forth.  The warps' rings run on
-// from one sequence into the next, and the sequences' partial sums meet at the end.  Registers: at most 168 (ATT_MAX_WARPS in the bounds), so that two
-// half-SM CTAs of six warps fit; at 173 8 sequences took 21.2 us for 13.0.
+// from one sequence into the next, and the sequences' partial sums meet at the end.  Registers with heads of 128: at most 168 (ATT_MAX_WARPS in the
+// bounds), so that two half-SM CTAs of six warps fit; at 173 8 sequences took 21.2 us for 13.0.  Heads of 64 need 128 and are scheduled worse under that
+// bound: 16 sequences of up to 6000 tokens 34.1 us, 38.3 with it.
 template <int D, bool PACKED>
-__global__ void __launch_bounds__(ATT_MAX_WARPS * 32) attention_decode_tc_kernel(
+__global__ void __launch_bounds__(PACKED || D > 64 ? ATT_MAX_WARPS * 32 : ATT_THREADS) attention_decode_tc_kernel(
     const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, const uint16_t* __restrict__ q,
     long long ld_q, const uint32_t* __restrict__ block_table, const uint32_t* __restrict__ seq_used_k,
     uint16_t* __restrict__ out, long long ld_o, int G, int num_kv_heads, int block_size, int max_blocks_per_seq,
