@@ -54,13 +54,15 @@ static inline AttPlan att_plan(int D, int G, int batch, int num_kv_heads, int bl
 
 // Whole sequences dealt to CTAs alone on their SMs, `bins` CTAs per kv head, back and forth by falling length (rank r goes to CTA r % bins in even
 // rounds, from the other end in odd ones): the longest CTA has little more than the mean or than the longest sequence.  Only where a CTA for each
-// sequence and kv head (two to an SM) would start a second round of them, up to three sequences a CTA.  With one round the small CTAs overlap the kernels
+// sequence and kv head (two to an SM, three of those with heads of 64 and a narrow table: 40 sequences of 64 tokens 5.0 us, dealt 9.8, of 300 8.2 and 11.5, but of 1000,
+// where they are two, 21.9 and 18.4) would start a second round of them, up to three sequences a CTA.  With one round the small CTAs overlap the kernels
 // before and after, which a CTA of a whole SM does not, and equally long sequences make whole rounds here: steps of the 3B Llama with 8 kv heads
 // at contexts of 2000, us packed / not, equal lengths and a quarter of it to all:  19 sequences 2208 / 1836, 1680 / 1791;  24 2290 / 2033, 1844 / 1915;
 // 32 2401 / 2347, 2041 / 2030;  37 2894 / 2546, 2205 / 2160;  38 2950 / 3111, 2232 / 2266;  48 3211 / 3326, 2587 / 2713;  52 3317 / 3381, 2689 / 2762;
 // four a CTA: 56 3796 / 3408, 2897 / 2956;  72 4126 / 4025, 3242 / 3217.  Contexts of 400: 24 1488 / 1386, 1390 / 1341;  48 1876 / 1907, 1712 / 1728.
 // (Lengths are the device's; the width of the table, which the host knows, says little of them.)
 constexpr int ATT_MAX_ITEMS = 3;
+constexpr size_t ATT_SMEM_SM = 228 * 1024;             // shared memory of an SM; each of its CTAs costs 1 KB beside its own
 constexpr size_t ATT_SMEM_BLOCK = 227 * 1024;          // shared memory that a CTA of sm_100a may have, dynamic and static together
 constexpr size_t ATT_SMEM_STATIC = 1024;               // of it the kernel's own arrays (AttShared, and the merge's weights) at most
 constexpr size_t ATT_SMEM_PACKED = ATT_SMEM_BLOCK - ATT_SMEM_STATIC;
@@ -78,7 +80,10 @@ struct AttBins {
 static inline AttBins att_bins(int D, int G, int batch, int num_kv_heads, int block_size, int max_blocks_per_seq, int sm_count, int nsplit) {
     AttBins p{};
     p.bins = sm_count / num_kv_heads;
-    if (nsplit > 1 || (long long)batch * num_kv_heads <= 2LL * sm_count || batch > ATT_MAX_ITEMS * p.bins) return p;
+    const AttPlan one = att_plan(D, G, batch, num_kv_heads, block_size, max_blocks_per_seq, sm_count);
+    const size_t ring = size_t(one.warps) * one.stages_per_warp * block_size * D * 4, part = size_t(one.warps) * G * (D + 2) * sizeof(float);
+    const long long per_sm = (long long)(ATT_SMEM_SM / ((ring > part ? ring : part) + one.fixed + ATT_SMEM_STATIC + 1024));
+    if (nsplit > 1 || (long long)batch * num_kv_heads <= per_sm * sm_count || batch > ATT_MAX_ITEMS * p.bins) return p;
     const int items = (batch + p.bins - 1) / p.bins;
     const size_t stage = size_t(block_size) * D * 4;
     p.table_cap = items * max_blocks_per_seq;

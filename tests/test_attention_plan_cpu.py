@@ -111,4 +111,10 @@ def test_packed_only_where_single_sequences_would_start_a_second_round(tmp_path)
             for batch in range(1, 500):
                 one_round, three = batch * heads <= 2 * SMS, batch <= 3 * (SMS // heads)
                 assert (items(3, batch, heads, blocks) > 0) == (three and not one_round), (heads, batch)
+    source.write_text('#include "attention_plan.h"\nextern "C" int items(int g, int b, int h, int mb) {\n'
+                      f'    return att_bins(64, g, b, h, 16, mb, {SMS}, 1).items;\n}}\n')
+    narrow = tmp_path / "narrow.so"
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, "-o", narrow, source], check=True)
+    heads64 = ctypes.CDLL(str(narrow)).items                  # three CTAs to an SM up to 23 blocks, two beyond
+    assert heads64(4, 48, 8, 19) == 0 and heads64(4, 48, 8, 63) == 3 and heads64(4, 37, 8, 63) == 0
     assert items(3, 37, 8, 128) == 0 and items(3, 38, 8, 128) == 3 and items(3, 54, 8, 128) == 3 and items(3, 55, 8, 128) == 0
