@@ -12,6 +12,9 @@ constexpr int ATT_MAX_STAGES = 24;
 constexpr size_t ATT_SMEM_BUDGET = 110 * 1024;
 constexpr size_t ATT_SMEM_BUDGET_ALONE = 200 * 1024;
 
+// The partial sums that the CTAs of a cluster leave with its first one.
+static inline size_t att_cluster_part(int D, int G, int nsplit) { return nsplit > 1 ? size_t(nsplit) * G * (D + 2) * sizeof(float) : 0; }
+
 struct AttPlan {
     int nsplit;                                        // CTAs that share a sequence and kv head
     int warps, stages_per_warp;                        // of the streaming kernel; no stages: the blocks do not fit it
@@ -22,14 +25,13 @@ struct AttPlan {
 static inline AttPlan att_plan(int D, int G, int batch, int num_kv_heads, int block_size, int max_blocks_per_seq, int sm_count) {
     AttPlan p;
     const size_t chunk = size_t(block_size) * D * 2;
-    const size_t part = size_t(ATT_SPLITS) * G * (D + 2) * sizeof(float);
     p.nsplit = ATT_SPLITS;                             // the most splits that still run as a single wave of two CTAs per SM
     while (p.nsplit > 1 && (long long)batch * num_kv_heads * p.nsplit > 2LL * sm_count) p.nsplit /= 2;
     // (Halving sequences for the width of their table, so that none is waited for alone, was measured and is not done: the width is a
     // capacity and not a length, and clusters of two start later.  32 sequences of 500 to 2048 tokens, in a stream of such calls, 39.7 us
     // whole and 41.1 halved, of 250 to 1000 in a table of 2048 21.6 and 33.2; 20 of 500 to 2048 36.9 and 30.2.)
     p.table_cap = max_blocks_per_seq / p.nsplit + 2;
-    p.fixed = part + size_t((p.table_cap + 1) & ~1) * 4 + ATT_MAX_STAGES * 8 + 1024 + 128;
+    p.fixed = att_cluster_part(D, G, p.nsplit) + size_t((p.table_cap + 1) & ~1) * 4 + ATT_MAX_STAGES * 8 + 1024 + 128;
     // alone on its SM: 8 warps and a deep ring; otherwise 4 or 6 warps and about half an SM's shared
     // memory.  The big CTA (48 K registers, ~200 KB) shares its SM with no CTA of the kernels before and after it in
     // the stream, so it pays only while the grid leaves most SMs to them: up to half the SMs.  (Llama-3.2-3B decode
@@ -38,8 +40,9 @@ static inline AttPlan att_plan(int D, int G, int batch, int num_kv_heads, int bl
     // and wants at least two of them, so that its next block loads while it works on the current one.
     const bool alone = 2LL * batch * num_kv_heads * p.nsplit <= sm_count;
     const size_t budget = alone ? ATT_SMEM_BUDGET_ALONE : ATT_SMEM_BUDGET;
-    // Six warps of two stages where a CTA has four blocks or more for each and they fit (the table of the cluster's sums grows with
-    // the query heads: beside it, 16-token blocks of 128 leave room for six up to 3 query heads per kv head), otherwise four of three
+    // Six warps of two stages where a CTA has four blocks or more for each and they fit (beside the cluster's sums, which grow with the query heads and
+    // which one CTA a sequence does without: with room kept for eight CTAs' sums all the same, tables of 129 blocks and more of 3 query heads left four
+    // warps, and a step of the 3B Llama at 32 sequences of up to 2048 tokens took 2168 us), otherwise four of three
     // (16 sequences of up to 2048 tokens 23.9 us with four warps, 20.8 with six; 4 sequences, 16 blocks a CTA, 13.0 and 14.6).
     // Large blocks: two, with one stage each if it must be.
     const int most = alone ? 8 : max_blocks_per_seq / p.nsplit >= 24 ? 6 : 4;
@@ -82,7 +85,8 @@ static inline AttBins att_bins(int D, int G, int batch, int num_kv_heads, int bl
     p.bins = sm_count / num_kv_heads;
     const AttPlan one = att_plan(D, G, batch, num_kv_heads, block_size, max_blocks_per_seq, sm_count);
     const size_t ring = size_t(one.warps) * one.stages_per_warp * block_size * D * 4, part = size_t(one.warps) * G * (D + 2) * sizeof(float);
-    const long long per_sm = (long long)(ATT_SMEM_SM / ((ring > part ? ring : part) + one.fixed + ATT_SMEM_STATIC + 1024));
+    const long long by_smem = (long long)(ATT_SMEM_SM / ((ring > part ? ring : part) + one.fixed + ATT_SMEM_STATIC + 1024));
+    const long long by_regs = 65536 / (one.warps * 32 * (D > 64 ? 168 : 128)), per_sm = by_smem < by_regs ? by_smem : by_regs;
     if (nsplit > 1 || (long long)batch * num_kv_heads <= per_sm * sm_count || batch > ATT_MAX_ITEMS * p.bins) return p;
     const int items = (batch + p.bins - 1) / p.bins;
     const size_t stage = size_t(block_size) * D * 4;

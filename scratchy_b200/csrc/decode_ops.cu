@@ -642,7 +642,9 @@ __global__ void __launch_bounds__(PACKED || D > 64 ? ATT_MAX_WARPS * 32 : ATT_TH
     float* warp_part = reinterpret_cast<float*>(ring);                     // aliases the ring once it is drained
     const size_t ring_bytes = PACKED ? size_t(stages) * 2 * chunk : max(size_t(stages) * 2 * chunk, size_t(nwarps) * G * STATE * sizeof(float));
     float* cl_part = reinterpret_cast<float*>(ring + ((ring_bytes + 127) & ~size_t(127)));        // [nsplit<=8][G][STATE]
-    uint32_t* blocks = reinterpret_cast<uint32_t*>(cl_part + ATT_SPLITS * G * STATE);
+    uint32_t nsplit;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(nsplit));
+    uint32_t* blocks = reinterpret_cast<uint32_t*>(cl_part + (nsplit > 1 ? int(nsplit) * G * STATE : 0));
     if (PACKED) {                                                          // sums of their own: [item][warp][G][STATE]
         warp_part = cl_part;
         blocks = reinterpret_cast<uint32_t*>(warp_part + size_t(items) * nwarps * G * STATE);
@@ -654,8 +656,6 @@ __global__ void __launch_bounds__(PACKED || D > 64 ? ATT_MAX_WARPS * 32 : ATT_TH
     static_assert(sizeof(AttShared) + sizeof(AttMergeShared) + 512 <= ATT_SMEM_STATIC, "what att_bins leaves for the static arrays");
 
     pdl_trigger();
-    uint32_t nsplit;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(nsplit));
     const int split = int(att_cluster_rank());
     const int kvh = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
