@@ -105,8 +105,8 @@ int32_t scr_affine_b4_embed(scr_ctx* ctx, const void* packed, const uint32_t* id
  * kernel pickers (crates/targets/metal/src/tape/quantized.rs:130-157,403-426,563-595):
  *   y[M,N] (bf16) = x[M,K] (bf16) @ dequant(W)[N,K]^T, f32 accumulation, one rounding,
  * the contraction of `cpu_reference::affine_qmm_t_b4` (crates/targets/metal/src/cpu_reference.rs:107-137).
- * The kernel is chosen from M, N and K: up to 16 tokens the matvec or, where the matrix is large for them (9 tokens from 4M weights on,
- * 5 from 40M, 3 where there are very many rows), the tensor-core GEMM for few tokens; tensor-core GEMMs above.  They add in
+ * The kernel is chosen from M, N and K: up to 16 tokens the matvec or, where the matrix is large for them (9 tokens from 4M weights on
+ * unless k is short, 5 from 40M, 3 where there are very many rows), the tensor-core GEMM for few tokens; tensor-core GEMMs above.  They add in
  * different orders: calls on either side of a choice agree to the rounding of the f32 sums, not bit for bit.
  * `bias_bf16` (may be NULL) is the linear's own bias [N], the `{prefix}.bias` tensor the loader
  * takes (crates/targets/metal/src/layers_quant.rs:318-351): it is added in f32 before the one
