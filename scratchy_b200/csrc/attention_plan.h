@@ -42,7 +42,7 @@ static inline AttPlan att_plan(int D, int G, int batch, int num_kv_heads, int bl
     const size_t budget = alone ? ATT_SMEM_BUDGET_ALONE : ATT_SMEM_BUDGET;
     // Six warps of two stages where a CTA has four blocks or more for each and they fit (beside the cluster's sums, which grow with the query heads and
     // which one CTA a sequence does without: with room kept for eight CTAs' sums all the same, tables of 129 blocks and more of 3 query heads left four
-    // warps, and a step of the 3B Llama at 32 sequences of up to 2048 tokens took 2168 us), otherwise four of three
+    // warps, and a step of the 3B Llama at 32 sequences of up to 2048 tokens took 2168 us for 2059), otherwise four of three
     // (16 sequences of up to 2048 tokens 23.9 us with four warps, 20.8 with six; 4 sequences, 16 blocks a CTA, 13.0 and 14.6).
     // Large blocks: two, with one stage each if it must be.
     const int most = alone ? 8 : max_blocks_per_seq / p.nsplit >= 24 ? 6 : 4;

@@ -558,8 +558,8 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_kernel(
 //
 // What bounds it: HBM (8 KB per block of 16 tokens and kv head), and the longest sequence's CTA.  Llama-3.2-3B at 32 sequences of
 // 512 to 2048 tokens, 153 MB per call, in a stream of calls: 57.6 us with the producer warp and a second MMA for the remainders,
-// 40.9 us with rings of the warps' own and a CTA for every sequence and kv head, 37.9 (4.0 TB/s) with two copies a block;
-// all of 2048 44.3 us (6.1 TB/s).  Whole sequences dealt to one CTA per SM (PACKED; their blocks in even shares to the warps)
+// 40.9 us with rings of the warps' own and a CTA for every sequence and kv head, 37.9 with two copies a block, 34.9
+// (4.4 TB/s) with six warps at that width of the table too; all of 2048 44.1 us (6.1 TB/s).  Whole sequences dealt to one CTA per SM (PACKED; their blocks in even shares to the warps)
 // are faster in such a stream, 31.6, but not between the kernels of a step (attention_plan.h): 48 sequences, which take them, 62.4 -> 48.3 us, all of 2048 81.9 -> 67.9.
 constexpr int ATT_ERR_FULL = 0x0A000001;
 
